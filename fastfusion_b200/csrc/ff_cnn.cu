@@ -519,71 +519,348 @@ __global__ void __launch_bounds__(128) k_conv_tc(const __grid_constant__ CUtenso
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
-template <int CIN, int COUT>
-constexpr size_t wgrad_smem_bytes() {
-  return sizeof(float) * ((size_t)CIN * PLANE + (size_t)COUT * GPLANE);
+// ------------------------------------------- tensor-core weight gradients
+//
+// dW[co][ci][ky][kx] = sum over pixels p of dy[p][co] * x[p + (ky-2, kx-2)][ci],
+// db[co] = sum of dy[co]: a GEMM whose contraction runs over the pixels, on
+// the 5th-generation tensor cores.  Both operands lie in shared memory pixel
+// after pixel with 8 channels (16 bytes) each, which is the M- and N-major
+// unswizzled canonical layout (core matrices of 8 pixels x 8 channels, 128
+// bytes; the next 8 pixels of K at LBO = 128, the next 8 channels at SBO).
+//   A (M = 128): 16 groups of 8 channels of x, the group stride running over
+//     (row, plane) of the tile, so one MMA holds 8 rows of 16 channels;
+//   B (N = G * NS): G rows of dy.  dy is FP32 and enters as three BF16 parts
+//     (top, middle and low 8 bits of the significand, by truncation), whose
+//     sum is dy exactly: with x in BF16 every product is exact, as in FP32;
+//   D[row j of x][row i of dy] is the gradient for ky = j - i; the shift kx is
+//     the start address of A's descriptor, one accumulator per kx.
+// The accumulators are emptied into FP32 registers after every tile (16 or
+// 8 MMAs each), so no long sum runs in the tensor core's accumulator.
+// Layer 1 has one plane of 8 channels: its second plane is the same pixels
+// one to the right, so that one accumulator serves two kx.
+//
+// What bounds it: shared-memory operand reads, (128 + N) x 32 bytes per MMA
+// (56 of 128-byte reads against 48 cycles of math at N = 96), so G = 2 rows of dy
+// per MMA for the 16-channel dy (5 x 96 columns of the 512 of tensor memory;
+// one row needs 220 operand-read cycles per 16 pixels, two 140) and 4 rows
+// for layer 3's single channel.  Measured on four 640x480 images: layers 2, 1 and 3 take 85,
+// 66 and 42 us (an MMA about 90 cycles, the flush of the accumulators a tenth),
+// with one (co, ci) pair per thread on the CUDA cores, 26 shared-memory reads
+// per 25 FMAs, 969, 371 and 472 us.  Errors against 64 bits (relative L2 of the
+// whole gradient): 2.2e-7 against 8.7e-7.
+enum WgKind { WG_L1 = 1, WG_L2 = 2, WG_L3 = 3 };
+constexpr int WG_THREADS = 256;
+constexpr int WG_W = 64, WG_R = 8;     // dy pixels of a tile
+constexpr int WG_XPX = 72;             // x pixels of a tile row: 64 + 4, whole 128-byte core matrices
+constexpr int WG_XROWS = WG_R + 6;     // 12 rows of x; the last MMA's unused groups reach two further
+constexpr int WG_XROW_BYTES = 2 * WG_XPX * 16;
+constexpr int WG_XBYTES = WG_XROWS * WG_XROW_BYTES;
+
+template <int KIND>
+struct WgTraits {
+  static constexpr int CO = KIND == WG_L3 ? 1 : 16;           // channels of dy
+  static constexpr int CI = KIND == WG_L1 ? CNN_IN : CNN_HID;  // channels of x
+  static constexpr int G = KIND == WG_L3 ? 4 : 2;              // rows of dy per MMA
+  static constexpr int NS = KIND == WG_L3 ? 8 : 48;            // columns of a dy row: its channels' three parts
+  static constexpr int N = G * NS;
+  static constexpr int NKX = KIND == WG_L1 ? 3 : 5;            // accumulators
+  static constexpr int KX_STEP = KIND == WG_L1 ? 2 : 1;
+  static constexpr int COLS = KIND == WG_L3 ? 256 : 512;       // tensor-memory columns allocated
+  static constexpr int GBYTES = WG_R * (NS / 8) * WG_W * 16;   // dy parts of a tile
+  static constexpr int BUF = WG_XBYTES + GBYTES;
+  static constexpr int DW = CO * CI * TAPS;
+  static constexpr int ACC = KIND == WG_L3 ? 2 : 16;           // accumulators per kx and thread
+  static_assert(NKX * N <= COLS, "accumulators fit the allocation");
+  static_assert(DW * 4 + 64 * 4 <= BUF, "the block's sums reuse a tile buffer");
+};
+// (the blocks that allocate all 512 columns leave no room for a second one)
+template <int KIND>
+constexpr size_t wg_smem_bytes() {
+  return 2 * (size_t)WgTraits<KIND>::BUF + 64;
+}
+static_assert((WG_XPX * 16) % 128 == 0 && WG_XBYTES % 128 == 0 && WgTraits<WG_L2>::BUF % 128 == 0 &&
+                  WgTraits<WG_L3>::BUF % 128 == 0,
+              "tile copies land on 128-byte boundaries");
+static_assert(wg_smem_bytes<WG_L1>() > 114 * 1024 && wg_smem_bytes<WG_L2>() > 114 * 1024, "one block per SM");
+
+// M = 128, D FP32, A and B BF16, both M/N-major
+template <int N>
+__host__ __device__ constexpr uint32_t wg_idesc() {
+  return tc_idesc<N>() | (1u << 15) | (1u << 16);
 }
 
-// Weight and bias gradients of a layer (CIN in, COUT out): dW[co][ci][tap] =
-// sum over pixels of x[p + tap] * dy[p][co], db[co] = sum of dy[co].  Each
-// thread owns one (co, ci) pair and a share of the tile's pixels, blocks
-// stride over the tiles of all images and add their sums once at the end.
-template <int CIN, int COUT, int CSTR>
-__global__ void __launch_bounds__(256) k_conv_wgrad(const __nv_bfloat16 *__restrict__ x,
-                                                    const float *__restrict__ dy, int W, int H, int n_img,
-                                                    float *__restrict__ dw, float *__restrict__ db) {
-  extern __shared__ __align__(16) float smem[];
-  float *s_x = smem;
-  float *s_g = smem + CIN * PLANE;
-  constexpr int P = CIN * COUT;
-  static_assert(P <= 256, "one pair per thread");
-  constexpr int G = 256 / P;
-  const int pair = threadIdx.x % P, grp = threadIdx.x / P;
-  const bool active = grp < G;
-  const int co = pair / CIN, ci = pair % CIN;
-  float acc[TAPS];
-#pragma unroll
-  for (int k = 0; k < TAPS; k++) acc[k] = 0.0f;
-  float accb = 0.0f;
-  const int tiles_x = (W + TX - 1) / TX, tiles_y = (H + TY - 1) / TY;
+// The three BF16 parts of v (bit patterns in the upper halves): v = hi + mid +
+// lo exactly; an infinity or a NaN stays in hi alone.
+__device__ __forceinline__ void split3_bf16(float v, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
+  hi = __float_as_uint(v) & 0xFFFF0000u;
+  float r = v - __uint_as_float(hi);
+  r = r == r ? r : 0.0f;
+  mid = __float_as_uint(r) & 0xFFFF0000u;
+  lo = __float_as_uint(r - __uint_as_float(mid));
+}
+// the upper halves of a and b as two BF16 words, a first
+__device__ __forceinline__ uint32_t pack_hi(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
+
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(addr));
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(const __grid_constant__ CUtensorMap tile,
+                                                         const float *__restrict__ dy, int W, int H, int n_img,
+                                                         float *__restrict__ dw, float *__restrict__ db) {
+  using T = WgTraits<KIND>;
+  extern __shared__ __align__(1024) uint8_t wsm[];
+  uint64_t *mbar = reinterpret_cast<uint64_t *>(wsm + 2 * T::BUF);  // [0], [1]: x of a buffer; [2]: MMAs
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mbar + 3);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
+                 "r"(T::COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    for (int k = 0; k < 3; k++)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(mbar + k)));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const int tiles_x = (W + WG_W - 1) / WG_W, tiles_y = (H + WG_R - 1) / WG_R;
   const int total = tiles_x * tiles_y * n_img;
-  for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
-    const int img = tile / (tiles_x * tiles_y), rest = tile % (tiles_x * tiles_y);
-    const int x0 = (rest % tiles_x) * TX, y0 = (rest / tiles_x) * TY;
-    __syncthreads();
-    load_tile<CIN, CSTR>(x, img, W, H, x0, y0, s_x);
-    for (int i = threadIdx.x; i < TX * TY; i += blockDim.x) {
-      const int gx = x0 + i % TX, gy = y0 + i / TX;
-      float v[COUT];
-      if (gx < W && gy < H) {
-        load_px<COUT, COUT>(dy + (((size_t)img * H + gy) * W + gx) * COUT, v);
-      } else {
+  struct Pos {
+    int img, x0, y0;
+  };
+  auto pos_of = [&](int t) {
+    Pos p;
+    p.img = t / (tiles_x * tiles_y);
+    const int rest = t % (tiles_x * tiles_y);
+    p.x0 = (rest % tiles_x) * WG_W;
+    p.y0 = (rest / tiles_x) * WG_R;
+    return p;
+  };
+  // x of a tile: (8 + 4) rows of two planes, each row of a plane one copy
+  // (zero outside the image), issued by the first 24 lanes of warp 1
+  auto load_x = [&](const Pos &p, int b) {
+    if (warp != 1) return;
+    const uint32_t bar = smem_addr(mbar + b), dst = smem_addr(wsm + b * T::BUF);
+    if (lane == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                   "r"((uint32_t)((WG_R + 4) * WG_XROW_BYTES))
+                   : "memory");
+    __syncwarp();
+    if (lane < 2 * (WG_R + 4)) {
+      const int r = lane >> 1, pl = lane & 1;
+      const uint32_t d = dst + (uint32_t)(r * WG_XROW_BYTES + pl * WG_XPX * 16);
+      if constexpr (KIND == WG_L1)
+        tma_load_4d(d, &tile, 0, p.x0 - 2 + pl, p.y0 - 2 + r, p.img, bar);
+      else
+        tma_load_5d(d, &tile, 0, pl, p.x0 - 2, p.y0 - 2 + r, p.img, bar);
+    }
+    __syncwarp();
+  };
+  // dy of a tile, split: [row][part, channel plane][pixel][8 channels]; zero
+  // outside the image.  The running sums of what a thread reads are its share
+  // of the bias gradient.
+  float bias[KIND == WG_L3 ? 1 : 4] = {};
+  auto load_g = [&](const Pos &p, int b) {
+    uint8_t *gs = wsm + b * T::BUF + WG_XBYTES;
+    const size_t base = (size_t)p.img * H * W;
+    if constexpr (KIND == WG_L3) {
 #pragma unroll
-        for (int c = 0; c < COUT; c++) v[c] = 0.0f;
+      for (int it = 0; it < WG_W * WG_R / WG_THREADS; it++) {
+        const int i = it * WG_THREADS + tid;
+        const int gx = p.x0 + i % WG_W, gy = p.y0 + i / WG_W;
+        const float v = (gx < W && gy < H) ? __ldg(dy + base + (size_t)gy * W + gx) : 0.0f;
+        bias[0] += v;
+        uint32_t h, m, l;
+        split3_bf16(v, h, m, l);
+        *reinterpret_cast<uint4 *>(gs + (size_t)i * 16) = make_uint4(pack_hi(h, m), l >> 16, 0u, 0u);
+      }
+    } else {
+      const int q = tid & 3;  // this thread's four channels
+      float4 f[8];
+#pragma unroll
+      for (int it = 0; it < 8; it++) {
+        const int px = it * (WG_THREADS / 4) + (tid >> 2);
+        const int gx = p.x0 + px % WG_W, gy = p.y0 + px / WG_W;
+        f[it] = (gx < W && gy < H)
+                    ? __ldg(reinterpret_cast<const float4 *>(dy + (base + (size_t)gy * W + gx) * 16) + q)
+                    : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
 #pragma unroll
-      for (int c = 0; c < COUT; c++) s_g[c * GPLANE + i] = v[c];
-    }
-    __syncthreads();
-    if (active) {
-      const float *pg = s_g + co * GPLANE;
-      const float *px = s_x + ci * PLANE;
-      for (int p = grp; p < TX * TY; p += G) {
-        const float g = pg[p];
-        const float *q = px + (p / TX) * SX + (p % TX);
+      for (int it = 0; it < 8; it++) {
+        const int px = it * (WG_THREADS / 4) + (tid >> 2);
+        const float v[4] = {f[it].x, f[it].y, f[it].z, f[it].w};
+        uint32_t h[4], m[4], l[4];
 #pragma unroll
-        for (int ky = 0; ky < 5; ky++)
-#pragma unroll
-          for (int kx = 0; kx < 5; kx++) acc[ky * 5 + kx] = fmaf(q[ky * SX + kx], g, acc[ky * 5 + kx]);
-        accb += g;
+        for (int k = 0; k < 4; k++) {
+          bias[k] += v[k];
+          split3_bf16(v[k], h[k], m[k], l[k]);
+        }
+        uint8_t *d = gs + (size_t)(px / WG_W) * (6 * WG_W * 16) + (size_t)(q >> 1) * (WG_W * 16) +
+                     (size_t)(px % WG_W) * 16 + (q & 1) * 8;
+        *reinterpret_cast<uint2 *>(d) = make_uint2(pack_hi(h[0], h[1]), pack_hi(h[2], h[3]));
+        *reinterpret_cast<uint2 *>(d + 2 * WG_W * 16) = make_uint2(pack_hi(m[0], m[1]), pack_hi(m[2], m[3]));
+        *reinterpret_cast<uint2 *>(d + 4 * WG_W * 16) = make_uint2(pack_hi(l[0], l[1]), pack_hi(l[2], l[3]));
       }
     }
-  }
-  if (active) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  };
+  // the tile's MMAs, by one thread once x has landed; returns whether it has
+  auto issue = [&](int b, uint32_t parity) -> uint32_t {
+    const uint32_t ok = mbar_wait(smem_addr(mbar + b), parity);
+    if (!ok) return 0u;
+    const uint32_t xb = smem_addr(wsm + b * T::BUF), gb = xb + WG_XBYTES;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    for (int ip = 0; ip < WG_R / T::G; ip++)
+      for (int ch = 0; ch < WG_W / 16; ch++) {
+        const uint64_t bd = tc_desc(gb + (uint32_t)(ip * T::G * (T::NS / 8) * WG_W * 16 + ch * 256), 128, WG_W * 16);
 #pragma unroll
-    for (int k = 0; k < TAPS; k++) atomicAdd(dw + (co * CIN + ci) * TAPS + k, acc[k]);
-    if (ci == 0) atomicAdd(db + co, accb);
+        for (int k = 0; k < T::NKX; k++) {
+          const uint64_t ad = tc_desc(
+              xb + (uint32_t)(ip * T::G * WG_XROW_BYTES + (ch * 16 + k * T::KX_STEP) * 16), 128, WG_XPX * 16);
+          asm volatile(
+              "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+              " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem + (uint32_t)(k * T::N)),
+              "l"(ad), "l"(bd), "r"(wg_idesc<T::N>()), "r"((ip | ch) ? 1u : 0u));
+        }
+      }
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                     smem_addr(mbar + 2))
+                 : "memory");
+    return 1u;
+  };
+  const int quad = warp & 3, half = warp >> 2;
+  const uint32_t trow = tmem + ((uint32_t)(32 * quad) << 16);
+  float acc[T::NKX][T::ACC];
+#pragma unroll
+  for (int k = 0; k < T::NKX; k++)
+#pragma unroll
+    for (int c = 0; c < T::ACC; c++) acc[k][c] = 0.0f;
+  int t = blockIdx.x;  // (below total: the grid has at most that many blocks)
+  {
+    const Pos first = pos_of(t);
+    load_x(first, 0);
+    load_g(first, 0);
   }
+  __syncthreads();
+  uint32_t pending_x = 0;  // (bit b: a copy into buffer b whose arrival nobody has waited for)
+  int it = 0;
+  bool bad = false;
+  for (; t < total; t += gridDim.x, it++) {
+    const int b = it & 1;
+    bool ok = tid != 0 || issue(b, (uint32_t)((it >> 1) & 1));
+    __syncwarp();
+    // the next tile's operands while the MMAs run (their buffer's last
+    // readers, the previous tile's MMAs, have finished)
+    const int tn = t + (int)gridDim.x;
+    pending_x = 0;
+    if (tn < total) {
+      const Pos nx = pos_of(tn);
+      load_x(nx, b ^ 1);
+      load_g(nx, b ^ 1);
+      pending_x = 1u;
+    }
+    const uint32_t done = mbar_wait(smem_addr(mbar + 2), (uint32_t)(it & 1));
+    ok = ok && done;
+    const bool read = __all_sync(0xffffffffu, done != 0u);  // (the reads of tensor memory are by whole warps)
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (read) {
+      if constexpr (KIND == WG_L3) {
+#pragma unroll
+        for (int k = 0; k < T::NKX; k++) {
+          uint32_t v[16];  // rows 2 half, 2 half + 1 of dy
+          tmem_ld16(trow + (uint32_t)(k * T::N + half * 16), v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 2; i++)
+            acc[k][i] += __uint_as_float(v[8 * i]) + (__uint_as_float(v[8 * i + 1]) + __uint_as_float(v[8 * i + 2]));
+        }
+      } else if (quad < 3) {  // (rows 6 and 7 of x meet neither row of dy)
+#pragma unroll
+        for (int k = 0; k < T::NKX; k++) {
+          uint32_t h[16], m[16], l[16];  // row `half` of dy
+          tmem_ld16(trow + (uint32_t)(k * T::N + half * T::NS), h);
+          tmem_ld16(trow + (uint32_t)(k * T::N + half * T::NS + 16), m);
+          tmem_ld16(trow + (uint32_t)(k * T::N + half * T::NS + 32), l);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int c = 0; c < 16; c++)
+            acc[k][c] += __uint_as_float(h[c]) + (__uint_as_float(m[c]) + __uint_as_float(l[c]));
+        }
+      }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    bad = __syncthreads_or(ok ? 0 : 1) != 0;
+    if (bad) break;
+  }
+  // A wait that gave up may leave copies or MMAs in flight: wait for them once
+  // more (bounded again) before their memory is given back; the gradients
+  // become NaN.
+  if (bad) {
+    mbar_wait(smem_addr(mbar + 2), (uint32_t)(it & 1));
+    mbar_wait(smem_addr(mbar + (it & 1)), (uint32_t)((it >> 1) & 1));
+    if (pending_x) mbar_wait(smem_addr(mbar + ((it & 1) ^ 1)), (uint32_t)(((it + 1) >> 1) & 1));
+    __syncthreads();
+  }
+  // the block's gradients in shared memory: row i of dy meets row j of x at
+  // ky = j - i, so each element is met once per i, in G steps
+  float *s_dw = reinterpret_cast<float *>(wsm);
+  float *s_db = s_dw + T::DW;
+  for (int i = tid; i < T::DW + T::CO; i += WG_THREADS) s_dw[i] = 0.0f;
+  __syncthreads();
+  const int m = 32 * quad + lane, j = m >> 4, pl = (m >> 3) & 1, c8 = m & 7;
+  const int ci = KIND == WG_L1 ? c8 : pl * 8 + c8;
+#pragma unroll
+  for (int i = 0; i < T::G; i++) {
+    const int ky = j - i;
+    const bool mine = KIND == WG_L3 ? (i >> 1) == half : i == half;
+    if (mine && ky >= 0 && ky < 5 && ci < T::CI) {
+#pragma unroll
+      for (int k = 0; k < T::NKX; k++) {
+        const int kx = k * T::KX_STEP + (KIND == WG_L1 ? pl : 0);
+        if (kx < 5) {
+          if constexpr (KIND == WG_L3) {
+            s_dw[ci * TAPS + ky * 5 + kx] += acc[k][i & 1];
+          } else {
+#pragma unroll
+            for (int co = 0; co < 16; co++) s_dw[(co * T::CI + ci) * TAPS + ky * 5 + kx] += acc[k][co];
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  // the bias: lanes of the same channels, then one add per warp
+  if constexpr (KIND == WG_L3) {
+    float v = bias[0];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) atomicAdd(s_db, v);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      float v = bias[k];
+#pragma unroll
+      for (int o = 16; o > 2; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane < 4) atomicAdd(s_db + 4 * lane + k, v);
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < T::DW; i += WG_THREADS) atomicAdd(dw + i, bad ? __int_as_float(0x7FC00000) : s_dw[i]);
+  for (int i = tid; i < T::CO; i += WG_THREADS) atomicAdd(db + i, bad ? __int_as_float(0x7FC00000) : s_db[i]);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(T::COLS));
 }
 
 // Network input per pixel: depth z (m), the unit normal from central
@@ -798,10 +1075,10 @@ cudaError_t set_tc_attr() {
   return cudaFuncSetAttribute(k_conv_tc<C, N, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)tc_smem_bytes<C, N>());
 }
-template <int CIN, int COUT, int CSTR>
+template <int KIND>
 cudaError_t set_wgrad_attr() {
-  return cudaFuncSetAttribute(k_conv_wgrad<CIN, COUT, CSTR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)wgrad_smem_bytes<CIN, COUT>());
+  return cudaFuncSetAttribute(k_wgrad_tc<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)wg_smem_bytes<KIND>());
 }
 
 cudaError_t ensure_attrs() {
@@ -818,9 +1095,9 @@ cudaError_t ensure_attrs() {
       set_tc_attr<CNN_HID, 16, CONV_CONF>(),
       set_conv_attr<1, CNN_HID, 1, float, true, CONV_MASK_F32>(),
       set_conv_attr<CNN_HID, CNN_HID, CNN_HID, float, true, CONV_MASK_F32>(),
-      set_wgrad_attr<CNN_HID, 1, CNN_HID>(),
-      set_wgrad_attr<CNN_HID, CNN_HID, CNN_HID>(),
-      set_wgrad_attr<CNN_IN, CNN_HID, CNN_IN_STRIDE>(),
+      set_wgrad_attr<WG_L1>(),
+      set_wgrad_attr<WG_L2>(),
+      set_wgrad_attr<WG_L3>(),
   };
   for (cudaError_t x : r)
     if (x != cudaSuccess) return x;
@@ -846,10 +1123,12 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// The tile of a k_conv_tc block over n images of W x H pixels, C = 8 or 16
-// BF16 channels per pixel: a (TC_ROWS + 4) x TC_COLS box of one 8-channel
-// plane, zero outside the image (dimensions: 8 channels, [plane], x, y, image).
-cudaError_t tile_map(CUtensorMap *m, const void *base, int C, int W, int H, int n) {
+// A tile over n images of W x H pixels, C = 8 or 16 BF16 channels per pixel: a
+// rows x cols box of one 8-channel plane (k_conv_tc: (TC_ROWS + 4) x TC_COLS;
+// k_wgrad_tc: one row of WG_XPX), zero outside the image (dimensions: 8
+// channels, [plane], x, y, image).
+cudaError_t tile_map(CUtensorMap *m, const void *base, int C, int W, int H, int n, int cols = TC_COLS,
+                     int rows = TC_TILE_ROWS) {
   const EncodeTiledFn f = encode_tiled();
   if (!f) return cudaErrorNotSupported;
   cuuint64_t dims[5], strides[4];
@@ -859,14 +1138,14 @@ cudaError_t tile_map(CUtensorMap *m, const void *base, int C, int W, int H, int 
     rank = 5;
     const cuuint64_t d[5] = {8, 2, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)n};
     const cuuint64_t st[4] = {16, 32, (cuuint64_t)W * 32, (cuuint64_t)W * H * 32};
-    const cuuint32_t b[5] = {8, 1, TC_COLS, TC_TILE_ROWS, 1};
+    const cuuint32_t b[5] = {8, 1, (cuuint32_t)cols, (cuuint32_t)rows, 1};
     for (int i = 0; i < 5; i++) dims[i] = d[i], box[i] = b[i];
     for (int i = 0; i < 4; i++) strides[i] = st[i];
   } else {
     rank = 4;
     const cuuint64_t d[4] = {8, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)n};
     const cuuint64_t st[3] = {16, (cuuint64_t)W * 16, (cuuint64_t)W * H * 16};
-    const cuuint32_t b[4] = {8, TC_COLS, TC_TILE_ROWS, 1};
+    const cuuint32_t b[4] = {8, (cuuint32_t)cols, (cuuint32_t)rows, 1};
     for (int i = 0; i < 4; i++) dims[i] = d[i], box[i] = b[i];
     for (int i = 0; i < 3; i++) strides[i] = st[i];
   }
@@ -888,12 +1167,15 @@ void conv(const TIN *in, int n, int W, int H, const __nv_bfloat16 *w, const __nv
       <<<conv_grid(W, H, n), 256, conv_smem_bytes<KIN, KOUT>(), s>>>(in, W, H, w, b, out, act, inv_tau);
 }
 
-template <int CIN, int COUT, int CSTR>
-void wgrad(const __nv_bfloat16 *x, const float *dy, int n, int W, int H, float *dw, float *db, cudaStream_t s) {
-  const int tiles = ((W + TX - 1) / TX) * ((H + TY - 1) / TY) * n;
+template <int KIND>
+cudaError_t wgrad(const __nv_bfloat16 *x, const float *dy, int n, int W, int H, float *dw, float *db, cudaStream_t s) {
+  CUtensorMap m;
+  const cudaError_t e = tile_map(&m, x, KIND == WG_L1 ? CNN_IN_STRIDE : CNN_HID, W, H, n, WG_XPX, 1);
+  if (e != cudaSuccess) return e;
+  const int tiles = ((W + WG_W - 1) / WG_W) * ((H + WG_R - 1) / WG_R) * n;
   note_launch();
-  k_conv_wgrad<CIN, COUT, CSTR>
-      <<<std::min(tiles, 148 * 2), 256, wgrad_smem_bytes<CIN, COUT>(), s>>>(x, dy, W, H, n, dw, db);
+  k_wgrad_tc<KIND><<<std::min(tiles, 148), WG_THREADS, wg_smem_bytes<KIND>(), s>>>(m, dy, W, H, n, dw, db);
+  return cudaGetLastError();
 }
 }  // namespace
 
@@ -939,13 +1221,13 @@ cudaError_t cnn_backward(const __nv_bfloat16 *params, const __nv_bfloat16 *feat,
   cudaError_t e = ensure_attrs();
   if (e != cudaSuccess) return e;
   // layer 3
-  wgrad<CNN_HID, 1, CNN_HID>(a2, dpred, n, W, H, grads + P_W3, grads + P_B3, s);
+  if ((e = wgrad<WG_L3>(a2, dpred, n, W, H, grads + P_W3, grads + P_B3, s)) != cudaSuccess) return e;
   conv<1, CNN_HID, 1, float, true, CONV_MASK_F32>(dpred, n, W, H, params + P_W3, nullptr, g2, a2, 0.0f, s);
   // layer 2
-  wgrad<CNN_HID, CNN_HID, CNN_HID>(a1, g2, n, W, H, grads + P_W2, grads + P_B2, s);
+  if ((e = wgrad<WG_L2>(a1, g2, n, W, H, grads + P_W2, grads + P_B2, s)) != cudaSuccess) return e;
   conv<CNN_HID, CNN_HID, CNN_HID, float, true, CONV_MASK_F32>(g2, n, W, H, params + P_W2, nullptr, g1, a1, 0.0f, s);
   // layer 1 (no gradient of the input)
-  wgrad<CNN_IN, CNN_HID, CNN_IN_STRIDE>(feat, g1, n, W, H, grads + P_W1, grads + P_B1, s);
+  if ((e = wgrad<WG_L1>(feat, g1, n, W, H, grads + P_W1, grads + P_B1, s)) != cudaSuccess) return e;
   return cudaGetLastError();
 }
 
