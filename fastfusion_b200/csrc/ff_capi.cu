@@ -135,8 +135,6 @@ struct ff_handle {
   // learned confidence weight (ff_set_confidence): BF16 parameters, and the
   // per-frame features, activations and confidence map
   __nv_bfloat16 *d_cnn_params = nullptr;
-  uint8_t *d_cnn_packed = nullptr;  // the weights as tensor-core operands
-  bool cnn_packed_ready = false;
   float conf_tau_cm = 0.0f;  // > 0: the learned weight is on
   __nv_bfloat16 *d_feat = nullptr, *d_a1 = nullptr, *d_a2 = nullptr;
   float *d_conf = nullptr;
@@ -727,7 +725,7 @@ ff_status ff_destroy(ff_handle *h) {
                   h->d_stamp, h->d_bstamp, h->d_queue_set[0], h->d_queue_set[1], h->d_cnt_set[0], h->d_cnt_set[1],
                   h->d_barrier, h->d_depth_set[0], h->d_depth_set[1], h->d_bgr_set[0], h->d_bgr_set[1], h->d_pxp,
                   h->d_pyp, h->d_vox, h->d_proc, h->d_bnd, h->d_pend, h->d_keys, h->d_sort_tmp, h->d_rcp_tab,
-                  h->d_cnn_params, h->d_cnn_packed, h->d_feat, h->d_a1, h->d_a2, h->d_conf_set[0], h->d_conf_set[1],
+                  h->d_cnn_params, h->d_feat, h->d_a1, h->d_a2, h->d_conf_set[0], h->d_conf_set[1],
                   h->d_batch_set[0], h->d_batch_set[1], h->d_upd_mask, h->d_upd_list, h->d_upd_count,
                   h->d_upd_total, h->d_ring_depth, h->d_ring_bgr, h->d_ring_conf, h->d_seq_vox, h->d_seq_proc,
                   h->d_seq_bnd, h->d_seq_cnt, h->d_loop_map, h->d_loop_slots, h->d_loop_st, h->d_loop_sdf,
@@ -1170,9 +1168,8 @@ static ff_status frame_prepare(ff_handle *h, const uint16_t *d_depth, const uint
     }
     const int pc = h->prof.begin(ST_CONFIDENCE, cs);
     CK(cnn_features(d_depth, 1, W, H, scaling, kf, h->d_feat, cs));
-    CK(cnn_forward(h->d_cnn_params, h->d_cnn_packed, h->cnn_packed_ready, h->d_feat, 1, W, H, h->d_a1, h->d_a2,
-                   h->d_conf, h->conf_tau_cm, &h->d_cnt->cnn_error, cs));
-    h->cnn_packed_ready = true;
+    CK(cnn_forward(h->d_cnn_params, h->d_feat, 1, W, H, h->d_a1, h->d_a2, h->d_conf, h->conf_tau_cm,
+                   &h->d_cnt->cnn_error, cs));
     if (h->inject == FF_INJECT_CONFIDENCE_TIMEOUT) {
       // the word the network sets when one of its waits gives up
       CK(cudaMemsetAsync(&h->d_cnt->cnn_error, 0xFF, sizeof(uint32_t), cs));
@@ -2408,8 +2405,6 @@ ff_status ff_set_confidence(ff_handle *h, const float *params, int n_params, flo
   std::vector<uint16_t> b(n_params);
   for (int i = 0; i < n_params; i++) b[i] = bf16_bits(params[i]);
   if (!h->d_cnn_params) CK(alloc(&h->d_cnn_params, (size_t)FF_CNN_PARAMS));
-  if (!h->d_cnn_packed) CK(alloc(&h->d_cnn_packed, (size_t)CNN_PACKED_BYTES));
-  h->cnn_packed_ready = false;  // packed by the next frame
   CK(cudaMemcpyAsync(h->d_cnn_params, b.data(), sizeof(uint16_t) * n_params, cudaMemcpyHostToDevice, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   h->conf_tau_cm = tau_m * 100.0f;
@@ -2487,9 +2482,9 @@ ff_status ff_cnn_forward(const void *d_params, void *d_packed, const void *d_fea
                          void *d_a1, void *d_a2, float *d_out, float tau_m, void *stream) {
   if (!d_params || !d_packed || !d_feat || !d_a1 || !d_a2 || !d_out || n <= 0 || width <= 0 || height <= 0)
     return cnn_bad("ff_cnn_forward: bad argument");
-  CKN(cnn_forward((const __nv_bfloat16 *)d_params, (uint8_t *)d_packed, false, (const __nv_bfloat16 *)d_feat, n,
-                  width, height, (__nv_bfloat16 *)d_a1, (__nv_bfloat16 *)d_a2, d_out,
-                  tau_m > 0.0f ? tau_m * 100.0f : 0.0f, nullptr, (cudaStream_t)stream));
+  CKN(cnn_forward((const __nv_bfloat16 *)d_params, (const __nv_bfloat16 *)d_feat, n, width, height,
+                  (__nv_bfloat16 *)d_a1, (__nv_bfloat16 *)d_a2, d_out, tau_m > 0.0f ? tau_m * 100.0f : 0.0f, nullptr,
+                  (cudaStream_t)stream));
   return FF_OK;
 }
 

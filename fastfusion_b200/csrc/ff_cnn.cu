@@ -33,232 +33,76 @@ constexpr int P_W1 = 0, P_B1 = P_W1 + CNN_HID * CNN_IN * TAPS, P_W2 = P_B1 + CNN
               P_B2 = P_W2 + CNN_HID * CNN_HID * TAPS, P_W3 = P_B2 + CNN_HID, P_B3 = P_W3 + CNN_HID * TAPS,
               P_TOTAL = P_B3 + 1;
 static_assert(P_TOTAL == CNN_PARAMS && CNN_HID == CNN_HIDDEN && CNN_IN_STRIDE == CNN_FEAT_CH, "parameter layout");
-static_assert(CNN_PACKED_BYTES == 65 * 512, "packed operand bytes");
 
-// output tile of a convolution block: 32 x 16 pixels, 256 threads, two
-// pixels (rows ty and ty + 8) per thread; input tile with a 2-pixel halo,
-// one plane per channel, planes padded to an odd length so that threads
-// reading different channels hit different banks
-constexpr int TX = 32, TY = 16, SX = TX + 4, SY = TY + 4, PLANE = SX * SY + 1;
-constexpr int GPLANE = TX * TY + 1;
-
-enum ConvMode { CONV_RELU_BF16 = 0, CONV_F32 = 1, CONV_CONF = 2, CONV_MASK_F32 = 3 };
-
-__device__ __forceinline__ float to_f(__nv_bfloat16 v) { return __bfloat162float(v); }
-__device__ __forceinline__ float to_f(float v) { return v; }
-
-// KIN channels of one pixel (CSTR elements apart) into v[]
-template <int KIN, int CSTR, typename T>
-__device__ __forceinline__ void load_px(const T *__restrict__ p, float *v) {
-  if constexpr (sizeof(T) == 2 && CSTR % 8 == 0) {
-    constexpr int NV = (KIN + 7) / 8;
-#pragma unroll
-    for (int k = 0; k < NV; k++) {
-      const uint4 u = __ldg(reinterpret_cast<const uint4 *>(p) + k);
-      const __nv_bfloat16 *b = reinterpret_cast<const __nv_bfloat16 *>(&u);
-#pragma unroll
-      for (int j = 0; j < 8; j++)
-        if (k * 8 + j < KIN) v[k * 8 + j] = __bfloat162float(b[j]);
-    }
-  } else if constexpr (sizeof(T) == 4 && CSTR % 4 == 0 && KIN % 4 == 0) {
-#pragma unroll
-    for (int k = 0; k < KIN / 4; k++) {
-      const float4 u = __ldg(reinterpret_cast<const float4 *>(p) + k);
-      v[4 * k] = u.x;
-      v[4 * k + 1] = u.y;
-      v[4 * k + 2] = u.z;
-      v[4 * k + 3] = u.w;
-    }
-  } else {
-#pragma unroll
-    for (int c = 0; c < KIN; c++) v[c] = to_f(p[c]);
-  }
-}
-
-// The input tile of block (x0, y0) of image img: KIN planes of SX x SYT
-// (PLANET floats apart).
-template <int KIN, int CSTR, typename T, int SYT = SY, int PLANET = PLANE>
-__device__ __forceinline__ void load_tile(const T *__restrict__ in, int img, int W, int H, int x0, int y0,
-                                          float *s_in) {
-  const size_t base = (size_t)img * W * H;
-  for (int i = threadIdx.x; i < SX * SYT; i += blockDim.x) {
-    const int gx = x0 + i % SX - 2, gy = y0 + i / SX - 2;
-    float v[KIN];
-    if (gx >= 0 && gx < W && gy >= 0 && gy < H) {
-      load_px<KIN, CSTR>(in + (base + (size_t)gy * W + gx) * CSTR, v);
-    } else {
-#pragma unroll
-      for (int c = 0; c < KIN; c++) v[c] = 0.0f;
-    }
-#pragma unroll
-    for (int c = 0; c < KIN; c++) s_in[c * PLANET + i] = v[c];
-  }
-}
-
-// Convolution tiles: 32 x (8 * RPT) output pixels, RPT rows per thread.
-constexpr int CONV_RPT = 4;
-__host__ __device__ constexpr int conv_ty(int rpt) { return 8 * rpt; }
-__host__ __device__ constexpr int conv_plane(int rpt) { return SX * (conv_ty(rpt) + 4) + 1; }
-__host__ __device__ constexpr int w_offset(int kin, int rpt) { return (kin * conv_plane(rpt) + 3) & ~3; }
-
-template <int KIN, int KOUT>
-constexpr size_t conv_smem_bytes() {
-  return sizeof(float) * ((size_t)w_offset(KIN, CONV_RPT) + (size_t)KIN * TAPS * KOUT);
-}
-
-// One 5x5 convolution layer over a 32 x (8 RPT) tile, each thread RPT
-// pixels of one column (rows ty, ty + 8, ...).  KIN channels are read, KOUT
-// produced.  TRANS: the gradient of a layer's input -- the layer (KOUT in,
-// KIN out) applied transposed, i.e. a correlation with its weights flipped.
-// Modes: ReLU to BF16 (forward hidden layers), FP32 (network output), the
-// confidence weight (inference), FP32 masked by the ReLU of an activation
-// (backward).  FP32 accumulation in channel-major, row, column order; the
-// weights of a tap are read as float4 broadcasts shared by the RPT pixels.
-template <int KIN, int KOUT, int CSTR, typename TIN, bool TRANS, int MODE>
-__global__ void __launch_bounds__(256) k_conv(const TIN *__restrict__ in, int W, int H,
-                                              const __nv_bfloat16 *__restrict__ w,
-                                              const __nv_bfloat16 *__restrict__ bias, void *__restrict__ out,
-                                              const __nv_bfloat16 *__restrict__ act, float inv_tau) {
-  constexpr int RPT = CONV_RPT, TYC = conv_ty(RPT), PL = conv_plane(RPT);
-  extern __shared__ __align__(16) float smem[];
-  float *s_in = smem;
-  float *s_w = smem + w_offset(KIN, RPT);  // [KIN][25][KOUT]
-  const int img = blockIdx.z;
-  const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TYC;
-  for (int i = threadIdx.x; i < KIN * TAPS * KOUT; i += blockDim.x) {
-    const int co = i % KOUT, rest = i / KOUT, tap = rest % TAPS, ci = rest / TAPS;
-    s_w[i] = TRANS ? __bfloat162float(w[(ci * KOUT + co) * TAPS + (TAPS - 1 - tap)])
-                   : __bfloat162float(w[(co * KIN + ci) * TAPS + tap]);
-  }
-  load_tile<KIN, CSTR, TIN, TYC + 4, PL>(in, img, W, H, x0, y0, s_in);
-  __syncthreads();
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  float acc[RPT][KOUT];
-#pragma unroll
-  for (int r = 0; r < RPT; r++)
-#pragma unroll
-    for (int co = 0; co < KOUT; co++) acc[r][co] = (MODE == CONV_MASK_F32) ? 0.0f : __bfloat162float(bias[co]);
-#pragma unroll 1
-  for (int ci = 0; ci < KIN; ci++) {
-    const float *pl = s_in + ci * PL + ty * SX + tx;
-    const float *wc = s_w + ci * TAPS * KOUT;
-#pragma unroll
-    for (int ky = 0; ky < 5; ky++) {
-#pragma unroll
-      for (int kx = 0; kx < 5; kx++) {
-        float u[RPT];
-#pragma unroll
-        for (int r = 0; r < RPT; r++) u[r] = pl[(ky + 8 * r) * SX + kx];
-        const float *wp = wc + (ky * 5 + kx) * KOUT;
-        if constexpr (KOUT % 4 == 0) {
-#pragma unroll
-          for (int co = 0; co < KOUT; co += 4) {
-            const float4 w4 = *reinterpret_cast<const float4 *>(wp + co);
-#pragma unroll
-            for (int r = 0; r < RPT; r++) {
-              acc[r][co] = fmaf(w4.x, u[r], acc[r][co]);
-              acc[r][co + 1] = fmaf(w4.y, u[r], acc[r][co + 1]);
-              acc[r][co + 2] = fmaf(w4.z, u[r], acc[r][co + 2]);
-              acc[r][co + 3] = fmaf(w4.w, u[r], acc[r][co + 3]);
-            }
-          }
-        } else {
-#pragma unroll
-          for (int co = 0; co < KOUT; co++) {
-            const float wv = wp[co];
-#pragma unroll
-            for (int r = 0; r < RPT; r++) acc[r][co] = fmaf(wv, u[r], acc[r][co]);
-          }
-        }
-      }
-    }
-  }
-  const int gx = x0 + tx;
-#pragma unroll
-  for (int r = 0; r < RPT; r++) {
-    const int gy = y0 + ty + 8 * r;
-    if (gx >= W || gy >= H) continue;
-    const float *a = acc[r];
-    const size_t px = ((size_t)img * H + gy) * W + gx;
-    if constexpr (MODE == CONV_RELU_BF16) {
-      static_assert(KOUT % 8 == 0, "vector store");
-#pragma unroll
-      for (int k = 0; k < KOUT / 8; k++) {
-        uint4 v;
-        __nv_bfloat16 *b = reinterpret_cast<__nv_bfloat16 *>(&v);
-#pragma unroll
-        for (int j = 0; j < 8; j++) b[j] = __float2bfloat16_rn(fmaxf(a[8 * k + j], 0.0f));
-        reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(out) + px * KOUT)[k] = v;
-      }
-    } else if constexpr (MODE == CONV_F32) {
-#pragma unroll
-      for (int co = 0; co < KOUT; co++) reinterpret_cast<float *>(out)[px * KOUT + co] = a[co];
-    } else if constexpr (MODE == CONV_CONF) {
-      static_assert(KOUT == 1, "confidence from one channel");
-      // (1 - r/tau)^2 on [0, tau], 0 beyond: weight falls to exactly zero for
-      // pixels whose predicted residual reaches tau
-      const float c = fmaxf(1.0f - fmaxf(a[0], 0.0f) * inv_tau, 0.0f);
-      reinterpret_cast<float *>(out)[px] = c * c;
-    } else {
-      static_assert(KOUT % 8 == 0, "vector load");
-#pragma unroll
-      for (int k = 0; k < KOUT / 8; k++) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4 *>(act + px * KOUT) + k);
-        const __nv_bfloat16 *b = reinterpret_cast<const __nv_bfloat16 *>(&v);
-        float4 o0, o1;
-        o0.x = __bfloat162float(b[0]) > 0.0f ? a[8 * k + 0] : 0.0f;
-        o0.y = __bfloat162float(b[1]) > 0.0f ? a[8 * k + 1] : 0.0f;
-        o0.z = __bfloat162float(b[2]) > 0.0f ? a[8 * k + 2] : 0.0f;
-        o0.w = __bfloat162float(b[3]) > 0.0f ? a[8 * k + 3] : 0.0f;
-        o1.x = __bfloat162float(b[4]) > 0.0f ? a[8 * k + 4] : 0.0f;
-        o1.y = __bfloat162float(b[5]) > 0.0f ? a[8 * k + 5] : 0.0f;
-        o1.z = __bfloat162float(b[6]) > 0.0f ? a[8 * k + 6] : 0.0f;
-        o1.w = __bfloat162float(b[7]) > 0.0f ? a[8 * k + 7] : 0.0f;
-        float4 *o = reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + px * KOUT) + 2 * k;
-        o[0] = o0;
-        o[1] = o1;
-      }
-    }
-  }
-}
+enum ConvMode { CONV_RELU_BF16 = 0, CONV_F32 = 1, CONV_CONF = 2 };
 
 // ------------------------------------------------ tensor-core convolution
 //
-// The forward layers as implicit GEMMs on the 5th-generation tensor cores:
-// per output row of a 128-pixel strip, D[128 pixels x 16] (FP32, in tensor
-// memory) accumulates one tcgen05.mma (M=128, N=16, K=16, BF16) per
-// tap (C = 16 input channels: the 16 channels of the tap) or per pair of
-// horizontally adjacent taps (C = 8: the 8 channels of two neighbouring
-// pixels).  Operands are read by the tensor core straight from shared
-// memory through descriptors of the K-major, unswizzled canonical layout:
-// 8 x 16-byte core matrices, rows (pixels) 16 bytes apart, 8-row groups 128
-// bytes apart (SBO), the two K halves LBO apart -- the two channel planes of
-// the tile (C = 16) or the next pixel (C = 8).  A tap's shift is the
-// descriptor's start address.  Layer 3 (16 -> 1) runs with N = 16 (the
-// smallest N of an M = 128 MMA): output channel 0 real, 1..15 zero weights.
+// The forward layers as streamed implicit GEMMs on the 5th-generation tensor
+// cores.  Output rows come in groups of four
+// ("quads"): for input row t of the eight that a quad reads and for kernel
+// column kx, one tcgen05.mma (M = 128 pixels, K = 16, BF16, FP32 accumulator
+// in tensor memory) adds
+//   D[pixel p][j * NB + co] += sum over ci of x[t][p + kx][ci] * w[co][ci][t - j][kx]
+// for all four output rows j at once (NB = 16 columns a row, or 1 for the
+// one-channel output), zero where t - j is no row of the kernel.  The shift kx
+// is the start address of the A descriptor; the columns of a t are a window
+// into one strip of column blocks per kx (3 zero blocks, the five ky from the
+// last to the first, 3 zero blocks), so they are the start address of B's.
+// Why: an M = 128 MMA reads (128 + N) x 32 bytes of operands from shared
+// memory, 128 bytes a cycle.  One MMA per tap with N = 16 takes 25 x 36 = 900
+// cycles a row; a quad takes 8 x 5 MMAs of 48 (N = 64), 480 a row, though 3 of
+// 8 of its columns' products are with zero blocks.  Every output is the sum of
+// its taps in raster order (K = 16 at a time, the zero blocks between them add
+// nothing), the order the activations' BF16 rounding is defined by.
 //
-// CTA: 128 threads, output tile 128 x TC_ROWS pixels; input tile
-// (TC_ROWS + 4) x TC_COLS pixels per plane, brought in with cp.async (zero
-// fill outside the image).  One thread issues the MMAs; all wait on an
-// mbarrier (bounded) and read the accumulators back with tcgen05.ld (warp
-// w: pixels 32w..32w+31).
+// Operands: K-major, unswizzled canonical layout (8 x 16-byte core matrices,
+// pixels 16 bytes apart, 8-pixel groups 128 (SBO), the two 8-channel halves
+// of K one plane apart (LBO); 8 channels: the halves are two neighbouring
+// pixels, 16 bytes apart, and serve two kx).
+//
+// A block streams down its strip: loader warps bring quads of input rows into a
+// ring in shared memory (each row once: only the 4 halo rows at a block's
+// ends are read twice), issuing threads run the MMAs of a quad as soon as
+// its two input quads are there, and epilogue warps empty the accumulators.
+// Four issuers, each with an accumulator of its own, since the MMAs of one
+// accumulator wait for one another and one thread issues an MMA in about 80
+// cycles.  The quads of all strips of all images are dealt out evenly, a
+// block's share running over from one strip to the next.  All waits are
+// bounded.
+//
+// Measured on four 640x480 images: layers 1, 2 and 3 take 25, 29 and 22 us
+// (an MMA about 75 cycles); a block per 128 x 8 pixels with one MMA per tap,
+// N = 16, took 34, 50 and 44 us.  On one image 11, 15 and 10 us against 13, 19
+// and 17.
+constexpr int TC_WAIT_LIMIT = 1 << 20;  // polls (a wait of these kernels takes microseconds)
+constexpr int CQ_OUT = 128;      // output pixels of a strip
+constexpr int CQ_PX = 136;       // input pixels of a ring row: 128 + 4, whole 128-byte core matrices
+constexpr int CQ_PLANE = CQ_PX * 16;  // bytes of one 8-channel plane of an input row
+constexpr int CQ_SLOTS = 5;      // quads of input rows in the ring
+constexpr int CQ_EPI_WARPS = 8, CQ_LOAD_WARPS = 8, CQ_MMA_WARPS = 4;
+constexpr int CQ_THREADS = 32 * (CQ_EPI_WARPS + CQ_LOAD_WARPS + CQ_MMA_WARPS);
 
-constexpr int TC_ROWS = 8;               // output rows per CTA
-constexpr int TC_COLS = 136;             // 128 + 4 halo + 4 (the pair of taps 4 and 5 reads one more pixel)
-constexpr int TC_TILE_ROWS = TC_ROWS + 4;
-constexpr int TC_PLANE = TC_TILE_ROWS * TC_COLS * 16;  // bytes of one 8-channel plane
-constexpr int TC_WAIT_LIMIT = 1 << 24;
-
+// C: input channels (8 or 16)
 template <int C>
-__host__ __device__ constexpr int tc_mmas_per_row() { return C == 16 ? 25 : 15; }
-template <int N>
-__host__ __device__ constexpr int tc_b_bytes() { return N * 32; }  // one K=16 x N operand (512 B)
-// at least 57 KB, so that at most 4 CTAs share an SM: 4 x 128 columns fill
-// the 512 of tensor memory, and no allocation has to wait for another CTA
-template <int C, int N>
-constexpr size_t tc_smem_bytes() {
-  return std::max<size_t>((size_t)(C / 8) * TC_PLANE + (size_t)tc_mmas_per_row<C>() * tc_b_bytes<N>() + 64,
-                          57 * 1024);
+struct CqIn {
+  static constexpr int PLANES = C / 8;
+  static constexpr int ROW = PLANES * CQ_PLANE;
+  static constexpr int QUAD = 4 * ROW;
+  static constexpr int NKX = C == 8 ? 3 : 5;  // MMAs per t
+};
+// NB: columns of an output row (its channels, 16 or 1)
+template <int C, int NB>
+struct CqAcc {
+  static constexpr int N = NB == 1 ? 16 : 64;  // columns of an MMA and of an accumulator
+  static constexpr int COLS = CQ_MMA_WARPS * N;
+  // columns of a kx's weight strip: 11 blocks (NB = 1: and the rest of the last window)
+  static constexpr int STRIP = NB == 1 ? 24 : 11 * 16;
+  static constexpr int WBYTES = CqIn<C>::NKX * STRIP * 32;
+};
+template <int C, int NB>
+constexpr size_t cq_smem_bytes() {
+  return (size_t)CQ_SLOTS * CqIn<C>::QUAD + CqAcc<C, NB>::WBYTES + 256;
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -292,11 +136,6 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap *m, 
       "l"(reinterpret_cast<uint64_t>(m)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
       : "memory");
 }
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-               "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
 __device__ __forceinline__ uint32_t mbar_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok = 0;
   for (int it = 0; it < TC_WAIT_LIMIT && !ok; it++) {
@@ -309,214 +148,699 @@ __device__ __forceinline__ uint32_t mbar_wait(uint32_t bar, uint32_t parity) {
   return ok;
 }
 
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, bool valid) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+// The three BF16 parts of v (bit patterns in the upper halves): v = hi + mid +
+// lo exactly; an infinity or a NaN stays in hi alone.
+__device__ __forceinline__ void split3_bf16(float v, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
+  hi = __float_as_uint(v) & 0xFFFF0000u;
+  float r = v - __uint_as_float(hi);
+  r = r == r ? r : 0.0f;
+  mid = __float_as_uint(r) & 0xFFFF0000u;
+  lo = __float_as_uint(r - __uint_as_float(mid));
 }
+// the upper halves of a and b as two BF16 words, a first
+__device__ __forceinline__ uint32_t pack_hi(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
 
-// Weight of operand element (n, k) of MMA j: layer with C input channels
-// (C = 8: taps paired along x), output channel n.
-template <int C>
-__device__ __forceinline__ float tc_weight(const __nv_bfloat16 *__restrict__ w, int cin, int cout, int j, int n,
-                                           int k) {
-  if (n >= cout) return 0.0f;
-  if (C == 16) return __bfloat162float(__ldg(w + (n * cin + k) * TAPS + j));
-  const int ky = j / 3, kx = 2 * (j % 3) + (k >> 3), ci = k & 7;
-  return (kx < 5 && ci < cin) ? __bfloat162float(__ldg(w + (n * cin + ci) * TAPS + ky * 5 + kx)) : 0.0f;
+__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(addr));
 }
-
-// The B operands of all three layers in their shared-memory layout (element
-// (n, k) of MMA j at j*512 + (k/8)*256 + (n/8)*128 + (n%8)*16 + (k%8)*2),
-// written once per parameter set by k_pack_tc and copied by each CTA.
-constexpr int TC_PACK_L1 = 0, TC_PACK_L2 = 15 * 512, TC_PACK_L3 = TC_PACK_L2 + 25 * 512,
-              TC_PACK_BYTES = TC_PACK_L3 + 25 * 512;
-
-__global__ void k_pack_tc(const __nv_bfloat16 *__restrict__ params, __nv_bfloat16 *__restrict__ packed) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= TC_PACK_BYTES / 2) return;
-  const int byte = 2 * i;
-  float v;
-  int rel, layer;
-  if (byte < TC_PACK_L2) rel = byte, layer = 1;
-  else if (byte < TC_PACK_L3) rel = byte - TC_PACK_L2, layer = 2;
-  else rel = byte - TC_PACK_L3, layer = 3;
-  const int j = rel / 512, q = rel % 512;
-  const int k = ((q / 256) << 3) | ((q % 16) / 2), n = ((q / 128) % 2) * 8 + (q % 128) / 16;
-  if (layer == 1) v = tc_weight<8>(params + P_W1, CNN_IN, CNN_HID, j, n, k);
-  else if (layer == 2) v = tc_weight<16>(params + P_W2, CNN_HID, CNN_HID, j, n, k);
-  else v = tc_weight<16>(params + P_W3, CNN_HID, 1, j, n, k);
-  packed[i] = __float2bfloat16_rn(v);
+__device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
 }
-
-template <int C, int N, int MODE>
-__global__ void __launch_bounds__(128) k_conv_tc(const __grid_constant__ CUtensorMap tile, int W, int H,
-                                                 const uint8_t *__restrict__ wpack,
-                                                 const __nv_bfloat16 *__restrict__ bias, void *__restrict__ out,
-                                                 float inv_tau, uint32_t *__restrict__ err) {
-  constexpr int NP = C / 8;  // channel planes
-  constexpr int NM = tc_mmas_per_row<C>();
-  constexpr int BB = tc_b_bytes<N>();
-  static_assert(N == 16, "M = 128 MMAs take N in steps of 16");
-  constexpr int TMEM_COLS = TC_ROWS * N;  // 128
-  extern __shared__ __align__(1024) uint8_t tsm[];
-  uint8_t *planes = tsm;                  // NP x [TC_TILE_ROWS][TC_COLS][8] bf16
-  uint8_t *wsm = tsm + NP * TC_PLANE;     // NM x [k half][N][8] bf16
-  uint64_t *mbar = reinterpret_cast<uint64_t *>(wsm + NM * BB);  // [0], [1]: MMA stages; [2]: loads
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(wsm + NM * BB + 24);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int img = blockIdx.z;
-  const int x0 = blockIdx.x * 128, y0 = blockIdx.y * TC_ROWS;
-
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
-                 "r"(TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+__device__ __forceinline__ void tc_commit(uint64_t *bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
+               : "memory");
+}
+// A bounded wait; one that gives up sets *stop, on which every later wait of
+// the block gives up at once.
+__device__ __forceinline__ bool tc_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *stop) {
+  const uint32_t addr = smem_addr(bar);
+  for (int it = 0; it < TC_WAIT_LIMIT; it++) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(addr), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if (*stop) return false;
   }
-  if (tid == 0) {
-    // stage barriers: one arrival per issuing warp (two warps per stage)
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(smem_addr(mbar)));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(smem_addr(mbar + 1)));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(mbar + 2)));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  *stop = 1u;
+  return false;
+}
+__device__ __forceinline__ void tc_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+// A block's share of the output quads: segments of consecutive quads of one
+// strip.
+struct CqSeg {
+  int64_t r, end;  // position in the quad space, strip after strip; the share's end
+  int img, x0, y0, len;  // first output pixel and row, quads
+};
+__device__ __forceinline__ void cq_seg(CqSeg &s, int quads, int strips) {
+  const int64_t strip = s.r / quads;
+  const int first = (int)(s.r - strip * quads);
+  s.img = (int)(strip / strips);
+  s.x0 = (int)(strip % strips) * CQ_OUT;
+  s.y0 = 4 * first;
+  s.len = (int)min((int64_t)(quads - first), s.end - s.r);
+}
+
+// Pixel (x, y) of image img as loaded: C BF16 channels, zero outside the image.
+template <int C>
+struct CqPx {
+  uint4 v[C / 8];
+};
+template <int C>
+__device__ __forceinline__ void cq_load_px(CqPx<C> &p, const __nv_bfloat16 *__restrict__ in, int img, int x, int y,
+                                           int W, int H) {
+  const bool inside = x >= 0 && x < W && y >= 0 && y < H;
+  const uint4 *q = reinterpret_cast<const uint4 *>(in) + (((int64_t)img * H + y) * W + x) * (C / 8);
+#pragma unroll
+  for (int k = 0; k < C / 8; k++) p.v[k] = inside ? __ldg(q + k) : make_uint4(0u, 0u, 0u, 0u);
+}
+// into position d of an input row (planes CQ_PLANE apart)
+template <int C>
+__device__ __forceinline__ void cq_store_px(const CqPx<C> &p, uint8_t *d) {
+#pragma unroll
+  for (int k = 0; k < C / 8; k++) *reinterpret_cast<uint4 *>(d + k * CQ_PLANE) = p.v[k];
+}
+
+// Element (column n, k) of MMA column kxi's weight strip.  Block i of a strip
+// holds ky = 7 - i (zero unless 0 .. 4), its columns the output channels; k is
+// the input channel (8 channels: of pixel kx = 2 kxi, then of kx + 1).
+template <int C, int NB>
+__device__ __forceinline__ __nv_bfloat16 cq_weight(const __nv_bfloat16 *__restrict__ w, int kxi, int n, int k) {
+  constexpr int CIN = C == 8 ? CNN_IN : CNN_HID;
+  const int co = n % NB, ky = 7 - n / NB, kx = C == 8 ? 2 * kxi + (k >> 3) : kxi, ci = k % C;
+  if (ky < 0 || ky > 4 || kx > 4 || ci >= CIN) return __float2bfloat16_rn(0.0f);
+  return __ldg(w + (co * CIN + ci) * TAPS + ky * 5 + kx);
+}
+
+template <int C, int NB, int MODE>
+__global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat16 *__restrict__ in, int W, int H, int n_img,
+                                                             const __nv_bfloat16 *__restrict__ w,
+                                                             const __nv_bfloat16 *__restrict__ bias,
+                                                             void *__restrict__ out, float inv_tau,
+                                                             uint32_t *__restrict__ err) {
+  using I = CqIn<C>;
+  using A = CqAcc<C, NB>;
+  extern __shared__ __align__(1024) uint8_t rsm[];
+  uint8_t *ring = rsm;
+  uint8_t *wsm = rsm + CQ_SLOTS * I::QUAD;  // [kx][k half][strip column][8] bf16
+  uint64_t *full = reinterpret_cast<uint64_t *>(wsm + A::WBYTES);
+  uint64_t *empty = full + CQ_SLOTS, *dfull = empty + CQ_SLOTS, *dempty = dfull + CQ_MMA_WARPS,
+           *drain = dempty + CQ_MMA_WARPS;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
+  volatile uint32_t *stop = tmem_slot + 1;
+  static_assert((2 * CQ_SLOTS + 2 * CQ_MMA_WARPS + 2) * 8 <= 256, "barrier words");
+  static_assert(I::QUAD % 128 == 0 && A::WBYTES % 16 == 0, "operand alignment");
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool loader = warp >= CQ_EPI_WARPS && warp < CQ_EPI_WARPS + CQ_LOAD_WARPS;
+  const int quads = (H + 3) / 4, strips = (W + CQ_OUT - 1) / CQ_OUT;
+  const int64_t total = (int64_t)strips * n_img * quads;
+  CqSeg seg;
+  seg.r = total * blockIdx.x / gridDim.x;
+  seg.end = total * (blockIdx.x + 1) / gridDim.x;
+
+  // Loaders: a quad's 4 x 132 pixels over 256 threads, two rows of one pixel
+  // column each and the last four columns by the first 16 (quad g of the
+  // block's sequence goes to ring slot g % SLOTS); the next quad in flight
+  // while they wait for its slot, the first of all while the block is set up.
+  const int lt = tid - 32 * CQ_EPI_WARPS;
+  const int lpx = lt & 127, lrow = (lt >> 7) * 2;
+  CqSeg c = seg;
+  int ci = 0;  // the segment's next input quad to fetch, 0 .. len
+  CqPx<C> p[3];
+  auto fetch = [&] {
+    if (c.r >= c.end) return;
+    const int gy = c.y0 - 2 + 4 * ci, gx = c.x0 - 2;
+    cq_load_px<C>(p[0], in, c.img, gx + lpx, gy + lrow, W, H);
+    cq_load_px<C>(p[1], in, c.img, gx + lpx, gy + lrow + 1, W, H);
+    if (lt < 16) cq_load_px<C>(p[2], in, c.img, gx + 128 + (lt & 3), gy + (lt >> 2), W, H);
+    if (++ci < c.len + 1) return;
+    c.r += c.len;
+    ci = 0;
+    if (c.r < c.end) cq_seg(c, quads, strips);
+  };
+  if (loader) {
+    if (c.r < c.end) cq_seg(c, quads, strips);
+    fetch();
+  } else {
+    // (a thread's weights in flight together)
+    constexpr int SETUP = CQ_THREADS - 32 * CQ_LOAD_WARPS, WN = A::WBYTES / 2, PER = (WN + SETUP - 1) / SETUP;
+    const int t = warp < CQ_EPI_WARPS ? tid : tid - 32 * CQ_LOAD_WARPS;
+#pragma unroll 8
+    for (int k = 0; k < PER; k++) {
+      const int i = t + k * SETUP, r = (i >> 3) / A::STRIP;
+      if (i < WN)
+        reinterpret_cast<__nv_bfloat16 *>(wsm)[i] =
+            cq_weight<C, NB>(w, r >> 1, (i >> 3) % A::STRIP, (r & 1) * 8 + (i & 7));
+    }
+    // (the ring's pixels 132 .. 135 are never written: the 8-channel layer's
+    // last tap pair reads pixel 132 against zero weights)
+    if constexpr (C == 8)
+      for (int i = t; i < 4 * CQ_SLOTS * 4; i += SETUP)
+        *reinterpret_cast<uint4 *>(ring + (i >> 2) * I::ROW + (132 + (i & 3)) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    if (warp == 0) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
+                   "r"(A::COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 32) {
+      auto init = [](uint64_t *b, uint32_t n) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(n));
+      };
+      for (int k = 0; k < CQ_SLOTS; k++) init(full + k, CQ_LOAD_WARPS), init(empty + k, CQ_MMA_WARPS);
+      for (int k = 0; k < CQ_MMA_WARPS; k++) init(dfull + k, 1), init(dempty + k, CQ_EPI_WARPS);
+      init(drain, CQ_MMA_WARPS);
+      *stop = 0u;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  const size_t img_base = (size_t)img * W * H;
-  const uint32_t pbase = smem_addr(planes), wbase = smem_addr(wsm), ld_bar = smem_addr(mbar + 2);
-  // the input tile (zero outside the image) and the weight operands, by the
-  // tensor-memory-access unit: one tile copy per 8-channel plane, one bulk copy
-  if (tid == 0) {
-    const uint32_t bytes = (uint32_t)(NP * TC_PLANE + NM * BB);
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(ld_bar), "r"(bytes) : "memory");
-    if constexpr (C == 16) {
-      tma_load_5d(pbase, &tile, 0, 0, x0 - 2, y0 - 2, img, ld_bar);
-      tma_load_5d(pbase + TC_PLANE, &tile, 0, 1, x0 - 2, y0 - 2, img, ld_bar);
-    } else {
-      tma_load_4d(pbase, &tile, 0, x0 - 2, y0 - 2, img, ld_bar);
-    }
-    bulk_load(wbase, wpack, (uint32_t)(NM * BB), ld_bar);
-  }
-  const uint32_t loaded = mbar_wait(ld_bar, 0);
-  if (!loaded && tid == 0 && err) atomicOr(err, ERR_SPIN_TIMEOUT);
 
-  // MMAs in two stages (output rows 0-3, then 4-7), one mbarrier each, so the
-  // read-back of the first overlaps the MMAs of the second; each warp's
-  // first lane issues the MMAs of two rows (four issuers share the tensor core)
-  auto issue = [&](int r0, int r1, uint64_t *bar) {
-    const uint32_t lbo = C == 16 ? (uint32_t)TC_PLANE : 16u;
-    for (int r = r0; r < r1; r++) {
-      for (int j = 0; j < NM; j++) {
-        const int ky = C == 16 ? j / 5 : j / 3;
-        const int kx = C == 16 ? j % 5 : 2 * (j % 3);
-        const uint64_t ad = tc_desc(pbase + (uint32_t)(((r + ky) * TC_COLS + kx) * 16), lbo, 128);
-        const uint64_t bd = tc_desc(wbase + (uint32_t)(j * BB), BB / 2, 128);
-        const uint32_t acc = j > 0 ? 1u : 0u;
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem + (uint32_t)(r * N)),
-            "l"(ad), "l"(bd), "r"(tc_idesc<N>()), "r"(acc));
-      }
+  if (loader) {
+    // input quads of the whole share: its output quads, and the halo of each segment
+    const int64_t segs = seg.r < seg.end ? (seg.end - 1) / quads - seg.r / quads + 1 : 0;
+    const uint32_t count = (uint32_t)(seg.end - seg.r + segs);
+    uint32_t sl = 0, par = 1;  // ring slot; parity of the wait for it (at once in the first turn)
+    for (uint32_t g = 0; g < count; g++) {
+      if (!tc_wait(empty + sl, par, stop)) break;
+      uint8_t *d = ring + sl * I::QUAD;
+      cq_store_px<C>(p[0], d + lrow * I::ROW + lpx * 16);
+      cq_store_px<C>(p[1], d + (lrow + 1) * I::ROW + lpx * 16);
+      if (lt < 16) cq_store_px<C>(p[2], d + (lt >> 2) * I::ROW + (128 + (lt & 3)) * 16);
+      __syncwarp();
+      if (lane == 0) tc_arrive(full + sl);
+      if (++sl == CQ_SLOTS) sl = 0, par ^= 1;
+      fetch();
     }
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_addr(bar))
-                 : "memory");
-  };
-  static_assert(TC_ROWS == 8, "two rows per warp, two warps per stage");
-  if (lane == 0 && loaded) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    issue(2 * warp, 2 * warp + 2, mbar + (warp >> 1));
-  }
-
-  auto wait_bar = [&](uint64_t *bar) -> uint32_t {
-    const uint32_t ok = loaded ? mbar_wait(smem_addr(bar), 0) : 0u;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (!ok && tid == 0 && err) atomicOr(err, ERR_SPIN_TIMEOUT);
-    return ok;
-  };
-  const int gx = x0 + 32 * warp + lane;
-  const uint32_t trow = tmem + ((uint32_t)(32 * warp) << 16);
-  // read back and store output rows [r0, r1) once their MMAs are done
-  auto epilogue = [&](int r0, int r1, uint32_t done) {
-    if constexpr (MODE == CONV_RELU_BF16) {
-      float b[16];
+  } else if (warp >= CQ_EPI_WARPS) {
+    if (lane == 0) {
+      // MMAs: of every segment, issuer m takes output quads m, m + 4, ... into
+      // its own accumulator.  Quad k reads input quads k and k + 1, there
+      // when the second is (the loaders take them in order).  Every issuer
+      // releases every input quad once, in order: by a commit after its last
+      // output quad that reads it, or, reading none of it, after it has
+      // passed; so no phase of a slot is missed.
+      const uint32_t m = (uint32_t)(warp - CQ_EPI_WARPS - CQ_LOAD_WARPS);
+      const uint32_t rbase = smem_addr(ring), wbase = smem_addr(wsm), acc = tmem + m * A::N;
+      uint32_t g = 0, dpar = 1;  // the segment's first input quad; parity of the wait for the accumulator
+      bool ok = true;
+      auto wait_full = [&](uint32_t gi) { return tc_wait(full + gi % CQ_SLOTS, (gi / CQ_SLOTS) & 1, stop); };
+      while (seg.r < seg.end && ok) {
+        cq_seg(seg, quads, strips);
+        const uint32_t len = (uint32_t)seg.len;
+        uint32_t q = 0;  // the segment's next input quad to release
+        for (uint32_t k = m;; k += CQ_MMA_WARPS) {
+          const uint32_t upto = k < len ? k : len + 1;
+          for (; q < upto && ok; q++) {
+            ok = wait_full(g + q);
+            if (ok) tc_arrive(empty + (g + q) % CQ_SLOTS);
+          }
+          if (k >= len || !ok) break;
+          const uint32_t gi = g + k;
+          ok = wait_full(gi + 1) && tc_wait(dempty + m, dpar, stop);
+          if (!ok) break;
+          dpar ^= 1;
+          // the loaders' stores, acquired through their barrier, ordered
+          // before the tensor core's reads
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t s0 = rbase + gi % CQ_SLOTS * I::QUAD, s1 = rbase + (gi + 1) % CQ_SLOTS * I::QUAD;
+          constexpr int KXS = C == 8 ? 32 : 16, LBO = C == 8 ? 16 : CQ_PLANE;
+          for (int t = 0; t < 8; t++) {
+            const uint32_t rb = (t < 4 ? s0 : s1) + (t & 3) * I::ROW;
+            const uint32_t wb = wbase + (uint32_t)((7 - t) * NB * 16);
 #pragma unroll
-      for (int c = 0; c < 16; c++) b[c] = __bfloat162float(bias[c]);
-#pragma unroll 1
-      for (int r = r0; r < r1; r++) {
-        uint32_t v[16];
-        if (done) {
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-              : "r"(trow + (uint32_t)(r * N)));
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        } else {
-#pragma unroll
-          for (int c = 0; c < 16; c++) v[c] = 0x7FC00000u;  // NaN: the accumulators were not read
+            for (int kx = 0; kx < I::NKX; kx++)
+              tc_mma(acc, tc_desc(rb + kx * KXS, LBO, 128), tc_desc(wb + kx * A::STRIP * 32, A::STRIP * 16, 128),
+                     tc_idesc<A::N>(), (kx || t) ? 1u : 0u);
+          }
+          tc_commit(dfull + m);
+          // the input quads this issuer's next output quad does not read
+          for (; q <= k + 1; q++) tc_commit(empty + (g + q) % CQ_SLOTS);
         }
-        const int gy = y0 + r;
-        if (gx < W && gy < H) {
-          uint4 o[2];
-          __nv_bfloat16 *ob = reinterpret_cast<__nv_bfloat16 *>(o);
-#pragma unroll
-          for (int c = 0; c < 16; c++) ob[c] = __float2bfloat16_rn(fmaxf(__uint_as_float(v[c]) + b[c], 0.0f));
-          uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(out) +
-                                                 (img_base + (size_t)gy * W + gx) * 16);
-          dst[0] = o[0];
-          dst[1] = o[1];
-        }
+        g += len + 1;
+        seg.r += seg.len;
       }
-    } else {
-      const float b0 = __bfloat162float(bias[0]);
-      constexpr int HALF = TC_ROWS / 2;
-      uint32_t v[HALF];
-      if (done) {
-        // column 0 (output channel 0) of each row's accumulator
-#pragma unroll
-        for (int k = 0; k < HALF; k++)
-          asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];"
-                       : "=r"(v[k])
-                       : "r"(trow + (uint32_t)((r0 + k) * N)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      } else {
-#pragma unroll
-        for (int k = 0; k < HALF; k++) v[k] = 0x7FC00000u;
-      }
-#pragma unroll
-      for (int k = 0; k < HALF; k++) {
-        const int gy = y0 + r0 + k;
-        if (gx >= W || gy >= H) continue;
-        const float a = __uint_as_float(v[k]) + b0;
-        float o = a;
-        if (MODE == CONV_CONF) {
-          const float c = fmaxf(1.0f - fmaxf(a, 0.0f) * inv_tau, 0.0f);
-          o = c * c;
-        }
-        reinterpret_cast<float *>(out)[img_base + (size_t)gy * W + gx] = o;
-      }
+      // every MMA and commit done before the block's memory is given back
+      tc_commit(drain);
+      uint32_t never = 0u;
+      tc_wait(drain, 0, &never);
     }
-  };
-  const uint32_t done0 = wait_bar(mbar);
-  epilogue(0, TC_ROWS / 2, done0);
-  const uint32_t done1 = wait_bar(mbar + 1);
-  epilogue(TC_ROWS / 2, TC_ROWS, done1);
-  // A wait that gave up may leave the tile copies or the MMAs in flight,
-  // writing this block's shared and tensor memory: wait for them once more
-  // (bounded again) before both are given back.  If that wait gives up too,
-  // the frame is already reported failed and its confidence map is not used.
-  if (!loaded) {
-    mbar_wait(ld_bar, 0);
   } else {
-    if (!done0) mbar_wait(smem_addr(mbar), 0);
-    if (!done1) mbar_wait(smem_addr(mbar + 1), 0);
+    // Epilogue: two groups of four warps, two rows of every quad each; the
+    // accumulators in turn, from the first in every segment
+    const int quad = warp & 3, row0 = (warp >> 2) * 2;
+    const uint32_t trow = tmem + ((uint32_t)(32 * quad) << 16);
+    float b[NB];
+#pragma unroll
+    for (int k = 0; k < NB; k++) b[k] = __bfloat162float(__ldg(bias + k));
+    uint32_t par = 0;  // bit d: parity of the next wait for accumulator d
+    while (seg.r < seg.end) {
+      cq_seg(seg, quads, strips);
+      uint32_t d = 0;
+      const int gx = seg.x0 + quad * 32 + lane;
+      for (int i = 0; i < seg.len; i++) {
+        const int gy = seg.y0 + 4 * i + row0;
+        const size_t px0 = ((size_t)seg.img * H + gy) * W + gx;
+        const bool inside[2] = {gx < W && gy < H, gx < W && gy + 1 < H};
+        const bool ok = tc_wait(dfull + d, (par >> d) & 1, stop);
+        __syncwarp();  // (the reads of tensor memory are by whole warps)
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        uint32_t v[2][16];
+        if constexpr (NB == 1) {
+          tmem_ld16(trow + d * A::N, v[0]);  // column j: output row j
+        } else {
+          tmem_ld16(trow + d * A::N + row0 * 16, v[0]);
+          tmem_ld16(trow + d * A::N + row0 * 16 + 16, v[1]);
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (lane == 0) tc_arrive(dempty + d);
+        par ^= 1u << d;
+        d = (d + 1) % CQ_MMA_WARPS;
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+          if (!inside[r]) continue;
+          const size_t px = px0 + (size_t)r * W;
+          if constexpr (NB == 1) {
+            float a = __uint_as_float(row0 ? v[0][2 + r] : v[0][r]) + b[0];
+            if (!ok) a = __uint_as_float(0x7FC00000u);  // NaN: the accumulators were not read
+            if (MODE == CONV_CONF) {
+              // (1 - r/tau)^2 on [0, tau], 0 beyond: weight falls to exactly zero
+              // for pixels whose predicted residual reaches tau
+              const float f = fmaxf(1.0f - fmaxf(a, 0.0f) * inv_tau, 0.0f);
+              a = ok ? f * f : a;
+            }
+            reinterpret_cast<float *>(out)[px] = a;
+          } else {
+            float a[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) a[k] = ok ? __uint_as_float(v[r][k]) + b[k] : __uint_as_float(0x7FC00000u);
+            uint4 o[2];
+            __nv_bfloat16 *ob = reinterpret_cast<__nv_bfloat16 *>(o);
+#pragma unroll
+            for (int k = 0; k < 16; k++) ob[k] = __float2bfloat16_rn(fmaxf(a[k], 0.0f));
+            uint4 *dst = reinterpret_cast<uint4 *>(reinterpret_cast<__nv_bfloat16 *>(out) + px * 16);
+            dst[0] = o[0];
+            dst[1] = o[1];
+          }
+        }
+        __syncwarp();
+      }
+      seg.r += seg.len;
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (*stop && tid == 0 && err) atomicOr(err, ERR_SPIN_TIMEOUT);
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(A::COLS));
+}
+
+// ------------------------------------------------ tensor-core input gradients
+//
+// The gradient of a layer's input, masked by the ReLU of the stored activation:
+// a correlation of the FP32 output gradient with the layer's weights, transposed
+// and flipped, as a streamed implicit GEMM.  Per output row of a strip, one
+// tcgen05.mma (M = 128 input pixels, N = 80, K = 16) per kernel row ky and BF16
+// part accumulates
+//   D[input pixel s][kx * 16 + ci] = sum over ky, co of g[row + ky][s][co] * w[co][ci][4 - ky][4 - kx],
+// all five kx side by side in N, and the epilogue adds
+//   out[j][ci] = sum over kx of D[j + kx][kx * 16 + ci]
+// across the lanes of a warp: a 32-pixel window belongs to each warp, so it
+// gives 28 outputs, and the four windows of a strip start 28 pixels apart.
+// Not as the forward layers: the gradient enters as three BF16 parts whose sum
+// it is exactly (split3_bf16), so the MMAs count three times, and all kx in N
+// take 15 of them a row where quads take 30; the fewer sums in the accumulator,
+// which rounds toward zero, also keep the error below that of FP32
+// multiply-adds (7.1e-8 and 8.5e-8 relative L2 for layers 3 and 2 against 64 bits;
+// 8.8e-8 and 2.4e-7 with FP32, 1.4e-7 and 2.2e-7 as quads).  Layer 3's
+// one-channel gradient has the three parts of its five rows ky in the K
+// dimension: its ring holds an output row's operand, one MMA a row.
+//
+// Streaming as in the forward layers, two rows at a time: loader warps bring
+// pairs of input rows into the ring, four issuers with an accumulator each take
+// the output rows in turn, two groups of epilogue warps the rows of a pair.
+//
+// Measured on four 640x480 images: layers 3 and 2 take 43 and 74 us, bound by
+// the epilogue's shuffles (64 per warp and row) and by the MMAs (15 a row,
+// about 107 cycles each); FP32 multiply-adds on the CUDA cores 50 and 366 us.
+constexpr int RC_OUT = 112;      // output pixels of a strip: 4 windows of 28
+constexpr int RC_SLOTS = 6;      // pairs of input rows in the ring
+constexpr int RC_PLANE = 128 * 16;  // bytes of one 8-channel plane of an input row
+constexpr int RC_EPI_WARPS = 8, RC_LOAD_WARPS = 4, RC_MMA_WARPS = 4;
+constexpr int RC_AHEAD = 2;      // pairs of input rows a loader has in flight
+constexpr int RC_THREADS = 32 * (RC_EPI_WARPS + RC_LOAD_WARPS + RC_MMA_WARPS);
+constexpr int RC_MIN_PAIRS = 2;  // pairs of output rows that are worth a block of their own
+
+enum RcInput { RC_F32_16 = 0, RC_F32_1 = 1 };
+
+template <int IN>
+struct RcIn {
+  static constexpr int PARTS = IN == RC_F32_16 ? 3 : 1;  // MMAs per kernel row
+  static constexpr int ROW = 2 * PARTS * RC_PLANE;
+  static constexpr int PAIR = 2 * ROW;
+  static constexpr int KY = IN == RC_F32_1 ? 1 : 5;    // ring rows of an output row
+  static constexpr int HALO = IN == RC_F32_1 ? 0 : 2;  // ring pairs of a segment beyond its output pairs
+};
+constexpr int RC_N = 80, RC_COLS = 512;  // columns of an accumulator (one per issuer), and allocated
+static_assert(RC_MMA_WARPS * RC_N <= RC_COLS, "accumulators fit the allocation");
+template <int IN>
+constexpr size_t rc_smem_bytes() {
+  return std::max<size_t>((size_t)RC_SLOTS * RcIn<IN>::PAIR + RcIn<IN>::KY * 2 * RC_N * 16 + 512,
+                          114 * 1024);  // (one block per SM: all of tensor memory)
+}
+
+// A block's share of the output row pairs: segments of consecutive pairs of
+// one strip (x0: its first output pixel).
+struct RcSeg {
+  int64_t r, end;  // position in the pair space, strip after strip; the share's end
+  int img, x0, y0, len;  // first output row, pairs
+};
+__device__ __forceinline__ void rc_seg(RcSeg &s, int pairs, int strips) {
+  const int64_t strip = s.r / pairs;
+  const int first = (int)(s.r - strip * pairs);
+  s.img = (int)(strip / strips);
+  s.x0 = (int)(strip % strips) * RC_OUT;
+  s.y0 = 2 * first;
+  s.len = (int)min((int64_t)(pairs - first), s.end - s.r);
+}
+
+// One pixel's channels as loaded.
+template <int IN>
+struct RcPx {
+  static constexpr int NV = IN == RC_F32_16 ? 4 : 2;
+  uint4 v[NV];
+};
+// Pixel px = (y, x) of an image of H rows; a one-channel input: rows y - 2 .. y + 2 of
+// its column (zero outside).
+template <int IN>
+__device__ __forceinline__ void rc_load_px(RcPx<IN> &p, const void *__restrict__ in, bool inside_x, int y, int H,
+                                           int W, size_t px) {
+#pragma unroll
+  for (int k = 0; k < RcPx<IN>::NV; k++) p.v[k] = make_uint4(0u, 0u, 0u, 0u);
+  if (!inside_x) return;
+  if constexpr (IN == RC_F32_1) {
+    const uint32_t *q = reinterpret_cast<const uint32_t *>(in) + px;
+    if (y - 2 >= 0 && y - 2 < H) p.v[0].x = __ldg(q - 2 * (int64_t)W);
+    if (y - 1 >= 0 && y - 1 < H) p.v[0].y = __ldg(q - (int64_t)W);
+    if (y < H) p.v[0].z = __ldg(q);
+    if (y + 1 < H) p.v[0].w = __ldg(q + W);
+    if (y + 2 < H) p.v[1].x = __ldg(q + 2 * (int64_t)W);
+  } else if (y >= 0 && y < H) {
+#pragma unroll
+    for (int k = 0; k < RcPx<IN>::NV; k++) p.v[k] = __ldg(reinterpret_cast<const uint4 *>(in) + px * RcPx<IN>::NV + k);
+  }
+}
+// into slot position d of an input row (planes RC_PLANE apart)
+template <int IN>
+__device__ __forceinline__ void rc_store_px(const RcPx<IN> &p, uint8_t *d) {
+  if constexpr (IN == RC_F32_1) {
+    // K = 3 ky + part, and a zero
+    uint32_t h[5], m[5], l[5];
+    split3_bf16(__uint_as_float(p.v[0].x), h[0], m[0], l[0]);
+    split3_bf16(__uint_as_float(p.v[0].y), h[1], m[1], l[1]);
+    split3_bf16(__uint_as_float(p.v[0].z), h[2], m[2], l[2]);
+    split3_bf16(__uint_as_float(p.v[0].w), h[3], m[3], l[3]);
+    split3_bf16(__uint_as_float(p.v[1].x), h[4], m[4], l[4]);
+    *reinterpret_cast<uint4 *>(d) =
+        make_uint4(pack_hi(h[0], m[0]), pack_hi(l[0], h[1]), pack_hi(m[1], l[1]), pack_hi(h[2], m[2]));
+    *reinterpret_cast<uint4 *>(d + RC_PLANE) =
+        make_uint4(pack_hi(l[2], h[3]), pack_hi(m[3], l[3]), pack_hi(h[4], m[4]), l[4] >> 16);
+  } else {
+#pragma unroll
+    for (int half = 0; half < 2; half++) {
+      uint32_t h[8], m[8], l[8];
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const uint4 u = p.v[2 * half + k];
+        split3_bf16(__uint_as_float(u.x), h[4 * k], m[4 * k], l[4 * k]);
+        split3_bf16(__uint_as_float(u.y), h[4 * k + 1], m[4 * k + 1], l[4 * k + 1]);
+        split3_bf16(__uint_as_float(u.z), h[4 * k + 2], m[4 * k + 2], l[4 * k + 2]);
+        split3_bf16(__uint_as_float(u.w), h[4 * k + 3], m[4 * k + 3], l[4 * k + 3]);
+      }
+      *reinterpret_cast<uint4 *>(d + half * RC_PLANE) =
+          make_uint4(pack_hi(h[0], h[1]), pack_hi(h[2], h[3]), pack_hi(h[4], h[5]), pack_hi(h[6], h[7]));
+      *reinterpret_cast<uint4 *>(d + (2 + half) * RC_PLANE) =
+          make_uint4(pack_hi(m[0], m[1]), pack_hi(m[2], m[3]), pack_hi(m[4], m[5]), pack_hi(m[6], m[7]));
+      *reinterpret_cast<uint4 *>(d + (4 + half) * RC_PLANE) =
+          make_uint4(pack_hi(l[0], l[1]), pack_hi(l[2], l[3]), pack_hi(l[4], l[5]), pack_hi(l[6], l[7]));
+    }
+  }
+}
+
+// Element (ky, k, n) of the weight operand: k the layer's output channel (a
+// one-channel gradient: k = 3 ky + part, the parts share a weight), column
+// n = kx * 16 + the layer's input channel.
+template <int IN>
+__device__ __forceinline__ __nv_bfloat16 rc_weight(const __nv_bfloat16 *__restrict__ w, int ky, int k, int n) {
+  if (IN == RC_F32_1 && k >= 15) return __float2bfloat16_rn(0.0f);
+  const int kx = n >> 4, ci = n & 15, co = IN == RC_F32_1 ? 0 : k, y = IN == RC_F32_1 ? k / 3 : ky;
+  return __ldg(w + (co * CNN_HID + ci) * TAPS + (TAPS - 1 - (y * 5 + kx)));
+}
+
+template <int IN>
+__global__ void __launch_bounds__(RC_THREADS, 1) k_grad_rows(const float *__restrict__ in, int W, int H, int n_img,
+                                                            const __nv_bfloat16 *__restrict__ w,
+                                                            float *__restrict__ out,
+                                                            const __nv_bfloat16 *__restrict__ act) {
+  using I = RcIn<IN>;
+  constexpr int N = RC_N;
+  extern __shared__ __align__(1024) uint8_t rsm[];
+  uint8_t *ring = rsm;
+  uint8_t *wsm = rsm + RC_SLOTS * I::PAIR;  // [ky][k half][n][8] bf16
+  uint64_t *full = reinterpret_cast<uint64_t *>(wsm + I::KY * 2 * N * 16);
+  uint64_t *empty = full + RC_SLOTS, *dfull = empty + RC_SLOTS, *dempty = dfull + RC_MMA_WARPS,
+           *drain = dempty + RC_MMA_WARPS;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
+  volatile uint32_t *stop = tmem_slot + 1;
+  static_assert((2 * RC_SLOTS + 2 * RC_MMA_WARPS + 2) * 8 <= 512, "barrier words");
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool loader = warp >= RC_EPI_WARPS && warp < RC_EPI_WARPS + RC_LOAD_WARPS;
+  const int pairs = (H + 1) / 2, strips = (W + RC_OUT - 1) / RC_OUT;
+  const int64_t total = (int64_t)strips * n_img * pairs;
+  RcSeg seg;
+  seg.r = total * blockIdx.x / gridDim.x;
+  seg.end = total * (blockIdx.x + 1) / gridDim.x;
+
+  // Loaders: one pixel of each of a pair's two input rows per thread (pair g of
+  // the block's sequence goes to ring slot g % RC_SLOTS), RC_AHEAD pairs in
+  // flight, the first of them while the block is set up.
+  const int slot = tid - 32 * RC_EPI_WARPS;
+  const int dx = (slot >> 5) * 28 + lane - 2;
+  RcSeg c = seg;
+  int ci = 0;  // the segment's next input pair to fetch, 0 .. len + HALO - 1
+  RcPx<IN> p[RC_AHEAD][2];
+  auto fetch = [&](RcPx<IN> (&q)[2]) {
+    if (c.r >= c.end) return;
+    const int gx = c.x0 + dx, gy = c.y0 - I::HALO + 2 * ci;
+    const bool in_x = gx >= 0 && gx < W;
+    const size_t px = ((size_t)c.img * H + gy) * W + gx;
+    rc_load_px<IN>(q[0], in, in_x, gy, H, W, px);
+    rc_load_px<IN>(q[1], in, in_x, gy + 1, H, W, px + W);
+    if (++ci < c.len + I::HALO) return;
+    c.r += c.len;
+    ci = 0;
+    if (c.r < c.end) rc_seg(c, pairs, strips);
+  };
+  if (loader) {
+    if (c.r < c.end) rc_seg(c, pairs, strips);
+#pragma unroll
+    for (int k = 0; k < RC_AHEAD; k++) fetch(p[k]);
+  } else {
+    // (all of a thread's weights in flight at once)
+    constexpr int SETUP = RC_THREADS - 32 * RC_LOAD_WARPS, WN = I::KY * 16 * N,
+                  PER = (WN + SETUP - 1) / SETUP;
+    const int t = warp < RC_EPI_WARPS ? tid : tid - 32 * RC_LOAD_WARPS;
+    __nv_bfloat16 v[PER];
+#pragma unroll
+    for (int k = 0; k < PER; k++) {
+      const int i = t + k * SETUP, n = (i >> 3) % N, r = (i >> 3) / N;
+      if (i < WN) v[k] = rc_weight<IN>(w, r >> 1, (r & 1) * 8 + (i & 7), n);
+    }
+#pragma unroll
+    for (int k = 0; k < PER; k++)
+      if (t + k * SETUP < WN) reinterpret_cast<__nv_bfloat16 *>(wsm)[t + k * SETUP] = v[k];
+    if (warp == 0) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
+                   "r"(RC_COLS));
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 32) {
+      auto init = [](uint64_t *b, uint32_t n) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(n));
+      };
+      for (int k = 0; k < RC_SLOTS; k++) init(full + k, RC_LOAD_WARPS), init(empty + k, RC_MMA_WARPS);
+      for (int k = 0; k < RC_MMA_WARPS; k++) init(dfull + k, 1), init(dempty + k, RC_EPI_WARPS / 2);
+      init(drain, RC_MMA_WARPS);
+      *stop = 0u;
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+
+  if (loader) {
+    // input pairs of the whole share: its output pairs, and the halo of each segment
+    const int64_t segs = seg.r < seg.end ? (seg.end - 1) / pairs - seg.r / pairs + 1 : 0;
+    const uint32_t count = (uint32_t)(seg.end - seg.r + I::HALO * segs);
+    // (a pair's registers are filled again in place: moving one that a load
+    // still owes would wait for that load)
+    bool ok = true;
+    uint8_t *const dst = ring + slot * 16;
+    uint32_t sl = 0, par = 1;  // ring slot; parity of the wait for it (at once in the first turn)
+    for (uint32_t g0 = 0; g0 < count && ok; g0 += RC_AHEAD) {
+#pragma unroll
+      for (int k = 0; k < RC_AHEAD; k++) {
+        if (g0 + (uint32_t)k >= count) break;
+        ok = tc_wait(empty + sl, par, stop);
+        if (!ok) break;
+        rc_store_px<IN>(p[k][0], dst + sl * I::PAIR);
+        rc_store_px<IN>(p[k][1], dst + sl * I::PAIR + I::ROW);
+        __syncwarp();
+        if (lane == 0) tc_arrive(full + sl);
+        if (++sl == RC_SLOTS) sl = 0, par ^= 1;
+        fetch(p[k]);
+      }
+    }
+  } else if (warp >= RC_EPI_WARPS) {
+    if (lane == 0) {
+      // MMAs: of every segment, issuer m takes output rows m, m + 4, ... into its
+      // own accumulator m (four chains of MMAs run side by side: those of one
+      // accumulator wait for one another).  Its row of output pair k reads input
+      // pairs k .. k + HALO, there when the last one is (the loaders take
+      // them in order).  Every issuer releases every input pair once, in order:
+      // by a commit after its last row that reads it, or, reading none of it,
+      // after it has passed; so no phase of a slot is missed.
+      const uint32_t m = (uint32_t)(warp - RC_EPI_WARPS - RC_LOAD_WARPS);
+      const uint32_t rbase = smem_addr(ring), wbase = smem_addr(wsm);
+      uint32_t g = 0, dpar = 1;  // the segment's first input pair; parity of the wait for the accumulator
+      bool ok = true;
+      auto wait_full = [&](uint32_t gi) { return tc_wait(full + gi % RC_SLOTS, (gi / RC_SLOTS) & 1, stop); };
+      while (seg.r < seg.end && ok) {
+        rc_seg(seg, pairs, strips);
+        const uint32_t len = (uint32_t)seg.len;
+        uint32_t p = 0;  // the segment's next input pair to release
+        for (uint32_t k = m >> 1;; k += 2) {
+          const uint32_t upto = k < len ? k : len + I::HALO;
+          for (; p < upto && ok; p++) {
+            ok = wait_full(g + p);
+            if (ok) tc_arrive(empty + (g + p) % RC_SLOTS);
+          }
+          if (k >= len || !ok) break;
+          const uint32_t gi = g + k;
+          const uint32_t r0 = rbase + gi % RC_SLOTS * I::PAIR, r1 = rbase + (gi + 1) % RC_SLOTS * I::PAIR,
+                         r2 = rbase + (gi + 2) % RC_SLOTS * I::PAIR;
+          // (without a halo the output row's operand is the one ring row r0)
+          const uint32_t rb[5] = {m & 1 ? r0 + I::ROW : r0, m & 1 ? r1 : r0 + I::ROW, m & 1 ? r1 + I::ROW : r1,
+                                  m & 1 ? r2 : r1 + I::ROW, m & 1 ? r2 + I::ROW : r2};
+          ok = wait_full(gi + I::HALO) && tc_wait(dempty + m, dpar, stop);
+          if (!ok) break;
+          dpar ^= 1;
+          // the loaders' stores, acquired through their barrier, ordered
+          // before the tensor core's reads
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          // (the lowest parts first: the accumulator rounds each sum toward
+          // zero, and the small parts' sums lose least while they are alone)
+#pragma unroll
+          for (int part = I::PARTS - 1; part >= 0; part--)
+#pragma unroll
+            for (int ky = 0; ky < I::KY; ky++)
+              tc_mma(tmem + m * N, tc_desc(rb[ky] + part * 2 * RC_PLANE, RC_PLANE, 128),
+                     tc_desc(wbase + (uint32_t)(ky * 2 * N * 16), N * 16, 128), tc_idesc<N>(),
+                     (ky || part < I::PARTS - 1) ? 1u : 0u);
+          tc_commit(dfull + m);
+          // the input pairs this issuer's next row does not read
+          const uint32_t last = (k + 2 < len && I::HALO > 1) ? k + 1 : k + I::HALO;
+          for (; p <= last; p++) tc_commit(empty + (g + p) % RC_SLOTS);
+        }
+        g += len + I::HALO;
+        seg.r += seg.len;
+      }
+      // every MMA and commit done before the block's memory is given back
+      tc_commit(drain);
+      uint32_t never = 0u;
+      tc_wait(drain, 0, &never);
+    }
+  } else {
+    // Epilogue: a group of four warps for each row of a pair; it takes
+    // accumulators row and row + 2 in turn, from row in every segment
+    const int quad = warp & 3, row = warp >> 2;
+    const uint32_t trow = tmem + ((uint32_t)(32 * quad) << 16);
+    uint32_t par = 0;  // bit d: parity of the next wait for accumulator d
+    while (seg.r < seg.end) {
+      rc_seg(seg, pairs, strips);
+      uint32_t d = (uint32_t)row;
+      const int gx = seg.x0 + quad * 28 + lane;
+      for (int i = 0; i < seg.len; i++) {
+        const int gy = seg.y0 + 2 * i + row;
+        const size_t px = ((size_t)seg.img * H + gy) * W + gx;
+        const bool inside = lane < 28 && gx < W && gy < H;
+        uint4 am[2];
+        if (inside) {
+          am[0] = __ldg(reinterpret_cast<const uint4 *>(act + px * 16));
+          am[1] = __ldg(reinterpret_cast<const uint4 *>(act + px * 16) + 1);
+        }
+        const bool ok = tc_wait(dfull + d, (par >> d) & 1, stop);
+        __syncwarp();  // (the reads of tensor memory are by whole warps)
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        uint32_t v[N / 16][16];
+#pragma unroll
+        for (int kx = 0; kx < N / 16; kx++) tmem_ld16(trow + d * N + kx * 16, v[kx]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        if (lane == 0) tc_arrive(dempty + d);
+        par ^= 1u << d;
+        d ^= 2;
+        float a[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+          a[k] = __uint_as_float(v[0][k]);
+#pragma unroll
+          for (int kx = 1; kx < 5; kx++) a[k] += __shfl_down_sync(0xffffffffu, __uint_as_float(v[kx][k]), kx);
+          if (!ok) a[k] = __uint_as_float(0x7FC00000u);  // NaN: the accumulators were not read
+        }
+        if (inside) {
+          const __nv_bfloat16 *ab = reinterpret_cast<const __nv_bfloat16 *>(am);
+          float4 *dst = reinterpret_cast<float4 *>(out + px * 16);
+#pragma unroll
+          for (int k = 0; k < 16; k += 4) {
+            float4 o;
+            o.x = __bfloat162float(ab[k]) > 0.0f ? a[k] : 0.0f;
+            o.y = __bfloat162float(ab[k + 1]) > 0.0f ? a[k + 1] : 0.0f;
+            o.z = __bfloat162float(ab[k + 2]) > 0.0f ? a[k + 2] : 0.0f;
+            o.w = __bfloat162float(ab[k + 3]) > 0.0f ? a[k + 3] : 0.0f;
+            dst[k / 4] = o;
+          }
+        }
+        __syncwarp();
+      }
+      seg.r += seg.len;
+    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(RC_COLS));
 }
 
 // ------------------------------------------- tensor-core weight gradients
@@ -587,26 +911,6 @@ static_assert(wg_smem_bytes<WG_L1>() > 114 * 1024 && wg_smem_bytes<WG_L2>() > 11
 template <int N>
 __host__ __device__ constexpr uint32_t wg_idesc() {
   return tc_idesc<N>() | (1u << 15) | (1u << 16);
-}
-
-// The three BF16 parts of v (bit patterns in the upper halves): v = hi + mid +
-// lo exactly; an infinity or a NaN stays in hi alone.
-__device__ __forceinline__ void split3_bf16(float v, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
-  hi = __float_as_uint(v) & 0xFFFF0000u;
-  float r = v - __uint_as_float(hi);
-  r = r == r ? r : 0.0f;
-  mid = __float_as_uint(r) & 0xFFFF0000u;
-  lo = __float_as_uint(r - __uint_as_float(mid));
-}
-// the upper halves of a and b as two BF16 words, a first
-__device__ __forceinline__ uint32_t pack_hi(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x7632); }
-
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(addr));
 }
 
 template <int KIND>
@@ -727,15 +1031,10 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(const __grid_constant__
         for (int k = 0; k < T::NKX; k++) {
           const uint64_t ad = tc_desc(
               xb + (uint32_t)(ip * T::G * WG_XROW_BYTES + (ch * 16 + k * T::KX_STEP) * 16), 128, WG_XPX * 16);
-          asm volatile(
-              "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
-              " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem + (uint32_t)(k * T::N)),
-              "l"(ad), "l"(bd), "r"(wg_idesc<T::N>()), "r"((ip | ch) ? 1u : 0u));
+          tc_mma(tmem + (uint32_t)(k * T::N), ad, bd, wg_idesc<T::N>(), (ip | ch) ? 1u : 0u);
         }
       }
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_addr(mbar + 2))
-                 : "memory");
+    tc_commit(mbar + 2);
     return 1u;
   };
   const int quad = warp & 3, half = warp >> 2;
@@ -1065,15 +1364,14 @@ namespace {
 std::mutex g_attr_mu;
 unsigned long long g_attr_done = 0;  // devices whose kernels have their shared-memory limits set
 
-template <int KIN, int KOUT, int CSTR, typename TIN, bool TRANS, int MODE>
+template <int C, int NB, int MODE>
 cudaError_t set_conv_attr() {
-  return cudaFuncSetAttribute(k_conv<KIN, KOUT, CSTR, TIN, TRANS, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)conv_smem_bytes<KIN, KOUT>());
+  return cudaFuncSetAttribute(k_conv_quads<C, NB, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)cq_smem_bytes<C, NB>());
 }
-template <int C, int N, int MODE>
-cudaError_t set_tc_attr() {
-  return cudaFuncSetAttribute(k_conv_tc<C, N, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)tc_smem_bytes<C, N>());
+template <int IN>
+cudaError_t set_grad_attr() {
+  return cudaFuncSetAttribute(k_grad_rows<IN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rc_smem_bytes<IN>());
 }
 template <int KIND>
 cudaError_t set_wgrad_attr() {
@@ -1089,12 +1387,12 @@ cudaError_t ensure_attrs() {
   const unsigned long long bit = 1ull << (dev & 63);
   if (g_attr_done & bit) return cudaSuccess;
   cudaError_t r[] = {
-      set_tc_attr<CNN_IN_STRIDE, 16, CONV_RELU_BF16>(),
-      set_tc_attr<CNN_HID, 16, CONV_RELU_BF16>(),
-      set_tc_attr<CNN_HID, 16, CONV_F32>(),
-      set_tc_attr<CNN_HID, 16, CONV_CONF>(),
-      set_conv_attr<1, CNN_HID, 1, float, true, CONV_MASK_F32>(),
-      set_conv_attr<CNN_HID, CNN_HID, CNN_HID, float, true, CONV_MASK_F32>(),
+      set_conv_attr<8, 16, CONV_RELU_BF16>(),
+      set_conv_attr<16, 16, CONV_RELU_BF16>(),
+      set_conv_attr<16, 1, CONV_F32>(),
+      set_conv_attr<16, 1, CONV_CONF>(),
+      set_grad_attr<RC_F32_1>(),
+      set_grad_attr<RC_F32_16>(),
       set_wgrad_attr<WG_L1>(),
       set_wgrad_attr<WG_L2>(),
       set_wgrad_attr<WG_L3>(),
@@ -1123,12 +1421,10 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// A tile over n images of W x H pixels, C = 8 or 16 BF16 channels per pixel: a
-// rows x cols box of one 8-channel plane (k_conv_tc: (TC_ROWS + 4) x TC_COLS;
-// k_wgrad_tc: one row of WG_XPX), zero outside the image (dimensions: 8
-// channels, [plane], x, y, image).
-cudaError_t tile_map(CUtensorMap *m, const void *base, int C, int W, int H, int n, int cols = TC_COLS,
-                     int rows = TC_TILE_ROWS) {
+// The copies of k_wgrad_tc over n images of W x H pixels, C = 8 or 16 BF16
+// channels per pixel: WG_XPX pixels of a row of one 8-channel plane, zero
+// outside the image (dimensions: 8 channels, [plane], x, y, image).
+cudaError_t tile_map(CUtensorMap *m, const void *base, int C, int W, int H, int n) {
   const EncodeTiledFn f = encode_tiled();
   if (!f) return cudaErrorNotSupported;
   cuuint64_t dims[5], strides[4];
@@ -1138,14 +1434,14 @@ cudaError_t tile_map(CUtensorMap *m, const void *base, int C, int W, int H, int 
     rank = 5;
     const cuuint64_t d[5] = {8, 2, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)n};
     const cuuint64_t st[4] = {16, 32, (cuuint64_t)W * 32, (cuuint64_t)W * H * 32};
-    const cuuint32_t b[5] = {8, 1, (cuuint32_t)cols, (cuuint32_t)rows, 1};
+    const cuuint32_t b[5] = {8, 1, WG_XPX, 1, 1};
     for (int i = 0; i < 5; i++) dims[i] = d[i], box[i] = b[i];
     for (int i = 0; i < 4; i++) strides[i] = st[i];
   } else {
     rank = 4;
     const cuuint64_t d[4] = {8, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)n};
     const cuuint64_t st[3] = {16, (cuuint64_t)W * 16, (cuuint64_t)W * H * 16};
-    const cuuint32_t b[4] = {8, (cuuint32_t)cols, (cuuint32_t)rows, 1};
+    const cuuint32_t b[4] = {8, WG_XPX, 1, 1};
     for (int i = 0; i < 4; i++) dims[i] = d[i], box[i] = b[i];
     for (int i = 0; i < 3; i++) strides[i] = st[i];
   }
@@ -1155,22 +1451,28 @@ cudaError_t tile_map(CUtensorMap *m, const void *base, int C, int W, int H, int 
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-dim3 conv_grid(int W, int H, int n) {
-  return dim3((W + TX - 1) / TX, (H + conv_ty(CONV_RPT) - 1) / conv_ty(CONV_RPT), n);
+template <int C, int NB, int MODE>
+void conv(const __nv_bfloat16 *in, int n, int W, int H, const __nv_bfloat16 *w, const __nv_bfloat16 *b, void *out,
+          float inv_tau, uint32_t *err, cudaStream_t s) {
+  const int64_t quads = (int64_t)((W + CQ_OUT - 1) / CQ_OUT) * n * ((H + 3) / 4);
+  note_launch();
+  k_conv_quads<C, NB, MODE><<<(int)std::min<int64_t>(148, quads), CQ_THREADS, cq_smem_bytes<C, NB>(), s>>>(
+      in, W, H, n, w, b, out, inv_tau, err);
 }
 
-template <int KIN, int KOUT, int CSTR, typename TIN, bool TRANS, int MODE>
-void conv(const TIN *in, int n, int W, int H, const __nv_bfloat16 *w, const __nv_bfloat16 *b, void *out,
-          const __nv_bfloat16 *act, float inv_tau, cudaStream_t s) {
+template <int IN>
+void input_grad(const float *g, int n, int W, int H, const __nv_bfloat16 *w, float *out, const __nv_bfloat16 *act,
+                cudaStream_t s) {
+  const int64_t pairs = (int64_t)((W + RC_OUT - 1) / RC_OUT) * n * ((H + 1) / 2);
+  const int grid = (int)std::min<int64_t>(148, (pairs + RC_MIN_PAIRS - 1) / RC_MIN_PAIRS);
   note_launch();
-  k_conv<KIN, KOUT, CSTR, TIN, TRANS, MODE>
-      <<<conv_grid(W, H, n), 256, conv_smem_bytes<KIN, KOUT>(), s>>>(in, W, H, w, b, out, act, inv_tau);
+  k_grad_rows<IN><<<grid, RC_THREADS, rc_smem_bytes<IN>(), s>>>(g, W, H, n, w, out, act);
 }
 
 template <int KIND>
 cudaError_t wgrad(const __nv_bfloat16 *x, const float *dy, int n, int W, int H, float *dw, float *db, cudaStream_t s) {
   CUtensorMap m;
-  const cudaError_t e = tile_map(&m, x, KIND == WG_L1 ? CNN_IN_STRIDE : CNN_HID, W, H, n, WG_XPX, 1);
+  const cudaError_t e = tile_map(&m, x, KIND == WG_L1 ? CNN_IN_STRIDE : CNN_HID, W, H, n);
   if (e != cudaSuccess) return e;
   const int tiles = ((W + WG_W - 1) / WG_W) * ((H + WG_R - 1) / WG_R) * n;
   note_launch();
@@ -1186,32 +1488,17 @@ cudaError_t cnn_features(const uint16_t *depth, int n, int W, int H, float scali
   return cudaGetLastError();
 }
 
-cudaError_t cnn_forward(const __nv_bfloat16 *params, uint8_t *packed, bool packed_ready, const __nv_bfloat16 *feat,
-                        int n, int W, int H, __nv_bfloat16 *a1, __nv_bfloat16 *a2, float *out, float tau_cm,
-                        uint32_t *err, cudaStream_t s) {
+cudaError_t cnn_forward(const __nv_bfloat16 *params, const __nv_bfloat16 *feat, int n, int W, int H,
+                        __nv_bfloat16 *a1, __nv_bfloat16 *a2, float *out, float tau_cm, uint32_t *err,
+                        cudaStream_t s) {
   cudaError_t e = ensure_attrs();
   if (e != cudaSuccess) return e;
-  if (!packed_ready) {
-    note_launch();
-    k_pack_tc<<<(TC_PACK_BYTES / 2 + 255) / 256, 256, 0, s>>>(params, reinterpret_cast<__nv_bfloat16 *>(packed));
-  }
-  CUtensorMap m_feat, m_a1, m_a2;
-  if ((e = tile_map(&m_feat, feat, CNN_IN_STRIDE, W, H, n)) != cudaSuccess ||
-      (e = tile_map(&m_a1, a1, CNN_HID, W, H, n)) != cudaSuccess ||
-      (e = tile_map(&m_a2, a2, CNN_HID, W, H, n)) != cudaSuccess)
-    return e;
-  const dim3 tg((W + 127) / 128, (H + TC_ROWS - 1) / TC_ROWS, n);
-  note_launch(3);
-  k_conv_tc<CNN_IN_STRIDE, 16, CONV_RELU_BF16><<<tg, 128, tc_smem_bytes<CNN_IN_STRIDE, 16>(), s>>>(
-      m_feat, W, H, packed + TC_PACK_L1, params + P_B1, a1, 0.0f, err);
-  k_conv_tc<CNN_HID, 16, CONV_RELU_BF16><<<tg, 128, tc_smem_bytes<CNN_HID, 16>(), s>>>(
-      m_a1, W, H, packed + TC_PACK_L2, params + P_B2, a2, 0.0f, err);
+  conv<8, 16, CONV_RELU_BF16>(feat, n, W, H, params + P_W1, params + P_B1, a1, 0.0f, err, s);
+  conv<16, 16, CONV_RELU_BF16>(a1, n, W, H, params + P_W2, params + P_B2, a2, 0.0f, err, s);
   if (tau_cm > 0.0f)
-    k_conv_tc<CNN_HID, 16, CONV_CONF><<<tg, 128, tc_smem_bytes<CNN_HID, 16>(), s>>>(
-        m_a2, W, H, packed + TC_PACK_L3, params + P_B3, out, 1.0f / tau_cm, err);
+    conv<16, 1, CONV_CONF>(a2, n, W, H, params + P_W3, params + P_B3, out, 1.0f / tau_cm, err, s);
   else
-    k_conv_tc<CNN_HID, 16, CONV_F32><<<tg, 128, tc_smem_bytes<CNN_HID, 16>(), s>>>(
-        m_a2, W, H, packed + TC_PACK_L3, params + P_B3, out, 0.0f, err);
+    conv<16, 1, CONV_F32>(a2, n, W, H, params + P_W3, params + P_B3, out, 0.0f, err, s);
   return cudaGetLastError();
 }
 
@@ -1222,10 +1509,10 @@ cudaError_t cnn_backward(const __nv_bfloat16 *params, const __nv_bfloat16 *feat,
   if (e != cudaSuccess) return e;
   // layer 3
   if ((e = wgrad<WG_L3>(a2, dpred, n, W, H, grads + P_W3, grads + P_B3, s)) != cudaSuccess) return e;
-  conv<1, CNN_HID, 1, float, true, CONV_MASK_F32>(dpred, n, W, H, params + P_W3, nullptr, g2, a2, 0.0f, s);
+  input_grad<RC_F32_1>(dpred, n, W, H, params + P_W3, g2, a2, s);
   // layer 2
   if ((e = wgrad<WG_L2>(a1, g2, n, W, H, grads + P_W2, grads + P_B2, s)) != cudaSuccess) return e;
-  conv<CNN_HID, CNN_HID, CNN_HID, float, true, CONV_MASK_F32>(g2, n, W, H, params + P_W2, nullptr, g1, a1, 0.0f, s);
+  input_grad<RC_F32_16>(g2, n, W, H, params + P_W2, g1, a1, s);
   // layer 1 (no gradient of the input)
   if ((e = wgrad<WG_L1>(feat, g1, n, W, H, grads + P_W1, grads + P_B1, s)) != cudaSuccess) return e;
   return cudaGetLastError();

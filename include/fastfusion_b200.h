@@ -465,8 +465,8 @@ ff_status ff_raycast_depth(ff_handle *h, const double K[4], const double R[9], c
  * width x height; feat bf16 [n][h][w][8]; a1, a2 bf16 [n][h][w][16]; pred /
  * dpred / target float [n][h][w]; g1, g2 float [n][h][w][16] (scratch);
  * params bf16 and grads / master / m / v float [FF_CNN_PARAMS]; packed:
- * FF_CNN_PACKED_BYTES of scratch that ff_cnn_forward fills with the weights
- * laid out as tensor-core operands (one per concurrent call).
+ * FF_CNN_PACKED_BYTES of scratch (not NULL; the kernels lay the weights out
+ * themselves and leave it as it is).
  * ff_cnn_forward writes the confidence when tau_m > 0, else the prediction.
  * ff_cnn_backward adds the parameter gradients of d(loss)/d(pred) to grads.
  * ff_cnn_mse: loss += sum over target >= 0 of (pred - target)^2 * inv_count,
