@@ -82,8 +82,8 @@ STAGE_KERNELS = {
     "finalize": "k_finalize_bitmap",
     "fuse": "k_fuse",
     "mesh_cells": "k_keep_cells+k_gen_levels+k_cell_keys+argsort (k_sort_small or k_rs_*)+k_merge_cells/k_gather_cells",
-    "mesh_count": "k_mesh_lattice<count>+k_mesh_corner<count>",
-    "mesh_emit": "k_mesh_lattice<emit>+k_mesh_corner<emit>+k_copy_clean",
+    "mesh_count": "k_mesh_count",
+    "mesh_emit": "k_mesh_emit",
     "confidence": "k_cnn_features+k_conv x3 (learned weight)",
 }
 

@@ -15,12 +15,12 @@
 //
 // Meshing.  A warp per interior/wall/edge cell gathers the cell's lattice of
 // samples (falling back along the parent-leaf chain where the weight is zero),
-// classifies the cubes, flags the lattice edges that carry a vertex, then
-// emits vertices and faces with warp prefix sums in the reference's per-type
-// loop orders (mesh_interleaved_meshcell.cpp:9-2478); a thread per corner
-// cell runs the reference's non-indexed single-cube path (:2480-2687).  A
-// count pass, an exclusive scan over cells and an emit pass write the
-// interleaved mesh without atomics, so it is identical run to run.
+// keeps their signs and validity as rows of bits, finds the lattice edges that
+// carry a vertex from those, then emits vertices and faces with warp prefix sums
+// in the reference's per-type loop orders (mesh_interleaved_meshcell.cpp:9-2478);
+// eight lanes per corner cell run the reference's non-indexed single-cube path
+// (:2480-2687).  A count pass, an exclusive scan over cells and an emit pass
+// write the interleaved mesh without atomics, so it is identical run to run.
 // Incremental: a cell whose leaves (and their parent chains) were not updated
 // since the previous mesh, and whose leaves did not change, copies its old
 // vertices and faces instead of being re-meshed.
@@ -54,28 +54,32 @@ __constant__ uint8_t c_edge_slot[12][4] = {{0, 0, 0, 0}, {1, 0, 0, 1}, {0, 1, 0,
 __constant__ uint8_t c_edge_a[12] = {0, 1, 2, 3, 4, 5, 6, 7, 0, 1, 2, 3};
 __constant__ uint8_t c_edge_b[12] = {1, 2, 3, 0, 5, 6, 7, 4, 4, 5, 6, 7};
 
+// loop nesting of the reference's vertex/face loops per cell type, outer to inner axis
+__constant__ uint8_t c_order[7][3] = {{2, 1, 0}, {2, 1, 0}, {2, 0, 1}, {1, 0, 2}, {0, 2, 1}, {1, 2, 0}, {2, 1, 0}};
+
 // The tables as the meshing kernels read them: from shared memory, since
 // the lanes of a warp index them by different cube cases.
 struct McTab {
   unsigned long long tri[256];
-  uint32_t slot[12];  // c_edge_slot packed: dx | dy << 8 | dz << 16 | axis << 24
+  // per cell type and cube edge: the lattice edge it lies on, 3 times the
+  // lattice position relative to the cube's (in the type's nesting: outer
+  // axis 64, middle 8, inner 1) plus the axis
+  uint16_t edge[7][12];
 };
 
 // Copy the tables into the block's shared memory (all threads of the block).
 __device__ __forceinline__ void load_mc(McTab &T) {
   for (int i = threadIdx.x; i < 256; i += blockDim.x) T.tri[i] = c_mc_tri[i];
-  for (int i = threadIdx.x; i < 12; i += blockDim.x)
-    T.slot[i] = (uint32_t)c_edge_slot[i][0] | ((uint32_t)c_edge_slot[i][1] << 8) |
-                ((uint32_t)c_edge_slot[i][2] << 16) | ((uint32_t)c_edge_slot[i][3] << 24);
+  for (int i = threadIdx.x; i < 7 * 12; i += blockDim.x) {
+    const int t = i / 12, e = i % 12;
+    T.edge[t][e] = (uint16_t)(3 * (64 * c_edge_slot[e][c_order[t][0]] + 8 * c_edge_slot[e][c_order[t][1]] +
+                                   c_edge_slot[e][c_order[t][2]]) +
+                              c_edge_slot[e][3]);
+  }
   __syncthreads();
 }
 __device__ __forceinline__ int mc_ntri(const McTab &T, int c) { return (int)(T.tri[c] >> 60); }
 __device__ __forceinline__ int mc_edge(const McTab &T, int c, int k) { return (int)((T.tri[c] >> (4 * k)) & 15ull); }
-// flat lattice-edge slot (3 * voxel index + axis) of a cube edge, relative to the cube's voxel index
-__device__ __forceinline__ int mc_slot(const McTab &T, int e) {
-  const uint32_t v = T.slot[e];
-  return 3 * ((int)(v & 255u) + 8 * (int)((v >> 8) & 255u) + 64 * (int)((v >> 16) & 255u)) + (int)(v >> 24);
-}
 
 // ---------------------------------------------------------------------------
 // Cell generation
@@ -1100,17 +1104,65 @@ struct Sample {
 // axis roles per type: 0 = lattice of spacing sizeMin, 1 = the two samples
 // either side of the shared boundary
 __constant__ uint8_t c_role[7][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {0, 0, 1}, {0, 1, 1}, {1, 0, 1}, {1, 1, 0}};
-// loop nesting of the reference's vertex/face loops, outer to inner axis
-__constant__ uint8_t c_order[7][3] = {{2, 1, 0}, {2, 1, 0}, {2, 0, 1}, {1, 0, 2}, {0, 2, 1}, {1, 2, 0}, {2, 1, 0}};
-
 struct CellGeom {
   int type, size, sizeMin, stretch;
-  int cnt[3];
+  int cnt[3];            // samples per axis
   int o[3];
+  int base[3], step[3];  // sample b of an axis lies at base + b step
   bool empty;
 };
 
-__device__ CellGeom cell_geom(const VoxSrc &m, const Cell &c) {
+// The parent chains of a lattice cell's sides (at most four): leaf and position
+// of each step, loaded once per cell into shared memory.  Most samples settle at
+// their side's first leaf, the others walk on along the same few leaves, so
+// the walk itself (a leaf's position and parent, dependent loads) is made once
+// instead of once per sample.
+constexpr int CHAIN_MAX = 6;  // steps kept (a longer chain is walked on from the last)
+struct Chain {
+  uint32_t leaf[4][CHAIN_MAX];
+  ushort4 pos[4][CHAIN_MAX];
+  uint32_t n[4];     // steps kept
+  uint32_t rest[4];  // the leaf after them (BRANCHINIT: none)
+};
+__device__ __forceinline__ int cell_sides(int type) { return type == 0 ? 1 : (type <= 3 ? 2 : 4); }
+
+// One thread per side of the cell (the first step's position is that of the
+// cell's leaf, whether or not the walk enters it).
+__device__ __forceinline__ void load_chain(const VoxSrc &m, const Cell &c, int side, Chain &ch) {
+  uint32_t leaf = c.L[0];
+#pragma unroll
+  for (int k = 1; k < 4; k++)
+    if (k == side) leaf = c.L[k];
+  int n = 0;
+  ch.pos[side][0] = m.leaf[leaf];
+  while (n < CHAIN_MAX && leaf < BRANCHINIT && leaf < m.leaves_used) {
+    const ushort4 p = m.leaf[leaf];
+    const uint32_t up = m.parent[leaf];
+    ch.leaf[side][n] = leaf;
+    ch.pos[side][n] = p;
+    n++;
+    leaf = up;
+  }
+  ch.n[side] = (uint32_t)n;
+  ch.rest[side] = n == CHAIN_MAX && leaf < m.leaves_used ? leaf : BRANCHINIT;  // (a shorter chain has ended)
+}
+
+// Step l of a side's chain; false when it has ended.
+__device__ __forceinline__ bool chain_step(const VoxSrc &m, const Chain &ch, int side, int l, uint32_t &leaf,
+                                           ushort4 &pos) {
+  if (l < (int)ch.n[side]) {
+    leaf = ch.leaf[side][l];
+    pos = ch.pos[side][l];
+    return true;
+  }
+  leaf = ch.rest[side];
+  for (int k = CHAIN_MAX; k < l && leaf < BRANCHINIT && leaf < m.leaves_used; k++) leaf = m.parent[leaf];
+  if (leaf >= BRANCHINIT || leaf >= m.leaves_used) return false;
+  pos = m.leaf[leaf];
+  return true;
+}
+
+__device__ __forceinline__ CellGeom cell_geom(const Cell &c, const Chain &ch) {
   CellGeom G;
   G.type = c.type;
   G.size = c.size;
@@ -1118,70 +1170,65 @@ __device__ CellGeom cell_geom(const VoxSrc &m, const Cell &c) {
   G.empty = false;
   for (int r = 0; r < 3; r++) G.o[r] = c.o[r];
   const int t = c.type;
+  const ushort4 lo = ch.pos[0][0];
   if (t == 0) {
-    G.sizeMin = m.leaf[c.L[0]].w;
+    G.sizeMin = lo.w;
     if (G.sizeMin > G.size || G.size / G.sizeMin > 8) G.empty = true;
-    const ushort4 lo = m.leaf[c.L[0]];
     const int ext = lo.w * 8;
     if (G.o[0] + G.size > lo.x + ext || G.o[0] < lo.x || G.o[1] + G.size > lo.y + ext || G.o[1] < lo.y ||
         G.o[2] + G.size > lo.z + ext || G.o[2] < lo.z)
       G.empty = true;
   } else if (t <= 3) {
-    const int a = m.leaf[c.L[0]].w, b = m.leaf[c.L[1]].w;
+    const int a = lo.w, b = ch.pos[1][0].w;
     G.sizeMin = min(a, b);
     G.stretch = a;
     if (G.stretch > G.size) G.empty = true;
   } else {
-    const int s0 = m.leaf[c.L[0]].w, s1 = m.leaf[c.L[1]].w, s2 = m.leaf[c.L[2]].w, s3 = m.leaf[c.L[3]].w;
+    const int s0 = lo.w, s1 = ch.pos[1][0].w, s2 = ch.pos[2][0].w, s3 = ch.pos[3][0].w;
     G.stretch = max(max(s0, s1), s2);
     G.sizeMin = min(min(s0, s1), min(s2, s3));
     if (G.stretch > G.size) G.empty = true;
   }
   if (G.sizeMin <= 0) G.empty = true;
-  for (int r = 0; r < 3; r++) G.cnt[r] = c_role[t][r] ? 2 : (G.empty ? 1 : (G.size + G.sizeMin - 1) / G.sizeMin);
-  for (int r = 0; r < 3; r++)
+#pragma unroll
+  for (int r = 0; r < 3; r++) {
+    const bool role = c_role[t][r] != 0;
+    G.cnt[r] = role ? 2 : (G.empty ? 1 : (G.size + G.sizeMin - 1) / G.sizeMin);
+    G.base[r] = role ? G.o[r] + G.size - G.stretch : G.o[r];
+    G.step[r] = role ? G.stretch : G.sizeMin;
     if (G.cnt[r] > 8) G.empty = true;  // a lattice never exceeds one brick
+  }
   return G;
 }
 
 __device__ __forceinline__ int sample_pos(const CellGeom &G, int r, int b) {
-  return c_role[G.type][r] ? (b ? G.o[r] + G.size : G.o[r] + G.size - G.stretch) : G.o[r] + b * G.sizeMin;
+  return (r == 0 ? G.base[0] : (r == 1 ? G.base[1] : G.base[2])) +
+         b * (r == 0 ? G.step[0] : (r == 1 ? G.step[1] : G.step[2]));
 }
 
-// One lattice sample of an interior/wall/edge cell; returns false when the
-// interior cell does not fit in a leaf of its chain (the reference then
-// leaves the cell's mesh empty).
+// The side of a cell that lattice sample (bx, by, bz) lies on.
+__device__ __forceinline__ int sample_side(int t, int bx, int by, int bz) {
+  if (t == 0) return 0;
+  if (t <= 3) return t == 1 ? bx : (t == 2 ? by : bz);
+  return t == 4 ? by + 2 * bz : (t == 5 ? bx + 2 * bz : bx + 2 * by);
+}
+
+// Whether an interior cell lies inside the leaf at lo.
+__device__ __forceinline__ bool cell_inside(const CellGeom &G, const ushort4 &lo) {
+  const int ext = lo.w * 8;
+  return !(G.o[0] + G.size > lo.x + ext || G.o[0] < lo.x || G.o[1] + G.size > lo.y + ext || G.o[1] < lo.y ||
+           G.o[2] + G.size > lo.z + ext || G.o[2] < lo.z);
+}
+
+// One step of a sample's walk: what leaf (at lo4) adds to it.
 template <bool COLOR>
-__device__ bool lattice_sample(const VoxSrc &m, const Cell &c, const CellGeom &G, int bx, int by, int bz, Sample &s) {
+__device__ __forceinline__ void sample_step(const VoxSrc &m, const CellGeom &G, uint32_t leaf, const ushort4 &lo4,
+                                            int bx, int by, int bz, Sample &s) {
   const int t = G.type;
   const int bb[3] = {bx, by, bz};
-  uint32_t first;
-  if (t == 0)
-    first = c.L[0];
-  else if (t <= 3)
-    first = c.L[bb[t - 1]];
-  else {
-    int p, q;
-    others(t - 4, p, q);
-    first = c.L[bb[p] + 2 * bb[q]];
-  }
-  s.w = 0.0f;
-  s.d = 0.0f;
-  s.c[0] = s.c[1] = s.c[2] = 0;
-  int guard = 0;
-  // (the parent is read only when the walk goes on: most samples settle at
-  // their first leaf)
-  for (uint32_t leaf = first; leaf < BRANCHINIT && s.w <= 0.0f && guard < 64;
-       leaf = s.w <= 0.0f ? m.parent[leaf] : BRANCHINIT, guard++) {
-    if (leaf >= m.leaves_used) break;
-    const ushort4 lo4 = m.leaf[leaf];
+  {
     const int lo[3] = {lo4.x, lo4.y, lo4.z};
     const int ls = lo4.w;
-    if (t == 0) {
-      const int ext = ls * 8;
-      for (int r = 0; r < 3; r++)
-        if (G.o[r] + G.size > lo[r] + ext || G.o[r] < lo[r]) return false;
-    }
     uint16_t ll[3], lh[3];
     float rr[3];
     // leaf scales are powers of two: divide by shifting (same truncating
@@ -1222,7 +1269,7 @@ __device__ bool lattice_sample(const VoxSrc &m, const Cell &c, const CellGeom &G
         s.d = d0;
 #pragma unroll
         for (int r = 0; r < 3; r++) s.c[r] = vcs<COLOR>(m, v0, r);
-        continue;
+        return;
       }
     }
     if (t == 0) {
@@ -1282,7 +1329,7 @@ __device__ bool lattice_sample(const VoxSrc &m, const Cell &c, const CellGeom &G
           s.d = d0;
 #pragma unroll
           for (int r = 0; r < 3; r++) s.c[r] = vcs<COLOR>(m, v0, r);
-          continue;
+          return;
         }
       }
       const float f[4] = {__fmul_rn(rbn, ran), __fmul_rn(rbn, ra), __fmul_rn(rb, ran), __fmul_rn(rb, ra)};
@@ -1343,49 +1390,153 @@ __device__ bool lattice_sample(const VoxSrc &m, const Cell &c, const CellGeom &G
       }
     }
   }
+}
+
+// One lattice sample of an interior/wall/edge cell; returns false when the
+// interior cell does not fit in a leaf of its chain (the reference then
+// leaves the cell's mesh empty).
+template <bool COLOR>
+__device__ __forceinline__ bool lattice_sample(const VoxSrc &m, const Chain &ch, const CellGeom &G, int bx, int by,
+                                               int bz, Sample &s) {
+  const int side = sample_side(G.type, bx, by, bz);
+  s.w = 0.0f;
+  s.d = 0.0f;
+  s.c[0] = s.c[1] = s.c[2] = 0;
+  uint32_t leaf;
+  ushort4 lo;
+  for (int l = 0; l < 64 && s.w <= 0.0f && chain_step(m, ch, side, l, leaf, lo); l++) {
+    if (G.type == 0 && !cell_inside(G, lo)) return false;
+    sample_step<COLOR>(m, G, leaf, lo, bx, by, bz, s);
+  }
   return true;
 }
 
-// An interior cell that is its leaf's whole brick: sample k (< 512) is
-// voxel k of the brick (lattice_sample's first step reads that one voxel).
-__device__ __forceinline__ bool brick_cell(const VoxSrc &m, const Cell &c, const CellGeom &G, uint32_t &leaf) {
-  if (G.type != 0) return false;
-  const uint32_t l0 = c.L[0];
-  if (l0 >= BRANCHINIT || l0 >= m.leaves_used) return false;
-  const ushort4 a = m.leaf[l0];
-  const int ls = a.w;
-  if (ls <= 0 || (ls & (ls - 1)) != 0 || G.sizeMin != ls || G.size != 8 * ls) return false;
-  if (G.o[0] != a.x || G.o[1] != a.y || G.o[2] != a.z) return false;
-  leaf = l0;
-  return true;
-}
-
-// Per-warp shared scratch of one lattice cell.  Only the zero test of a
-// sample's weight is needed after sampling; colours and vertex numbers are
-// used by the emit pass alone, so the count pass's scratch stops before them
-// (more warps per SM).
-// Edge flags are bytes: plain stores, where bits would need atomics.
-struct WarpScratch {
-  float sd[512];           // SDF of each lattice sample
-  uint8_t wzero[512];      // the sample's weight is zero
-  uint8_t cube_case[512];  // marching-cubes case of each cube
-  uint8_t edge_set[512 * 3];  // lattice-edge slots (3 per voxel) that carry a vertex
-  uint16_t sc[512 * 3];    // emit pass: colour (R, G, B) of each sample
-  uint16_t vidx[512 * 3];  // emit pass: the vertex number of each such slot
-  uint16_t vlist[512 * 3];  // emit pass: the vertex-carrying slots in vertex order
+// A lattice cell in its type's loop nesting: rows along the inner axis, row
+// 8 iA + iB for the outer and middle positions (iA, iB), sample 8 row + iF.
+// Everything but the samples' values is bit arithmetic on the rows: bit iF of
+// byte `row` is the sign of sample iF, a cube's validity, a lattice edge's vertex.
+//
+// What bounds the passes: instruction issue.  Sampling each lattice position
+// through the general step and looking every cube up from its eight samples took
+// about 10,000 instructions per warp for an interior cell, 45 and 43 us for the
+// count and emit passes at 5,000 dirty cells of 6,300 (two cells per warp: a
+// single wave).  With the rows a cube's tests are a few operations for eight
+// cubes, the cases of the mixed cubes alone are looked up, and a sample on its
+// leaf's lattice is three table reads and its voxel.  With the corner cells and
+// the clean cells' copies inside the emit pass (they were two more launches, the
+// copies the longest of the three) a 640x480 frame's mesh stage after the cell
+// generation went from 161 to 126 us (count 72 and 75 with its scan and the
+// host's wait, emit 90 and 52), ten frames' from 169 to 135 us.
+struct Nest {
+  int A, B, F;     // axes, outer to inner
+  int nA, nB, nF;  // samples
+  uint32_t corner; // nibble q: bit of cube corner q among (4 dA + 2 dB + dF)
 };
-constexpr size_t SCRATCH_COUNT_BYTES = offsetof(WarpScratch, sc);
-constexpr size_t SCRATCH_EMIT_BYTES = sizeof(WarpScratch);
+__device__ __forceinline__ Nest nest_of(const CellGeom &G) {
+  Nest N;
+  const uint8_t *ord = c_order[G.type];
+  N.A = ord[0], N.B = ord[1], N.F = ord[2];
+  auto cnt = [&](int r) { return r == 0 ? G.cnt[0] : (r == 1 ? G.cnt[1] : G.cnt[2]); };
+  N.nA = cnt(N.A), N.nB = cnt(N.B), N.nF = cnt(N.F);
+  constexpr int xyz[8] = {0, 1, 3, 2, 4, 5, 7, 6};  // corner q's offsets, x in bit 0
+  N.corner = 0;
+#pragma unroll
+  for (int q = 0; q < 8; q++)
+    N.corner |= (uint32_t)((((xyz[q] >> N.A) & 1) << 2) | (((xyz[q] >> N.B) & 1) << 1) | ((xyz[q] >> N.F) & 1)) << (4 * q);
+  return N;
+}
+// sample 8 row + f as (x, y, z)
+__device__ __forceinline__ void nest_xyz(const Nest &N, int p, int &x, int &y, int &z) {
+  const int a = p >> 6, b = (p >> 3) & 7, f = p & 7;
+  x = N.A == 0 ? a : (N.B == 0 ? b : f);
+  y = N.A == 1 ? a : (N.B == 1 ? b : f);
+  z = N.A == 2 ? a : (N.B == 2 ? b : f);
+}
+// The marching-cubes case of the cube at bit f of four neighbouring rows.
+__device__ __forceinline__ int cube_case(const Nest &N, uint32_t s00, uint32_t s01, uint32_t s10, uint32_t s11, int f) {
+  const uint32_t pb = ((s00 >> f) & 3u) | (((s01 >> f) & 3u) << 2) | (((s10 >> f) & 3u) << 4) | (((s11 >> f) & 3u) << 6);
+  int c = 0;
+#pragma unroll
+  for (int q = 0; q < 8; q++) c |= (int)((pb >> ((N.corner >> (4 * q)) & 15u)) & 1u) << q;
+  return c;
+}
+
+// The voxel a sample lies on at its side's first leaf: per side and nest
+// direction (inner, middle, outer), the position's share of the voxel index, or
+// VOX_OFF where the sample does not lie on that leaf's lattice (power-of-two
+// scales) or inside its brick: such a sample takes the general walk.
+constexpr uint32_t VOX_OFF = 0x8000u;
+struct VoxTab {
+  uint16_t e[4][3][8];
+};
+__device__ __forceinline__ void load_vox_tab(const CellGeom &G, const Nest &N, const Chain &ch, VoxTab &tab, int lane) {
+  const int sides = cell_sides(G.type);
+  for (int i = lane; i < 24 * sides; i += 32) {
+    const int side = i / 24, dir = (i >> 3) % 3, b = i & 7;
+    const int r = dir == 0 ? N.F : (dir == 1 ? N.B : N.A);
+    const ushort4 lo = ch.pos[side][0];
+    const int num = sample_pos(G, r, b) - (r == 0 ? (int)lo.x : (r == 1 ? (int)lo.y : (int)lo.z)), ls = lo.w;
+    uint32_t e = VOX_OFF;
+    if (ch.n[side] && ls > 0 && (ls & (ls - 1)) == 0 && num >= 0) {
+      const int q = num >> (__ffs(ls) - 1);
+      if (q < 8 && (c_role[G.type][r] || (num & (ls - 1)) == 0)) e = (uint32_t)q << (3 * r);
+    }
+    tab.e[side][dir][b] = (uint16_t)e;
+  }
+}
+// The side of sample (a, b, f): the two samples across a wall lie along the inner
+// axis, the four around an edge along the inner (bit 0) and the middle one.
+__device__ __forceinline__ int nest_side(int type, int b, int f) { return type == 0 ? 0 : (type <= 3 ? f : f + 2 * b); }
+__device__ __forceinline__ uint32_t vox_of(const VoxTab &tab, int side, int a, int b, int f) {
+  return (uint32_t)tab.e[side][2][a] | tab.e[side][1][b] | tab.e[side][0][f];  // (the shares' bits are disjoint)
+}
+// What a sample's voxel at its side's first leaf decides: true when the walk ends
+// there, with weight or because the chain does (s.d and s.w are then d and w).
+__device__ __forceinline__ bool settles(int type, float d, float w, bool single) {
+  return isfinite(d) && (type < 1 || type > 3 || isfinite(w)) && (single || !(__fadd_rn(0.0f, w) <= 0.0f));
+}
+__device__ __forceinline__ bool single_step(const Chain &ch, int side) {
+  return ch.n[side] == 1 && ch.rest[side] == BRANCHINIT;
+}
+// An interior cell that is its leaf's whole brick: sample k is voxel k.
+__device__ __forceinline__ bool whole_brick(const CellGeom &G, const Chain &ch) {
+  const ushort4 lo = ch.pos[0][0];
+  return G.type == 0 && ch.n[0] && (lo.w & (lo.w - 1)) == 0 && G.sizeMin == lo.w && G.size == 8 * lo.w &&
+         G.o[0] == lo.x && G.o[1] == lo.y && G.o[2] == lo.z;
+}
+
+// Per-warp shared scratch of one lattice cell; the count pass's stops before
+// the members of the emit pass alone.
+struct LatScratch {
+  Chain chain;
+  VoxTab tab;
+  uint8_t S[80];       // rows: negative samples (padding: neighbours of the last row)
+  uint8_t Z[80];       // rows: samples without weight
+  uint8_t Vp[16 + 64];  // rows of valid cubes, after nine zero rows and more (neighbours of the first row)
+  uint16_t slow[512];  // samples that take the general walk; emit pass: the samples to read, then the cubes
+  // emit pass
+  uint8_t mF[80], mB[80], mA[80];  // rows: lattice edges along F, B, A with a vertex
+  uint8_t code[352];               // case of each listed cube
+  uint16_t face0[352];             // first face of each listed cube
+  float sd[512];                   // SDF of the samples read
+  uint16_t sc[512 * 3];            // their colours
+  uint16_t vlist[1536];            // the vertex-carrying lattice edges in vertex order
+  uint16_t vidx[1536];             // the vertex of each
+};
+constexpr size_t SCRATCH_COUNT_BYTES = offsetof(LatScratch, mF);
+constexpr size_t SCRATCH_EMIT_BYTES = sizeof(LatScratch);
 static_assert(SCRATCH_COUNT_BYTES % 16 == 0 && SCRATCH_EMIT_BYTES % 16 == 0, "scratch alignment");
+static_assert(offsetof(LatScratch, S) % 4 == 0 && offsetof(LatScratch, Z) % 4 == 0 && offsetof(LatScratch, Vp) % 4 == 0,
+              "word reads of the rows");
 
-__device__ __forceinline__ int edge_bit(const WarpScratch &W, int slot) { return W.edge_set[slot]; }
+constexpr int MESH_WARPS = 4, MESH_THREADS = 32 * MESH_WARPS;
 
-constexpr int MESH_WARPS = 4;
-
-// Output of the count pass / input of the emit pass, per cell.
+// Output of the count pass / input of the emit pass, per cell: its counts, and
+// per listed lattice cell its rows of signs and of valid cubes.
 struct CellOut {
   uint32_t nv, nf;
 };
+constexpr int CELL_ROWS = 128;  // bytes: 64 rows of signs, 64 of valid cubes
 
 // A position k < 512 of a lattice of extents n0 (fastest) x n1 x n2 split
 // into its three coordinates.  The quotients are products with ceil(2^16 / d)
@@ -1412,22 +1563,6 @@ __device__ __forceinline__ void split3(const Lat3 &L, int k, int &c0, int &c1, i
   c2 = (int)q01;
 }
 
-// lattice-order position k -> lattice index, for the cell type's loop nesting
-// (L: the extents in that nesting, fastest first)
-__device__ __forceinline__ int lattice_idx(const CellGeom &G, int k, const Lat3 &L, int &b0, int &b1, int &b2) {
-  const uint8_t *ord = c_order[G.type];
-  int i0, i1, i2;
-  split3(L, k, i2, i1, i0);
-  int bb[3];
-  bb[ord[0]] = i0;
-  bb[ord[1]] = i1;
-  bb[ord[2]] = i2;
-  b0 = bb[0];
-  b1 = bb[1];
-  b2 = bb[2];
-  return (bb[2] * 8 + bb[1]) * 8 + bb[0];
-}
-
 __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
   int x = v;
 #pragma unroll
@@ -1439,285 +1574,341 @@ __device__ __forceinline__ int warp_excl_scan(int v, int lane, int &total) {
   return x - v;
 }
 
-// emit = false: count vertices/faces of each cell into out[]; emit = true:
-// write them at vbase/fbase.
-// The next cell for this warp (work: a counter that starts at zero).
-__device__ __forceinline__ uint32_t next_cell(uint32_t *work, int lane) {
-  uint32_t v = 0;
-  if (lane == 0) v = atomicAdd(work, 1u);
-  return __shfl_sync(0xffffffffu, v, 0);
+// The dirty cells of an update by kind: lattice cells (interior, walls, edges) and
+// corner cells.  Their order does not matter (the two passes see the same lists).
+struct MeshLists {
+  const uint32_t *lattice, *corner;
+  const uint32_t *n_lattice, *n_corner;  // device counts
+};
+
+// The next item for this warp (work: a counter that starts at zero), asked for
+// before the current one is processed: lane 0 holds the answer.
+__device__ __forceinline__ uint32_t ask_item(uint32_t *work, int lane) { return lane == 0 ? atomicAdd(work, 1u) : 0u; }
+
+// Count pass, one lattice cell by a warp.
+__device__ __forceinline__ void count_cell(const VoxSrc &m, const Cell &c, uint32_t cid, uint8_t *cell_rows,
+                                           CellOut *out, LatScratch &W, const McTab &T, int lane) {
+  if (!owns_cell(m, c)) {  // another part meshes it
+    if (lane == 0) out[cid] = CellOut{0u, 0u};
+    return;
+  }
+  if (lane < cell_sides(c.type)) load_chain(m, c, lane, W.chain);
+  __syncwarp();
+  const CellGeom geo = cell_geom(c, W.chain);
+  if (geo.empty) {
+    if (lane == 0) out[cid] = CellOut{0u, 0u};
+    return;
+  }
+  const Nest N = nest_of(geo);
+  const int nsamp = N.nA * N.nB * N.nF;
+  const bool brick = whole_brick(geo, W.chain);
+  int nslow = 0;
+  if (brick) {
+    // the brick's voxels in order, 16 loads per lane in flight; a ballot is four
+    // rows, kept by lane j for the j-th 32 samples
+    const bool single = single_step(W.chain, 0);
+    const size_t v0 = (size_t)W.chain.leaf[0][0] * 512 + lane;
+    uint32_t sw = 0, zw = 0;
+#pragma unroll 1
+    for (int h = 0; h < 2; h++) {
+      float dv[8], wv[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) dv[j] = vd(m, v0 + 256 * h + 32 * j), wv[j] = vw(m, v0 + 256 * h + 32 * j);
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const bool ok = settles(0, dv[j], wv[j], single);
+        const unsigned neg = __ballot_sync(0xffffffffu, ok && dv[j] < 0.0f),
+                       zero = __ballot_sync(0xffffffffu, ok && __fadd_rn(0.0f, wv[j]) == 0.0f),
+                       slow = __ballot_sync(0xffffffffu, !ok);
+        if (lane == 8 * h + j) sw = neg, zw = zero;
+        if (slow) {
+          if (!ok) W.slow[nslow + __popc(slow & ((1u << lane) - 1u))] = (uint16_t)(256 * h + 32 * j + lane);
+          nslow += __popc(slow);
+        }
+      }
+    }
+    if (lane < 16) {
+      reinterpret_cast<uint32_t *>(W.S)[lane] = sw;
+      reinterpret_cast<uint32_t *>(W.Z)[lane] = zw;
+    }
+  } else {
+    load_vox_tab(geo, N, W.chain, W.tab, lane);
+    if (lane < 16) {
+      reinterpret_cast<uint32_t *>(W.S)[lane] = 0;
+      reinterpret_cast<uint32_t *>(W.Z)[lane] = 0;
+    }
+    __syncwarp();
+    // every sample's voxel, four per lane in flight
+    const Lat3 Ls = lat3(N.nF, N.nB);
+#pragma unroll 1
+    for (int k0 = 0; k0 < nsamp; k0 += 128) {
+      float dv[4], wv[4];
+      int p[4];
+      bool one[4];
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int k = k0 + 32 * j + lane;
+        p[j] = -1;
+        dv[j] = __int_as_float(0x7fc00000);
+        wv[j] = 0.0f;
+        one[j] = false;
+        if (k < nsamp) {
+          int a, b, f;
+          split3(Ls, k, f, b, a);
+          p[j] = (a * 8 + b) * 8 + f;
+          const int side = nest_side(geo.type, b, f);
+          const uint32_t v = vox_of(W.tab, side, a, b, f);
+          if (v < VOX_OFF) {
+            const size_t vi = (size_t)W.chain.leaf[side][0] * 512 + v;
+            dv[j] = vd(m, vi);
+            wv[j] = vw(m, vi);
+            one[j] = single_step(W.chain, side);
+          }
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        if (k0 + 32 * j >= nsamp) break;
+        const bool ok = p[j] < 0 || settles(geo.type, dv[j], wv[j], one[j]);
+        if (ok && p[j] >= 0) {
+          const uint32_t bit = 1u << (p[j] & 31);
+          if (dv[j] < 0.0f) atomicOr(reinterpret_cast<uint32_t *>(W.S) + (p[j] >> 5), bit);
+          if (__fadd_rn(0.0f, wv[j]) == 0.0f) atomicOr(reinterpret_cast<uint32_t *>(W.Z) + (p[j] >> 5), bit);
+        }
+        const unsigned slow = __ballot_sync(0xffffffffu, !ok);
+        if (slow) {
+          if (!ok) W.slow[nslow + __popc(slow & ((1u << lane) - 1u))] = (uint16_t)p[j];
+          nslow += __popc(slow);
+        }
+      }
+    }
+  }
+  __syncwarp();
+  // the samples that walk on
+  bool fit = true;
+  for (int k = lane; k < nslow; k += 32) {
+    const int p = W.slow[k];
+    int x, y, z;
+    nest_xyz(N, p, x, y, z);
+    Sample s;
+    fit &= lattice_sample<false>(m, W.chain, geo, x, y, z, s);  // (no colour: the count pass needs none)
+    const uint32_t bit = 1u << (p & 31);
+    if (s.d < 0.0f) atomicOr(reinterpret_cast<uint32_t *>(W.S) + (p >> 5), bit);
+    if (s.w == 0.0f) atomicOr(reinterpret_cast<uint32_t *>(W.Z) + (p >> 5), bit);
+  }
+  fit = __all_sync(0xffffffffu, fit);
+  if (m.samples && lane == 0) atomicAdd(m.samples, (unsigned long long)nsamp);
+  if (!fit) {
+    if (lane == 0) out[cid] = CellOut{0u, 0u};
+    return;
+  }
+  const uint32_t cubeF = ((1u << N.nF) - 1u) >> 1;
+  if (lane < 20) reinterpret_cast<uint32_t *>(W.Vp)[lane] = 0;
+  __syncwarp();
+  // cubes: valid where all eight samples have weight; the cases of the mixed ones
+  uint32_t tri = 0;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int r = lane + 32 * h;
+    if ((r >> 3) >= N.nA - 1 || (r & 7) >= N.nB - 1) continue;
+    const uint32_t s00 = W.S[r], s01 = W.S[r + 1], s10 = W.S[r + 8], s11 = W.S[r + 9];
+    const uint32_t zz = W.Z[r] | W.Z[r + 1] | W.Z[r + 8] | W.Z[r + 9];
+    const uint32_t valid = ~(zz | (zz >> 1)) & cubeF;
+    const uint32_t any = s00 | s01 | s10 | s11, all = s00 & s01 & s10 & s11;
+    W.Vp[16 + r] = (uint8_t)valid;
+    for (uint32_t u = valid & (any | (any >> 1)) & ~(all & (all >> 1)); u; u &= u - 1)
+      tri += (uint32_t)mc_ntri(T, cube_case(N, s00, s01, s10, s11, __ffs(u) - 1));
+  }
+  __syncwarp();
+  // a vertex on every lattice edge whose ends differ in sign and that belongs to
+  // a valid cube (every such edge of a cube carries one of its triangles' vertices)
+  uint32_t verts = 0;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int r = lane + 32 * h;
+    uint32_t mF, mB, mA;
+    const uint8_t *V = W.Vp + 16 + r;
+    const uint32_t s = W.S[r], vF = V[0] | V[-1] | V[-8] | V[-9], vB = V[0] | V[-8], vA = V[0] | V[-1];
+    mF = (s ^ (s >> 1)) & vF & cubeF;
+    mB = (s ^ W.S[r + 1]) & (vB | (vB << 1));
+    mA = (s ^ W.S[r + 8]) & (vA | (vA << 1));
+    verts += (uint32_t)(__popc(mF) + __popc(mB & 255u) + __popc(mA & 255u));
+  }
+  // kept for the emit pass
+  reinterpret_cast<uint32_t *>(cell_rows)[lane] =
+      lane < 16 ? reinterpret_cast<const uint32_t *>(W.S)[lane] : reinterpret_cast<const uint32_t *>(W.Vp + 16)[lane - 16];
+  verts = __reduce_add_sync(0xffffffffu, verts);
+  tri = __reduce_add_sync(0xffffffffu, tri);
+  if (lane == 0) out[cid] = CellOut{verts, tri};
 }
 
-// (register caps: the count pass's 4.6 KB of scratch per warp leaves room
-// for 8 blocks per SM at 64 registers; the emit pass's 13.5 KB for 4)
-template <bool EMIT>
-__global__ void __launch_bounds__(32 * MESH_WARPS, EMIT ? 4 : 8) k_mesh_lattice(VoxSrc m, const Cell *__restrict__ cells,
-                                                                  uint32_t first, uint32_t ncell,
-                                                                  const uint32_t *__restrict__ list, const uint32_t *list_n, CellOut *out,
-                                                                  const uint64_t *vbase, const uint64_t *fbase,
-                                                                  float *xyz, uint8_t *rgb, uint32_t *faces,
-                                                                  uint32_t *work, uint8_t *__restrict__ cases) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ McTab T;
-  pdl_trigger();
-  load_mc(T);  // (constant tables: before the wait for the kernel ahead)
-  pdl_wait();
-  WarpScratch &W = *reinterpret_cast<WarpScratch *>(smem_raw + (size_t)(threadIdx.x >> 5) *
-                                                                      (EMIT ? SCRATCH_EMIT_BYTES : SCRATCH_COUNT_BYTES));
-  const int lane = threadIdx.x & 31;
-  // the dirty cells: a list of ids, or all cells of [first, first + ncell).
-  // Emit: warps take the next cell from a shared counter (cells differ in
-  // cost); count: a fixed stride (its cells are cheap next to the fetch).
-  const uint32_t n = list ? *list_n : ncell;
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t ci = EMIT ? next_cell(work, lane) : gw; ci < n; ci = EMIT ? next_cell(work, lane) : ci + nw) {
-    const uint32_t cid = list ? list[ci] : first + ci;
-    // emit: a cell that the count pass found without vertices writes nothing
-    if (EMIT && out[cid].nv == 0) continue;
-    const Cell c = cells[cid];
-    if (!owns_cell(m, c)) {
-      // another part meshes it
-      if (!EMIT && lane == 0) out[cid] = CellOut{0u, 0u};
-      continue;
-    }
-    const CellGeom G = cell_geom(m, c);
-    if (G.empty) {
-      if (!EMIT && lane == 0) out[cid] = CellOut{0u, 0u};
-      continue;
-    }
-    const int n3[3] = {G.cnt[0], G.cnt[1], G.cnt[2]};
-    const int nsamp = n3[0] * n3[1] * n3[2];
-    const int nc3[3] = {n3[0] - 1, n3[1] - 1, n3[2] - 1};
-    const int ncube = nc3[0] * nc3[1] * nc3[2];
-    // (the lattices of samples and cubes are split by Lat3s made just
-    // before each loop: in memory order, or in the cell type's loop nesting)
-    const uint8_t *ord = c_order[G.type];
-    // the count pass's marching-cubes case of every cube of this cell
-    uint4 *const cell_cases = reinterpret_cast<uint4 *>(cases + (size_t)ci * 512);
-    if (EMIT) {
-      // Only the samples at the ends of lattice edges that carry a vertex
-      // are read: the edge slots follow from the stored cube cases, and the
-      // samples are the same function of the volume as in the count pass
-      // (which found every sample of this cell inside its leaves).
-      reinterpret_cast<uint4 *>(W.cube_case)[lane] = cell_cases[lane];
-      for (int k = lane; k < 384; k += 32) reinterpret_cast<uint32_t *>(W.edge_set)[k] = 0;
-      for (int k = lane; k < 128; k += 32) reinterpret_cast<uint32_t *>(W.wzero)[k] = 0;  // "needed" flags
-      __syncwarp();
-      const Lat3 Lc = lat3(nc3[0], nc3[1]);
-      for (int k = lane; k < ncube; k += 32) {
-        int bx, by, bz;
-        split3(Lc, k, bx, by, bz);
-        const int idx = (bz * 8 + by) * 8 + bx;
-        const int ci8 = W.cube_case[idx];
-        const int nt = mc_ntri(T, ci8);
-        for (int q = 0; q < 3 * nt; q++) {
-          const int slot = 3 * idx + mc_slot(T, mc_edge(T, ci8, q));
-          const int si = slot / 3, a = slot - 3 * si;
-          W.edge_set[slot] = 1;
-          W.wzero[si] = 1;
-          W.wzero[si + (a == 0 ? 1 : (a == 1 ? 8 : 64))] = 1;
-        }
-      }
-      __syncwarp();
-      // compact list of the needed sample indices (in vidx, free until the
-      // vertex loop below)
-      uint16_t *need = W.vidx;
-      int nneed = 0;
-      for (int k0 = 0; k0 < 512; k0 += 32) {
-        const bool nd = W.wzero[k0 + lane] != 0;
-        const unsigned b = __ballot_sync(0xffffffffu, nd);
-        if (nd) need[nneed + __popc(b & ((1u << lane) - 1u))] = (uint16_t)(k0 + lane);
-        nneed += __popc(b);
-      }
-      __syncwarp();
-      if (lane == 0) atomicAdd(m.samples, (unsigned long long)nneed);
-      for (int k = lane; k < nneed; k += 32) {
-        const int si = need[k];
-        Sample s;
-        lattice_sample<true>(m, c, G, si & 7, (si >> 3) & 7, si >> 6, s);
-        W.sd[si] = s.d;
-        W.sc[3 * si] = s.c[0];
-        W.sc[3 * si + 1] = s.c[1];
-        W.sc[3 * si + 2] = s.c[2];
-      }
-      __syncwarp();
-    } else {
-      bool fit = true;
-      const Lat3 Ls = lat3(n3[0], n3[1]);
-      uint32_t bl;
-      if (brick_cell(m, c, G, bl)) {
-        // the brick's voxels in order; a sample that its voxel does not
-        // settle (no weight, or not finite) takes the general path
-        const size_t vb0 = (size_t)bl * 512;
-        for (int k = lane; k < 512; k += 32) {
-          const float d0 = vd(m, vb0 + k), w0 = vw(m, vb0 + k);
-          if (isfinite(d0)) {
-            const float w = __fadd_rn(0.0f, w0);
-            if (!(w <= 0.0f)) {
-              W.sd[k] = d0;
-              W.wzero[k] = 0;
-              continue;
-            }
-          }
-          Sample s;
-          fit &= lattice_sample<false>(m, c, G, k & 7, (k >> 3) & 7, k >> 6, s);
-          W.sd[k] = s.d;
-          W.wzero[k] = s.w == 0.0f;
-        }
-      } else
-      for (int k = lane; k < nsamp; k += 32) {
-        int bx, by, bz;
-        split3(Ls, k, bx, by, bz);
-        Sample s;
-        fit &= lattice_sample<false>(m, c, G, bx, by, bz, s);  // (no colour: the count pass needs none)
-        const int si = (bz * 8 + by) * 8 + bx;
-        W.sd[si] = s.d;
-        W.wzero[si] = s.w == 0.0f;
-      }
-      for (int k = lane; k < 384; k += 32) reinterpret_cast<uint32_t *>(W.edge_set)[k] = 0;
-      fit = __all_sync(0xffffffffu, fit);
-      __syncwarp();
-      if (lane == 0) atomicAdd(m.samples, (unsigned long long)nsamp);
-      if (!fit) {
-        if (lane == 0) out[cid] = CellOut{0u, 0u};
-        continue;
-      }
-      uint32_t tri = 0;  // this lane's cubes' triangles
-      const Lat3 Lc = lat3(nc3[0], nc3[1]);
-      for (int k = lane; k < ncube; k += 32) {
-        int bx, by, bz;
-        split3(Lc, k, bx, by, bz);
-        const int idx = (bz * 8 + by) * 8 + bx;
-        const int off[8] = {0, 1, 9, 8, 64, 65, 73, 72};
-        bool zero = false;
-        int ci8 = 0;
+// Emit pass, one lattice cell by a warp.
+__device__ __forceinline__ void emit_cell(const VoxSrc &m, const Cell &c, const uint8_t *cell_rows, uint64_t vb,
+                                          uint64_t fb, float *xyz, uint8_t *rgb, uint32_t *faces, LatScratch &W,
+                                          const McTab &T, int lane) {
+  const uint32_t kept = reinterpret_cast<const uint32_t *>(cell_rows)[lane];
+  if (lane < cell_sides(c.type)) load_chain(m, c, lane, W.chain);
+  if (lane < 16) reinterpret_cast<uint32_t *>(W.S)[lane] = kept;
+  else reinterpret_cast<uint32_t *>(W.Vp + 16)[lane - 16] = kept;
+  if (lane < 4) {
+    reinterpret_cast<uint32_t *>(W.Vp)[lane] = 0;
+    reinterpret_cast<uint32_t *>(W.S + 64)[lane] = 0;
+  }
+  __syncwarp();
+  const CellGeom geo = cell_geom(c, W.chain);
+  const Nest N = nest_of(geo);
+  load_vox_tab(geo, N, W.chain, W.tab, lane);
+  const uint32_t cubeF = ((1u << N.nF) - 1u) >> 1;
+  // The rows' vertex-carrying edges, mixed cubes and samples at the edges' ends
+  // (a lane the rows 2 lane and 2 lane + 1, so that a scan over the lanes runs in
+  // row order).  Only those samples are read: the same function of the volume as
+  // in the count pass (which found every sample inside its leaves).
+  uint32_t act[2];
+  int nv = 0, ncube = 0, ntri = 0;
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-          zero |= W.wzero[idx + off[q]] != 0;
-          if (W.sd[idx + off[q]] < 0.0f) ci8 |= 1 << q;
-        }
-        if (zero) ci8 = 0;
-        W.cube_case[idx] = (uint8_t)ci8;
-        const int nt = mc_ntri(T, ci8);
-        tri += (uint32_t)nt;
-        for (int q = 0; q < 3 * nt; q++) {
-          const int slot = 3 * idx + mc_slot(T, mc_edge(T, ci8, q));
-          W.edge_set[slot] = 1;  // lanes that set the same slot store the same byte
-        }
-      }
-      __syncwarp();
-      // kept for the emit pass (entries of cubes outside the lattice unused)
-      cell_cases[lane] = reinterpret_cast<const uint4 *>(W.cube_case)[lane];
-      // The counts need no order: a vertex per edge slot that carries one
-      // (every such slot lies at a lattice sample, and the flags outside the
-      // lattice are clear), a face per triangle of the lattice's cubes.
-      uint32_t verts = 0;
-      for (int k = lane; k < 384; k += 32) verts += (uint32_t)__popc(reinterpret_cast<const uint32_t *>(W.edge_set)[k]);
-      verts = __reduce_add_sync(0xffffffffu, verts);
-      tri = __reduce_add_sync(0xffffffffu, tri);
-      if (lane == 0) out[cid] = CellOut{verts, tri};
-      __syncwarp();
-      continue;
-    }
-    // (the emit pass from here) vertices, in the reference's loop order of
-    // this cell type: the slots that carry one listed in that order first
-    // (a warp scan per 32 samples), then one lane per vertex
-    uint32_t vrun = 0;
-    const uint64_t vb = EMIT ? vbase[cid] : 0;
-    const Lat3 Lso = lat3(n3[ord[2]], n3[ord[1]]);
-    for (int k0 = 0; k0 < nsamp; k0 += 32) {
-      const int k = k0 + lane;
-      int b0 = 0, b1 = 0, b2 = 0, idx = 0, cntv = 0;
-      if (k < nsamp) {
-        idx = lattice_idx(G, k, Lso, b0, b1, b2);
-        cntv = edge_bit(W, 3 * idx) + edge_bit(W, 3 * idx + 1) + edge_bit(W, 3 * idx + 2);
-      }
-      int tot;
-      const int ex = warp_excl_scan(cntv, lane, tot);
-      uint32_t at = vrun + (uint32_t)ex;
-      for (int a = 0; a < 3 && cntv; a++)
-        if (edge_bit(W, 3 * idx + a)) W.vlist[at++] = (uint16_t)(3 * idx + a);
-      vrun += (uint32_t)tot;
-    }
-    __syncwarp();
-    for (uint32_t q = lane; q < vrun; q += 32) {
-      const int slot = W.vlist[q];
-      const int idx = slot / 3, a = slot - 3 * idx;
-      const int bb[3] = {idx & 7, (idx >> 3) & 7, idx >> 6};
-      float P0[3];
+  for (int h = 0; h < 2; h++) {
+    const int r = 2 * lane + h;
+    const uint8_t *V = W.Vp + 16 + r;
+    const uint32_t s = W.S[r], vF = V[0] | V[-1] | V[-8] | V[-9], vB = V[0] | V[-8], vA = V[0] | V[-1];
+    const uint32_t mF = (s ^ (s >> 1)) & vF & cubeF, mB = (s ^ W.S[r + 1]) & (vB | (vB << 1)) & 255u,
+                   mA = (s ^ W.S[r + 8]) & (vA | (vA << 1)) & 255u;
+    W.mF[r] = (uint8_t)mF;
+    W.mB[r] = (uint8_t)mB;
+    W.mA[r] = (uint8_t)mA;
+    nv += __popc(mF) + __popc(mB) + __popc(mA);
+    const uint32_t any = s | W.S[r + 1] | W.S[r + 8] | W.S[r + 9], all = s & W.S[r + 1] & W.S[r + 8] & W.S[r + 9];
+    act[h] = V[0] & (any | (any >> 1)) & ~(all & (all >> 1));
+    ncube += __popc(act[h]);
+  }
+  __syncwarp();
+  uint32_t need[2];
+  int nneed = 0;
 #pragma unroll
-      for (int r = 0; r < 3; r++) P0[r] = __fadd_rn(m.offset[r], __fmul_rn((float)sample_pos(G, r, bb[r]), m.scale));
-      const int step = a == 0 ? 1 : (a == 1 ? 8 : 64);
-      float P1[3] = {P0[0], P0[1], P0[2]};
-      const int q2 = sample_pos(G, a, bb[a]) + (c_role[G.type][a] ? G.stretch : G.sizeMin);
-      P1[a] = __fadd_rn(m.offset[a], __fmul_rn((float)q2, m.scale));
-      float v[3];
-      uint16_t col[3];
-      const float d0 = W.sd[idx], d1 = W.sd[idx + step];
-      vinterp(P0, P1, (double)d0, (double)d1, v);
-      cinterp(&W.sc[3 * idx], &W.sc[3 * (idx + step)], d0, d1, col);
-      const uint64_t gi = vb + q;
-      xyz[3 * gi] = v[0];
-      xyz[3 * gi + 1] = v[1];
-      xyz[3 * gi + 2] = v[2];
-      rgb[3 * gi] = (uint8_t)(col[0] / 256);
-      rgb[3 * gi + 1] = (uint8_t)(col[1] / 256);
-      rgb[3 * gi + 2] = (uint8_t)(col[2] / 256);
-      W.vidx[slot] = (uint16_t)q;
-    }
-    __syncwarp();
-    // faces, cube by cube in the same nesting
-    uint32_t frun = 0;
-    const uint64_t fb = EMIT ? fbase[cid] : 0;
-    const Lat3 Lco = lat3(nc3[ord[2]], nc3[ord[1]]);
-    for (int k0 = 0; k0 < ncube; k0 += 32) {
-      const int k = k0 + lane;
-      int idx = 0, nt = 0, ci8 = 0;
-      if (k < ncube) {
-        int b0, b1, b2;
-        idx = lattice_idx(G, k, Lco, b0, b1, b2);
-        ci8 = W.cube_case[idx];
-        nt = mc_ntri(T, ci8);
-      }
-      int tot;
-      int ex = warp_excl_scan(nt, lane, tot);
-      if (EMIT) {
-        for (int t = 0; t < nt; t++) {
-          const uint64_t gf = fb + frun + (uint32_t)ex + t;
+  for (int h = 0; h < 2; h++) {
+    const int r = 2 * lane + h;
+    const uint32_t f = W.mF[r];
+    need[h] = f | (f << 1) | W.mB[r] | (r >= 1 ? W.mB[r - 1] : 0) | W.mA[r] | (r >= 8 ? W.mA[r - 8] : 0);
+    nneed += __popc(need[h]);
+  }
+  int all_need, all_v, all_cubes;
+  int at = warp_excl_scan(nneed, lane, all_need);
 #pragma unroll
-          for (int q = 0; q < 3; q++)
-            faces[3 * gf + q] = (uint32_t)(vb + W.vidx[3 * idx + mc_slot(T, mc_edge(T, ci8, 3 * t + q))]);
-        }
-      }
-      frun += (uint32_t)tot;
+  for (int h = 0; h < 2; h++)
+    for (uint32_t u = need[h]; u; u &= u - 1) W.slow[at++] = (uint16_t)(8 * (2 * lane + h) + __ffs(u) - 1);
+  // vertices: the lattice edges that carry one in the reference's loop order of
+  // this cell type, the three axes of a sample in turn
+  at = warp_excl_scan(nv, lane, all_v);
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int r = 2 * lane + h;
+    const uint32_t mF = W.mF[r], mB = W.mB[r], mA = W.mA[r];
+    const uint32_t m0 = N.F == 0 ? mF : (N.B == 0 ? mB : mA), m1 = N.F == 1 ? mF : (N.B == 1 ? mB : mA),
+                   m2 = N.F == 2 ? mF : (N.B == 2 ? mB : mA);
+    for (uint32_t u = m0 | m1 | m2; u; u &= u - 1) {
+      const int f = __ffs(u) - 1, slot = 3 * (8 * r + f);
+      if ((m0 >> f) & 1u) W.vidx[slot] = (uint16_t)at, W.vlist[at++] = (uint16_t)slot;
+      if ((m1 >> f) & 1u) W.vidx[slot + 1] = (uint16_t)at, W.vlist[at++] = (uint16_t)(slot + 1);
+      if ((m2 >> f) & 1u) W.vidx[slot + 2] = (uint16_t)at, W.vlist[at++] = (uint16_t)(slot + 2);
     }
-    __syncwarp();
+  }
+  __syncwarp();
+  if (m.samples && lane == 0) atomicAdd(m.samples, (unsigned long long)all_need);
+  for (int k = lane; k < all_need; k += 32) {
+    const int p = W.slow[k];
+    int x, y, z;
+    nest_xyz(N, p, x, y, z);
+    const int side = nest_side(geo.type, (p >> 3) & 7, p & 7);
+    const uint32_t v = vox_of(W.tab, side, p >> 6, (p >> 3) & 7, p & 7);
+    Sample s;
+    bool settled = false;
+    if (v < VOX_OFF) {
+      const size_t vi = (size_t)W.chain.leaf[side][0] * 512 + v;
+      const float d = vd(m, vi), w = vw(m, vi);
+      s.c[0] = vc(m, vi, 0);
+      s.c[1] = vc(m, vi, 1);
+      s.c[2] = vc(m, vi, 2);
+      s.d = d;
+      settled = settles(geo.type, d, w, single_step(W.chain, side));
+    }
+    if (!settled) lattice_sample<true>(m, W.chain, geo, x, y, z, s);
+    W.sd[p] = s.d;
+    W.sc[3 * p] = s.c[0];
+    W.sc[3 * p + 1] = s.c[1];
+    W.sc[3 * p + 2] = s.c[2];
+  }
+  __syncwarp();
+  // (slow, free now, takes the mixed cubes) where each cube's faces start
+  at = warp_excl_scan(ncube, lane, all_cubes);
+  const int cube0 = at;
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int r = 2 * lane + h;
+    const uint32_t s00 = W.S[r], s01 = W.S[r + 1], s10 = W.S[r + 8], s11 = W.S[r + 9];
+    for (uint32_t u = act[h]; u; u &= u - 1) {
+      const int f = __ffs(u) - 1, cs = cube_case(N, s00, s01, s10, s11, f);
+      W.slow[at] = (uint16_t)(8 * r + f);
+      W.code[at] = (uint8_t)cs;
+      W.face0[at++] = (uint16_t)ntri;
+      ntri += mc_ntri(T, cs);
+    }
+  }
+  int all_tri;
+  const int face0 = warp_excl_scan(ntri, lane, all_tri);
+  for (int q = cube0; q < at; q++) W.face0[q] = (uint16_t)(W.face0[q] + face0);
+  for (int q = lane; q < all_v; q += 32) {
+    const int slot = W.vlist[q];
+    const int p = slot / 3, a = slot - 3 * p;
+    int b[3];
+    nest_xyz(N, p, b[0], b[1], b[2]);
+    float P0[3];
+#pragma unroll
+    for (int r = 0; r < 3; r++) P0[r] = __fadd_rn(m.offset[r], __fmul_rn((float)sample_pos(geo, r, b[r]), m.scale));
+    const int to = p + (a == N.F ? 1 : (a == N.B ? 8 : 64));
+    float P1[3] = {P0[0], P0[1], P0[2]};
+#pragma unroll
+    for (int r = 0; r < 3; r++)
+      if (r == a) P1[r] = __fadd_rn(m.offset[r], __fmul_rn((float)sample_pos(geo, r, b[r] + 1), m.scale));
+    float v[3];
+    uint16_t col[3];
+    const float d0 = W.sd[p], d1 = W.sd[to];
+    vinterp(P0, P1, (double)d0, (double)d1, v);
+    cinterp(&W.sc[3 * p], &W.sc[3 * to], d0, d1, col);
+    const uint64_t gi = vb + q;
+    xyz[3 * gi] = v[0];
+    xyz[3 * gi + 1] = v[1];
+    xyz[3 * gi + 2] = v[2];
+    rgb[3 * gi] = (uint8_t)(col[0] / 256);
+    rgb[3 * gi + 1] = (uint8_t)(col[1] / 256);
+    rgb[3 * gi + 2] = (uint8_t)(col[2] / 256);
+  }
+  __syncwarp();
+  // faces, cube by cube in the same nesting
+  for (int q = lane; q < all_cubes; q += 32) {
+    const int base = 3 * (int)W.slow[q], cs = W.code[q], nt = mc_ntri(T, cs);
+    const uint64_t gf = fb + W.face0[q];
+    for (int k = 0; k < 3 * nt; k++)
+      faces[3 * gf + k] = (uint32_t)(vb + W.vidx[base + T.edge[geo.type][mc_edge(T, cs, k)]]);
   }
 }
 
 // addBrickMiddle_indexed_incremental: eight lanes per corner cell, one per
-// sample (the samples' parent-leaf walks are chains of dependent loads: in
-// one thread they would run one after the other), then the cell's first lane
-// runs the single-cube marching cubes on the gathered samples.
+// sample (the samples' parent-leaf walks are chains of dependent loads: in one
+// thread they would run one after the other), then the cube's edges and
+// triangles over the same lanes.  One cell for each eight lanes of the warp;
+// S: a scratch of the eight lanes.
 constexpr int CORNER_LANES = 8;
+struct CornerScratch {
+  float v[12][3];     // vertex on each cube edge the surface cuts
+  uint16_t c[12][4];  // its colour
+};
+static_assert(4 * sizeof(CornerScratch) <= SCRATCH_COUNT_BYTES, "corner scratch fits a warp's lattice scratch");
 
 template <bool EMIT>
-__global__ void k_mesh_corner(VoxSrc m, const Cell *__restrict__ cells, uint32_t first, uint32_t ncell,
-                              const uint32_t *__restrict__ list, const uint32_t *list_n, CellOut *out,
-                              const uint64_t *vbase, const uint64_t *fbase, float *xyz, uint8_t *rgb,
-                              uint32_t *faces) {
-  __shared__ McTab T;
-  pdl_trigger();
-  load_mc(T);  // (constant tables: before the wait for the kernel ahead)
-  pdl_wait();
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t i = t / CORNER_LANES;
-  const int k = (int)(t % CORNER_LANES);  // this lane's sample
+__device__ __forceinline__ void corner_cell(const VoxSrc &m, const Cell &c, uint32_t cid, CellOut *out, uint64_t vb,
+                                            uint64_t fb, float *xyz, uint8_t *rgb, uint32_t *faces, CornerScratch &S,
+                                            const McTab &T) {
+  const int k = (int)(threadIdx.x & 7u);  // this lane's sample
   const unsigned gmask = 0xffu << (threadIdx.x & 24u);
-  if (i >= (list ? *list_n : ncell)) return;
-  const uint32_t cid = list ? list[i] : first + i;
-  const Cell c = cells[cid];
   if (!owns_cell(m, c)) {
     if (!EMIT && k == 0) out[cid] = CellOut{0u, 0u};
     return;
@@ -1730,10 +1921,7 @@ __global__ void k_mesh_corner(VoxSrc m, const Cell *__restrict__ cells, uint32_t
     if (!EMIT && k == 0) out[cid] = CellOut{0u, 0u};
     return;
   }
-  {
-    const unsigned act = __activemask();
-    if ((threadIdx.x & 31u) == (unsigned)(__ffs(act) - 1)) atomicAdd(m.samples, (unsigned long long)__popc(act));
-  }
+  if (m.samples && k == 0) atomicAdd(m.samples, (unsigned long long)CORNER_LANES);
   float dk = 0.0f, wk = 0.0f;
   uint16_t ck[3] = {0, 0, 0};
   {
@@ -1754,86 +1942,270 @@ __global__ void k_mesh_corner(VoxSrc m, const Cell *__restrict__ cells, uint32_t
       for (int r = 0; r < 3; r++) ck[r] = vcs<EMIT>(m, vi, r);  // (the count pass needs no colour)
     }
   }
-  // every lane of the cell gets all eight samples
-  float d[8], w[8];
-  uint16_t col[8][3];
-  const uint32_t ck01 = (uint32_t)ck[0] | ((uint32_t)ck[1] << 16);
-#pragma unroll
-  for (int j = 0; j < 8; j++) {
-    d[j] = __shfl_sync(gmask, dk, j, CORNER_LANES);
-    w[j] = __shfl_sync(gmask, wk, j, CORNER_LANES);
-    const uint32_t a01 = __shfl_sync(gmask, ck01, j, CORNER_LANES);
-    const uint32_t a2 = __shfl_sync(gmask, (uint32_t)ck[2], j, CORNER_LANES);
-    col[j][0] = (uint16_t)(a01 & 0xffffu);
-    col[j][1] = (uint16_t)(a01 >> 16);
-    col[j][2] = (uint16_t)a2;
-  }
-  if (k != 0) return;
-  const int mcv[8] = {0, 1, 3, 2, 4, 5, 7, 6};
+  __syncwarp(gmask);
+  // every lane of the cell gets all eight samples, cube corner j from sample mcv[j]
   float val[8];
+  uint16_t col[8][3];
   bool zero = false;
   int ci8 = 0;
-  for (int k = 0; k < 8; k++) {
-    val[k] = d[mcv[k]];
-    zero |= w[mcv[k]] == 0.0f;
-    if (val[k] < 0.0f) ci8 |= 1 << k;
+  const uint32_t ck01 = (uint32_t)ck[0] | ((uint32_t)ck[1] << 16);
+  constexpr int mcv[8] = {0, 1, 3, 2, 4, 5, 7, 6};
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    val[j] = __shfl_sync(gmask, dk, mcv[j], CORNER_LANES);
+    zero |= __shfl_sync(gmask, wk, mcv[j], CORNER_LANES) == 0.0f;
+    if (val[j] < 0.0f) ci8 |= 1 << j;
+    if (EMIT) {
+      const uint32_t a01 = __shfl_sync(gmask, ck01, mcv[j], CORNER_LANES);
+      const uint32_t a2 = __shfl_sync(gmask, (uint32_t)ck[2], mcv[j], CORNER_LANES);
+      col[j][0] = (uint16_t)(a01 & 0xffffu);
+      col[j][1] = (uint16_t)(a01 >> 16);
+      col[j][2] = (uint16_t)a2;
+    }
   }
   if (zero) ci8 = 0;
   const float sx = __fmul_rn(m.scale, (float)stretch);
   float O[3];
   for (int r = 0; r < 3; r++) O[r] = __fadd_rn(m.offset[r], __fmul_rn((float)(c.o[r] + c.size - stretch), m.scale));
-  float P[8][3];
-  for (int k = 0; k < 8; k++) {
-    const int bx = (k == 1 || k == 2 || k == 5 || k == 6), by = (k == 2 || k == 3 || k == 6 || k == 7), bz = k >= 4;
-    P[k][0] = __fadd_rn(O[0], __fmul_rn((float)bx, sx));
-    P[k][1] = __fadd_rn(O[1], __fmul_rn((float)by, sx));
-    P[k][2] = __fadd_rn(O[2], __fmul_rn((float)bz, sx));
-  }
-  float vl[12][3];
-  uint16_t cl[12][3];
-  for (int e = 0; e < 12; e++) {
+  // edges k and (lanes 0-3) k + 8 of the cube
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int e = k + 8 * h;
+    if (e >= 12) break;
     const int a = c_edge_a[e], b = c_edge_b[e];
-    if (((ci8 >> a) & 1) != ((ci8 >> b) & 1)) {
-      vinterp(P[a], P[b], (double)val[a], (double)val[b], vl[e]);
-      if (EMIT) cinterp(col[mcv[a]], col[mcv[b]], val[a], val[b], cl[e]);
+    if (((ci8 >> a) & 1) == ((ci8 >> b) & 1)) continue;
+    float va = 0.0f, vb_ = 0.0f, Pa[3], Pb[3];
+    uint16_t ca[3] = {0, 0, 0}, cb[3] = {0, 0, 0};
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      if (j == a) {
+        va = val[j];
+        if (EMIT) ca[0] = col[j][0], ca[1] = col[j][1], ca[2] = col[j][2];
+      }
+      if (j == b) {
+        vb_ = val[j];
+        if (EMIT) cb[0] = col[j][0], cb[1] = col[j][1], cb[2] = col[j][2];
+      }
     }
+    // corner q lies at (x, y, z) of the cube: x for 1, 2, 5, 6; y for 2, 3, 6, 7; z from 4
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const int ba = r == 0 ? ((a + 1) >> 1) & 1 : (r == 1 ? (a >> 1) & 1 : a >> 2);
+      const int bb = r == 0 ? ((b + 1) >> 1) & 1 : (r == 1 ? (b >> 1) & 1 : b >> 2);
+      Pa[r] = __fadd_rn(O[r], __fmul_rn((float)ba, sx));
+      Pb[r] = __fadd_rn(O[r], __fmul_rn((float)bb, sx));
+    }
+    vinterp(Pa, Pb, (double)va, (double)vb_, S.v[e]);
+    if (EMIT) cinterp(ca, cb, va, vb_, S.c[e]);
   }
+  __syncwarp(gmask);
+  // one triangle per lane (at most five), degenerate ones dropped
   const int nt = mc_ntri(T, ci8);
-  uint32_t kept = 0;
-  const uint64_t vb = EMIT ? vbase[cid] : 0, fb = EMIT ? fbase[cid] : 0;
-  for (int t = 0; t < nt; t++) {
-    const int e0 = mc_edge(T, ci8, 3 * t), e1 = mc_edge(T, ci8, 3 * t + 1), e2 = mc_edge(T, ci8, 3 * t + 2);
-    const float *v0 = vl[e0], *v1 = vl[e1], *v2 = vl[e2];
+  bool keep = k < nt;
+  int es[3] = {0, 0, 0};
+  if (keep) {
+#pragma unroll
+    for (int q = 0; q < 3; q++) es[q] = mc_edge(T, ci8, 3 * k + q);
+    const float *v0 = S.v[es[0]], *v1 = S.v[es[1]], *v2 = S.v[es[2]];
     const bool deg = (v0[0] == v1[0] && v0[1] == v1[1] && v0[2] == v1[2]) ||
                      (v2[0] == v1[0] && v2[1] == v1[1] && v2[2] == v1[2]) ||
                      (v0[0] == v2[0] && v0[1] == v2[1] && v0[2] == v2[2]);
-    if (deg) continue;
-    if (EMIT) {
-      const int es[3] = {e0, e1, e2};
-      for (int q = 0; q < 3; q++) {
-        const uint64_t gi = vb + 3 * kept + q;
-        for (int r = 0; r < 3; r++) {
-          xyz[3 * gi + r] = vl[es[q]][r];
-          rgb[3 * gi + r] = (uint8_t)(cl[es[q]][r] / 256);
-        }
-        faces[3 * (fb + kept) + q] = (uint32_t)gi;
+    keep = !deg;
+  }
+  const unsigned kept = __ballot_sync(gmask, keep);
+  if (EMIT && keep) {
+    const uint32_t at = (uint32_t)__popc(kept & ((1u << (threadIdx.x & 31u)) - 1u));
+    for (int q = 0; q < 3; q++) {
+      const uint64_t gi = vb + 3 * at + q;
+      for (int r = 0; r < 3; r++) {
+        xyz[3 * gi + r] = S.v[es[q]][r];
+        rgb[3 * gi + r] = (uint8_t)(S.c[es[q]][r] / 256);
+      }
+      faces[3 * (fb + at) + q] = (uint32_t)gi;
+    }
+  }
+  if (!EMIT && k == 0) {
+    const uint32_t n = (uint32_t)__popc(kept);
+    out[cid] = CellOut{3 * n, n};
+  }
+  __syncwarp(gmask);
+}
+
+// n bytes (any alignment) from src to dst by a warp: dst's aligned words, each
+// from the one or two words of src that hold it, and the ends byte by byte.
+// src's word that holds the last byte may be read whole.
+__device__ __forceinline__ void copy_bytes(uint8_t *dst, const uint8_t *src, uint64_t n, int lane) {
+  const uint64_t head = min((uint64_t)((4 - ((uintptr_t)dst & 3)) & 3), n);
+  if ((uint64_t)lane < head) dst[lane] = src[lane];
+  const uint64_t words = (n - head) / 4;
+  const uint8_t *sp = src + head;
+  const uint32_t sh = (uint32_t)((uintptr_t)sp & 3) * 8;
+  const uint32_t *sw = reinterpret_cast<const uint32_t *>((uintptr_t)sp & ~(uintptr_t)3);
+  uint32_t *dw = reinterpret_cast<uint32_t *>(dst + head);
+#pragma unroll 4
+  for (uint64_t k = lane; k < words; k += 32) dw[k] = __funnelshift_r(sw[k], sh ? sw[k + 1] : 0u, sh);
+  const uint64_t done = head + 4 * words;
+  if ((uint64_t)lane < n - done) dst[done + lane] = src[done + lane];
+}
+
+// n words by a warp, `add` added to each (ADD), eight in flight per lane.
+template <bool ADD>
+__device__ __forceinline__ void copy_words(uint32_t *dst, const uint32_t *src, uint32_t n, uint32_t add, int lane) {
+  constexpr int U = 8;
+  for (uint32_t k0 = lane; k0 < n; k0 += 32 * U) {
+    uint32_t v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) v[u] = k0 + 32 * u < n ? src[k0 + 32 * u] : 0u;
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (k0 + 32 * u < n) dst[k0 + 32 * u] = ADD ? v[u] + add : v[u];
+  }
+}
+
+// The clean cells' mesh of the previous update: where it lies, and its cells.
+struct CleanCopy {
+  const uint8_t *dirty;
+  const int32_t *old_index;
+  const uint64_t *old_vbase, *old_fbase;
+  const float *old_xyz;
+  const uint8_t *old_rgb;
+  const uint32_t *old_faces;
+  uint32_t n;  // cells (0: nothing to copy)
+};
+
+// Cells [CLEAN_CELLS i, CLEAN_CELLS (i + 1)): the clean ones copy their previous
+// vertices and faces (faces re-based).  Neighbours that were neighbours before, shifted by the same
+// number of vertices and faces, are one copy.
+constexpr uint32_t CLEAN_CELLS = 8;
+__device__ __forceinline__ void copy_clean(const CleanCopy &C, uint32_t i, const CellOut *out, const uint64_t *vbase,
+                                           const uint64_t *fbase, float *xyz, uint8_t *rgb, uint32_t *faces,
+                                           int lane) {
+  const uint32_t id = CLEAN_CELLS * i + lane;
+  bool clean = lane < (int)CLEAN_CELLS && id < C.n && !C.dirty[id];
+  uint64_t v0 = 0, f0 = 0, ov = 0, of = 0;
+  CellOut o = {0u, 0u};
+  if (clean) {
+    const int32_t j = C.old_index[id];
+    o = out[id];
+    v0 = vbase[id];
+    f0 = fbase[id];
+    ov = C.old_vbase[j];
+    of = C.old_fbase[j];
+  }
+  const uint64_t sv = v0 - ov, sf = f0 - of;
+  const uint64_t psv = __shfl_up_sync(0xffffffffu, sv, 1), psf = __shfl_up_sync(0xffffffffu, sf, 1);
+  const unsigned cl = __ballot_sync(0xffffffffu, clean);
+  const bool joins = clean && lane > 0 && ((cl >> (lane - 1)) & 1u) && sv == psv && sf == psf;
+  const unsigned heads = __ballot_sync(0xffffffffu, clean && !joins);
+  for (unsigned hs = heads; hs; hs &= hs - 1) {
+    const int a = __ffs(hs) - 1;
+    // the run's last cell: before the next head or the next cell that is not clean
+    const unsigned stop = (heads | ~cl) & ~((2u << a) - 1u);
+    const int z = stop ? __ffs(stop) - 2 : 31;
+    const uint64_t va = __shfl_sync(0xffffffffu, v0, a), fa = __shfl_sync(0xffffffffu, f0, a);
+    const uint64_t oa = __shfl_sync(0xffffffffu, ov, a), ofa = __shfl_sync(0xffffffffu, of, a);
+    const uint64_t vz = __shfl_sync(0xffffffffu, v0 + o.nv, z), fz = __shfl_sync(0xffffffffu, f0 + o.nf, z);
+    const uint64_t nv = vz - va, nf = fz - fa;
+    copy_words<false>(reinterpret_cast<uint32_t *>(xyz) + 3 * va, reinterpret_cast<const uint32_t *>(C.old_xyz) + 3 * oa,
+                      (uint32_t)(3 * nv), 0u, lane);
+    copy_bytes(rgb + 3 * va, C.old_rgb + 3 * oa, 3 * nv, lane);
+    copy_words<true>(faces + 3 * fa, C.old_faces + 3 * ofa, (uint32_t)(3 * nf), (uint32_t)(va - oa), lane);
+  }
+}
+
+// Count pass: vertices and faces of the dirty cells into out, the lattice cells'
+// rows into cell_rows (CELL_ROWS bytes each, in list order).  Lattice cells by a
+// warp each, corner cells by eight lanes each, from one shared counter; in the
+// emit pass the clean cells too, CLEAN_CELLS to a warp.
+__global__ void __launch_bounds__(MESH_THREADS, 8) k_mesh_count(VoxSrc m, const Cell *__restrict__ cells, MeshLists L,
+                                                               CellOut *out, uint8_t *__restrict__ cell_rows,
+                                                               uint32_t *work) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ McTab T;
+  pdl_trigger();
+  load_mc(T);  // (constant tables: before the wait for the kernel ahead)
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  LatScratch &W = *reinterpret_cast<LatScratch *>(smem_raw + (size_t)(threadIdx.x >> 5) * SCRATCH_COUNT_BYTES);
+  const uint32_t nl = *L.n_lattice, nc = *L.n_corner, items = nl + (nc + 3) / 4;
+  uint32_t it = __shfl_sync(0xffffffffu, ask_item(work, lane), 0);
+  while (it < items) {
+    const uint32_t next = ask_item(work, lane);
+    if (it < nl) {
+      const uint32_t cid = L.lattice[it];
+      count_cell(m, cells[cid], cid, cell_rows + (size_t)it * CELL_ROWS, out, W, T, lane);
+    } else {
+      const uint32_t i = 4 * (it - nl) + (uint32_t)(lane >> 3);
+      if (i < nc) {
+        const uint32_t cid = L.corner[i];
+        corner_cell<false>(m, cells[cid], cid, out, 0, 0, nullptr, nullptr, nullptr,
+                           reinterpret_cast<CornerScratch *>(&W)[lane >> 3], T);
       }
     }
-    kept++;
+    __syncwarp();
+    it = __shfl_sync(0xffffffffu, next, 0);
   }
-  if (!EMIT) out[cid] = CellOut{3 * kept, kept};
+}
+
+// Emit pass: every cell's vertices and faces at their final offsets.
+__global__ void __launch_bounds__(MESH_THREADS, 4) k_mesh_emit(VoxSrc m, const Cell *__restrict__ cells, MeshLists L,
+                                                              CellOut *out, const uint64_t *vbase,
+                                                              const uint64_t *fbase, float *xyz, uint8_t *rgb,
+                                                              uint32_t *faces, uint32_t *work,
+                                                              const uint8_t *__restrict__ cell_rows, CleanCopy C) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ McTab T;
+  pdl_trigger();
+  load_mc(T);
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  LatScratch &W = *reinterpret_cast<LatScratch *>(smem_raw + (size_t)(threadIdx.x >> 5) * SCRATCH_EMIT_BYTES);
+  const uint32_t nl = *L.n_lattice, nc = *L.n_corner;
+  const uint32_t corners = nl + (nc + 3) / 4, items = corners + (C.n + CLEAN_CELLS - 1) / CLEAN_CELLS;
+  uint32_t it = __shfl_sync(0xffffffffu, ask_item(work, lane), 0);
+  while (it < items) {
+    const uint32_t next = ask_item(work, lane);
+    if (it < nl) {
+      const uint32_t cid = L.lattice[it];
+      if (out[cid].nv)
+        emit_cell(m, cells[cid], cell_rows + (size_t)it * CELL_ROWS, vbase[cid], fbase[cid], xyz, rgb, faces, W, T, lane);
+    } else if (it < corners) {
+      const uint32_t i = 4 * (it - nl) + (uint32_t)(lane >> 3);
+      if (i < nc) {
+        const uint32_t cid = L.corner[i];
+        if (out[cid].nv)
+          corner_cell<true>(m, cells[cid], cid, out, vbase[cid], fbase[cid], xyz, rgb, faces,
+                            reinterpret_cast<CornerScratch *>(&W)[lane >> 3], T);
+      }
+    } else {
+      copy_clean(C, it - corners, out, vbase, fbase, xyz, rgb, faces, lane);
+    }
+    __syncwarp();
+    it = __shfl_sync(0xffffffffu, next, 0);
+  }
 }
 
 // ---------------------------------------------------------------------------
 // Incremental bookkeeping
 // ---------------------------------------------------------------------------
 
-// a cell is dirty if it is new, its leaves changed, or a leaf on any of its
-// parent chains was updated since the previous mesh
+// The dirty lists as the marking fills them.
+struct DirtyLists {
+  uint32_t *lattice, *corner;
+  uint32_t *n_lattice, *n_corner;
+};
+__device__ __forceinline__ void list_dirty(const DirtyLists &D, uint32_t i, int type) {
+  if (type < 7) D.lattice[claim(D.n_lattice)] = i;
+  else D.corner[claim(D.n_corner)] = i;
+}
+
+// A cell is dirty if it is new, its leaves changed, or a leaf on any of its
+// parent chains was updated since the previous mesh.  A clean cell's counts are
+// the previous update's.
 __global__ void k_mark_dirty(const Cell *cells, uint32_t n, const Cell *old_cells, uint32_t n_old,
                              const uint64_t *old_keys, const uint32_t *stamp, const uint32_t *parent,
                              uint32_t leaves_used, uint32_t since, uint8_t *dirty, int32_t *old_index,
-                             uint32_t *n_dirty, uint32_t first_corner, uint32_t *list, uint32_t *n_list, int B) {
+                             DirtyLists D, const CellOut *old_out, CellOut *out, int B) {
   pdl_enter();
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -1865,12 +2237,15 @@ __global__ void k_mark_dirty(const Cell *cells, uint32_t n, const Cell *old_cell
   }
   dirty[i] = d ? 1 : 0;
   old_index[i] = found;
-  if (d) {
-    atomicAdd(n_dirty, 1u);
-    // lattice cells listed from the front, corner cells from first_corner
-    if (i < first_corner) list[claim(n_list)] = i;
-    else list[first_corner + claim(n_list + 1)] = i;
-  }
+  if (d) list_dirty(D, i, c.type);
+  else out[i] = old_out[found];
+}
+
+// The first update: every cell is dirty.
+__global__ void k_mark_all(const Cell *cells, uint32_t n, DirtyLists D) {
+  pdl_enter();
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) list_dirty(D, i, cells[i].type);
 }
 
 // ---------------------------------------------------------------------------
@@ -1983,36 +2358,6 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_count_tile_apply(const CellOut
   }
 }
 
-// clean cells copy their previous vertices and faces (faces re-based)
-__global__ void k_copy_clean(const uint8_t *dirty, const int32_t *old_index, uint32_t n, const CellOut *out,
-                             const uint64_t *vbase, const uint64_t *fbase, const uint64_t *old_vbase,
-                             const uint64_t *old_fbase, const float *old_xyz, const uint8_t *old_rgb,
-                             const uint32_t *old_faces, float *xyz, uint8_t *rgb, uint32_t *faces) {
-  pdl_enter();
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = warp; i < n; i += nwarps) {
-    if (dirty[i]) continue;
-    const int32_t j = old_index[i];
-    const uint64_t nv = out[i].nv, nf = out[i].nf;
-    const uint64_t v0 = vbase[i], f0 = fbase[i], ov0 = old_vbase[j], of0 = old_fbase[j];
-    for (uint64_t k = lane; k < 3 * nv; k += 32) {
-      xyz[3 * v0 + k] = old_xyz[3 * ov0 + k];
-      rgb[3 * v0 + k] = old_rgb[3 * ov0 + k];
-    }
-    for (uint64_t k = lane; k < 3 * nf; k += 32) faces[3 * f0 + k] = (uint32_t)(old_faces[3 * of0 + k] - ov0 + v0);
-  }
-}
-
-__global__ void k_fill_counts_from_old(const uint8_t *dirty, const int32_t *old_index, uint32_t n,
-                                       const CellOut *old_out, CellOut *out) {
-  pdl_enter();
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || dirty[i]) return;
-  out[i] = old_out[old_index[i]];
-}
-
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
@@ -2080,7 +2425,8 @@ struct MeshImpl {
   // one axis), and its cell count
   size_t peak[5] = {0, 0, 0, 0, 0};
   int key_bits = 0;                   // bits per origin coordinate of old_keys / keys
-  // words 8 n_cells, 9 error, 10 n_dirty, 11 n_corners, 12-13 samples;
+  // words 8 n_cells, 9 error, 11 n_corners, 12-13 and 18-19 samples, 14-15
+  // dirty cells, 17 and 22 work counters, 20-21 kept cells, 24-25 barrier;
   // from LEVEL_COUNTS: QK item counters per generation level
   uint32_t *d_count = nullptr;
   uint32_t *h_count = nullptr;
@@ -2107,8 +2453,8 @@ struct MeshImpl {
   size_t cap_oi = 0;
   uint32_t *dlist = nullptr;  // dirty cell ids: lattice cells, then (from first_corner) corner cells
   size_t cap_dlist = 0;
-  uint8_t *cases = nullptr;  // count pass -> emit pass: 512 cube cases per dirty lattice cell
-  size_t cap_cases = 0;
+  uint8_t *cell_rows = nullptr;  // count pass -> emit pass: CELL_ROWS bytes per dirty lattice cell
+  size_t cap_cell_rows = 0;
   void *scan_tmp = nullptr;
   size_t scan_tmp_bytes = 0;
   // previous mesh (the current output moves here before the next update)
@@ -2169,6 +2515,9 @@ static int key_bits_for(uint32_t n) {
 constexpr int KEPT_WORD = 20;
 // d_count words 24, 25: the grid barrier of the one-launch traversal
 constexpr int GEN_BARRIER_WORD = 24;
+// the dirty lists' counts (lattice cells, corner cells) and the count and emit
+// passes' work counters
+constexpr int DIRTY_WORD = 14, COUNT_WORK_WORD = 17, EMIT_WORK_WORD = 22;
 
 static int generate_cells(MeshImpl &I, const MeshInputs &in, bool incr, cudaStream_t s, uint32_t &ncells,
                           std::string &err) {
@@ -2471,9 +2820,9 @@ int mesh_update(MeshState &M, const MeshInputs &in, cudaStream_t s, std::string 
   vs.shard = in.shard;
   vs.shards = in.shards;
   for (int r = 0; r < 3; r++) vs.shift[r] = in.shift[r];
-  // d_count words 12-13 hold the sample counter (8-byte aligned)
-  vs.samples = reinterpret_cast<unsigned long long *>(I.d_count + 12);
-  MCK(cudaMemsetAsync(I.d_count + 12, 0, 2 * sizeof(uint32_t), s));
+  // the passes count the samples they read (profiling) in d_count words 12-13
+  // and 18-19; all these words are zero since the cell generation began
+  vs.samples = P.on ? reinterpret_cast<unsigned long long *>(I.d_count + 12) : nullptr;
 
   MCK(grow_buf(I.out, I.cap_out, ncells, s));
   MCK(grow_buf(I.dirty, I.cap_dirty, ncells, s));
@@ -2490,60 +2839,54 @@ int mesh_update(MeshState &M, const MeshInputs &in, cudaStream_t s, std::string 
   // buffers of the count pass and the scans, ahead of the kernels (nothing
   // but kernels between them on the stream)
   const uint32_t ntiles = (ncells + SCAN_TILE - 1) / SCAN_TILE;
-  MCK(grow_buf(I.cases, I.cap_cases, (size_t)first_corner * 512, s));
+  MCK(grow_buf(I.cell_rows, I.cap_cell_rows, (size_t)first_corner * CELL_ROWS, s));
   MCK(grow_buf(I.nv, I.cap_nv, std::max<uint32_t>(ntiles, 1), s));  // tile sums of the vertex counts
   MCK(grow_buf(I.nf, I.cap_nf, std::max<uint32_t>(ntiles, 1), s));  // and of the face counts
   // programmatic dependent launches, unless the stage profile's events lie
   // between the kernels
   const bool pdl = !P.on;
   // dirty cells: all on the first update, otherwise those whose inputs changed
-  MCK(cudaMemsetAsync(I.d_count + 10, 0, sizeof(uint32_t), s));
-  MCK(cudaMemsetAsync(I.d_count + 14, 0, 2 * sizeof(uint32_t), s));
+  DirtyLists D;
+  D.lattice = I.dlist;
+  D.corner = I.dlist + first_corner;
+  D.n_lattice = I.d_count + DIRTY_WORD;
+  D.n_corner = I.d_count + DIRTY_WORD + 1;
   if (ncells) {
-    if (incremental) {
-      note_launch(2);
+    note_launch(1);
+    if (incremental)
       k_mark_dirty<<<(ncells + 255) / 256, 256, 0, s>>>(I.cells, ncells, I.old_cells, I.n_old, I.old_keys, in.stamp,
-                                                        in.parent, in.leaves_used, I.since, I.dirty, I.old_index,
-                                                        I.d_count + 10, first_corner, I.dlist, I.d_count + 14,
-                                                        kb);
-      MCK(launch_pdl(pdl, k_fill_counts_from_old, dim3((ncells + 255) / 256), dim3(256), 0, s, I.dirty, I.old_index,
-                     ncells, I.old_out, I.out));
-    } else {
-      MCK(cudaMemsetAsync(I.dirty, 1, ncells, s));
-    }
+                                                        in.parent, in.leaves_used, I.since, I.dirty, I.old_index, D,
+                                                        I.old_out, I.out, kb);
+    else
+      k_mark_all<<<(ncells + 255) / 256, 256, 0, s>>>(I.cells, ncells, D);
   }
+  MeshLists L;
+  L.lattice = D.lattice;
+  L.corner = D.corner;
+  L.n_lattice = D.n_lattice;
+  L.n_corner = D.n_corner;
   const size_t smem_count = SCRATCH_COUNT_BYTES * MESH_WARPS, smem_emit = SCRATCH_EMIT_BYTES * MESH_WARPS;
   static std::atomic<unsigned long long> attr_devices{0};
   int dev = 0;
   MCK(cudaGetDevice(&dev));
   const unsigned long long dbit = 1ull << (dev & 63);
   if (!(attr_devices.load() & dbit)) {
-    MCK(cudaFuncSetAttribute(k_mesh_lattice<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_count));
-    MCK(cudaFuncSetAttribute(k_mesh_lattice<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_emit));
+    MCK(cudaFuncSetAttribute(k_mesh_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_count));
+    MCK(cudaFuncSetAttribute(k_mesh_emit, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_emit));
     attr_devices.fetch_or(dbit);
   }
-  const uint32_t *lat_list = incremental ? I.dlist : nullptr;
-  const uint32_t *cor_list = incremental ? I.dlist + first_corner : nullptr;
   pi = P.begin(ST_MESH_COUNT, s);
-  const int lat_blocks = std::max(1, std::min<int>(148 * 8, (int)((first_corner + MESH_WARPS - 1) / MESH_WARPS)));
-  note_launch((first_corner ? 1 : 0) + (ncells > first_corner ? 1 : 0) + (ncells ? 1 : 0));
+  // blocks: as many as are resident at once, at most one per 4 cells
+  const auto blocks = [&](int per_sm, uint32_t items) {
+    return dim3((unsigned)std::max(1, std::min<int>(148 * per_sm, (int)((items + MESH_WARPS - 1) / MESH_WARPS))));
+  };
   // (the kernels from here to the totals' copy follow one another on the
-  // stream: each after the first is a programmatic dependent of the one
-  // before; the dirty marking is one when the volume's cells were kept)
-  bool chained = pdl && incremental && ncells;
-  if (first_corner) {
-    MCK(launch_pdl(chained, k_mesh_lattice<false>, dim3(lat_blocks), dim3(32 * MESH_WARPS), smem_count, s, vs,
-                   (const Cell *)I.cells, 0u, first_corner, lat_list, (const uint32_t *)(I.d_count + 14), I.out,
-                   (const uint64_t *)nullptr, (const uint64_t *)nullptr, (float *)nullptr, (uint8_t *)nullptr,
-                   (uint32_t *)nullptr, I.d_count + 16, I.cases));
-    chained = pdl;
-  }
-  if (ncells > first_corner) {
-    MCK(launch_pdl(chained, k_mesh_corner<false>, dim3(((ncells - first_corner) * CORNER_LANES + 127) / 128),
-                   dim3(128), 0, s, vs, (const Cell *)I.cells, first_corner, ncells - first_corner, cor_list,
-                   (const uint32_t *)(I.d_count + 15), I.out, (const uint64_t *)nullptr, (const uint64_t *)nullptr,
-                   (float *)nullptr, (uint8_t *)nullptr, (uint32_t *)nullptr));
-    chained = pdl;
+  // stream: each is a programmatic dependent of the one before)
+  bool chained = pdl && ncells;
+  if (ncells) {
+    note_launch(1);
+    MCK(launch_pdl(chained, k_mesh_count, blocks(8, ncells), dim3(MESH_THREADS), smem_count, s, vs,
+                   (const Cell *)I.cells, L, I.out, I.cell_rows, I.d_count + COUNT_WORK_WORD));
   }
   const int pi_count = pi;
   P.end(pi_count, 0.0, s);
@@ -2567,7 +2910,7 @@ int mesh_update(MeshState &M, const MeshInputs &in, cudaStream_t s, std::string 
   MCK(cudaMemcpyAsync(h_tot + 0, I.vbase + ncells, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   MCK(cudaMemcpyAsync(h_tot + 1, I.fbase + ncells, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   MCK(cudaMemcpyAsync(h_tot + 2, I.d_count + 12, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  MCK(cudaMemcpyAsync(I.h_count + HOST_TOTALS + 6, I.d_count + 10, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  MCK(cudaMemcpyAsync(I.h_count + DIRTY_WORD, I.d_count + DIRTY_WORD, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   MCK(cudaMemcpyAsync(I.h_count + HOST_TOTALS + 7, I.d_count + 9, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   MCK(cudaStreamSynchronize(s));
   if (I.h_count[HOST_TOTALS + 7] & ERR_CELL_KEY) {
@@ -2591,7 +2934,7 @@ int mesh_update(MeshState &M, const MeshInputs &in, cudaStream_t s, std::string 
   }
   const uint64_t tot[2] = {h_tot[0], h_tot[1]};
   const unsigned long long nsamples = h_tot[2];
-  const uint32_t ndirty = incremental ? I.h_count[HOST_TOTALS + 6] : ncells;
+  const uint32_t ndirty = I.h_count[DIRTY_WORD] + I.h_count[DIRTY_WORD + 1];
   // count pass: SDF and weight of every sample of the dirty cells (the emit
   // pass reads colour as well: sample_bytes)
   const double sample_bytes = vs.fp16 ? 10.0 : 14.0;
@@ -2607,31 +2950,23 @@ int mesh_update(MeshState &M, const MeshInputs &in, cudaStream_t s, std::string 
   MCK(grow_buf(M.d_rgb, I.cap_rgb, 3 * tot[0] + 3, s));
   MCK(grow_buf(M.d_faces, I.cap_faces, 3 * tot[1] + 3, s));
   // the emit pass counts the samples it reads in d_count words 18-19
-  vs.samples = reinterpret_cast<unsigned long long *>(I.d_count + 18);
+  vs.samples = P.on ? reinterpret_cast<unsigned long long *>(I.d_count + 18) : nullptr;
   pi = P.begin(ST_MESH_EMIT, s);
-  note_launch((first_corner ? 1 : 0) + (ncells > first_corner ? 1 : 0) + (incremental && ncells ? 1 : 0));
-  // (the emit kernels after the first: programmatic dependents of the one
-  // before)
-  chained = false;
-  if (first_corner) {
-    k_mesh_lattice<true><<<lat_blocks, 32 * MESH_WARPS, smem_emit, s>>>(vs, I.cells, 0, first_corner, lat_list,
-                                                                   I.d_count + 14, I.out, I.vbase, I.fbase, M.d_xyz,
-                                                                   M.d_rgb, M.d_faces, I.d_count + 17, I.cases);
-    chained = pdl;
+  CleanCopy C;
+  C.dirty = I.dirty;
+  C.old_index = I.old_index;
+  C.old_vbase = I.old_vbase;
+  C.old_fbase = I.old_fbase;
+  C.old_xyz = I.old_xyz;
+  C.old_rgb = I.old_rgb;
+  C.old_faces = I.old_faces;
+  C.n = incremental ? ncells : 0u;
+  if (ncells) {
+    note_launch(1);
+    k_mesh_emit<<<blocks(4, ncells), MESH_THREADS, smem_emit, s>>>(vs, I.cells, L, I.out, I.vbase, I.fbase, M.d_xyz,
+                                                                  M.d_rgb, M.d_faces, I.d_count + EMIT_WORK_WORD,
+                                                                  I.cell_rows, C);
   }
-  if (ncells > first_corner) {
-    MCK(launch_pdl(chained, k_mesh_corner<true>, dim3(((ncells - first_corner) * CORNER_LANES + 127) / 128),
-                   dim3(128), 0, s, vs, (const Cell *)I.cells, first_corner, ncells - first_corner, cor_list,
-                   (const uint32_t *)(I.d_count + 15), I.out, (const uint64_t *)I.vbase, (const uint64_t *)I.fbase,
-                   M.d_xyz, M.d_rgb, M.d_faces));
-    chained = pdl;
-  }
-  if (incremental && ncells)
-    MCK(launch_pdl(chained, k_copy_clean, dim3(148 * 8), dim3(256), 0, s, (const uint8_t *)I.dirty,
-                   (const int32_t *)I.old_index, ncells, (const CellOut *)I.out, (const uint64_t *)I.vbase,
-                   (const uint64_t *)I.fbase, (const uint64_t *)I.old_vbase, (const uint64_t *)I.old_fbase,
-                   (const float *)I.old_xyz, (const uint8_t *)I.old_rgb, (const uint32_t *)I.old_faces, M.d_xyz,
-                   M.d_rgb, M.d_faces));
   // emit pass: the samples it reads (the ends of vertex-carrying lattice
   // edges, corner cells' 8) and the whole mesh written (xyz 12 B + rgb 3 B
   // per vertex, 12 B per face); the sample count arrives with the final sync
@@ -2783,7 +3118,7 @@ void mesh_free(MeshState &M) {
                     I.vertq[1], I.d_count, I.raw, I.cells, I.old_cells, I.keys, I.keys_sorted, I.old_keys,
                     I.vals, I.vals_sorted, I.sort_tmp, I.out, I.old_out, I.nv, I.nf, I.vbase, I.fbase,
                     I.old_vbase, I.old_fbase, I.dirty, I.old_index, I.scan_tmp, I.old_xyz, I.old_rgb,
-                    I.old_faces, I.dlist, I.cases, I.keep, I.keep_tiles, I.mkeys, I.top_cellq, I.top_faceq,
+                    I.old_faces, I.dlist, I.cell_rows, I.keep, I.keep_tiles, I.mkeys, I.top_cellq, I.top_faceq,
                     I.top_edgeq, I.top_vertq, I.d_top_count};
     for (void *p : ptrs)
       if (p) cudaFreeAsync(p, 0);
@@ -2824,12 +3159,11 @@ void mesh_note_frame(MeshState &) {}
 
 cudaError_t prewarm_mesh_kernels() {
   const void *fns[] = {(const void *)k_gen_levels,         (const void *)k_cell_keys,
-                       (const void *)k_gather_cells,       (const void *)k_mesh_lattice<false>,
-                       (const void *)k_mesh_lattice<true>, (const void *)k_mesh_corner<false>,
-                       (const void *)k_mesh_corner<true>,  (const void *)k_mark_dirty,
-                       (const void *)k_count_tile_sums,    (const void *)k_copy_clean,
+                       (const void *)k_gather_cells,       (const void *)k_mesh_count,
+                       (const void *)k_mesh_emit,          (const void *)k_mark_all,
+                       (const void *)k_mark_dirty,         (const void *)k_count_tile_sums,
                        (const void *)k_count_tile_scan,    (const void *)k_count_tile_apply,
-                       (const void *)k_fill_counts_from_old, (const void *)k_export_cells,
+                       (const void *)k_export_cells,
                        (const void *)k_keep_cells,         (const void *)k_keep_tile_scan,
                        (const void *)k_keep_apply,         (const void *)k_merge_cells,
                        (const void *)k_load_top};
