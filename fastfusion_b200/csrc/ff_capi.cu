@@ -1680,8 +1680,12 @@ static ff_status ensure_seq(ff_handle *h, int W, int H, int frames) {
 // and leaf base, or halts it), one read-back of every frame's counters, and
 // the host's bookkeeping frame by frame.  done: frames finished (a frame
 // halted by an earlier one that grew the volume is not; the caller runs it
-// again).
-static ff_status sequence_chunk(ff_handle *h, int c, const uint16_t *const *d_depth, const uint8_t *const *d_bgr,
+// again).  after_pass: an update pass may have been launched since the map's
+// stream was last ordered after one; it takes the marks of its frames away as it
+// goes, so this chunk's first marks wait for it (the de-duplication and the first
+// insert overlap it).
+static ff_status sequence_chunk(ff_handle *h, bool after_pass, int c, const uint16_t *const *d_depth,
+                                const uint8_t *const *d_bgr,
                                 int W, int H, const double *K, const double *R, const double *t, float scaling,
                                 float maxcam, int32_t *queued, int &done) {
   done = 0;
@@ -1726,8 +1730,10 @@ static ff_status sequence_chunk(ff_handle *h, int c, const uint16_t *const *d_de
     launch_insert(h->d_batch, (uint32_t)(h->h_batch->pix_end[k] - (k ? h->h_batch->pix_end[k - 1] : 0u)), s, block,
                   k, k + 1, pdl && k > 0);
     h->prof.end(pi, 0.0, s);
+    const bool wait = after_pass && k == 0;
+    if (wait) CK(cudaStreamWaitEvent(s, h->ev_ring_free, 0));
     pi = h->prof.begin(ST_FINALIZE, s);
-    if (!launch_finalize_small(h->d_batch, 1, (uint32_t)pix, h->cfg.device, s, k, pdl))
+    if (!launch_finalize_small(h->d_batch, 1, (uint32_t)pix, h->cfg.device, s, k, pdl && !wait))
       return set_err(h, FF_ERR_CUDA, "leaf finalisation could not be launched");
     h->prof.end(pi, 0.0, s);
   }
@@ -1798,7 +1804,8 @@ ff_status ff_add_map_sequence_u16_device(ff_handle *h, int n, const uint16_t *co
       if (st != FF_OK) break;
     }
     int done = 0;
-    st = sequence_chunk(h, c, d_depth + i, d_bgr + i, width, height, K + 4 * i, R + 9 * i, t + 3 * i, scaling,
+    // (an earlier chunk of the call may have launched its pass)
+    st = sequence_chunk(h, i > 0, c, d_depth + i, d_bgr + i, width, height, K + 4 * i, R + 9 * i, t + 3 * i, scaling,
                         maxcam, queued ? queued + i : nullptr, done);
     i += done;
   }
