@@ -91,8 +91,8 @@ STAGE_KERNELS = {
 # stage -> the algorithmic bytes its roofline counts (per launch)
 STAGE_BYTES = {
     "grow": "octree and leaf positions read and written",
-    "dedupe": "W*H*2 B: the depth image read (voxel keys and flags it writes stay in L2)",
-    "insert": "16 B per octree level probed per processed pixel (counted on the device)",
+    "dedupe": "W*H*2 B: the depth image read (the list of cells it writes stays in L2)",
+    "insert": "16 B per octree level probed per listed cell (counted on the device)",
     "finalize": "8 B per new brick",
     "fuse": "14,336 B per queued brick per frame (512 voxels x (4 SDF + 4 weight + 6 colour) B, read and written; "
             "10,240 B with FP16 storage)",

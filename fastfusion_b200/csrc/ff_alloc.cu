@@ -111,22 +111,25 @@ __device__ __forceinline__ int4 project_point(float d, float px, float py, const
 // key k = v & -8 differs from s(x,y-1) and from s(x-1,y), where
 // s = k if processed and -1 otherwise (traversal_wrapper_functions.cpp:636-639,
 // 688-690).  This is a recurrence over the two predecessors only, so it has a
-// unique solution.  Each warp solves one 32x32 tile exactly, given the state
-// of the column to its left and the row above it, rows top to bottom.  The
-// key comparisons never change, so they are made once, as bit masks: per lane
-// valid(r), up(r) = k(x,r)==k(x,r-1), left(r) = k(x,r)==k(x-1,r).  In a row,
-// a(x) = valid && !(p(x,r-1) && up) and p(x) = a(x) && !(p(x-1) && left(x)):
-// p copies a(x) at a lane that is not chained to its left neighbour
-// (a(x)==0 or left(x)==0) and alternates along a chain, so one ballot of the
-// chained lanes and one of the chain starts give the row.  Tiles exchange
-// boundary bits and repeat until no boundary changes; a chain of dependencies
-// crosses at most tilesX+tilesY tiles, which bounds the number of rounds.
+// unique solution.  Each warp solves one tile, 32 pixels wide, exactly, given
+// the state of the column to its left and the row above it.  The key
+// comparisons never change, so they are made once, as a word per row (bit:
+// column): valid V, U = k(x,r)==k(x,r-1), L = k(x,r)==k(x-1,r).  A row is then a
+// dozen word operations: a = V & ~(p(r-1) & U), and p(x) = a(x) && !(p(x-1) &&
+// L(x)).  p(x) = a(x) where x is not chained to its left neighbour (a & L == 0)
+// and alternates along a chain, so p is known from the parity of each chain's
+// start, carried along the chain by an addition (solve_row).  Tiles exchange
+// their right columns' and bottom rows' p and repeat until none changes; a chain
+// of dependencies crosses at most tilesX+tilesY tiles, which bounds the number
+// of rounds.
 
 __device__ __forceinline__ void grid_barrier(uint32_t *bar, uint32_t nblocks, Counters *cnt, uint32_t limit) {
   grid_barrier_bounded(bar, nblocks, &cnt->error, ERR_DEDUPE_TIMEOUT, limit);
 }
 
-constexpr int DD_WARPS = 4;  // tiles (warps) per block
+constexpr int DD_WARPS = 8;  // tiles (warps) per block
+// warps that share one launch, per SM (the launch bounds below keep them resident)
+constexpr int DD_BLOCKS_PER_SM = 3;
 // tile height: 16 rows (more, shorter tiles shorten each warp's chain of
 // rows), or 32 when the image has more 16-row tiles than resident warps
 constexpr int DD_ROWS_SHORT = 16, DD_ROWS_TALL = 32;
@@ -136,41 +139,208 @@ __device__ __forceinline__ bool same3(int a0, int a1, int a2, int b0, int b1, in
   return a0 == b0 && a1 == b1 && a2 == b2;
 }
 
-// Tiles are 32 pixels wide and DD_ROWS high.  bnd layout: right-column keys
-// [ntiles][32] int4 (DD_ROWS used), bottom-row keys [ntiles][32]
-// int4 (written once, before the first barrier), then processed bits of the
-// right column and of the bottom row, [2 rounds][ntiles] uint32 each.
+// p of a row from a and the chained positions c (c & ~a == 0, bit 0 not in c).
+// A chain's p is 1 at every second position from its start, the first one where
+// a(start) is 1, the next where it is 0: even positions for starts in q, odd
+// ones for the others.  The addition of the lowest chained position above a start
+// in q carries through that chain, and clears it.
+__device__ __forceinline__ uint32_t solve_row(uint32_t a, uint32_t c) {
+  constexpr uint32_t EVEN = 0x55555555u;
+  const uint32_t q = ~c & ~(a ^ EVEN);
+  const uint32_t e = q | (c & ~(c + ((q << 1) & c)));
+  return ~(e ^ EVEN);
+}
+
+// The cells the processed pixels ask for.  A descent of the octree ends at the
+// cell of edge h that holds the pixel's voxel (h: the smallest power of two
+// not below the pixel's target, at most half the volume), and pixels of the
+// same cell make the same descent: only the cell's first pixel matters to its
+// leaf's index, and half the pixels of a surface are processed, some hundred
+// per cell.  So each tile lists its cells, with the first pixel that asked, for
+// the insert to look up.  A cell may be listed more than once (its pixels in two
+// tiles, or a hash slot taken over): the insert keeps the smallest pixel.
+constexpr int CELL_TAB = 64;
+template <int DD_ROWS>
+struct TileScratch {
+  uint16_t depth[DD_ROWS][32];
+  uint16_t item[DD_ROWS * 32];       // pixels to look at: 32 row + column
+  unsigned long long tab[CELL_TAB];  // cells listed, by hash; a later one of the same slot takes it over
+};
+
+// Lane r's word of row r's processed pixels, less those that share a cell with
+// an earlier processed pixel two steps away: same-cell steps to the left (SL)
+// and up (SU), in the tile.  Processed pixels of a cell are two steps apart (a
+// neighbour of the same cell is not processed), so about one per cell is left.
+__device__ __forceinline__ uint32_t first_of_cells(uint32_t P, uint32_t SL, uint32_t SU, int lane) {
+  const uint32_t full = 0xffffffffu;
+  uint32_t P1 = __shfl_up_sync(full, P, 1), SL1 = __shfl_up_sync(full, SL, 1), SU1 = __shfl_up_sync(full, SU, 1);
+  uint32_t P2 = __shfl_up_sync(full, P, 2);
+  if (lane < 1) P1 = SL1 = SU1 = 0;
+  if (lane < 2) P2 = 0;
+  const uint32_t ll = SL & (SL << 1) & (P << 2), lu = SL & (SU << 1) & (P1 << 1);
+  const uint32_t uu = SU & SU1 & P2, ul = SU & SL1 & (P1 << 1), ur = SU & (SL1 >> 1) & (P1 >> 1);
+  return P & ~(ll | lu | uu | ul | ur);
+}
+
+// List the cells of a tile's pixels in `word` (lane r: row r), rows top to bottom
+// and columns left to right.  True if any of the pixels lies within a brick of
+// where the frame's bounding box leaves the volume.
+template <int DD_ROWS>
+__device__ __forceinline__ bool list_cells(const MapFrame &F, TileScratch<DD_ROWS> &T, int x0, int y0, uint32_t word,
+                                           float px, float py_lane) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t full = 0xffffffffu;
+  uint32_t at = (uint32_t)__popc(word);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(full, at, o);
+    if (lane >= o) at += t;
+  }
+  const uint32_t total = __shfl_sync(full, at, 31);
+  at -= (uint32_t)__popc(word);
+  for (uint32_t w = word; w; w &= w - 1) T.item[at++] = (uint16_t)(32 * lane + __ffs(w) - 1);
+  for (int k = lane; k < CELL_TAB; k += 32) T.tab[k] = ~0ull;
+  __syncwarp();
+  const CamF cam = F.p;
+  const float scaling = F.scaling, maxcam = F.maxcam;
+  const uint32_t n = F.n;
+  const bool pow2 = (n & (n - 1)) == 0;
+  const int margin = (int)F.bw + 7;
+  bool near_face = false;
+  uint32_t kept = 0;
+  // (two or four groups of pixels at a time were slower: the code runs once or
+  // twice a launch, and what it waits for is its own instructions)
+  for (uint32_t j0 = 0; j0 < total; j0 += 32) {
+    const bool have = j0 + lane < total;
+    const int code = have ? T.item[j0 + lane] : 0;
+    const int r = code >> 5, c = code & 31;
+    const float ix = __shfl_sync(full, px, c), iy = __shfl_sync(full, py_lane, r);
+    const int4 v = project_point((float)T.depth[r][c], ix, iy, cam, scaling, maxcam);
+    near_face |= have && (min(v.x, min(v.y, v.z)) < margin || max(v.x, max(v.y, v.z)) >= (int)n - margin);
+    const uint32_t cx = (uint16_t)v.x, cy = (uint16_t)v.y, cz = (uint16_t)v.z, target = (uint32_t)v.w;
+    bool add = have && v.x >= 0 && cx < n && v.y >= 0 && cy < n && v.z >= 0 && cz < n;
+    // (a volume whose side is no power of two has no such cells: voxel and target name the descent)
+    uint32_t lg = target;
+    int sh = 0;
+    if (pow2) {
+      lg = min(32 - __clz(target - 1), 30 - __clz(n));
+      sh = (int)lg & 31;
+    }
+    const uint32_t k0 = (cx >> sh) | (cy >> sh) << 16, k1 = (cz >> sh) | lg << 16;
+    const unsigned long long key = (unsigned long long)k1 << 32 | k0;
+    const uint32_t slot = ((k0 ^ k1 * 0x85EBCA6Bu) * 0x9E3779B1u) >> 26;
+    add = add && T.tab[slot] != key;
+    // the first pixel of each key not listed yet (few: a shuffle each)
+    unsigned f = 0;
+    for (unsigned m = __ballot_sync(full, add); m;) {
+      const int lead = __ffs(m) - 1;
+      const unsigned long long lead_key = __shfl_sync(full, key, lead);
+      m &= ~__ballot_sync(full, key == lead_key);
+      f |= 1u << lead;
+    }
+    if (!f) continue;
+    if ((f >> lane) & 1u) {
+      T.tab[slot] = key;
+      T.item[kept + __popc(f & ((1u << lane) - 1u))] = (uint16_t)code;  // (at or before this pass's items)
+    }
+    kept += (uint32_t)__popc(f);
+    __syncwarp();
+  }
+  near_face = __any_sync(full, near_face);
+  if (!kept) return near_face;
+  uint32_t base = 0;
+  if (lane == 0) base = atomicAdd(&F.cnt->cands, kept);
+  base = __shfl_sync(full, base, 0);
+  for (uint32_t j0 = 0; j0 < kept; j0 += 32) {
+    const int code = j0 + lane < kept ? T.item[j0 + lane] : 0;
+    const int r = code >> 5, c = code & 31;
+    const float ix = __shfl_sync(full, px, c), iy = __shfl_sync(full, py_lane, r);
+    const int4 v = project_point((float)T.depth[r][c], ix, iy, cam, scaling, maxcam);
+    if (j0 + lane < kept)
+      F.cand[base + j0 + lane] =
+          make_uint4((uint32_t)(uint16_t)v.x | (uint32_t)(uint16_t)v.y << 16,
+                     (uint32_t)(uint16_t)v.z | (uint32_t)v.w << 16, (uint32_t)(y0 + r) * (uint32_t)F.W + (uint32_t)(x0 + c), 0u);
+  }
+  return near_face;
+}
+
+// Same-cell words of a tile whose pixels have several cell sizes: lane r's row's
+// U and L, less the steps between pixels of different sizes.
+template <int DD_ROWS>
+__device__ __forceinline__ void same_size(const TileScratch<DD_ROWS> &T, float scaling, float maxcam, uint32_t &SU,
+                                          uint32_t &SL) {
+  const int lane = threadIdx.x & 31;
+  int above = -1;
+#pragma unroll 2
+  for (int r = 0; r < DD_ROWS; r++) {
+    const int4 v = project_point((float)T.depth[r][lane], 0.0f, 0.0f, CamF(), scaling, maxcam);
+    const int lg = v.w < 0 ? -1 : __clz(v.w - 1);
+    const int left = __shfl_up_sync(0xffffffffu, lg, 1);
+    const uint32_t eu = __ballot_sync(0xffffffffu, lg == above), el = __ballot_sync(0xffffffffu, lg == left);
+    if (lane == r) SU &= eu, SL &= el;
+    above = lg;
+  }
+}
+
+// A tile whose pixels come close to the volume's faces: the frame's bounding
+// box over its processed pixels (lane r's word: row r).
+template <int DD_ROWS>
+__device__ __forceinline__ void tile_box(const MapFrame &F, const TileScratch<DD_ROWS> &T, int rows, uint32_t word,
+                                         float px, float py_lane) {
+  const int lane = threadIdx.x & 31;
+  const int n = (int)F.n, bw = (int)F.bw;
+  int lo[3] = {0, 0, 0}, hi[3] = {n - 1, n - 1, n - 1};
+#pragma unroll 1
+  for (int r = 0; r < rows; r++) {
+    const uint32_t row = __shfl_sync(0xffffffffu, word, r);
+    const float py = __shfl_sync(0xffffffffu, py_lane, r);
+    if (!((row >> lane) & 1u)) continue;
+    const int4 v = project_point((float)T.depth[r][lane], px, py, F.p, F.scaling, F.maxcam);
+    const int vv[3] = {v.x, v.y, v.z};
+#pragma unroll
+    for (int a = 0; a < 3; a++) lo[a] = min(lo[a], vv[a] - bw), hi[a] = max(hi[a], vv[a] + bw);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    const int l = __reduce_min_sync(0xffffffffu, lo[a]), h = __reduce_max_sync(0xffffffffu, hi[a]);
+    if (lane == 0 && l < 0) atomicMin(&F.cnt->box_min[a], l);
+    if (lane == 0 && h >= n) atomicMax(&F.cnt->box_max[a], h);
+  }
+}
+
+// Tiles are 32 pixels wide and DD_ROWS high, a warp each.  bnd: processed bits
+// of the right column and of the bottom row, [2 rounds][ntiles] each.
 // bar: [0] arrivals, [1] generation, [4..6] per-round change counters (rotating)
 // One launch for all frames of a batch: warps are dealt out over the maps'
 // tiles in order; the rounds and their barrier are shared (a map whose tiles
 // have settled recomputes the same bits until every map has).
 // Maps [m0, m1) of the batch (their tiles must all be resident at once).
+//
+// What bounds it: latency -- a few warps per scheduler, three to five rounds
+// with a grid barrier (2 us) each.  A row of a tile used to be solved across the
+// lanes with two ballots and a search for the chain's start (240 ns a row); the
+// word operations take 20 ns and leave the barriers.
 template <int DD_ROWS>
-__device__ __forceinline__ void dedupe_body(const BatchDesc *__restrict__ bd, int m0, int m1, uint32_t *bar) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t base = m0 ? bd->tile_end[m0 - 1] : 0u;
+__device__ __forceinline__ void dedupe_body(const BatchDesc *__restrict__ bd, const TileEnds &ends, int m0, int m1,
+                                            uint32_t *bar) {
+  __shared__ TileScratch<DD_ROWS> scratch[DD_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t base = m0 ? ends.end[m0 - 1] : 0u;
   const uint32_t gtile = base + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   int m = m0;
-  while (m < m1 - 1 && gtile >= bd->tile_end[m]) m++;
+  while (m < m1 - 1 && gtile >= ends.end[m]) m++;
+  const bool active = gtile < ends.end[m1 - 1];  // (the others only join the barriers)
   const MapFrame &F = bd->f[m];
-  const int tile = (int)(gtile - (m ? bd->tile_end[m - 1] : 0u));
-  const bool active = gtile < bd->tile_end[m1 - 1];  // warps past the last tile only join the barriers
+  const int tile = (int)(gtile - (m ? ends.end[m - 1] : 0u));
   const uint16_t *__restrict__ depth = F.depth;
-  const float *__restrict__ pxp = F.pxp;
-  const float *__restrict__ pyp = F.pyp;
   const CamF cam = F.p;
   const float scaling = F.scaling, maxcam = F.maxcam;
-  int4 *vox = F.vox;
   const int W = F.W, H = F.H, tilesX = F.tilesX, tilesY = F.tilesY;
-  int4 *bnd = F.bnd;
-  uint8_t *processed = F.proc;
-  Counters *cnt = F.cnt;
   const int ntiles = tilesX * tilesY;
-  int4 *keyR = bnd, *keyB = bnd + (size_t)ntiles * 32;
-  uint32_t *pR = reinterpret_cast<uint32_t *>(bnd + (size_t)2 * ntiles * 32);
-  uint32_t *pB = pR + 2 * (size_t)ntiles;
+  uint32_t *pR = F.bnd, *pB = pR + 2 * (size_t)ntiles;
   const int tx = active ? tile % tilesX : 0, ty = active ? tile / tilesX : 0;
-  const int x = tx * 32 + lane;
+  const int x0 = tx * 32, y0 = ty * DD_ROWS, x = x0 + lane;
   // each map's counters for this frame (read from the first barrier on)
   if (blockIdx.x == 0 && (int)threadIdx.x < m1 - m0) {
     const MapFrame &G = bd->f[m0 + threadIdx.x];
@@ -187,49 +357,59 @@ __device__ __forceinline__ void dedupe_body(const BatchDesc *__restrict__ bd, in
       c->box_max[r] = (int)G.n - 1;
     }
   }
-  const int rows = active ? min(DD_ROWS, H - ty * DD_ROWS) : 0;
-  // project the tile (voxel keys for the insert that follows) and make the
-  // key comparisons; the tile's depth and row factors are fetched first so
-  // the loads overlap
-  uint16_t dv[DD_ROWS];
+  const int rows = active ? min(DD_ROWS, H - y0) : 0;
+  // Project the tile and make the key comparisons: the tile's depth and the row
+  // above it, and (a lane per row) the column to its left.
   const bool col_ok = active && x < W;
+  const bool row_ok = lane < rows, left_ok = row_ok && tx > 0;
+  const uint16_t *dcol = depth + (size_t)y0 * W + x;
+  TileScratch<DD_ROWS> &T = scratch[warp];
+  uint16_t d_above = 0, d_left = 0;
+  if (col_ok && ty > 0) d_above = __ldg(dcol - W);
+  if (left_ok) d_left = __ldg(&depth[(size_t)(y0 + lane) * W + x0 - 1]);
+  uint16_t dv[DD_ROWS];
 #pragma unroll
-  for (int r = 0; r < DD_ROWS; r++) dv[r] = (col_ok && r < rows) ? __ldg(&depth[(size_t)(ty * DD_ROWS + r) * W + x]) : 0;
-  const float px = col_ok ? __ldg(&pxp[x]) : 0.0f;
-  const float py_lane = (active && lane < rows) ? __ldg(&pyp[ty * DD_ROWS + lane]) : 0.0f;
-  uint32_t valid = 0, up = 0, left = 0;
-  int c0 = 0, c1 = 0, c2 = 0;     // key at (lane 0, row = lane): compared with the left tile
-  int t0 = 0, t1 = 0, t2 = 0;     // key at (lane, row 0): compared with the tile above
-  int u0 = 0, u1 = 0, u2 = 0;     // key of the previous row
+  for (int r = 0; r < DD_ROWS; r++) dv[r] = col_ok && r < rows ? __ldg(dcol + (size_t)r * W) : (uint16_t)0;
+  const float px = col_ok ? __ldg(&F.pxp[x]) : 0.0f;
+  const float px_left = left_ok ? __ldg(&F.pxp[x0 - 1]) : 0.0f;
+  const float py_lane = row_ok ? __ldg(&F.pyp[y0 + lane]) : 0.0f;
+  const float py_above = active && ty > 0 ? __ldg(&F.pyp[y0 - 1]) : 0.0f;
 #pragma unroll
-  for (int r = 0; r < DD_ROWS; r++) {
-    if (r >= rows) break;
-    const int y = ty * DD_ROWS + r;
-    const float py = __shfl_sync(0xffffffffu, py_lane, r);
-    int4 v = make_int4(0, 0, 0, -1);
-    if (x < W) {
-      v = project_point((float)dv[r], px, py, cam, scaling, maxcam);
-      vox[(size_t)y * W + x] = v;
-    }
-    const int k0 = v.x & -8, k1 = v.y & -8, k2 = v.z & -8;
-    const int l0 = __shfl_up_sync(0xffffffffu, k0, 1);
-    const int l1 = __shfl_up_sync(0xffffffffu, k1, 1);
-    const int l2 = __shfl_up_sync(0xffffffffu, k2, 1);
-    const int f0 = __shfl_sync(0xffffffffu, k0, 0);
-    const int f1 = __shfl_sync(0xffffffffu, k1, 0);
-    const int f2 = __shfl_sync(0xffffffffu, k2, 0);
-    if (lane == r) c0 = f0, c1 = f1, c2 = f2;
-    if (r == 0) t0 = k0, t1 = k1, t2 = k2;
-    if (x < W && v.w >= 0) valid |= 1u << r;
-    if (r > 0 && same3(k0, k1, k2, u0, u1, u2)) up |= 1u << r;
-    if (lane > 0 && same3(k0, k1, k2, l0, l1, l2)) left |= 1u << r;
-    u0 = k0, u1 = k1, u2 = k2;
-    if (lane == 31) keyR[(size_t)tile * 32 + r] = make_int4(k0, k1, k2, 0);
-    if (r == rows - 1) keyB[(size_t)tile * 32 + lane] = make_int4(k0, k1, k2, 0);
+  for (int r = 0; r < DD_ROWS; r++) T.depth[r][lane] = dv[r];
+  __syncwarp();
+  const float px_first = __shfl_sync(0xffffffffu, px, 0);
+  // this lane's row: its first pixel has the key of the left tile's last one
+  bool eq_left = false;
+  if (left_ok) {
+    const int4 a = project_point((float)d_left, px_left, py_lane, cam, scaling, maxcam);
+    const int4 b = project_point((float)T.depth[lane][0], px_first, py_lane, cam, scaling, maxcam);
+    eq_left = same3(a.x & -8, a.y & -8, a.z & -8, b.x & -8, b.y & -8, b.z & -8);
   }
-  uint32_t eq_left = 0;  // row bits: lane 0's key equals the left tile's right column
-  bool eq_above = false;  // this lane's row-0 key equals the above tile's bottom row
-  uint32_t bits = 0, last_r = 0, last_b = 0;
+  uint32_t V = 0, U = 0, L = 0;  // the masks of row `lane`
+  int4 u = project_point((float)d_above, px, py_above, cam, scaling, maxcam);  // the row before
+  uint32_t target_min = 0xffffffffu;  // (an invalid pixel's is -1)
+  int target_max = -1;
+#pragma unroll 4
+  for (int r = 0; r < DD_ROWS; r++) {
+    const float py = __shfl_sync(0xffffffffu, py_lane, r);
+    const int4 v = project_point((float)T.depth[r][lane], px, py, cam, scaling, maxcam);  // (invalid past the image: depth 0)
+    const int l0 = __shfl_up_sync(0xffffffffu, v.x, 1);
+    const int l1 = __shfl_up_sync(0xffffffffu, v.y, 1);
+    const int l2 = __shfl_up_sync(0xffffffffu, v.z, 1);
+    const int du = (v.x ^ u.x) | (v.y ^ u.y) | (v.z ^ u.z), dl = (v.x ^ l0) | (v.y ^ l1) | (v.z ^ l2);
+    const uint32_t rv = __ballot_sync(0xffffffffu, v.w >= 0);
+    const uint32_t ru = __ballot_sync(0xffffffffu, (du & -8) == 0);
+    const uint32_t rl = __ballot_sync(0xffffffffu, (dl & -8) == 0) & ~1u;
+    if (lane == r) V = rv, U = ru, L = rl;
+    target_min = min(target_min, (uint32_t)v.w);
+    target_max = max(target_max, v.w);
+    u = v;
+  }
+  // the tile's pixels ask for cells of one size
+  const bool one_size = __clz((int)__reduce_min_sync(0xffffffffu, target_min) - 1) ==
+                        __clz(__reduce_max_sync(0xffffffffu, target_max) - 1);
+  uint32_t word = 0;  // the processed pixels of row `lane`
+  uint32_t last_r = 0, last_b = 0, last_left = 0, last_above = 0;
   const int max_rounds = bd->max_rounds;
   volatile uint32_t *chg = bar + 4;
   int round = 0;
@@ -240,43 +420,31 @@ __device__ __forceinline__ void dedupe_body(const BatchDesc *__restrict__ bd, in
     if (active) {
       uint32_t left_p = 0, above_p = 0;
       if (round > 0) {
-        if (round == 1) {
-          // boundary keys were published before the first barrier
-          bool eq = false;
-          if (tx > 0 && lane < rows) {
-            const int4 k = keyR[(size_t)(tile - 1) * 32 + lane];
-            eq = same3(k.x, k.y, k.z, c0, c1, c2);
-          }
-          eq_left = __ballot_sync(0xffffffffu, eq);
-          if (ty > 0) {
-            const int4 k = keyB[(size_t)(tile - tilesX) * 32 + lane];
-            eq_above = same3(k.x, k.y, k.z, t0, t1, t2);
-          }
+        if (tx > 0) left_p = __ldcg(&pR[(size_t)in * ntiles + tile - 1]);
+        if (ty > 0) above_p = __ldcg(&pB[(size_t)in * ntiles + tile - tilesX]);
+      }
+      if (round == 0 || left_p != last_left || above_p != last_above) {
+        const uint32_t vl = V & ~((left_p >> lane) & (uint32_t)eq_left);  // (chained to a processed pixel of the left tile)
+        uint32_t p = above_p, rb = 0, bb = 0;
+#pragma unroll 8
+        for (int r = 0; r < DD_ROWS; r++) {
+          const uint32_t rv = __shfl_sync(0xffffffffu, vl, r), ru = __shfl_sync(0xffffffffu, U, r),
+                         rl = __shfl_sync(0xffffffffu, L, r);
+          const uint32_t a = rv & ~(p & ru);
+          p = solve_row(a, a & rl);
+          rb |= (p >> 31) << r;
+          if (r == rows - 1) bb = p;
+          if (lane == r) word = p;
         }
-        if (tx > 0) left_p = pR[(size_t)in * ntiles + tile - 1];
-        if (ty > 0) above_p = pB[(size_t)in * ntiles + tile - tilesX];
+        changed = round == 0 || rb != last_r || bb != last_b;
+        last_r = rb;
+        last_b = bb;
+        last_left = left_p;
+        last_above = above_p;
       }
-      const uint32_t below = (2u << lane) - 1u;  // lanes 0..lane
-      int ap = (int)((above_p >> lane) & 1u) & (int)eq_above;  // p above, where its key matches
-      bits = 0;
-      for (int r = 0; r < rows; r++) {
-        const int a = ((valid >> r) & 1u) && !(ap && (r == 0 || ((up >> r) & 1u)));
-        const int start_p = lane == 0 ? (a && !(((left_p & eq_left) >> r) & 1u)) : a;
-        const uint32_t chained = __ballot_sync(0xffffffffu, lane > 0 && a && ((left >> r) & 1u));
-        const uint32_t start_bits = __ballot_sync(0xffffffffu, start_p);
-        const int st = 31 - __clz(~chained & below);
-        const int p = (int)((start_bits >> st) & 1u) ^ ((lane - st) & 1);
-        bits |= (uint32_t)p << r;
-        ap = p;
-      }
-      const uint32_t rb = __shfl_sync(0xffffffffu, bits, 31);
-      const uint32_t bb = __ballot_sync(0xffffffffu, (bits >> (rows - 1)) & 1u);
-      changed = round == 0 || rb != last_r || bb != last_b;
-      last_r = rb;
-      last_b = bb;
       if (lane == 0) {
-        pR[(size_t)out * ntiles + tile] = rb;
-        pB[(size_t)out * ntiles + tile] = bb;
+        pR[(size_t)out * ntiles + tile] = last_r;
+        pB[(size_t)out * ntiles + tile] = last_b;
       }
     }
     if (changed && lane == 0) atomicAdd((uint32_t *)&chg[round % 3], 1u);
@@ -297,15 +465,19 @@ __device__ __forceinline__ void dedupe_body(const BatchDesc *__restrict__ bd, in
   // (round + 2) % 3 was last read before this round's barrier (after a
   // barrier that gave up or no convergence, the host clears the words)
   if (converged && blockIdx.x == 0 && threadIdx.x == 0) chg[(round + 2) % 3] = 0;
-  uint32_t nproc = 0;
-  if (active && x < W) {
-    for (int r = 0; r < rows; r++) processed[(size_t)(ty * DD_ROWS + r) * W + x] = (uint8_t)((bits >> r) & 1u);
-    nproc = (uint32_t)__popc(rows >= 32 ? bits : (bits & ((1u << rows) - 1u)));
-  }
-  // the frame's processed pixels, counted once per tile (the insert that
-  // follows no longer adds them per warp on the counters' cache line)
-  nproc = __reduce_add_sync(0xffffffffu, nproc);
+  // the frame's processed pixels, counted once per tile
+  const uint32_t nproc = __reduce_add_sync(0xffffffffu, active ? (uint32_t)__popc(word) : 0u);
   if (active && lane == 0 && nproc) atomicAdd(&F.cnt->processed, nproc);
+  if (active && converged && nproc) {
+    uint32_t look = word;
+    if ((F.n & (F.n - 1)) == 0) {  // (else there are no cells, see list_cells)
+      uint32_t SU = U, SL = L;
+      if (!one_size) same_size(T, scaling, maxcam, SU, SL);
+      look = first_of_cells(word, SL, SU, lane);
+    }
+    const bool near_face = list_cells(F, T, x0, y0, look, px, py_lane);
+    if (near_face) tile_box(F, T, rows, word, px, py_lane);
+  }
   if (blockIdx.x == 0 && (int)threadIdx.x < m1 - m0) {
     Counters *c = bd->f[m0 + threadIdx.x].cnt;
     c->dedupe_iters = round + 1;
@@ -315,24 +487,23 @@ __device__ __forceinline__ void dedupe_body(const BatchDesc *__restrict__ bd, in
 }
 
 template <int DD_ROWS>
-// (register budget for 6 blocks per SM: a 10-frame sequence of 640x480
-// frames fits one cooperative launch)
-__global__ void __launch_bounds__(32 * DD_WARPS, 6) k_dedupe(const BatchDesc *__restrict__ bd, int m0, int m1,
-                                                          uint32_t *bar) {
-  dedupe_body<DD_ROWS>(bd, m0, m1, bar);
+// (a 10-frame sequence of 640x480 frames fits one cooperative launch)
+__global__ void __launch_bounds__(32 * DD_WARPS, DD_BLOCKS_PER_SM) k_dedupe(
+    const BatchDesc *__restrict__ bd, const __grid_constant__ TileEnds ends, int m0, int m1, uint32_t *bar) {
+  dedupe_body<DD_ROWS>(bd, ends, m0, m1, bar);
 }
 
 // One map's frame, its descriptor a launch parameter: block 0 also stores it
 // to `out`, where the frame's later kernels read it.
 template <int DD_ROWS>
-__global__ void __launch_bounds__(32 * DD_WARPS) k_dedupe_one(const __grid_constant__ BatchDesc1 desc,
+__global__ void __launch_bounds__(32 * DD_WARPS, DD_BLOCKS_PER_SM) k_dedupe_one(const __grid_constant__ BatchDesc1 desc,
                                                               BatchDesc *out, uint32_t *bar) {
   if (blockIdx.x == 0) {
     const uint2 *src = reinterpret_cast<const uint2 *>(&desc);
     uint2 *dst = reinterpret_cast<uint2 *>(out);
     for (int k = threadIdx.x; k < (int)(sizeof(BatchDesc1) / 8); k += blockDim.x) dst[k] = src[k];
   }
-  dedupe_body<DD_ROWS>(reinterpret_cast<const BatchDesc *>(&desc), 0, 1, bar);
+  dedupe_body<DD_ROWS>(reinterpret_cast<const BatchDesc *>(&desc), desc.ends, 0, 1, bar);
 }
 
 int dedupe_tiles(int W, int H, int *tilesX, int *tilesY, int rows) {
@@ -344,47 +515,28 @@ int dedupe_tiles(int W, int H, int *tilesX, int *tilesY, int rows) {
 
 size_t dedupe_boundary_elems(int W, int H) {
   // sized for the lowest tiles (the largest count)
-  const size_t ntiles = (size_t)dedupe_tiles(W, H, nullptr, nullptr, DD_ROWS_LOW);
-  return ntiles * 32 * 2 + ntiles;  // keys of the right column and bottom row, then 4 bit words per tile
+  return 4 * (size_t)dedupe_tiles(W, H, nullptr, nullptr, DD_ROWS_LOW);
 }
 
-template <int ROWS>
-static cudaError_t resident_dedupe_warps(int device, int &warps) {
-  static int resident[64] = {};
-  const int dslot = device & 63;
-  if (!resident[dslot]) {
-    int per_sm = 0, per_sm_one = 0, sms = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dedupe<ROWS>, 32 * DD_WARPS, 0);
-    if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_one, k_dedupe_one<ROWS>, 32 * DD_WARPS, 0);
-    if (e != cudaSuccess) return e;
-    per_sm = std::min(per_sm, per_sm_one);  // (both launch forms use one capacity)
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e != cudaSuccess) return e;
-    resident[dslot] = per_sm * sms;
-  }
-  warps = resident[dslot] * DD_WARPS;
-  return cudaSuccess;
-}
-
-cudaError_t dedupe_capacity(int device, int rows, uint32_t &tiles) {
-  int warps = 0;
-  cudaError_t e = rows == DD_ROWS_SHORT  ? resident_dedupe_warps<DD_ROWS_SHORT>(device, warps)
-                  : rows == DD_ROWS_LOW ? resident_dedupe_warps<DD_ROWS_LOW>(device, warps)
-                                        : resident_dedupe_warps<DD_ROWS_TALL>(device, warps);
-  tiles = (uint32_t)warps;
+// Tiles that one launch takes (and so the largest image): the warps that the
+// launch bounds keep resident.
+cudaError_t dedupe_capacity(int device, uint32_t &tiles) {
+  int sms = 0;
+  const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  tiles = (uint32_t)(sms * DD_BLOCKS_PER_SM * DD_WARPS);
   return e;
 }
 
-cudaError_t launch_dedupe(const BatchDesc *d_batch, int m0, int m1, uint32_t tiles, int rows, uint32_t *barrier,
+cudaError_t launch_dedupe(const BatchDesc *h_batch, const BatchDesc *d_batch, int m0, int m1, uint32_t tiles, int rows, uint32_t *barrier,
                           int device, cudaStream_t s) {
   uint32_t cap = 0;
-  cudaError_t e = dedupe_capacity(device, rows, cap);
+  cudaError_t e = dedupe_capacity(device, cap);
   if (e != cudaSuccess) return e;
   // one warp per tile, all resident at once
   const int blocks = (int)((tiles + DD_WARPS - 1) / DD_WARPS);
   if ((uint32_t)blocks * DD_WARPS > cap || blocks < 1) return cudaErrorInvalidConfiguration;
-  void *args[] = {(void *)&d_batch, (void *)&m0, (void *)&m1, (void *)&barrier};
+  TileEnds ends = h_batch->ends;
+  void *args[] = {(void *)&d_batch, (void *)&ends, (void *)&m0, (void *)&m1, (void *)&barrier};
   note_launch();
   const void *fn = rows == DD_ROWS_SHORT  ? (const void *)k_dedupe<DD_ROWS_SHORT>
                    : rows == DD_ROWS_LOW ? (const void *)k_dedupe<DD_ROWS_LOW>
@@ -395,7 +547,7 @@ cudaError_t launch_dedupe(const BatchDesc *d_batch, int m0, int m1, uint32_t til
 cudaError_t launch_dedupe_one(const BatchDesc *h_desc, BatchDesc *d_batch, uint32_t tiles, int rows,
                               uint32_t *barrier, int device, cudaStream_t s) {
   uint32_t cap = 0;
-  cudaError_t e = dedupe_capacity(device, rows, cap);
+  cudaError_t e = dedupe_capacity(device, cap);
   if (e != cudaSuccess) return e;
   const int blocks = (int)((tiles + DD_WARPS - 1) / DD_WARPS);
   if ((uint32_t)blocks * DD_WARPS > cap || blocks < 1 || h_desc->n != 1) return cudaErrorInvalidConfiguration;
@@ -455,32 +607,22 @@ __device__ __forceinline__ uint32_t wait_unlocked(uint32_t *tree, uint32_t ptr, 
 // side (16 bits of voxel coordinates) plus the root.
 constexpr int DESCENT_MAX = 18;
 
-// One processed pixel of the frame F (voxel key v): bounding-box growth,
-// then (inside the volume) the descent of queryPointDepthSingle_func_subtree:
-// queue the existing coarser leaves on the path, allocate missing branches,
-// claim the final leaf.  Returns the number of octree levels probed; sets
-// *created when this pixel wrote a new branch or leaf slot into the octree,
-// and records the branches it passed (root first) in path[0, *npath).
-__device__ __forceinline__ uint32_t insert_descend(const MapFrame &F, int i, int4 v, Counters *cnt, bool *created,
-                                                   uint32_t *path, int *npath) {
+// One cell of the frame F's list (a voxel v in it, the target, its first pixel
+// i): the descent of queryPointDepthSingle_func_subtree: queue the existing
+// coarser leaves on the path, allocate missing branches, claim the final leaf.
+// Returns the number of octree levels probed; sets *created when it wrote a
+// new branch or leaf slot into the octree, and records the branches it passed
+// (root first) in path[0, *npath).
+__device__ __forceinline__ uint32_t insert_descend(const MapFrame &F, uint32_t i, uint32_t x, uint32_t y, uint32_t z,
+                                                   uint32_t target, Counters *cnt, bool *created, uint32_t *path,
+                                                   int *npath) {
   const uint32_t n = F.n;
-  const int bw = (int)F.bw;
   uint32_t *tree = F.tree;
   const uint32_t leaves_max = F.leaves_max, branches_max = F.branches_max, frame = F.frame;
   uint32_t *stamp = F.stamp, *queue = F.queue;
   PendingLeaf *pend = F.pend;
   const uint32_t pend_cap = F.pend_cap;
   uint32_t probed = 0;
-  int vv[3] = {v.x, v.y, v.z};
-#pragma unroll
-  for (int r = 0; r < 3; r++) {
-    int lo = vv[r] - bw, hi = vv[r] + bw;
-    if (lo < 0) atomicMin(&cnt->box_min[r], lo);
-    if (hi >= (int)n) atomicMax(&cnt->box_max[r], hi);
-  }
-  if (!(v.x >= 0 && (uint16_t)v.x < n && v.y >= 0 && (uint16_t)v.y < n && v.z >= 0 && (uint16_t)v.z < n)) return 0;
-  const uint32_t x = (uint16_t)v.x, y = (uint16_t)v.y, z = (uint16_t)v.z;
-  const uint32_t target = (uint32_t)v.w;
   uint32_t ox = 0, oy = 0, oz = 0;
   uint32_t half = (uint16_t)(n >> 1);
   uint32_t branch = 0;
@@ -548,7 +690,7 @@ __device__ __forceinline__ uint32_t insert_descend(const MapFrame &F, int i, int
       }
       PendingLeaf pl;
       pl.slot = ptr;
-      pl.first_pixel = (uint32_t)i;
+      pl.first_pixel = i;
       pl.pos = make_ushort4((uint16_t)(ox + half * ((co & 1) != 0)), (uint16_t)(oy + half * ((co & 2) != 0)),
                             (uint16_t)(oz + half * ((co & 4) != 0)), (uint16_t)(half / BL));
       pend[rec] = pl;
@@ -563,7 +705,7 @@ __device__ __forceinline__ uint32_t insert_descend(const MapFrame &F, int i, int
   cur = wait_unlocked(tree, ptr, cur, cnt, &ok, F.spin_limit);
   if (!ok) return probed;
   if (cur >= PENDING && cur < PENDING + pend_cap) {
-    atomicMin(&pend[cur - PENDING].first_pixel, (uint32_t)i);
+    atomicMin(&pend[cur - PENDING].first_pixel, i);
   } else if (cur < leaves_max) {
     queue_leaf(cur, frame, stamp, queue, cnt);
   }
@@ -571,9 +713,9 @@ __device__ __forceinline__ uint32_t insert_descend(const MapFrame &F, int i, int
 }
 
 // Mark every branch on the descent's path (root first, down to the branch
-// that holds the pixel's slot, or to the last one reached when the descent
+// that holds the cell's slot, or to the last one reached when the descent
 // stopped early) with the frame: the branches whose subtree gained a branch
-// or a leaf.  Only pixels that created something do it; the loads of the
+// or a leaf.  Only cells that created something do it; the loads of the
 // stamps are independent, so they overlap.
 __device__ __forceinline__ void stamp_path(const MapFrame &F, const uint32_t *path, int np) {
   for (int k = 0; k < np; k++) {
@@ -582,54 +724,53 @@ __device__ __forceinline__ void stamp_path(const MapFrame &F, const uint32_t *pa
   }
 }
 
-__device__ __forceinline__ uint32_t insert_pixel(const MapFrame &F, int i, int4 v, Counters *cnt) {
-  bool created = false;
-  uint32_t path[DESCENT_MAX];
-  int np = 0;
-  const uint32_t probed = insert_descend(F, i, v, cnt, &created, path, &np);
-  if (created) stamp_path(F, path, np);
-  return probed;
-}
-
-// One thread per pixel of every frame of the batch (each map's pixels padded
-// to whole warps, so a warp never spans two maps).  At most 40 registers: six
+// The cells the frames' de-duplication listed: blocks over x stride over a
+// frame's list, y is the frame of the batch.  Bound by the latency of a descent
+// (some eight dependent octree reads): a thread per processed pixel, 140,000 of
+// a 640x480 frame where the list has 3,000 to 4,000 cells, took 27.6 us with its
+// launch and 80.9 us at 1280x960; the list takes 12.4 and 12.7 us.  At most 40 registers: six
 // 256-thread blocks per SM instead of five (a few bytes of spill), for any
 // block size the tuning picks.
-__global__ void __maxnreg__(40) k_insert(const BatchDesc *__restrict__ bd, int m0, int m1) {
+__global__ void __maxnreg__(40) k_insert(const BatchDesc *__restrict__ bd, int m0) {
   pdl_enter();
-  const int nmaps = min(bd->n, m1);
-  const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x + (m0 ? bd->pix_end[m0 - 1] : 0u);
-  if (g >= bd->pix_end[nmaps - 1]) return;
-  int mi = m0;
-  while (mi < nmaps - 1 && g >= bd->pix_end[mi]) mi++;
-  const MapFrame &F = bd->f[mi];
-  const int i = (int)(g - (mi ? bd->pix_end[mi - 1] : 0u));
-  const int npix = (int)F.npix;
-  const int4 *__restrict__ vox = F.vox;
-  const uint8_t *__restrict__ processed = F.proc;
+  const MapFrame &F = bd->f[m0 + blockIdx.y];
   Counters *cnt = F.cnt;
   // a de-duplication that did not complete leaves the frame out, and so does
   // a sequence halted by an earlier frame: the octree is not touched
   if (ld_volatile(&cnt->error) & (ERR_DEDUPE_FAILED | ERR_SEQ_HALT)) return;
-  bool act = i < npix && processed[i];
-  unsigned m = __ballot_sync(0xffffffffu, act);
-  if (!act) return;
-  // octree levels this pixel probes on its descent, summed per warp when the
-  // stage profile is on (the algorithmic bytes of the insert: 16 B per level
-  // -- the node's leaf and child slots, the leaf's frame stamp and its queue
-  // entry, 4 B each)
-  const uint32_t levels = insert_pixel(F, i, vox[i], cnt);
-  if (F.count_levels) {
-    const uint32_t sum = __reduce_add_sync(m, levels);
-    if ((threadIdx.x & 31) == __ffs(m) - 1) atomicAdd(&cnt->levels, sum);
+  const uint32_t cands = ld_volatile(&cnt->cands);
+  const int lane = threadIdx.x & 31;
+  for (uint32_t j0 = blockIdx.x * blockDim.x + threadIdx.x - lane; j0 < cands; j0 += gridDim.x * blockDim.x) {
+    uint32_t levels = 0;
+    if (j0 + lane < cands) {
+      const uint4 c = F.cand[j0 + lane];
+      bool created = false;
+      uint32_t path[DESCENT_MAX];
+      int np = 0;
+      levels = insert_descend(F, c.z, c.x & 0xFFFFu, c.x >> 16, c.y & 0xFFFFu, c.y >> 16, cnt, &created, path, &np);
+      if (created) stamp_path(F, path, np);
+    }
+    __syncwarp();
+    // octree levels probed, when the stage profile is on (the algorithmic
+    // bytes of the insert: 16 B per level -- the node's leaf and child slots,
+    // the leaf's frame stamp and its queue entry, 4 B each)
+    if (F.count_levels) {
+      levels = __reduce_add_sync(0xffffffffu, levels);
+      if (lane == 0) atomicAdd(&cnt->levels, levels);
+    }
   }
 }
 
-void launch_insert(const BatchDesc *d_batch, uint32_t pix, cudaStream_t s, int block, int m0, int m1, bool pdl) {
-  if (!pix) return;
+// Enough blocks for a list as long as the image (every pixel its own cell),
+// but no more than are resident at once.
+void launch_insert(const BatchDesc *d_batch, uint32_t npix, int sm_count, cudaStream_t s, int block, int m0, int nmaps,
+                   bool pdl) {
+  if (!npix || nmaps < 1) return;
   if (block < 64 || block > 1024 || block % 32) block = 256;
+  const int resident = std::max(1, 1536 / block) * sm_count;
+  const int blocks = std::max(1, std::min((int)((npix + block - 1) / block), resident / nmaps));
   note_launch();
-  launch_pdl(pdl, k_insert, dim3((pix + block - 1) / block), dim3(block), 0, s, d_batch, m0, m1);
+  launch_pdl(pdl, k_insert, dim3(blocks, nmaps), dim3(block), 0, s, d_batch, m0);
 }
 
 // ------------------------------------------------- pending leaf order -----

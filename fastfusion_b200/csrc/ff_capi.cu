@@ -114,9 +114,8 @@ struct ff_handle {
   uint16_t *d_depth = nullptr;
   uint8_t *d_bgr = nullptr;
   float *d_pxp = nullptr, *d_pyp = nullptr;
-  int4 *d_vox = nullptr;
-  uint8_t *d_proc = nullptr;
-  int4 *d_bnd = nullptr;
+  uint4 *d_cand = nullptr;
+  uint32_t *d_bnd = nullptr;
   size_t bnd_elems = 0;
   PendingLeaf *d_pend = nullptr;
   // 6 x cap_pix words: pending-leaf sort keys (u64), sorted keys (u64), order; finalisation ranks
@@ -188,9 +187,8 @@ struct ff_handle {
   // counters (device, and a pinned mirror)
   int seq_frames = 0;
   size_t seq_pix = 0, seq_bnd = 0;
-  int4 *d_seq_vox = nullptr;
-  uint8_t *d_seq_proc = nullptr;
-  int4 *d_seq_bnd = nullptr;
+  uint4 *d_seq_cand = nullptr;
+  uint32_t *d_seq_bnd = nullptr;
   Counters *d_seq_cnt = nullptr, *h_seq_cnt = nullptr;
   int pi_insert = -1;  // profile record of the last insert launch this map led
 
@@ -468,8 +466,7 @@ static ff_status ensure_image(ff_handle *h, int W, int H) {
       h->d_depth_set[k] = nullptr;
       h->d_bgr_set[k] = nullptr;
     }
-    cudaFree(h->d_vox);
-    cudaFree(h->d_proc);
+    cudaFree(h->d_cand);
     cudaFree(h->d_pend);
     cudaFree(h->d_keys);
     cudaFree(h->d_sort_tmp);
@@ -478,8 +475,7 @@ static ff_status ensure_image(ff_handle *h, int W, int H) {
       CK(alloc(&h->d_bgr_set[k], (size_t)npix * 3));
     }
     select_set(h, h->set);
-    CK(alloc(&h->d_vox, npix));
-    CK(alloc(&h->d_proc, npix));
+    CK(alloc(&h->d_cand, npix));
     CK(alloc(&h->d_pend, npix));
     CK(alloc(&h->d_keys, (size_t)npix * 6));
     h->sort_tmp_bytes = pending_sort_bytes(npix);
@@ -724,10 +720,10 @@ ff_status ff_destroy(ff_handle *h) {
   void *ptrs[] = {h->d_tree, h->d_leaf, h->d_parent, h->d_sdf, h->d_wgt, h->d_sdf16, h->d_wgt16, h->d_col,
                   h->d_stamp, h->d_bstamp, h->d_queue_set[0], h->d_queue_set[1], h->d_cnt_set[0], h->d_cnt_set[1],
                   h->d_barrier, h->d_depth_set[0], h->d_depth_set[1], h->d_bgr_set[0], h->d_bgr_set[1], h->d_pxp,
-                  h->d_pyp, h->d_vox, h->d_proc, h->d_bnd, h->d_pend, h->d_keys, h->d_sort_tmp, h->d_rcp_tab,
+                  h->d_pyp, h->d_cand, h->d_bnd, h->d_pend, h->d_keys, h->d_sort_tmp, h->d_rcp_tab,
                   h->d_cnn_params, h->d_feat, h->d_a1, h->d_a2, h->d_conf_set[0], h->d_conf_set[1],
                   h->d_batch_set[0], h->d_batch_set[1], h->d_upd_mask, h->d_upd_list, h->d_upd_count,
-                  h->d_upd_total, h->d_ring_depth, h->d_ring_bgr, h->d_ring_conf, h->d_seq_vox, h->d_seq_proc,
+                  h->d_upd_total, h->d_ring_depth, h->d_ring_bgr, h->d_ring_conf, h->d_seq_cand,
                   h->d_seq_bnd, h->d_seq_cnt, h->d_loop_map, h->d_loop_slots, h->d_loop_st, h->d_loop_sdf,
                   h->d_loop_wgt, h->d_loop_col};
   for (void *p : ptrs)
@@ -1026,7 +1022,6 @@ struct FramePlan {
   bool counters_early = false;
 };
 
-static uint32_t pad32(uint32_t v) { return (v + 31u) & ~31u; }
 
 // Host part before the launches; fills the frame's descriptor.
 // side: a single-map frame whose update runs on fuse_stream; its confidence
@@ -1115,8 +1110,7 @@ static ff_status frame_prepare(ff_handle *h, const uint16_t *d_depth, const uint
   mf.queue = h->d_queue;
   mf.rank = h->d_keys + 5 * h->cap_pix;
   mf.pend = h->d_pend;
-  mf.vox = h->d_vox;
-  mf.proc = h->d_proc;
+  mf.cand = h->d_cand;
   mf.bnd = h->d_bnd;
   mf.cnt = h->d_cnt;
   mf.branches_init = h->branches_used;  // (the counters are set up on the device)
@@ -1195,7 +1189,7 @@ static ff_status frame_prepare(ff_handle *h, const uint16_t *d_depth, const uint
 }
 
 // The launch plan of a batch: tile height, the groups of whole maps that
-// share one cooperative de-duplication launch, padded pixel total.
+// share one cooperative de-duplication launch, pixels of the largest image.
 struct LaunchPlan {
   int rows = 16;
   uint32_t pix = 0;
@@ -1211,18 +1205,15 @@ static ff_status frame_plan(ff_handle *lead, int n, LaunchPlan &lp) {
   B.n = n;
   // 16-row tiles when they fit one cooperative launch, else 32-row tiles in
   // as many launches (groups of whole maps) as needed
-  uint32_t tiles16 = 0, cap16 = 0, cap32 = 0;
+  uint32_t tiles16 = 0, cap = 0;
   for (int i = 0; i < n; i++) tiles16 += (uint32_t)dedupe_tiles(B.f[i].W, B.f[i].H, nullptr, nullptr, 16);
-  CK(dedupe_capacity(lead->cfg.device, 16, cap16));
-  CK(dedupe_capacity(lead->cfg.device, 32, cap32));
-  int rows = tiles16 <= cap16 ? 16 : 32;
-  if (lead->tune.dedupe_rows == 32 || (lead->tune.dedupe_rows == 16 && tiles16 <= cap16)) rows = lead->tune.dedupe_rows;
-  uint32_t cap = rows == 16 ? cap16 : cap32;
+  CK(dedupe_capacity(lead->cfg.device, cap));
+  int rows = tiles16 <= cap ? 16 : 32;
+  if (lead->tune.dedupe_rows == 32 || (lead->tune.dedupe_rows == 16 && tiles16 <= cap)) rows = lead->tune.dedupe_rows;
   if (lead->tune.dedupe_rows == 8) {
-    uint32_t tiles8 = 0, cap8 = 0;
+    uint32_t tiles8 = 0;
     for (int i = 0; i < n; i++) tiles8 += (uint32_t)dedupe_tiles(B.f[i].W, B.f[i].H, nullptr, nullptr, 8);
-    CK(dedupe_capacity(lead->cfg.device, 8, cap8));
-    if (tiles8 <= cap8) rows = 8, cap = cap8;
+    if (tiles8 <= cap) rows = 8;
   }
   for (int i = 0; i < n; i++) {
     const uint32_t nt = (uint32_t)dedupe_tiles(B.f[i].W, B.f[i].H, &B.f[i].tilesX, &B.f[i].tilesY, rows);
@@ -1233,9 +1224,8 @@ static ff_status frame_plan(ff_handle *lead, int n, LaunchPlan &lp) {
   for (int i = 0; i < n; i++) {
     rounds = std::max(rounds, B.f[i].tilesX + B.f[i].tilesY + 1);
     tiles += (uint32_t)(B.f[i].tilesX * B.f[i].tilesY);
-    pix += pad32(B.f[i].npix);
-    B.tile_end[i] = tiles;
-    B.pix_end[i] = pix;
+    pix = std::max(pix, B.f[i].npix);
+    B.ends.end[i] = tiles;
   }
   B.max_rounds = rounds;
   lp.rows = rows;
@@ -1280,7 +1270,7 @@ static ff_status frame_issue(ff_handle *lead, int n, const LaunchPlan &lp, bool 
                          s));
   else
     for (size_t g = 0; g < lp.groups.size(); g++)
-      CK(launch_dedupe(lead->d_batch, (int)lp.groups[g][0], (int)lp.groups[g][1], lp.groups[g][2], lp.rows,
+      CK(launch_dedupe(lead->h_batch, lead->d_batch, (int)lp.groups[g][0], (int)lp.groups[g][1], lp.groups[g][2], lp.rows,
                        lead->d_barrier + 8 * g, lead->cfg.device, s));
   lead->prof.end(pi, lp.npix * 2, s);  // the depth image read (the keys and flags it writes stay in L2)
   if (!insert) {
@@ -1293,7 +1283,8 @@ static ff_status frame_issue(ff_handle *lead, int n, const LaunchPlan &lp, bool 
     lead->fin_pending = false;
   }
   pi = lead->prof.begin(ST_INSERT, s);
-  launch_insert(lead->d_batch, lp.pix, s, lead->tune.insert_block > 0 ? lead->tune.insert_block : 256);
+  launch_insert(lead->d_batch, lp.pix, lead->sm_count, s, lead->tune.insert_block > 0 ? lead->tune.insert_block : 256,
+                0, n);
   // 16 B per octree level probed, counted on the device (set after the frame)
   lead->prof.end(pi, 0.0, s);
   lead->pi_insert = pi;
@@ -1451,8 +1442,7 @@ static ff_status frame_finish(ff_handle *h, const FramePlan &plan, MapFrame &mf,
     mf.nq_host = nq;
     h->h_batch->n = 1;
     h->h_batch->max_rounds = 1;
-    h->h_batch->tile_end[0] = 0;
-    h->h_batch->pix_end[0] = 0;
+    h->h_batch->ends.end[0] = 0;
     h->h_batch->f[0] = mf;
     CK(cudaMemcpyAsync(h->d_batch, h->h_batch, batch_desc_bytes(1), cudaMemcpyHostToDevice, s));
     pi_fuse = h->prof.begin(ST_FUSE, s);
@@ -1653,15 +1643,12 @@ static ff_status ensure_seq(ff_handle *h, int W, int H, int frames) {
   if (frames <= h->seq_frames && pix <= h->seq_pix && bnd <= h->seq_bnd) return FF_OK;
   const int nf = std::max(frames, h->seq_frames);
   const size_t np = std::max(pix, h->seq_pix), nb = std::max(bnd, h->seq_bnd);
-  cudaFree(h->d_seq_vox);
-  cudaFree(h->d_seq_proc);
+  cudaFree(h->d_seq_cand);
   cudaFree(h->d_seq_bnd);
-  h->d_seq_vox = nullptr;
-  h->d_seq_proc = nullptr;
+  h->d_seq_cand = nullptr;
   h->d_seq_bnd = nullptr;
   h->seq_frames = 0;
-  CK(alloc(&h->d_seq_vox, np * nf));
-  CK(alloc(&h->d_seq_proc, np * nf));
+  CK(alloc(&h->d_seq_cand, np * nf));
   CK(alloc(&h->d_seq_bnd, nb * nf));
   if (!h->d_seq_cnt) {
     CK(alloc(&h->d_seq_cnt, (size_t)BATCH_MAX));
@@ -1705,8 +1692,7 @@ static ff_status sequence_chunk(ff_handle *h, bool after_pass, int c, const uint
     h->cnn_on_side = false;
     FCK(sp);
     MapFrame &F = mf[k];
-    F.vox = h->d_seq_vox + (size_t)k * h->seq_pix;
-    F.proc = h->d_seq_proc + (size_t)k * h->seq_pix;
+    F.cand = h->d_seq_cand + (size_t)k * h->seq_pix;
     F.bnd = h->d_seq_bnd + (size_t)k * h->seq_bnd;
     F.cnt = h->d_seq_cnt + k;
     F.frame = frame0 + 1 + (uint32_t)k;
@@ -1727,8 +1713,7 @@ static ff_status sequence_chunk(ff_handle *h, bool after_pass, int c, const uint
   for (int k = 0; k < c; k++) {
     int pi = h->prof.begin(ST_INSERT, s);
     pi_ins[k] = pi;
-    launch_insert(h->d_batch, (uint32_t)(h->h_batch->pix_end[k] - (k ? h->h_batch->pix_end[k - 1] : 0u)), s, block,
-                  k, k + 1, pdl && k > 0);
+    launch_insert(h->d_batch, lp.pix, h->sm_count, s, block, k, 1, pdl && k > 0);
     h->prof.end(pi, 0.0, s);
     const bool wait = after_pass && k == 0;
     if (wait) CK(cudaStreamWaitEvent(s, h->ev_ring_free, 0));

@@ -39,9 +39,8 @@ struct MapFrame {
   // octree subtrees unchanged since its previous update)
   uint32_t *bstamp;
   PendingLeaf *pend;
-  int4 *vox;
-  uint8_t *proc;
-  int4 *bnd;
+  uint4 *cand;  // the frame's cells: x | y << 16, z | target << 16, first pixel (at most one per pixel)
+  uint32_t *bnd;
   Counters *cnt;
   const uint32_t *rcp_tab;
   int rcp_shift;
@@ -165,11 +164,15 @@ void launch_halo_unpack(const void *in, uint64_t n, uint32_t leaves_max, float *
 
 constexpr int BATCH_MAX = 32;
 
+// Inclusive prefix of each map's de-duplication tiles.
+struct TileEnds {
+  uint32_t end[BATCH_MAX];
+};
+
 struct BatchDesc {
   int n;                          // maps in the batch
   int max_rounds;                 // de-duplication round limit (largest image)
-  uint32_t tile_end[BATCH_MAX];   // inclusive prefix of each map's de-duplication tiles
-  uint32_t pix_end[BATCH_MAX];    // inclusive prefix of each map's pixels, each padded to 32
+  TileEnds ends;
   MapFrame f[BATCH_MAX];
 };
 
@@ -182,8 +185,7 @@ inline size_t batch_desc_bytes(int n) { return offsetof(BatchDesc, f) + sizeof(M
 struct BatchDesc1 {
   int n;
   int max_rounds;
-  uint32_t tile_end[BATCH_MAX];
-  uint32_t pix_end[BATCH_MAX];
+  TileEnds ends;
   MapFrame f[1];
 };
 static_assert(offsetof(BatchDesc1, f) == offsetof(BatchDesc, f) && sizeof(BatchDesc1) == offsetof(BatchDesc, f) +
@@ -207,15 +209,15 @@ void launch_first_bbox(const uint16_t *depth, int W, int H, const CamF &p, float
 // can be resident, then 32-row tiles (dedupe_tile_rows).
 int dedupe_tiles(int W, int H, int *tilesX, int *tilesY, int rows);
 // Tiles one cooperative de-duplication launch holds (all warps resident).
-cudaError_t dedupe_capacity(int device, int rows, uint32_t &tiles);
-// int4 elements of the boundary buffer launch_dedupe needs for a W x H image.
+cudaError_t dedupe_capacity(int device, uint32_t &tiles);
+// Words of the boundary buffer launch_dedupe needs for a W x H image.
 size_t dedupe_boundary_elems(int W, int H);
-// Per-pixel voxel coordinates, validity and target brick scale (written to
-// each frame's vox), then the row/column de-duplication of brick keys
-// (traversal_wrapper_functions.cpp:613-639, 688-690), for every frame of the
-// batch in one cooperative launch per group of maps [m0, m1) whose `tiles`
-// fit the launch.  barrier: 8 zeroed uint32 words per launch.
-cudaError_t launch_dedupe(const BatchDesc *d_batch, int m0, int m1, uint32_t tiles, int rows, uint32_t *barrier,
+// Per-pixel voxel coordinates, the row/column de-duplication of brick keys
+// (traversal_wrapper_functions.cpp:613-639, 688-690) and the list of the cells
+// its pixels ask for, for every frame of the batch in one cooperative launch
+// per group of maps [m0, m1) whose `tiles` fit the launch (h_batch: the
+// descriptor on the host).  barrier: 8 zeroed uint32 words per launch.
+cudaError_t launch_dedupe(const BatchDesc *h_batch, const BatchDesc *d_batch, int m0, int m1, uint32_t tiles, int rows, uint32_t *barrier,
                           int device, cudaStream_t s);
 // The same for a one-map descriptor h_desc in host memory: passed as the
 // launch's parameter (no upload of its own) and stored to d_batch by the
@@ -223,12 +225,12 @@ cudaError_t launch_dedupe(const BatchDesc *d_batch, int m0, int m1, uint32_t til
 cudaError_t launch_dedupe_one(const BatchDesc *h_desc, BatchDesc *d_batch, uint32_t tiles, int rows,
                               uint32_t *barrier, int device, cudaStream_t s);
 
-// Octree descent / allocation of every processed pixel of the batch's maps
-// [m0, m1) (pixels [pix_end[m0 - 1], pix_end[m1 - 1]), pix = their count).
+// Octree descent / allocation of the listed cells of the batch's maps
+// [m0, m0 + nmaps); npix: pixels of the largest image.
 // pdl: launched as a programmatic dependent of the stream's previous kernel
 // (which must be a kernel), as in the chained frames of a sequence.
-void launch_insert(const BatchDesc *d_batch, uint32_t pix, cudaStream_t s, int block = 256, int m0 = 0,
-                   int m1 = BATCH_MAX, bool pdl = false);
+void launch_insert(const BatchDesc *d_batch, uint32_t npix, int sm_count, cudaStream_t s, int block, int m0, int nmaps,
+                   bool pdl = false);
 
 // Sort scratch size for `n` pending leaves.
 size_t pending_sort_bytes(int n);
