@@ -701,10 +701,9 @@ __device__ void save_top(const GenQueues &Q, int lv, const TopCache &T) {
 }
 
 // (the cache's counts fit the queues: the queues only grow while it is valid)
-__global__ void k_load_top(GenQueues Q, int lv, TopCache T) {
-  pdl_enter();
+// Thread t0 of `stride`.
+__device__ __forceinline__ void load_top(const GenQueues &Q, int lv, const TopCache &T, uint32_t t0, uint32_t stride) {
   const int b = lv & 1;
-  const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   if (t0 == 0) {
     uint32_t *c = Q.lvl + QK * lv;
     for (int k = 0; k < QK; k++) c[k] = T.count[k];
@@ -887,10 +886,18 @@ __device__ __forceinline__ uint32_t block_scan_keep(uint32_t v, uint32_t *total)
 }
 
 // keep[i] = 1 if previous cell i is kept; per tile of KEEP_THREADS cells, the
-// number kept (tile_sum).
+// number kept (tile_sum).  The blocks past the tiles put the kept top levels'
+// items (of level top_level) into the traversal's queues: two short kernels
+// that do not need one another, in one launch.
 __global__ void __launch_bounds__(KEEP_THREADS) k_keep_cells(GenCtx g, uint32_t n, const Cell *__restrict__ old_cells,
-                                                            uint32_t n_old, uint32_t *keep, uint32_t *tile_sum) {
+                                                            uint32_t n_old, uint32_t *keep, uint32_t *tile_sum,
+                                                            uint32_t ntiles, GenQueues Q, int top_level, TopCache T) {
   pdl_enter();
+  if (blockIdx.x >= ntiles) {
+    load_top(Q, top_level, T, (blockIdx.x - ntiles) * KEEP_THREADS + threadIdx.x,
+             (gridDim.x - ntiles) * KEEP_THREADS);
+    return;
+  }
   const uint32_t i = blockIdx.x * KEEP_THREADS + threadIdx.x;
   uint32_t k = 0;
   if (i < n_old) {
@@ -911,7 +918,10 @@ __global__ void __launch_bounds__(KEEP_THREADS) k_keep_cells(GenCtx g, uint32_t 
 }
 
 // Exclusive scan of the tile sums in one block (any number of tiles, in
-// chunks of the block size).
+// chunks of the block size), for lists of more than SUM_CELLS cells: up to that
+// the blocks that use the sums (512 at most) add up the ones before theirs, a
+// read or two per thread, which costs less than a launch (2 to 3 us).
+constexpr uint32_t SUM_CELLS = 1u << 17;
 __global__ void __launch_bounds__(KEEP_SCAN_THREADS) k_keep_tile_scan(uint32_t *tile_sum, uint32_t ntiles) {
   pdl_enter();
   __shared__ uint32_t warp_sum[KEEP_SCAN_THREADS / 32];
@@ -946,20 +956,30 @@ __global__ void __launch_bounds__(KEEP_SCAN_THREADS) k_keep_tile_scan(uint32_t *
 // keep[] becomes the exclusive prefix of the kept flags, with the total at
 // keep[n_old]; counts[0] = cells kept, counts[1] = cells kept before the
 // previous list's first corner cell.
+// scanned: tile_sum holds exclusive prefixes (else the tiles' own sums).
 __global__ void __launch_bounds__(KEEP_THREADS) k_keep_apply(uint32_t *keep, uint32_t n_old, const uint32_t *tile_sum,
-                                                            uint32_t ntiles, uint32_t first_corner_old,
+                                                            uint32_t ntiles, bool scanned, uint32_t first_corner_old,
                                                             uint32_t *counts) {
   pdl_enter();
   const uint32_t i = blockIdx.x * KEEP_THREADS + threadIdx.x;
   const uint32_t k = i < n_old ? keep[i] : 0u;
+  uint32_t before = 0;
+  if (scanned) {
+    before = tile_sum[blockIdx.x];
+  } else {
+    uint32_t sum = 0;
+    for (uint32_t j = threadIdx.x; j < blockIdx.x; j += KEEP_THREADS) sum += tile_sum[j];
+    (void)block_scan_keep(sum, &before);
+    __syncthreads();
+  }
   uint32_t total;
-  const uint32_t ex = block_scan_keep(k, &total) + tile_sum[blockIdx.x];
+  const uint32_t ex = block_scan_keep(k, &total) + before;
   if (i < n_old) keep[i] = ex;
   if (i == first_corner_old) counts[1] = ex;
   if (blockIdx.x == ntiles - 1 && threadIdx.x == 0) {
-    keep[n_old] = tile_sum[blockIdx.x] + total;
-    counts[0] = tile_sum[blockIdx.x] + total;
-    if (first_corner_old >= n_old) counts[1] = tile_sum[blockIdx.x] + total;
+    keep[n_old] = before + total;
+    counts[0] = before + total;
+    if (first_corner_old >= n_old) counts[1] = before + total;
   }
 }
 
@@ -2147,17 +2167,29 @@ __global__ void __launch_bounds__(MESH_THREADS, 8) k_mesh_count(VoxSrc m, const 
   }
 }
 
+// What the emit pass, launched ahead of the host's look at the totals, looks at
+// itself: the output buffers' elements and the cells' error word.
+struct EmitRoom {
+  uint32_t ncells;
+  uint64_t vertex_elems, face_elems;
+  const uint32_t *error;
+};
+
 // Emit pass: every cell's vertices and faces at their final offsets.
 __global__ void __launch_bounds__(MESH_THREADS, 4) k_mesh_emit(VoxSrc m, const Cell *__restrict__ cells, MeshLists L,
                                                               CellOut *out, const uint64_t *vbase,
                                                               const uint64_t *fbase, float *xyz, uint8_t *rgb,
                                                               uint32_t *faces, uint32_t *work,
-                                                              const uint8_t *__restrict__ cell_rows, CleanCopy C) {
+                                                              const uint8_t *__restrict__ cell_rows, CleanCopy C,
+                                                              EmitRoom room) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ McTab T;
   pdl_trigger();
   load_mc(T);
   pdl_wait();
+  if (3 * vbase[room.ncells] + 3 > room.vertex_elems || 3 * fbase[room.ncells] + 3 > room.face_elems ||
+      (*room.error & (ERR_CELL_KEY | ERR_CELL_MERGE)))
+    return;
   const int lane = threadIdx.x & 31;
   LatScratch &W = *reinterpret_cast<LatScratch *>(smem_raw + (size_t)(threadIdx.x >> 5) * SCRATCH_EMIT_BYTES);
   const uint32_t nl = *L.n_lattice, nc = *L.n_corner;
@@ -2302,10 +2334,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_count_tile_sums(const CellOut 
   }
 }
 
-// One block: tile sums -> exclusive tile offsets (in place), totals to
-// vbase[n] and fbase[n].
-__global__ void __launch_bounds__(SCAN_THREADS) k_count_tile_scan(uint64_t *tile_v, uint64_t *tile_f, uint32_t ntiles,
-                                                                  uint64_t *vbase, uint64_t *fbase, uint32_t n) {
+// One block: tile sums -> exclusive tile offsets (in place); for more than
+// SUM_CELLS cells only.
+__global__ void __launch_bounds__(SCAN_THREADS) k_count_tile_scan(uint64_t *tile_v, uint64_t *tile_f, uint32_t ntiles) {
   pdl_enter();
   __shared__ uint64_t carry_v, carry_f;
   if (threadIdx.x == 0) carry_v = carry_f = 0;
@@ -2323,16 +2354,27 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_count_tile_scan(uint64_t *tile
     if (threadIdx.x == 0) carry_v += ta, carry_f += tb;
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    vbase[n] = carry_v;
-    fbase[n] = carry_f;
-  }
 }
 
+// Per-cell bases, and their totals to vbase[n] and fbase[n].  The last block
+// also hands the host what it waits for, through its pinned memory (five small
+// copies cost the stream 10 us): the totals and the counter words below 32.
+// scanned: the tile sums are exclusive prefixes (else the tiles' own sums).
 __global__ void __launch_bounds__(SCAN_THREADS) k_count_tile_apply(const CellOut *__restrict__ out, uint32_t n,
                                                                    const uint64_t *tile_v, const uint64_t *tile_f,
-                                                                   uint64_t *vbase, uint64_t *fbase) {
+                                                                   bool scanned, uint64_t *vbase, uint64_t *fbase,
+                                                                   const uint32_t *words, uint32_t *host_words,
+                                                                   uint64_t *host_totals) {
   pdl_enter();
+  uint64_t before_v = 0, before_f = 0;
+  if (scanned) {
+    before_v = tile_v[blockIdx.x], before_f = tile_f[blockIdx.x];
+  } else {
+    uint64_t a = 0, b = 0, pa, pb;
+    for (uint32_t j = threadIdx.x; j < blockIdx.x; j += SCAN_THREADS) a += tile_v[j], b += tile_f[j];
+    block_scan2(a, b, pa, pb, &before_v, &before_f);
+    __syncthreads();
+  }
   const uint32_t i0 = blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_PER_THREAD;
   uint32_t cv[SCAN_PER_THREAD], cf[SCAN_PER_THREAD];
   uint64_t a = 0, b = 0;
@@ -2344,9 +2386,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_count_tile_apply(const CellOut
     a += cv[k];
     b += cf[k];
   }
-  uint64_t pa, pb;
-  block_scan2(a, b, pa, pb, nullptr, nullptr);
-  uint64_t ov = tile_v[blockIdx.x] + pa, of = tile_f[blockIdx.x] + pb;
+  uint64_t pa, pb, ta, tb;
+  block_scan2(a, b, pa, pb, &ta, &tb);
+  uint64_t ov = before_v + pa, of = before_f + pb;
 #pragma unroll
   for (int k = 0; k < SCAN_PER_THREAD; k++) {
     if (i0 + k < n) {
@@ -2355,6 +2397,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_count_tile_apply(const CellOut
     }
     ov += cv[k];
     of += cf[k];
+  }
+  if (blockIdx.x != gridDim.x - 1) return;
+  if (threadIdx.x < LEVEL_COUNTS) host_words[threadIdx.x] = words[threadIdx.x];
+  if (threadIdx.x == 0) {
+    vbase[n] = host_totals[0] = before_v + ta;
+    fbase[n] = host_totals[1] = before_f + tb;
   }
 }
 
@@ -2463,6 +2511,7 @@ struct MeshImpl {
   uint32_t *old_faces = nullptr;
   size_t cap_oxyz = 0, cap_orgb = 0, cap_ofaces = 0;
   size_t cap_xyz = 0, cap_rgb = 0, cap_faces = 0;
+  cudaEvent_t ev_totals = nullptr;  // after the totals' hand-over to the host
   uint32_t since = 0;
   // incremental cell list: the previous update's leaf and branch counts and
   // growth count; per previous cell its kept flag, then their prefix; merged
@@ -2577,17 +2626,6 @@ static int generate_cells(MeshImpl &I, const MeshInputs &in, bool incr, cudaStre
     g.prev_branches = I.prev_branches;
     g.incr = incr ? 1 : 0;
     g.expand_all = 0;  // (set per level by the traversal)
-    if (incr) {
-      // the previous cells whose sides did not change, and their positions
-      // among the kept (words KEPT_WORD, KEPT_WORD + 1: kept, kept before the
-      // first corner cell)
-      // (the scan and the apply: programmatic dependents of the kernel before)
-      note_launch(3);
-      k_keep_cells<<<keep_tiles, KEEP_THREADS, 0, s>>>(g, in.n, I.old_cells, n_old, I.keep, I.keep_tiles);
-      MCK(launch_pdl(pdl, k_keep_tile_scan, dim3(1), dim3(KEEP_SCAN_THREADS), 0, s, I.keep_tiles, keep_tiles));
-      MCK(launch_pdl(pdl, k_keep_apply, dim3(keep_tiles), dim3(KEEP_THREADS), 0, s, I.keep, n_old,
-                     (const uint32_t *)I.keep_tiles, keep_tiles, first_corner_old, I.d_count + KEPT_WORD));
-    }
     // The top levels: an incremental update whose frames created nothing
     // near the root starts from the kept level-MESH_TOP_LEVELS items;
     // otherwise the top levels run (in an incremental update expanding every
@@ -2624,10 +2662,19 @@ static int generate_cells(MeshImpl &I, const MeshInputs &in, bool incr, cudaStre
       for (int k = 0; k < 4; k++) T.cap[k] = (uint32_t)(k == 1 || k == 2 ? I.cap_top[k] / 3 : I.cap_top[k]);
     }
     I.gen_start_level = (uint32_t)lv0;
-    if (use_top) {
-      note_launch(1);
-      // (after the keep test's last kernel: a programmatic dependent)
-      MCK(launch_pdl(pdl, k_load_top, dim3(148 * 2), dim3(256), 0, s, Q, (int)LC, T));
+    if (incr) {
+      // the previous cells whose sides did not change, and their positions
+      // among the kept (words KEPT_WORD, KEPT_WORD + 1: kept, kept before the
+      // first corner cell)
+      // (the scan and the apply: programmatic dependents of the kernel before)
+      const bool scan = n_old > SUM_CELLS;
+      note_launch(scan ? 3 : 2);
+      k_keep_cells<<<keep_tiles + (use_top ? 148 : 0), KEEP_THREADS, 0, s>>>(g, in.n, I.old_cells, n_old, I.keep,
+                                                                           I.keep_tiles, keep_tiles, Q, (int)LC, T);
+      if (scan)
+        MCK(launch_pdl(pdl, k_keep_tile_scan, dim3(1), dim3(KEEP_SCAN_THREADS), 0, s, I.keep_tiles, keep_tiles));
+      MCK(launch_pdl(pdl, k_keep_apply, dim3(keep_tiles), dim3(KEEP_THREADS), 0, s, I.keep, n_old,
+                     (const uint32_t *)I.keep_tiles, keep_tiles, scan, first_corner_old, I.d_count + KEPT_WORD));
     }
     // An item of level l holds slots of depth l at most, and it expands only
     // if one of them is subdivided, so the last level with items is the
@@ -2891,34 +2938,71 @@ int mesh_update(MeshState &M, const MeshInputs &in, cudaStream_t s, std::string 
   const int pi_count = pi;
   P.end(pi_count, 0.0, s);
   MCK(cudaGetLastError());
-  // exclusive scans of vertex and face counts -> per-cell bases (totals at ncells)
+  // exclusive scans of vertex and face counts -> per-cell bases (totals at
+  // ncells); totals, dirty counts, samples and errors to the pinned counter mirror
+  uint64_t *h_tot = reinterpret_cast<uint64_t *>(I.h_count + HOST_TOTALS);
   {
-    note_launch(ntiles ? 3 : 1);
+    const bool scan = ncells > SUM_CELLS;
+    note_launch((ntiles ? 2 : 1) + (scan ? 1 : 0));
     if (ntiles) {
       MCK(launch_pdl(chained, k_count_tile_sums, dim3(ntiles), dim3(SCAN_THREADS), 0, s, (const CellOut *)I.out,
                      ncells, I.nv, I.nf));
       chained = pdl;
     }
-    MCK(launch_pdl(chained, k_count_tile_scan, dim3(1), dim3(SCAN_THREADS), 0, s, I.nv, I.nf, ntiles, I.vbase,
-                   I.fbase, ncells));
-    if (ntiles)
-      MCK(launch_pdl(pdl, k_count_tile_apply, dim3(ntiles), dim3(SCAN_THREADS), 0, s, (const CellOut *)I.out, ncells,
-                     (const uint64_t *)I.nv, (const uint64_t *)I.nf, I.vbase, I.fbase));
+    if (scan) MCK(launch_pdl(pdl, k_count_tile_scan, dim3(1), dim3(SCAN_THREADS), 0, s, I.nv, I.nf, ntiles));
+    MCK(launch_pdl(chained, k_count_tile_apply, dim3(std::max(ntiles, 1u)), dim3(SCAN_THREADS), 0, s,
+                   (const CellOut *)I.out, ncells, (const uint64_t *)I.nv, (const uint64_t *)I.nf, scan, I.vbase,
+                   I.fbase, (const uint32_t *)I.d_count, I.h_count, h_tot));
   }
-  // totals, dirty count and samples through the pinned counter mirror
-  uint64_t *h_tot = reinterpret_cast<uint64_t *>(I.h_count + HOST_TOTALS);
-  MCK(cudaMemcpyAsync(h_tot + 0, I.vbase + ncells, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  MCK(cudaMemcpyAsync(h_tot + 1, I.fbase + ncells, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  MCK(cudaMemcpyAsync(h_tot + 2, I.d_count + 12, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-  MCK(cudaMemcpyAsync(I.h_count + DIRTY_WORD, I.d_count + DIRTY_WORD, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  MCK(cudaMemcpyAsync(I.h_count + HOST_TOTALS + 7, I.d_count + 9, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  MCK(cudaStreamSynchronize(s));
-  if (I.h_count[HOST_TOTALS + 7] & ERR_CELL_KEY) {
+  // The previous output becomes the copy source; the new output is written
+  // fresh, by an emit pass launched ahead of the host's wait for the totals:
+  // it does nothing when the buffers are too small for them (or the cells are
+  // in error), and the host then grows them and launches it again.  With the
+  // totals handed over by the scan, a 640x480 frame and its update take 456 us
+  // instead of 490.  Not with the stage profile on, which times one emit pass per
+  // update.
+  const auto swap_outputs = [&]() {
+    std::swap(I.old_xyz, M.d_xyz);
+    std::swap(I.cap_oxyz, I.cap_xyz);
+    std::swap(I.old_rgb, M.d_rgb);
+    std::swap(I.cap_orgb, I.cap_rgb);
+    std::swap(I.old_faces, M.d_faces);
+    std::swap(I.cap_ofaces, I.cap_faces);
+  };
+  const auto launch_emit = [&]() {
+    CleanCopy C;
+    C.dirty = I.dirty;
+    C.old_index = I.old_index;
+    C.old_vbase = I.old_vbase;
+    C.old_fbase = I.old_fbase;
+    C.old_xyz = I.old_xyz;
+    C.old_rgb = I.old_rgb;
+    C.old_faces = I.old_faces;
+    C.n = incremental ? ncells : 0u;
+    EmitRoom room;
+    room.ncells = ncells;
+    room.vertex_elems = std::min(I.cap_xyz, I.cap_rgb);
+    room.face_elems = I.cap_faces;
+    room.error = I.d_count + 9;
+    note_launch(1);
+    k_mesh_emit<<<blocks(4, ncells), MESH_THREADS, smem_emit, s>>>(vs, I.cells, L, I.out, I.vbase, I.fbase, M.d_xyz,
+                                                                  M.d_rgb, M.d_faces, I.d_count + EMIT_WORK_WORD,
+                                                                  I.cell_rows, C, room);
+  };
+  if (!I.ev_totals) MCK(cudaEventCreateWithFlags(&I.ev_totals, cudaEventDisableTiming));
+  MCK(cudaEventRecord(I.ev_totals, s));
+  swap_outputs();
+  const bool ahead = !P.on && ncells && I.cap_xyz && I.cap_rgb && I.cap_faces;
+  if (ahead) launch_emit();
+  MCK(cudaEventSynchronize(I.ev_totals));
+  const uint32_t cell_error = I.h_count[9];
+  if (cell_error & (ERR_CELL_KEY | ERR_CELL_MERGE)) swap_outputs();  // (nothing was written)
+  if (cell_error & ERR_CELL_KEY) {
     mesh_invalidate(M);
     err = "meshing: a mesh cell lies outside the volume";
     return 6;
   }
-  if (I.h_count[HOST_TOTALS + 7] & ERR_CELL_MERGE) {
+  if (cell_error & ERR_CELL_MERGE) {
     // the kept and the new cells overlap: build this update from the whole
     // octree instead (every cell generated and meshed again)
     if (!incr_cells) {
@@ -2933,40 +3017,20 @@ int mesh_update(MeshState &M, const MeshInputs &in, cudaStream_t s, std::string 
     return rc;
   }
   const uint64_t tot[2] = {h_tot[0], h_tot[1]};
-  const unsigned long long nsamples = h_tot[2];
+  const unsigned long long nsamples = *reinterpret_cast<const uint64_t *>(I.h_count + 12);
   const uint32_t ndirty = I.h_count[DIRTY_WORD] + I.h_count[DIRTY_WORD + 1];
   // count pass: SDF and weight of every sample of the dirty cells (the emit
   // pass reads colour as well: sample_bytes)
   const double sample_bytes = vs.fp16 ? 10.0 : 14.0;
   P.set_bytes(pi_count, (double)nsamples * (vs.fp16 ? 4.0 : 8.0));
-  // the previous output becomes the copy source; the new output is written fresh
-  std::swap(I.old_xyz, M.d_xyz);
-  std::swap(I.cap_oxyz, I.cap_xyz);
-  std::swap(I.old_rgb, M.d_rgb);
-  std::swap(I.cap_orgb, I.cap_rgb);
-  std::swap(I.old_faces, M.d_faces);
-  std::swap(I.cap_ofaces, I.cap_faces);
+  const bool room = 3 * tot[0] + 3 <= I.cap_xyz && 3 * tot[0] + 3 <= I.cap_rgb && 3 * tot[1] + 3 <= I.cap_faces;
   MCK(grow_buf(M.d_xyz, I.cap_xyz, 3 * tot[0] + 3, s));
   MCK(grow_buf(M.d_rgb, I.cap_rgb, 3 * tot[0] + 3, s));
   MCK(grow_buf(M.d_faces, I.cap_faces, 3 * tot[1] + 3, s));
   // the emit pass counts the samples it reads in d_count words 18-19
   vs.samples = P.on ? reinterpret_cast<unsigned long long *>(I.d_count + 18) : nullptr;
   pi = P.begin(ST_MESH_EMIT, s);
-  CleanCopy C;
-  C.dirty = I.dirty;
-  C.old_index = I.old_index;
-  C.old_vbase = I.old_vbase;
-  C.old_fbase = I.old_fbase;
-  C.old_xyz = I.old_xyz;
-  C.old_rgb = I.old_rgb;
-  C.old_faces = I.old_faces;
-  C.n = incremental ? ncells : 0u;
-  if (ncells) {
-    note_launch(1);
-    k_mesh_emit<<<blocks(4, ncells), MESH_THREADS, smem_emit, s>>>(vs, I.cells, L, I.out, I.vbase, I.fbase, M.d_xyz,
-                                                                  M.d_rgb, M.d_faces, I.d_count + EMIT_WORK_WORD,
-                                                                  I.cell_rows, C);
-  }
+  if (ncells && !(ahead && room)) launch_emit();
   // emit pass: the samples it reads (the ends of vertex-carrying lattice
   // edges, corner cells' 8) and the whole mesh written (xyz 12 B + rgb 3 B
   // per vertex, 12 B per face); the sample count arrives with the final sync
@@ -3123,6 +3187,7 @@ void mesh_free(MeshState &M) {
     for (void *p : ptrs)
       if (p) cudaFreeAsync(p, 0);
     if (I.h_count) cudaFreeHost(I.h_count);
+    if (I.ev_totals) cudaEventDestroy(I.ev_totals);
     if (I.h_top_count) cudaFreeHost(I.h_top_count);
     delete &I;
     M.impl = nullptr;
@@ -3165,8 +3230,7 @@ cudaError_t prewarm_mesh_kernels() {
                        (const void *)k_count_tile_scan,    (const void *)k_count_tile_apply,
                        (const void *)k_export_cells,
                        (const void *)k_keep_cells,         (const void *)k_keep_tile_scan,
-                       (const void *)k_keep_apply,         (const void *)k_merge_cells,
-                       (const void *)k_load_top};
+                       (const void *)k_keep_apply,         (const void *)k_merge_cells};
   for (const void *f : fns) {
     cudaFuncAttributes a;
     cudaError_t e = cudaFuncGetAttributes(&a, f);

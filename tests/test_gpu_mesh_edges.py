@@ -65,3 +65,29 @@ def test_incremental_equals_first_update(lib_built, storage):
     assert np.array_equal(ma.vertices.view(np.uint32), mb.vertices.view(np.uint32))
     assert np.array_equal(ma.faces, mb.faces)
     assert np.array_equal(ma.colors, mb.colors)
+
+
+def test_large_cell_lists(lib_built):
+    """Cell lists past the size up to which blocks add up the sums before theirs
+    (131,072 cells), incrementally and from scratch: every pixel of a noise image
+    its own brick."""
+    rng = np.random.default_rng(5)
+    w, h = 512, 384
+    K = np.array([w * 0.9, w * 0.9, w / 2 - 0.5, h / 2 - 0.5])
+    a = _gpu(leaves_max=600000, branches_max=1 << 25, storage="fp16")
+    b = _gpu(leaves_max=600000, branches_max=1 << 25, storage="fp16")
+    for k in range(3):
+        depth = np.rint(rng.uniform(0.5, 4.5, (h, w)) / SCALING).astype(np.uint16)
+        bgr = rng.integers(0, 256, (h, w, 3), dtype=np.uint8)
+        for m in (a, b):
+            m.addMap(depth, _cam(K, np.eye(3), np.zeros(3)), bgr, SCALING, 5.0)
+        a.updateMeshes()
+    b.updateMeshes()
+    assert a.stats()["mesh_cells"] > 1 << 17
+    ma, mb = a.getMeshInterleavedMarchingCubes(), b.getMeshInterleavedMarchingCubes()
+    assert len(ma.vertices) > 0
+    assert np.array_equal(ma.vertices.view(np.uint32), mb.vertices.view(np.uint32))
+    assert np.array_equal(ma.faces, mb.faces)
+    assert np.array_equal(ma.colors, mb.colors)
+    a.close()
+    b.close()
