@@ -1249,23 +1249,33 @@ __global__ void k_cnn_adam(float *__restrict__ master, __nv_bfloat16 *__restrict
 
 constexpr int RAYCAST_MAX_STEPS = 4096;
 
-// The finest leaf holding voxel (x, y, z), or UINT32_MAX.
-__device__ __forceinline__ uint32_t finest_leaf(const uint32_t *__restrict__ tree, uint32_t n, uint32_t leaves_max,
-                                                uint32_t x, uint32_t y, uint32_t z) {
-  uint32_t ox = 0, oy = 0, oz = 0, half = n >> 1, branch = 0, best = UINT32_MAX;
+// The octree slot at the end of a voxel's descent: every voxel of its box has
+// the same finest leaf (UINT32_MAX: none).
+struct RaySlot {
+  uint32_t x, y, z, edge;  // (edge 0: no voxel)
+  uint32_t leaf;
+};
+__device__ __forceinline__ bool in_slot(const RaySlot &S, uint32_t x, uint32_t y, uint32_t z) {
+  return x - S.x < S.edge && y - S.y < S.edge && z - S.z < S.edge;
+}
+__device__ __forceinline__ RaySlot ray_slot(const uint32_t *__restrict__ tree, uint32_t n, uint32_t leaves_max,
+                                            uint32_t x, uint32_t y, uint32_t z) {
+  RaySlot S{0, 0, 0, 0, UINT32_MAX};
+  uint32_t half = n >> 1, branch = 0;
   for (int level = 0; level < 16 && half >= (uint32_t)BL; level++) {
-    const uint32_t co = (x >= ox + half) * 1u + (y >= oy + half) * 2u + (z >= oz + half) * 4u;
+    const uint32_t co = (x >= S.x + half) * 1u + (y >= S.y + half) * 2u + (z >= S.z + half) * 4u;
     const uint32_t leaf = __ldg(tree + branch + co);
-    if (leaf < leaves_max) best = leaf;
+    if (leaf < leaves_max) S.leaf = leaf;
     const uint32_t child = __ldg(tree + branch + co + 8);
+    S.x += half * ((co & 1) != 0);
+    S.y += half * ((co & 2) != 0);
+    S.z += half * ((co & 4) != 0);
+    S.edge = half;
     if (child >= PENDING) break;  // BRANCHINIT (no child)
-    ox += half * ((co & 1) != 0);
-    oy += half * ((co & 2) != 0);
-    oz += half * ((co & 4) != 0);
     branch = child;
     half >>= 1;
   }
-  return best;
+  return S;
 }
 
 // Depth (m) of the first surface crossing of pixel (x, y)'s ray within
@@ -1276,10 +1286,19 @@ __device__ __forceinline__ uint32_t finest_leaf(const uint32_t *__restrict__ tre
 // samples weighted, linearly interpolated -- or, entering a weighted band
 // from unallocated space with 0 <= s < the truncation distance, t - s.
 // 0 where the pixel has no depth, -1 where no surface lies in the window.
-__global__ void k_raycast(RaycastMap m, CamF p, int W, int H, const uint16_t *__restrict__ depth, float scaling,
-                          float window, float step, float *__restrict__ out) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-  if (x >= W) return;
+//
+// What bounds it: the latency of dependent loads, sample after sample: a descent
+// of the octree (eight levels) and 16 voxel loads each.  Samples half a voxel
+// apart mostly stay in the octree slot and the voxel cube of the sample before,
+// so a thread keeps both, with the cube's values; a warp takes 8x4 pixels, whose
+// rays share bricks.  640x480, 0.15 m either side in steps of 2.5 mm: 473 -> 293 us.
+constexpr int RAY_THREADS = 128, RAY_W = 16, RAY_H = 8;  // pixels of a block: warps of 8x4, two by two
+__global__ void __launch_bounds__(RAY_THREADS) k_raycast(RaycastMap m, CamF p, int W, int H,
+                                                        const uint16_t *__restrict__ depth, float scaling,
+                                                        float window, float step, float *__restrict__ out) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int x = blockIdx.x * RAY_W + 8 * (warp & 1) + (lane & 7), y = blockIdx.y * RAY_H + 4 * (warp >> 1) + (lane >> 3);
+  if (x >= W || y >= H) return;
   const float d0 = scaling * (float)__ldg(depth + (size_t)y * W + x);
   float res = 0.0f;
   if (d0 > 0.0f) {
@@ -1288,6 +1307,13 @@ __global__ void k_raycast(RaycastMap m, CamF p, int W, int H, const uint16_t *__
     const float t0 = fmaxf(d0 - window, 0.05f), t1 = d0 + window;
     bool prev_ok = false;
     float prev_s = 0.0f, prev_t = 0.0f, band = 0.0f;
+    RaySlot slot{0, 0, 0, 0, UINT32_MAX};
+    // the slot's leaf: its origin and voxel size, the cube of 8 voxels last
+    // read (its number in the brick, values, all weighted), the voxel last read
+    float ox = 0.0f, oy = 0.0f, oz = 0.0f, ls = 1.0f;
+    int cube = -1, voxel = -1;
+    float cv[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f}, vv = 0.0f;
+    bool cube_ok = false, voxel_ok = false;
     const int nsteps = min((int)((t1 - t0) / step) + 1, RAYCAST_MAX_STEPS);
     for (int k = 0; k < nsteps; k++) {
       const float t = t0 + (float)k * step;
@@ -1299,29 +1325,44 @@ __global__ void k_raycast(RaycastMap m, CamF p, int W, int H, const uint16_t *__
       float s = 0.0f;
       const int ix = __float2int_rn(gx), iy = __float2int_rn(gy), iz = __float2int_rn(gz);
       if (ix >= 0 && iy >= 0 && iz >= 0 && ix < (int)m.n && iy < (int)m.n && iz < (int)m.n) {
-        const uint32_t leaf = finest_leaf(m.tree, m.n, m.leaves_max, ix, iy, iz);
-        if (leaf != UINT32_MAX) {
-          const ushort4 o = __ldg(m.leaf + leaf);
-          const float ls = (float)o.w;
-          band = 0.99f * m.thr * ls;
-          const float ux = (gx - (float)o.x) / ls, uy = (gy - (float)o.y) / ls, uz = (gz - (float)o.z) / ls;
+        if (!in_slot(slot, ix, iy, iz)) {
+          const uint32_t before = slot.leaf;
+          slot = ray_slot(m.tree, m.n, m.leaves_max, ix, iy, iz);
+          if (slot.leaf != before) {
+            cube = voxel = -1;
+            if (slot.leaf != UINT32_MAX) {
+              const ushort4 o = __ldg(m.leaf + slot.leaf);
+              ox = (float)o.x, oy = (float)o.y, oz = (float)o.z, ls = (float)o.w;
+              band = 0.99f * m.thr * ls;
+            }
+          }
+        }
+        if (slot.leaf != UINT32_MAX) {
+          const float ux = (gx - ox) / ls, uy = (gy - oy) / ls, uz = (gz - oz) / ls;
           const int fx0 = (int)floorf(ux), fy0 = (int)floorf(uy), fz0 = (int)floorf(uz);
-          const size_t base = (size_t)leaf * 512;
+          const size_t base = (size_t)slot.leaf * 512;
           if (fx0 >= 0 && fy0 >= 0 && fz0 >= 0 && fx0 < 7 && fy0 < 7 && fz0 < 7) {
             // trilinear inside the brick when its 8 voxels are all weighted
-            const float ax = ux - (float)fx0, ay = uy - (float)fy0, az = uz - (float)fz0;
-            float acc = 0.0f;
-            bool all = true;
+            const int first = (fz0 * 8 + fy0) * 8 + fx0;
+            if (first != cube) {
+              cube = first;
+              cube_ok = true;
 #pragma unroll
-            for (int c = 0; c < 8; c++) {
-              const int dx = c & 1, dy = (c >> 1) & 1, dz = c >> 2;
-              const size_t vi = base + ((fz0 + dz) * 8 + fy0 + dy) * 8 + fx0 + dx;
-              const float w = m.fp16 ? __half2float(m.wgt16[vi]) : m.wgt[vi];
-              const float v = m.fp16 ? __half2float(m.sdf16[vi]) : m.sdf[vi];
-              all = all && w > 0.0f;
-              acc += (dx ? ax : 1.0f - ax) * (dy ? ay : 1.0f - ay) * (dz ? az : 1.0f - az) * v;
+              for (int c = 0; c < 8; c++) {
+                const size_t vi = base + first + ((c >> 2) * 8 + ((c >> 1) & 1)) * 8 + (c & 1);
+                const float w = m.fp16 ? __half2float(m.wgt16[vi]) : m.wgt[vi];
+                cv[c] = m.fp16 ? __half2float(m.sdf16[vi]) : m.sdf[vi];
+                cube_ok = cube_ok && w > 0.0f;
+              }
             }
-            if (all) {
+            if (cube_ok) {
+              const float ax = ux - (float)fx0, ay = uy - (float)fy0, az = uz - (float)fz0;
+              float acc = 0.0f;
+#pragma unroll
+              for (int c = 0; c < 8; c++) {
+                const int dx = c & 1, dy = (c >> 1) & 1, dz = c >> 2;
+                acc += (dx ? ax : 1.0f - ax) * (dy ? ay : 1.0f - ay) * (dz ? az : 1.0f - az) * cv[c];
+              }
               s = acc;
               ok = true;
             }
@@ -1330,10 +1371,15 @@ __global__ void k_raycast(RaycastMap m, CamF p, int W, int H, const uint16_t *__
             const int lx = min(max(__float2int_rn(ux), 0), 7);
             const int ly = min(max(__float2int_rn(uy), 0), 7);
             const int lz = min(max(__float2int_rn(uz), 0), 7);
-            const size_t vi = base + (lz * 8 + ly) * 8 + lx;
-            const float w = m.fp16 ? __half2float(m.wgt16[vi]) : m.wgt[vi];
-            if (w > 0.0f) {
-              s = m.fp16 ? __half2float(m.sdf16[vi]) : m.sdf[vi];
+            const int at = (lz * 8 + ly) * 8 + lx;
+            if (at != voxel) {
+              voxel = at;
+              const float w = m.fp16 ? __half2float(m.wgt16[base + at]) : m.wgt[base + at];
+              vv = m.fp16 ? __half2float(m.sdf16[base + at]) : m.sdf[base + at];
+              voxel_ok = w > 0.0f;
+            }
+            if (voxel_ok) {
+              s = vv;
               ok = true;
             }
           }
@@ -1537,7 +1583,7 @@ cudaError_t cnn_adam(float *master, __nv_bfloat16 *params, float *grads, float *
 cudaError_t launch_raycast(const RaycastMap &m, const CamF &p, int W, int H, const uint16_t *depth, float scaling,
                            float window, float step, float *out, cudaStream_t s) {
   note_launch();
-  k_raycast<<<dim3((W + 127) / 128, H), 128, 0, s>>>(m, p, W, H, depth, scaling, window, step, out);
+  k_raycast<<<dim3((W + RAY_W - 1) / RAY_W, (H + RAY_H - 1) / RAY_H), RAY_THREADS, 0, s>>>(m, p, W, H, depth, scaling, window, step, out);
   return cudaGetLastError();
 }
 
