@@ -72,7 +72,7 @@ struct ff_handle {
   cudaStream_t fuse_stream = nullptr;
   cudaEvent_t ev_alloc = nullptr;  // the frame's insert done (map stream)
   cudaEvent_t ev_cnn_in = nullptr, ev_cnn_done = nullptr;  // the confidence network on fuse_stream
-  bool cnn_on_side = false;  // a sequence's frames: their networks on fuse_stream, beside the allocation chain
+  bool chunk_network = false;  // a sequence's frames: their networks run together, beside the allocation chain
   bool cnn_pending = false;
   cudaEvent_t ev_fin = nullptr;    // the frame's finalisation done (fuse_stream)
   bool fin_pending = false;
@@ -137,7 +137,8 @@ struct ff_handle {
   float conf_tau_cm = 0.0f;  // > 0: the learned weight is on
   __nv_bfloat16 *d_feat = nullptr, *d_a1 = nullptr, *d_a2 = nullptr;
   float *d_conf = nullptr;
-  size_t conf_cap = 0;  // pixels the buffers hold
+  size_t conf_cap = 0;  // pixels a confidence map holds
+  size_t net_cap = 0;   // pixels the network's activations hold (of one image or several)
   int conf_w = 0, conf_h = 0;  // size of the last confidence map
 
   // iterations after which a device-side wait gives up (ff_set_spin_limit),
@@ -1023,6 +1024,33 @@ struct FramePlan {
 };
 
 
+// The network's buffers: activations of `pixels`, confidence maps of `npx`.
+static ff_status ensure_network(ff_handle *h, size_t pixels, size_t npx) {
+  if (pixels > h->net_cap) {
+    cudaFree(h->d_feat);
+    cudaFree(h->d_a1);
+    cudaFree(h->d_a2);
+    h->d_feat = h->d_a1 = h->d_a2 = nullptr;
+    h->net_cap = 0;
+    CK(alloc(&h->d_feat, pixels * CNN_FEAT_CH));
+    CK(alloc(&h->d_a1, pixels * CNN_HIDDEN));
+    CK(alloc(&h->d_a2, pixels * CNN_HIDDEN));
+    h->net_cap = pixels;
+  }
+  if (npx > h->conf_cap) {
+    for (int k = 0; k < 2; k++) {
+      cudaFree(h->d_conf_set[k]);
+      h->d_conf_set[k] = nullptr;
+    }
+    h->conf_cap = 0;
+    CK(alloc(&h->d_conf_set[0], npx));
+    CK(alloc(&h->d_conf_set[1], npx));
+    h->d_conf = h->d_conf_set[h->set];
+    h->conf_cap = npx;
+  }
+  return FF_OK;
+}
+
 // Host part before the launches; fills the frame's descriptor.
 // side: a single-map frame whose update runs on fuse_stream; its confidence
 // network (learned weight) runs there too, overlapping the de-duplication and
@@ -1128,32 +1156,15 @@ static ff_status frame_prepare(ff_handle *h, const uint16_t *d_depth, const uint
     mf.upd_count = h->d_upd_count;
     mf.upd_slot = h->cur_slot;
   }
-  if (h->conf_tau_cm > 0.0f) {
+  if (h->conf_tau_cm > 0.0f && !h->chunk_network) {
     // the frame's confidence map, ahead of the launches that read it on this stream
     const size_t npx = (size_t)W * H;
-    if (npx > h->conf_cap) {
-      cudaFree(h->d_feat);
-      cudaFree(h->d_a1);
-      cudaFree(h->d_a2);
-      h->d_feat = h->d_a1 = h->d_a2 = nullptr;
-      for (int k = 0; k < 2; k++) {
-        cudaFree(h->d_conf_set[k]);
-        h->d_conf_set[k] = nullptr;
-      }
-      h->conf_cap = 0;
-      CK(alloc(&h->d_feat, npx * CNN_FEAT_CH));
-      CK(alloc(&h->d_a1, npx * CNN_HIDDEN));
-      CK(alloc(&h->d_a2, npx * CNN_HIDDEN));
-      CK(alloc(&h->d_conf_set[0], npx));
-      CK(alloc(&h->d_conf_set[1], npx));
-      h->d_conf = h->d_conf_set[h->set];
-      h->conf_cap = npx;
-    }
+    FCK(ensure_network(h, npx, npx));
     // a waiting frame's confidence map lives in its ring slot until the pass
     if (h->cur_slot >= 0) h->d_conf = h->d_ring_conf + (size_t)h->cur_slot * h->ring_pix;
     const float kf[4] = {(float)K[0], (float)K[1], (float)K[2], (float)K[3]};
     cudaStream_t cs = s;
-    if ((side && plan.one_sync) || h->cnn_on_side) {
+    if (side && plan.one_sync) {
       // after the depth image is ready on the map's stream; the network
       // feeds only the voxel update, so the frame's allocation need not wait
       cs = h->fuse_stream;
@@ -1179,7 +1190,7 @@ static ff_status frame_prepare(ff_handle *h, const uint16_t *d_depth, const uint
     h->conf_h = H;
     mf.conf = h->d_conf;
   }
-  if (h->inject == FF_INJECT_CONFIDENCE_TIMEOUT) {
+  if (h->inject == FF_INJECT_CONFIDENCE_TIMEOUT && !(h->conf_tau_cm > 0.0f)) {
     // no network this frame: the word is set all the same (the frame's
     // counter set-up keeps it; the update and the host read it)
     CK(cudaMemsetAsync(&h->d_cnt->cnn_error, 0xFF, sizeof(uint32_t), s));
@@ -1661,6 +1672,61 @@ static ff_status ensure_seq(ff_handle *h, int W, int H, int frames) {
   return FF_OK;
 }
 
+// The learned weight's networks of a chunk of c frames.  One image's layers are
+// too short to fill the GPU (45 to 60 us a frame at 640x480, a chain of four
+// launches each, and ten of them were longer than everything else the sequence
+// did); as many images run together as keep the activations, 80 B per pixel, in
+// the 126 MB L2 (12 us a frame).
+constexpr size_t NETWORK_PIXELS = 1250000;
+static int network_images(int c, size_t npx) {
+  return (int)std::min<size_t>(c, std::max<size_t>(1, NETWORK_PIXELS / npx));
+}
+
+// Buffers, and where each frame's confidence map goes: the chunk's maps follow
+// one another from its first ring slot on (a slot holds an image at least).
+static ff_status network_buffers(ff_handle *h, int c, int W, int H, MapFrame *mf) {
+  const size_t npx = (size_t)W * H;
+  FCK(ensure_network(h, npx * network_images(c, npx), npx));
+  for (int k = 0; k < c; k++) {
+    h->d_conf = h->d_ring_conf + (size_t)h->upd_pending * h->ring_pix + npx * k;
+    mf[k].conf = h->h_batch->f[k].conf = h->d_conf;
+  }
+  h->conf_w = W;
+  h->conf_h = H;
+  return FF_OK;
+}
+
+static ff_status network_launch(ff_handle *h, int c, int W, int H, const uint16_t *const *d_depth, const double *K,
+                                float scaling, const MapFrame *mf) {
+  const size_t npx = (size_t)W * H;
+  cudaStream_t cs = h->fuse_stream;
+  CK(cudaStreamWaitEvent(cs, h->ev_cnn_in, 0));
+  const int group = network_images(c, npx);
+  for (int i = 0; i < c; i += group) {
+    const int m = std::min(group, c - i);
+    FeatureImages images;
+    for (int k = 0; k < m; k++) {
+      images.depth[k] = d_depth[i + k];
+      for (int j = 0; j < 4; j++) images.K[k][j] = (float)K[4 * (i + k) + j];
+    }
+    const int pc = h->prof.begin(ST_CONFIDENCE, cs);
+    CK(cnn_features_of(images, m, W, H, scaling, h->d_feat, cs));
+    CK(cnn_forward(h->d_cnn_params, h->d_feat, m, W, H, h->d_a1, h->d_a2, const_cast<float *>(mf[i].conf),
+                   h->conf_tau_cm, &h->d_seq_cnt[0].cnn_error, cs));
+    // depth -> features -> a1 -> a2 -> confidence, each written once and read once
+    h->prof.end(pc, (double)npx * m * ((2 + 16) + (16 + 32) + (32 + 32) + (32 + 4)), cs);
+  }
+  CK(cnn_spread_error(h->d_seq_cnt, c, cs));
+  if (h->inject == FF_INJECT_CONFIDENCE_TIMEOUT) {
+    // the first frame's network reports a wait that gave up
+    CK(cudaMemsetAsync(&h->d_seq_cnt[0].cnn_error, 0xFF, sizeof(uint32_t), cs));
+    h->inject = 0;
+  }
+  CK(cudaEventRecord(h->ev_cnn_done, cs));
+  h->cnn_pending = true;
+  return FF_OK;
+}
+
 // One chunk of a sequence: frames [0, c) of the arrays, all de-duplicated in
 // one set of cooperative launches, then inserted and finalised frame after
 // frame on the device (each finalisation hands the next frame its branch count
@@ -1686,10 +1752,10 @@ static ff_status sequence_chunk(ff_handle *h, bool after_pass, int c, const uint
     h->cur_slot = h->upd_pending + k;
     h->d_cnt = h->d_seq_cnt + k;
     h->h_cnt = h->h_seq_cnt + k;
-    h->cnn_on_side = true;
+    h->chunk_network = true;
     const ff_status sp = frame_prepare(h, d_depth[k], d_bgr[k], W, H, K + 4 * k, R + 9 * k, t + 3 * k, scaling,
                                        maxcam, mf[k], plan[k]);
-    h->cnn_on_side = false;
+    h->chunk_network = false;
     FCK(sp);
     MapFrame &F = mf[k];
     F.cand = h->d_seq_cand + (size_t)k * h->seq_pix;
@@ -1700,9 +1766,13 @@ static ff_status sequence_chunk(ff_handle *h, bool after_pass, int c, const uint
     F.next_cnt = k + 1 < c ? h->d_seq_cnt + k + 1 : nullptr;
     h->h_batch->f[k] = F;
   }
+  if (h->conf_tau_cm > 0.0f) FCK(network_buffers(h, c, W, H, mf.data()));
   LaunchPlan lp;
   FCK(frame_plan(h, c, lp));
+  // the networks wait for the depth images only, not for the de-duplication
+  if (h->conf_tau_cm > 0.0f) CK(cudaEventRecord(h->ev_cnn_in, s));
   FCK(frame_issue(h, c, lp, false));
+  if (h->conf_tau_cm > 0.0f) FCK(network_launch(h, c, W, H, d_depth, K, scaling, mf.data()));
   const int block = h->tune.insert_block > 0 ? h->tune.insert_block : 256;
   std::vector<int> pi_ins(c, -1);
   // The chain's kernels follow one another directly on the stream: each is

@@ -1165,11 +1165,12 @@ __global__ void __launch_bounds__(WG_THREADS) k_wgrad_tc(const __grid_constant__
 // Network input per pixel: depth z (m), the unit normal from central
 // differences of the back-projected neighbours (zero unless all four are
 // valid), and the validity flag.
-__global__ void k_cnn_features(const uint16_t *__restrict__ depth, int W, int H, float scaling, float fx, float fy,
-                               float cx, float cy, __nv_bfloat16 *__restrict__ feat) {
+__global__ void k_cnn_features(const __grid_constant__ FeatureImages images, int W, int H, float scaling,
+                               __nv_bfloat16 *__restrict__ feat) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, img = blockIdx.z;
   if (x >= W) return;
-  const uint16_t *d = depth + (size_t)img * W * H;
+  const uint16_t *__restrict__ d = images.depth[img];
+  const float fx = images.K[img][0], fy = images.K[img][1], cx = images.K[img][2], cy = images.K[img][3];
   auto zat = [&](int xx, int yy) -> float {
     return (xx < 0 || yy < 0 || xx >= W || yy >= H) ? 0.0f : scaling * (float)__ldg(d + (size_t)yy * W + xx);
   };
@@ -1527,10 +1528,40 @@ cudaError_t wgrad(const __nv_bfloat16 *x, const float *dy, int n, int W, int H, 
 }
 }  // namespace
 
+cudaError_t cnn_features_of(const FeatureImages &images, int n, int W, int H, float scaling, __nv_bfloat16 *feat,
+                            cudaStream_t s) {
+  if (n < 1 || n > FEATURE_IMAGES_MAX) return cudaErrorInvalidValue;
+  note_launch();
+  k_cnn_features<<<dim3((W + 127) / 128, H, n), 128, 0, s>>>(images, W, H, scaling, feat);
+  return cudaGetLastError();
+}
+
 cudaError_t cnn_features(const uint16_t *depth, int n, int W, int H, float scaling, const float K[4],
                          __nv_bfloat16 *feat, cudaStream_t s) {
+  const size_t pix = (size_t)W * H;
+  for (int i = 0; i < n; i += FEATURE_IMAGES_MAX) {
+    FeatureImages images;
+    const int m = std::min(n - i, FEATURE_IMAGES_MAX);
+    for (int k = 0; k < m; k++) {
+      images.depth[k] = depth + (size_t)(i + k) * pix;
+      for (int c = 0; c < 4; c++) images.K[k][c] = K[c];
+    }
+    const cudaError_t e = cnn_features_of(images, m, W, H, scaling, feat + (size_t)i * pix * CNN_FEAT_CH, s);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+// A batch's error word (the first frame's) in every frame of it: which image's
+// wait gave up is not known.
+__global__ void k_cnn_spread_error(Counters *cnt, int n) {
+  const uint32_t e = cnt[0].cnn_error;
+  if (e && (int)threadIdx.x < n) cnt[threadIdx.x].cnn_error = e;
+}
+
+cudaError_t cnn_spread_error(Counters *cnt, int n, cudaStream_t s) {
   note_launch();
-  k_cnn_features<<<dim3((W + 127) / 128, H, n), 128, 0, s>>>(depth, W, H, scaling, K[0], K[1], K[2], K[3], feat);
+  k_cnn_spread_error<<<1, 32, 0, s>>>(cnt, n);
   return cudaGetLastError();
 }
 

@@ -305,6 +305,16 @@ struct RaycastMap {
   float thr;  // truncation distance (m) of scale-1 bricks
 };
 
+// The images of one feature launch: depth and intrinsics of each.
+constexpr int FEATURE_IMAGES_MAX = 32;
+struct FeatureImages {
+  const uint16_t *depth[FEATURE_IMAGES_MAX];
+  float K[FEATURE_IMAGES_MAX][4];
+};
+cudaError_t cnn_features_of(const FeatureImages &images, int n, int W, int H, float scaling, __nv_bfloat16 *feat,
+                            cudaStream_t s);
+// The first frame's network error word copied to the other n - 1 frames' (n <= 32).
+cudaError_t cnn_spread_error(Counters *cnt, int n, cudaStream_t s);
 cudaError_t cnn_features(const uint16_t *depth, int n, int W, int H, float scaling, const float K[4],
                          __nv_bfloat16 *feat, cudaStream_t s);
 // tau_cm > 0: out = the confidence weight; else out = the network's output.
