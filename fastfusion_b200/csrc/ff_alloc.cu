@@ -128,8 +128,12 @@ __device__ __forceinline__ void grid_barrier(uint32_t *bar, uint32_t nblocks, Co
 }
 
 constexpr int DD_WARPS = 8;  // tiles (warps) per block
-// warps that share one launch, per SM (the launch bounds below keep them resident)
-constexpr int DD_BLOCKS_PER_SM = 3;
+// blocks that share one launch, per SM (the launch bounds below keep them
+// resident): at 64 registers, so that eight maps of mixed sizes (3,750 tiles of 32
+// rows) fit one launch (91 us in two, 74 in one), and three 1280x960 frames
+constexpr int DD_BLOCKS_PER_SM = 4;
+// the largest image, in warps per SM
+constexpr int DD_IMAGE_WARPS_PER_SM = 24;
 // tile height: 16 rows (more, shorter tiles shorten each warp's chain of
 // rows), or 32 when the image has more 16-row tiles than resident warps
 constexpr int DD_ROWS_SHORT = 16, DD_ROWS_TALL = 32;
@@ -518,12 +522,12 @@ size_t dedupe_boundary_elems(int W, int H) {
   return 4 * (size_t)dedupe_tiles(W, H, nullptr, nullptr, DD_ROWS_LOW);
 }
 
-// Tiles that one launch takes (and so the largest image): the warps that the
-// launch bounds keep resident.
-cudaError_t dedupe_capacity(int device, uint32_t &tiles) {
+// Tiles that one launch takes: the warps that the launch bounds keep resident.
+cudaError_t dedupe_capacity(int device, uint32_t &tiles, uint32_t *image_tiles) {
   int sms = 0;
   const cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   tiles = (uint32_t)(sms * DD_BLOCKS_PER_SM * DD_WARPS);
+  if (image_tiles) *image_tiles = (uint32_t)(sms * DD_IMAGE_WARPS_PER_SM);
   return e;
 }
 
@@ -724,6 +728,38 @@ __device__ __forceinline__ void stamp_path(const MapFrame &F, const uint32_t *pa
   }
 }
 
+// Deferred update: mark each brick of the frame's queue (nq entries: the
+// q0 the insert queued, then the new leaves in rank order, indices from
+// leaves_before) with the frame's bit, and list the bricks no earlier frame
+// of the pass has marked.  Thread t of `threads` (whole warps; every thread of
+// a warp runs the same number of iterations, so the list slots are claimed with
+// one atomic per warp).
+__device__ __forceinline__ void mark_queue(const MapFrame &F, uint32_t q0, uint32_t nq, uint32_t leaves_before,
+                                           uint32_t t, uint32_t threads) {
+  const uint32_t bit = 1u << F.upd_slot;
+  for (uint32_t j0 = t & ~31u; j0 < nq; j0 += threads) {
+    const uint32_t j = j0 + (t & 31u);
+    bool add = false;
+    uint32_t b = 0;
+    if (j < nq) {
+      b = j < q0 ? F.queue[j] : leaves_before + (j - q0);
+      // a part of a sharded map updates the bricks it owns; the queue holds
+      // each brick once, so the old mask lacks this bit
+      if (F.shards <= 1 || owns_brick(F, F.leaf[b])) add = atomicOr(&F.upd_mask[b], bit) == 0u;
+    }
+    const unsigned ball = __ballot_sync(0xffffffffu, add);
+    uint32_t at = 0;
+    if ((t & 31) == 0 && ball) at = atomicAdd(F.upd_count, (uint32_t)__popc(ball));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (add) F.upd_list[at + __popc(ball & ((1u << (t & 31)) - 1u))] = b;
+  }
+}
+
+// Blocks of a chained frame's insert that mark the frame before it, whose leaves
+// are placed by then: four dependent round trips (4 us) that the chain of
+// frames would wait for in that frame's finalisation overlap the descents here.
+constexpr int MARK_BLOCKS = 8;
+
 // The cells the frames' de-duplication listed: blocks over x stride over a
 // frame's list, y is the frame of the batch.  Bound by the latency of a descent
 // (some eight dependent octree reads): a thread per processed pixel, 140,000 of
@@ -731,8 +767,17 @@ __device__ __forceinline__ void stamp_path(const MapFrame &F, const uint32_t *pa
 // launch and 80.9 us at 1280x960; the list takes 12.4 and 12.7 us.  At most 40 registers: six
 // 256-thread blocks per SM instead of five (a few bytes of spill), for any
 // block size the tuning picks.
-__global__ void __maxnreg__(40) k_insert(const BatchDesc *__restrict__ bd, int m0) {
+__global__ void __maxnreg__(40) k_insert(const BatchDesc *__restrict__ bd, int m0, int markers) {
   pdl_enter();
+  const uint32_t blocks = gridDim.x - (uint32_t)markers;
+  if (blockIdx.x >= blocks) {
+    const MapFrame &P = bd->f[m0 - 1];
+    const Counters *c = P.cnt;
+    const uint32_t error = ld_volatile(&c->error), aside = ld_volatile(&c->aside), nq = ld_volatile(&c->queued);
+    if (P.upd_mask && !aside && !(error & (ERR_SEQ_HALT | ERR_DEDUPE_FAILED | ERR_PENDING_OVERFLOW)))
+      mark_queue(P, nq, nq, 0u, (blockIdx.x - blocks) * blockDim.x + threadIdx.x, (uint32_t)markers * blockDim.x);
+    return;
+  }
   const MapFrame &F = bd->f[m0 + blockIdx.y];
   Counters *cnt = F.cnt;
   // a de-duplication that did not complete leaves the frame out, and so does
@@ -740,7 +785,7 @@ __global__ void __maxnreg__(40) k_insert(const BatchDesc *__restrict__ bd, int m
   if (ld_volatile(&cnt->error) & (ERR_DEDUPE_FAILED | ERR_SEQ_HALT)) return;
   const uint32_t cands = ld_volatile(&cnt->cands);
   const int lane = threadIdx.x & 31;
-  for (uint32_t j0 = blockIdx.x * blockDim.x + threadIdx.x - lane; j0 < cands; j0 += gridDim.x * blockDim.x) {
+  for (uint32_t j0 = blockIdx.x * blockDim.x + threadIdx.x - lane; j0 < cands; j0 += blocks * blockDim.x) {
     uint32_t levels = 0;
     if (j0 + lane < cands) {
       const uint4 c = F.cand[j0 + lane];
@@ -764,13 +809,14 @@ __global__ void __maxnreg__(40) k_insert(const BatchDesc *__restrict__ bd, int m
 // Enough blocks for a list as long as the image (every pixel its own cell),
 // but no more than are resident at once.
 void launch_insert(const BatchDesc *d_batch, uint32_t npix, int sm_count, cudaStream_t s, int block, int m0, int nmaps,
-                   bool pdl) {
+                   bool pdl, bool chained) {
   if (!npix || nmaps < 1) return;
   if (block < 64 || block > 1024 || block % 32) block = 256;
   const int resident = std::max(1, 1536 / block) * sm_count;
   const int blocks = std::max(1, std::min((int)((npix + block - 1) / block), resident / nmaps));
   note_launch();
-  launch_pdl(pdl, k_insert, dim3(blocks, nmaps), dim3(block), 0, s, d_batch, m0);
+  const int markers = chained ? MARK_BLOCKS : 0;
+  launch_pdl(pdl, k_insert, dim3(blocks + markers, nmaps), dim3(block), 0, s, d_batch, m0, markers);
 }
 
 // ------------------------------------------------- pending leaf order -----
@@ -921,33 +967,6 @@ __device__ __forceinline__ void chain_next(const MapFrame &F, Counters *cnt, uin
   if (halt) atomicOr(&nx->error, ERR_SEQ_HALT);
 }
 
-// Deferred update: mark each brick of the frame's queue (nq entries: the
-// q0 the insert queued, then the new leaves in rank order, indices from
-// leaves_before) with the frame's bit, and list the bricks no earlier frame
-// of the pass has marked.  Every thread of the block runs the same number of
-// iterations, so the list slots are claimed with one atomic per warp.
-__device__ __forceinline__ void finalize_mark(const MapFrame &F, uint32_t q0, uint32_t nq, uint32_t leaves_before,
-                                              int t) {
-  const uint32_t bit = 1u << F.upd_slot;
-  const uint32_t rounds = (nq + FIN_THREADS - 1) / FIN_THREADS;
-  for (uint32_t it = 0; it < rounds; it++) {
-    const uint32_t j = it * FIN_THREADS + (uint32_t)t;
-    bool add = false;
-    uint32_t b = 0;
-    if (j < nq) {
-      b = j < q0 ? F.queue[j] : leaves_before + (j - q0);
-      // a part of a sharded map updates the bricks it owns; the queue holds
-      // each brick once, so the old mask lacks this bit
-      if (F.shards <= 1 || owns_brick(F, F.leaf[b])) add = atomicOr(&F.upd_mask[b], bit) == 0u;
-    }
-    const unsigned ball = __ballot_sync(0xffffffffu, add);
-    uint32_t at = 0;
-    if ((t & 31) == 0 && ball) at = atomicAdd(F.upd_count, (uint32_t)__popc(ball));
-    at = __shfl_sync(0xffffffffu, at, 0);
-    if (add) F.upd_list[at + __popc(ball & ((1u << (t & 31)) - 1u))] = b;
-  }
-}
-
 __global__ void __launch_bounds__(FIN_THREADS) k_finalize_bitmap(const BatchDesc *__restrict__ bd, int m0) {
   extern __shared__ uint32_t fin_smem[];
   // (the next frame's insert is scheduled once this has started: it overlaps
@@ -989,8 +1008,9 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize_bitmap(const BatchDesc
   if (t == 0) aside_flag = fuse_deferred(F) ? 1 : 0;
   __syncthreads();
   const bool stand_aside = aside_flag != 0;
-  const bool mark = F.upd_mask && !stand_aside;
-  if (mark && F.shards <= 1) finalize_mark(F, q0, q0 + nplaced, leaves_before, t);
+  // (a frame with another after it in its chain is marked beside that one's insert)
+  const bool mark = F.upd_mask && !stand_aside && !F.next_cnt;
+  if (mark && F.shards <= 1) mark_queue(F, q0, q0 + nplaced, leaves_before, t, FIN_THREADS);
   uint32_t *rank = F.rank, *tree = F.tree, *stamp = F.stamp, *queue = F.queue;
   ushort4 *leaf = F.leaf;
   const uint32_t nwords = (npix + 31) / 32;
@@ -1042,10 +1062,11 @@ __global__ void __launch_bounds__(FIN_THREADS) k_finalize_bitmap(const BatchDesc
   // (the new leaves' parents: k_parents_frames, after this kernel)
   if (mark && F.shards > 1) {
     __syncthreads();  // the new leaves' positions
-    finalize_mark(F, q0, q0 + nplaced, leaves_before, t);
+    mark_queue(F, q0, q0 + nplaced, leaves_before, t, FIN_THREADS);
   }
   if (t == 0) {
     cnt->queued = q0 + nplaced;
+    cnt->aside = stand_aside ? 1u : 0u;
     Counters *nx = F.next_cnt;
     if (nx) {
       // the next frame of a sequence starts from this one's counts

@@ -1296,9 +1296,9 @@ static ff_status frame_plan(ff_handle *lead, int n, LaunchPlan &lp) {
   B.n = n;
   // 16-row tiles when they fit one cooperative launch, else 32-row tiles in
   // as many launches (groups of whole maps) as needed
-  uint32_t tiles16 = 0, cap = 0;
+  uint32_t tiles16 = 0, cap = 0, image_tiles = 0;
   for (int i = 0; i < n; i++) tiles16 += (uint32_t)dedupe_tiles(B.f[i].W, B.f[i].H, nullptr, nullptr, 16);
-  CK(dedupe_capacity(lead->cfg.device, cap));
+  CK(dedupe_capacity(lead->cfg.device, cap, &image_tiles));
   int rows = tiles16 <= cap ? 16 : 32;
   if (lead->tune.dedupe_rows == 32 || (lead->tune.dedupe_rows == 16 && tiles16 <= cap)) rows = lead->tune.dedupe_rows;
   if (lead->tune.dedupe_rows == 8) {
@@ -1308,7 +1308,7 @@ static ff_status frame_plan(ff_handle *lead, int n, LaunchPlan &lp) {
   }
   for (int i = 0; i < n; i++) {
     const uint32_t nt = (uint32_t)dedupe_tiles(B.f[i].W, B.f[i].H, &B.f[i].tilesX, &B.f[i].tilesY, rows);
-    if (nt > cap) return set_err(lead, FF_ERR_BAD_ARG, "image too large for the de-duplication launch");
+    if (nt > (rows == 32 ? image_tiles : cap)) return set_err(lead, FF_ERR_BAD_ARG, "image too large for the de-duplication launch");
   }
   int rounds = 1;
   uint32_t tiles = 0, pix = 0;
@@ -1841,6 +1841,7 @@ static ff_status sequence_chunk(ff_handle *h, bool after_pass, int c, const uint
     F.cand = h->d_seq_cand + (size_t)k * h->seq_pix;
     F.bnd = h->d_seq_bnd + (size_t)k * h->seq_bnd;
     F.cnt = h->d_seq_cnt + k;
+    F.queue = h->d_queue_set[k & 1];  // (marked while the next frame's insert fills the other)
     F.frame = frame0 + 1 + (uint32_t)k;
     F.chain = k > 0 ? 1u : 0u;
     F.next_cnt = k + 1 < c ? h->d_seq_cnt + k + 1 : nullptr;
@@ -1863,7 +1864,7 @@ static ff_status sequence_chunk(ff_handle *h, bool after_pass, int c, const uint
   for (int k = 0; k < c; k++) {
     int pi = h->prof.begin(ST_INSERT, s);
     pi_ins[k] = pi;
-    launch_insert(h->d_batch, lp.pix, h->sm_count, s, block, k, 1, pdl && k > 0);
+    launch_insert(h->d_batch, lp.pix, h->sm_count, s, block, k, 1, pdl && k > 0, k > 0);
     h->prof.end(pi, 0.0, s);
     const bool wait = after_pass && k == 0;
     if (wait) CK(cudaStreamWaitEvent(s, h->ev_ring_free, 0));

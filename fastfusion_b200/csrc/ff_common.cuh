@@ -109,6 +109,7 @@ struct Counters {
   uint32_t cnn_error;  // the confidence network's bounded waits (kept by the frame's counter set-up)
   uint32_t levels;     // octree levels the insert probed, summed over the frame's cells
   uint32_t leaves_base;  // a sequence's later frame: leaves before it (set by the previous frame's finalisation)
+  uint32_t aside;        // the finalisation left the frame's update to the host (fuse_deferred)
   uint32_t cands;        // entries of the frame's list of cells (the insert's work)
   uint32_t top_created;  // a branch or leaf was created in a slot within MESH_TOP_LEVELS of the root
 };

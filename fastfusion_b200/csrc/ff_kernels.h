@@ -209,7 +209,8 @@ void launch_first_bbox(const uint16_t *depth, int W, int H, const CamF &p, float
 // can be resident, then 32-row tiles (dedupe_tile_rows).
 int dedupe_tiles(int W, int H, int *tilesX, int *tilesY, int rows);
 // Tiles one cooperative de-duplication launch holds (all warps resident).
-cudaError_t dedupe_capacity(int device, uint32_t &tiles);
+// image_tiles: tiles of the largest image that is taken.
+cudaError_t dedupe_capacity(int device, uint32_t &tiles, uint32_t *image_tiles = nullptr);
 // Words of the boundary buffer launch_dedupe needs for a W x H image.
 size_t dedupe_boundary_elems(int W, int H);
 // Per-pixel voxel coordinates, the row/column de-duplication of brick keys
@@ -226,11 +227,12 @@ cudaError_t launch_dedupe_one(const BatchDesc *h_desc, BatchDesc *d_batch, uint3
                               uint32_t *barrier, int device, cudaStream_t s);
 
 // Octree descent / allocation of the listed cells of the batch's maps
-// [m0, m0 + nmaps); npix: pixels of the largest image.
+// [m0, m0 + nmaps); npix: pixels of the largest image.  chained: frame m0 follows
+// frame m0 - 1 of its sequence, which is marked for the deferred update beside it.
 // pdl: launched as a programmatic dependent of the stream's previous kernel
 // (which must be a kernel), as in the chained frames of a sequence.
 void launch_insert(const BatchDesc *d_batch, uint32_t npix, int sm_count, cudaStream_t s, int block, int m0, int nmaps,
-                   bool pdl = false);
+                   bool pdl = false, bool chained = false);
 
 // Sort scratch size for `n` pending leaves.
 size_t pending_sort_bytes(int n);
