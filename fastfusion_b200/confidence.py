@@ -36,7 +36,7 @@ import numpy as np
 from fastfusion_b200 import fusion, scene
 
 N_PARAMS = 8833
-PACKED_BYTES = 33280   # FF_CNN_PACKED_BYTES: the weights as tensor-core operands
+PACKED_BYTES = 33280   # FF_CNN_PACKED_BYTES: scratch that the forward call takes (no longer written)
 LAYOUT = ((0, 2000), (2000, 16), (2016, 6400), (8416, 16), (8432, 400), (8832, 1))  # W1 b1 W2 b2 W3 b3
 UNIT_M = 0.01          # the network predicts centimetres
 CAP_CM = 15.0          # target cap and the raycast window

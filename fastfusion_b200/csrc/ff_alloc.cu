@@ -324,7 +324,9 @@ __device__ __forceinline__ void tile_box(const MapFrame &F, const TileScratch<DD
 // What bounds it: latency -- a few warps per scheduler, three to five rounds
 // with a grid barrier (2 us) each.  A row of a tile used to be solved across the
 // lanes with two ballots and a search for the chain's start (240 ns a row); the
-// word operations take 20 ns and leave the barriers.
+// word operations take 20 ns and leave the barriers.  With the list of cells
+// (5 us) a 640x480 frame's launch takes 24 us (37 before, without a list), ten
+// frames' 51 us (64), ten 1280x960 frames' launches 244 us (336).
 template <int DD_ROWS>
 __device__ __forceinline__ void dedupe_body(const BatchDesc *__restrict__ bd, const TileEnds &ends, int m0, int m1,
                                             uint32_t *bar) {
