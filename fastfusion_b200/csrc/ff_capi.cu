@@ -1933,16 +1933,19 @@ ff_status ff_add_map_sequence_u16_device(ff_handle *h, int n, const uint16_t *co
   h->fin_pending = false;
   select_set(h, 0);
   ff_status st = FF_OK;
+  bool after_pass = false;  // a pass may have been launched since the map's stream was ordered after one (above)
   for (int i = 0; i < n && st == FF_OK;) {
     const int c = std::min(n - i, std::min(BATCH_MAX, h->upd_batch));
     if (h->upd_pending + c > h->upd_batch) {
+      // frames waiting, before the call too, that the chunk does not fit beside
       st = flush_updates(h);
       if (st != FF_OK) break;
+      after_pass = true;
     }
     int done = 0;
-    // (an earlier chunk of the call may have launched its pass)
-    st = sequence_chunk(h, i > 0, c, d_depth + i, d_bgr + i, width, height, K + 4 * i, R + 9 * i, t + 3 * i, scaling,
-                        maxcam, queued ? queued + i : nullptr, done);
+    st = sequence_chunk(h, after_pass, c, d_depth + i, d_bgr + i, width, height, K + 4 * i, R + 9 * i, t + 3 * i,
+                        scaling, maxcam, queued ? queued + i : nullptr, done);
+    after_pass = true;  // (the chunk's last frame may have launched one)
     i += done;
   }
   // the sequence's frames are read where the caller keeps them: their update
