@@ -461,9 +461,8 @@ static ff_status grow(ff_handle *h, const int *box_min, const int *box_max) {
 // up to MAP_POOL_KEEP; above that it goes back at the next synchronisation, and
 // all of it does when an allocation fails.
 //
-// Both calls behave as cudaMalloc and cudaFree do: the memory can be used on
-// every stream at once (the pool's stream has waited for the block's last use),
-// and nothing that was launched before still uses what is freed.
+// The memory can be used on every stream at once, as cudaMalloc's: the pool's
+// stream has waited for the block's last use.
 constexpr uint64_t MAP_POOL_KEEP = 1ull << 30;
 struct MapPool {
   cudaMemPool_t pool = nullptr;
@@ -518,21 +517,44 @@ static cudaError_t dev_malloc(void **p, size_t bytes) {
   return cudaStreamSynchronize(P.stream);
 }
 
-// n pointers (null ones are skipped) after everything launched so far.
-static void dev_free(void *const *ptrs, size_t n) {
-  MapPool P;
-  bool synced = false;
-  for (size_t k = 0; k < n; k++) {
-    if (!ptrs[k]) continue;
-    if (!synced) {
-      cudaDeviceSynchronize();
-      synced = true;
-      if (map_pool(P) != cudaSuccess) return;
+// Everything launched for the map has run: a map's memory is used on its own
+// streams (a batch of maps runs on the first one's, and its call returns after
+// the work).  Not the whole device's streams: another thread may be recording
+// one of them, and a device synchronisation is refused then.
+static cudaError_t map_idle(const ff_handle *h) {
+  for (cudaStream_t s : {h->stream, h->fuse_stream, h->copy_stream, h->mesh_stream})
+    if (s && cudaStreamSynchronize(s) != cudaSuccess) {
+      cudaGetLastError();
+      return cudaDeviceSynchronize();  // (a caller's stream that is gone, or an error that stays)
     }
-    cudaFreeAsync(ptrs[k], P.stream);
-  }
+  return cudaSuccess;
 }
-static void dev_free(void *p) { dev_free(&p, 1); }
+
+// Give n blocks of the map back (null ones are skipped); the next map, of any
+// thread, may get them at once.  On an error the rest stays the map's: a block
+// whose last use could not be waited for is never given out.
+static cudaError_t dev_free(const ff_handle *h, void **ptrs, size_t n) {
+  if (std::all_of(ptrs, ptrs + n, [](void *p) { return !p; })) return cudaSuccess;
+  MapPool P;
+  cudaError_t e = map_idle(h);
+  if (e == cudaSuccess) e = map_pool(P);
+  for (size_t k = 0; k < n && e == cudaSuccess; k++) {
+    if (ptrs[k]) e = cudaFreeAsync(ptrs[k], P.stream);
+    if (e == cudaSuccess) ptrs[k] = nullptr;
+  }
+  // (the pool gives back what it does not keep when its stream is waited for)
+  return e == cudaSuccess ? cudaStreamSynchronize(P.stream) : e;
+}
+
+// Give buffers of the map back and clear their pointers.
+template <typename... T>
+static cudaError_t drop(const ff_handle *h, T *&...p) {
+  void *ptrs[] = {(void *)p...};
+  const cudaError_t e = dev_free(h, ptrs, sizeof...(p));
+  size_t k = 0;
+  ((p = (T *)ptrs[k++]), ...);
+  return e;
+}
 
 template <typename T>
 static cudaError_t alloc(T **p, size_t count) {
@@ -545,16 +567,8 @@ static cudaError_t alloc(T **p, size_t count) {
 static ff_status ensure_image(ff_handle *h, int W, int H) {
   int npix = W * H;
   if (npix > h->cap_pix) {
-    for (int k = 0; k < 2; k++) {
-      dev_free(h->d_depth_set[k]);
-      dev_free(h->d_bgr_set[k]);
-      h->d_depth_set[k] = nullptr;
-      h->d_bgr_set[k] = nullptr;
-    }
-    dev_free(h->d_cand);
-    dev_free(h->d_pend);
-    dev_free(h->d_keys);
-    dev_free(h->d_sort_tmp);
+    CK(drop(h, h->d_depth_set[0], h->d_depth_set[1], h->d_bgr_set[0], h->d_bgr_set[1], h->d_cand, h->d_pend,
+            h->d_keys, h->d_sort_tmp));
     for (int k = 0; k < 2; k++) {
       CK(alloc(&h->d_depth_set[k], npix));
       CK(alloc(&h->d_bgr_set[k], (size_t)npix * 3));
@@ -569,7 +583,7 @@ static ff_status ensure_image(ff_handle *h, int W, int H) {
   }
   const size_t bnd_need = dedupe_boundary_elems(W, H);
   if (bnd_need > h->bnd_elems) {
-    dev_free(h->d_bnd);
+    CK(drop(h, h->d_bnd));
     h->bnd_elems = bnd_need;
     CK(alloc(&h->d_bnd, h->bnd_elems));
   }
@@ -592,24 +606,19 @@ static ff_status ensure_ring(ff_handle *h, int W, int H) {
   const int slots = std::max(h->upd_batch, h->ring_slots);
   const size_t pix = std::max(npix, h->ring_pix);
   if (pix > h->ring_pix || slots > h->ring_slots) {
-    dev_free(h->d_ring_depth);
-    dev_free(h->d_ring_bgr);
-    h->d_ring_depth = nullptr;
-    h->d_ring_bgr = nullptr;
+    CK(drop(h, h->d_ring_depth, h->d_ring_bgr));
     h->ring_pix = 0;
     CK(alloc(&h->d_ring_depth, pix * slots));
     CK(alloc(&h->d_ring_bgr, pix * 3 * slots));
     if (h->d_ring_conf) {
-      dev_free(h->d_ring_conf);
-      h->d_ring_conf = nullptr;
+      CK(drop(h, h->d_ring_conf));
       h->ring_conf_pix = 0;
     }
     h->ring_pix = pix;
     h->ring_slots = slots;
   }
   if (need_conf && h->ring_conf_pix < h->ring_pix) {
-    dev_free(h->d_ring_conf);
-    h->d_ring_conf = nullptr;
+    CK(drop(h, h->d_ring_conf));
     CK(alloc(&h->d_ring_conf, h->ring_pix * h->ring_slots));
     h->ring_conf_pix = h->ring_pix;
   }
@@ -810,7 +819,7 @@ ff_status ff_destroy(ff_handle *h) {
                   h->d_upd_total, h->d_ring_depth, h->d_ring_bgr, h->d_ring_conf, h->d_seq_cand,
                   h->d_seq_bnd, h->d_seq_cnt, h->d_loop_map, h->d_loop_slots, h->d_loop_st, h->d_loop_sdf,
                   h->d_loop_wgt, h->d_loop_col, h->d_hseq_depth, h->d_hseq_bgr};
-  dev_free(ptrs, sizeof(ptrs) / sizeof(ptrs[0]));
+  if (dev_free(h, ptrs, sizeof(ptrs) / sizeof(ptrs[0])) != cudaSuccess) cudaGetLastError();  // (not given out again)
   for (int k = 0; k < 2; k++) {
     if (h->h_cnt_set[k]) cudaFreeHost(h->h_cnt_set[k]);
     if (h->h_batch_set[k]) cudaFreeHost(h->h_batch_set[k]);
@@ -912,11 +921,7 @@ ff_status ff_loop_begin(ff_handle *h, uint32_t capacity) {
   cudaStream_t s = h->stream;
   CK(cudaStreamSynchronize(s));
   if (capacity != h->loop_cap) {
-    dev_free(h->d_loop_sdf);
-    dev_free(h->d_loop_wgt);
-    dev_free(h->d_loop_col);
-    h->d_loop_sdf = h->d_loop_wgt = nullptr;
-    h->d_loop_col = nullptr;
+    CK(drop(h, h->d_loop_sdf, h->d_loop_wgt, h->d_loop_col));
     h->loop_cap = 0;
     CK(alloc(&h->d_loop_sdf, (size_t)capacity * 512));
     CK(alloc(&h->d_loop_wgt, (size_t)capacity * 512));
@@ -949,8 +954,7 @@ ff_status ff_loop_delete_frame(ff_handle *h, const float *d_depth, const uint8_t
   FCK(settle(h));
   cudaStream_t s = h->stream;
   if (n_queue > h->loop_slots_cap) {
-    dev_free(h->d_loop_slots);
-    h->d_loop_slots = nullptr;
+    CK(drop(h, h->d_loop_slots));
     h->loop_slots_cap = 0;
     CK(alloc(&h->d_loop_slots, (size_t)n_queue));
     h->loop_slots_cap = n_queue;
@@ -1107,10 +1111,7 @@ struct FramePlan {
 // The network's buffers: activations of `pixels`, confidence maps of `npx`.
 static ff_status ensure_network(ff_handle *h, size_t pixels, size_t npx) {
   if (pixels > h->net_cap) {
-    dev_free(h->d_feat);
-    dev_free(h->d_a1);
-    dev_free(h->d_a2);
-    h->d_feat = h->d_a1 = h->d_a2 = nullptr;
+    CK(drop(h, h->d_feat, h->d_a1, h->d_a2));
     h->net_cap = 0;
     CK(alloc(&h->d_feat, pixels * CNN_FEAT_CH));
     CK(alloc(&h->d_a1, pixels * CNN_HIDDEN));
@@ -1118,10 +1119,7 @@ static ff_status ensure_network(ff_handle *h, size_t pixels, size_t npx) {
     h->net_cap = pixels;
   }
   if (npx > h->conf_cap) {
-    for (int k = 0; k < 2; k++) {
-      dev_free(h->d_conf_set[k]);
-      h->d_conf_set[k] = nullptr;
-    }
+    CK(drop(h, h->d_conf_set[0], h->d_conf_set[1]));
     h->conf_cap = 0;
     CK(alloc(&h->d_conf_set[0], npx));
     CK(alloc(&h->d_conf_set[1], npx));
@@ -1160,9 +1158,7 @@ static ff_status frame_prepare(ff_handle *h, const uint16_t *d_depth, const uint
     std::vector<float> px(W), py(H);
     for (int x = 0; x < W; x++) px[x] = ((float)x - p.cx) / p.fx;
     for (int y = 0; y < H; y++) py[y] = ((float)y - p.cy) / p.fy;
-    dev_free(h->d_pxp);
-    dev_free(h->d_pyp);
-    h->d_pxp = h->d_pyp = nullptr;
+    CK(drop(h, h->d_pxp, h->d_pyp));
     CK(alloc(&h->d_pxp, W));
     CK(alloc(&h->d_pyp, H));
     CK(cudaMemcpyAsync(h->d_pxp, px.data(), sizeof(float) * W, cudaMemcpyHostToDevice, s));
@@ -1734,10 +1730,7 @@ static ff_status ensure_seq(ff_handle *h, int W, int H, int frames) {
   if (frames <= h->seq_frames && pix <= h->seq_pix && bnd <= h->seq_bnd) return FF_OK;
   const int nf = std::max(frames, h->seq_frames);
   const size_t np = std::max(pix, h->seq_pix), nb = std::max(bnd, h->seq_bnd);
-  dev_free(h->d_seq_cand);
-  dev_free(h->d_seq_bnd);
-  h->d_seq_cand = nullptr;
-  h->d_seq_bnd = nullptr;
+  CK(drop(h, h->d_seq_cand, h->d_seq_bnd));
   h->seq_frames = 0;
   CK(alloc(&h->d_seq_cand, np * nf));
   CK(alloc(&h->d_seq_bnd, nb * nf));
@@ -1980,10 +1973,7 @@ ff_status ff_add_map_sequence_u16(ff_handle *h, int n, const uint16_t *const *de
   const size_t npix = (size_t)width * height;
   const size_t frames = (size_t)std::min(n, BATCH_MAX);
   if (frames > h->hseq_frames || npix > h->hseq_pix) {
-    dev_free(h->d_hseq_depth);
-    dev_free(h->d_hseq_bgr);
-    h->d_hseq_depth = nullptr;
-    h->d_hseq_bgr = nullptr;
+    CK(drop(h, h->d_hseq_depth, h->d_hseq_bgr));
     h->hseq_frames = h->hseq_pix = 0;
     CK(alloc(&h->d_hseq_depth, frames * npix));
     CK(alloc(&h->d_hseq_bgr, frames * npix * 3));
@@ -2145,7 +2135,10 @@ ff_status ff_add_maps_u16_device(ff_handle *const *maps, int n, const uint16_t *
   }
   if (!use_graph) {
     st = issue();
-    if (st != FF_OK) return st;
+    if (st != FF_OK) {
+      cudaStreamSynchronize(lead->stream);  // (what was launched uses every map's memory)
+      return st;
+    }
   }
   CK(cudaStreamSynchronize(lead->stream));
   double bricks = 0, pending = 0;

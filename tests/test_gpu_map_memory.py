@@ -1,0 +1,67 @@
+"""The maps' device memory beside what else the process does."""
+import threading
+
+import numpy as np
+import pytest
+
+from tests.helpers import MAXCAM, SCALING, circle_frames
+
+pytestmark = pytest.mark.gpu
+
+
+def _make(leaves=30000):
+    from fastfusion_b200.fusion import FusionMipMapCPU
+    return FusionMipMapCPU(0, 0, 0, 0.005, 0.01, 0, True, leaves_max=leaves, branches_max=1 << 21, rcp="exact")
+
+
+def _fuse(m, n=4, wh=(160, 120)):
+    from fastfusion_b200.fusion import CameraInfo
+    K, frames = circle_frames(0, n, *wh)
+    m.addMapSequence([f[0] for f in frames], [CameraInfo(K, f[2], f[3]) for f in frames], [f[1] for f in frames],
+                     SCALING, MAXCAM)
+    return [np.array(x) for x in (*m.bricks(), *m.leaves())]
+
+
+def _same(a, b):
+    return all(x.shape == y.shape and x.tobytes() == y.tobytes() for x, y in zip(a, b))
+
+
+def test_closing_and_growing_while_another_thread_records(lib_built):
+    """A thread records a stream (thread-local mode, as this library's own
+    recordings) while another closes a map, makes one and grows its buffers: the
+    recording stays whole and the maps are right."""
+    import torch
+    m = _make()
+    want = _fuse(m)
+    x = torch.zeros(1000, device="cuda")
+    s = torch.cuda.Stream()
+    g = torch.cuda.CUDAGraph()
+    got, errors = [], []
+
+    def other():
+        try:
+            m.close()
+            k = _make()
+            _fuse(k, 2, (97, 61))
+            k.close()
+            k = _make()
+            got.append(_fuse(k))
+            k.close()
+        except Exception as e:  # (reported by the main thread)
+            errors.append(repr(e))
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        g.capture_begin(capture_error_mode="thread_local")
+        x.add_(1.0)
+        t = threading.Thread(target=other)
+        t.start()
+        t.join()
+        x.add_(1.0)
+        g.capture_end()
+    assert not errors, errors
+    for _ in range(3):
+        g.replay()
+    torch.cuda.synchronize()
+    assert float(x[0]) == 6.0
+    assert _same(got[0], want)
