@@ -219,6 +219,7 @@ static thread_local std::string g_create_error;
   do {                                                                                \
     cudaError_t e_ = (call);                                                          \
     if (e_ != cudaSuccess) {                                                          \
+      cudaGetLastError(); /* (reported here, not by the next call again) */           \
       h->err = std::string(#call) + ": " + cudaGetErrorString(e_);                    \
       return FF_ERR_CUDA;                                                             \
     }                                                                                 \
@@ -569,6 +570,8 @@ static ff_status ensure_image(ff_handle *h, int W, int H) {
   if (npix > h->cap_pix) {
     CK(drop(h, h->d_depth_set[0], h->d_depth_set[1], h->d_bgr_set[0], h->d_bgr_set[1], h->d_cand, h->d_pend,
             h->d_keys, h->d_sort_tmp));
+    h->cap_pix = 0;  // (until all of them are there)
+    select_set(h, h->set);
     for (int k = 0; k < 2; k++) {
       CK(alloc(&h->d_depth_set[k], npix));
       CK(alloc(&h->d_bgr_set[k], (size_t)npix * 3));
@@ -584,8 +587,9 @@ static ff_status ensure_image(ff_handle *h, int W, int H) {
   const size_t bnd_need = dedupe_boundary_elems(W, H);
   if (bnd_need > h->bnd_elems) {
     CK(drop(h, h->d_bnd));
+    h->bnd_elems = 0;
+    CK(alloc(&h->d_bnd, bnd_need));
     h->bnd_elems = bnd_need;
-    CK(alloc(&h->d_bnd, h->bnd_elems));
   }
   return FF_OK;
 }
@@ -610,15 +614,14 @@ static ff_status ensure_ring(ff_handle *h, int W, int H) {
     h->ring_pix = 0;
     CK(alloc(&h->d_ring_depth, pix * slots));
     CK(alloc(&h->d_ring_bgr, pix * 3 * slots));
-    if (h->d_ring_conf) {
-      CK(drop(h, h->d_ring_conf));
-      h->ring_conf_pix = 0;
-    }
+    CK(drop(h, h->d_ring_conf));
+    h->ring_conf_pix = 0;
     h->ring_pix = pix;
     h->ring_slots = slots;
   }
   if (need_conf && h->ring_conf_pix < h->ring_pix) {
     CK(drop(h, h->d_ring_conf));
+    h->ring_conf_pix = 0;
     CK(alloc(&h->d_ring_conf, h->ring_pix * h->ring_slots));
     h->ring_conf_pix = h->ring_pix;
   }
@@ -928,7 +931,8 @@ ff_status ff_loop_begin(ff_handle *h, uint32_t capacity) {
     CK(alloc(&h->d_loop_col, (size_t)capacity * 1536));
     h->loop_cap = capacity;
   }
-  if (!h->d_loop_map) {
+  if (!h->h_loop_st) {
+    CK(drop(h, h->d_loop_map, h->d_loop_st));
     CK(alloc(&h->d_loop_map, (size_t)h->cfg.leaves_max));
     CK(alloc(&h->d_loop_st, (size_t)4));
     CK(cudaMallocHost((void **)&h->h_loop_st, 4 * sizeof(uint32_t)));
@@ -1121,6 +1125,7 @@ static ff_status ensure_network(ff_handle *h, size_t pixels, size_t npx) {
   if (npx > h->conf_cap) {
     CK(drop(h, h->d_conf_set[0], h->d_conf_set[1]));
     h->conf_cap = 0;
+    h->d_conf = nullptr;
     CK(alloc(&h->d_conf_set[0], npx));
     CK(alloc(&h->d_conf_set[1], npx));
     h->d_conf = h->d_conf_set[h->set];
@@ -1159,6 +1164,7 @@ static ff_status frame_prepare(ff_handle *h, const uint16_t *d_depth, const uint
     for (int x = 0; x < W; x++) px[x] = ((float)x - p.cx) / p.fx;
     for (int y = 0; y < H; y++) py[y] = ((float)y - p.cy) / p.fy;
     CK(drop(h, h->d_pxp, h->d_pyp));
+    h->img_w = h->img_h = 0;
     CK(alloc(&h->d_pxp, W));
     CK(alloc(&h->d_pyp, H));
     CK(cudaMemcpyAsync(h->d_pxp, px.data(), sizeof(float) * W, cudaMemcpyHostToDevice, s));
@@ -1734,7 +1740,8 @@ static ff_status ensure_seq(ff_handle *h, int W, int H, int frames) {
   h->seq_frames = 0;
   CK(alloc(&h->d_seq_cand, np * nf));
   CK(alloc(&h->d_seq_bnd, nb * nf));
-  if (!h->d_seq_cnt) {
+  if (!h->h_seq_cnt) {
+    CK(drop(h, h->d_seq_cnt));
     CK(alloc(&h->d_seq_cnt, (size_t)BATCH_MAX));
     CK(cudaMemset(h->d_seq_cnt, 0, sizeof(Counters) * BATCH_MAX));
     CK(cudaMallocHost((void **)&h->h_seq_cnt, sizeof(Counters) * BATCH_MAX));

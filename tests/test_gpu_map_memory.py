@@ -65,3 +65,37 @@ def test_closing_and_growing_while_another_thread_records(lib_built):
     torch.cuda.synchronize()
     assert float(x[0]) == 6.0
     assert _same(got[0], want)
+
+
+def test_image_that_does_not_fit_leaves_the_map_usable(lib_built):
+    """The buffers of a larger image cannot be allocated (the device is full): the
+    call fails, again too, and the map goes on with the image size it had, is
+    closed, and leaves the next map unharmed."""
+    import torch
+    from fastfusion_b200.fusion import CameraInfo, FFError
+    k = _make()
+    want = _fuse(k, 8)
+    k.close()
+    K, frames = circle_frames(0, 8, 160, 120)
+    cams = [CameraInfo(K, R, t) for _, _, R, t in frames]
+    m = _make()
+    for (depth, bgr, _, _), cam in list(zip(frames, cams))[:3]:
+        m.addMap(depth, cam, bgr, SCALING, MAXCAM)
+    large = np.full((6000, 8000), 5000, np.uint16)  # 66 B of buffers per pixel, 3.2 GB
+    colour = np.zeros((6000, 8000, 3), np.uint8)
+    other = _make()
+    torch.cuda.synchronize()
+    full = torch.empty(torch.cuda.mem_get_info()[0] - (600 << 20), dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        with pytest.raises(FFError) as e:
+            m.addMap(large, cams[3], colour, SCALING, MAXCAM)
+        assert "out of memory" in str(e.value)
+    for (depth, bgr, _, _), cam in list(zip(frames, cams))[3:5]:
+        m.addMap(depth, cam, bgr, SCALING, MAXCAM)
+    m.addMapSequence([f[0] for f in frames[5:]], cams[5:], [f[1] for f in frames[5:]], SCALING, MAXCAM)
+    assert _same([np.array(x) for x in (*m.bricks(), *m.leaves())], want)
+    m.close()
+    del full
+    torch.cuda.empty_cache()
+    assert _same(_fuse(other, 8), want)
+    other.close()
