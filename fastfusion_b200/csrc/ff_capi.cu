@@ -140,7 +140,8 @@ struct ff_handle {
   float *d_conf = nullptr;
   size_t conf_cap = 0;  // pixels a confidence map holds
   size_t net_cap = 0;   // pixels the network's activations hold (of one image or several)
-  int conf_w = 0, conf_h = 0;  // size of the last confidence map
+  const float *conf_last = nullptr;  // the last finished frame's map (ff_get_confidence_map): a ring slot or a set's
+  int conf_w = 0, conf_h = 0;        // and its size
 
   // iterations after which a device-side wait gives up (ff_set_spin_limit),
   // and a failure the next frame reports as if a device wait had given up
@@ -615,12 +616,14 @@ static ff_status ensure_ring(ff_handle *h, int W, int H) {
     CK(alloc(&h->d_ring_depth, pix * slots));
     CK(alloc(&h->d_ring_bgr, pix * 3 * slots));
     CK(drop(h, h->d_ring_conf));
+    h->conf_last = nullptr;
     h->ring_conf_pix = 0;
     h->ring_pix = pix;
     h->ring_slots = slots;
   }
   if (need_conf && h->ring_conf_pix < h->ring_pix) {
     CK(drop(h, h->d_ring_conf));
+    h->conf_last = nullptr;
     h->ring_conf_pix = 0;
     CK(alloc(&h->d_ring_conf, h->ring_pix * h->ring_slots));
     h->ring_conf_pix = h->ring_pix;
@@ -1124,6 +1127,7 @@ static ff_status ensure_network(ff_handle *h, size_t pixels, size_t npx) {
   }
   if (npx > h->conf_cap) {
     CK(drop(h, h->d_conf_set[0], h->d_conf_set[1]));
+    h->conf_last = nullptr;
     h->conf_cap = 0;
     h->d_conf = nullptr;
     CK(alloc(&h->d_conf_set[0], npx));
@@ -1268,8 +1272,6 @@ static ff_status frame_prepare(ff_handle *h, const uint16_t *d_depth, const uint
       CK(cudaEventRecord(h->ev_cnn_done, cs));
       h->cnn_pending = true;
     }
-    h->conf_w = W;
-    h->conf_h = H;
     mf.conf = h->d_conf;
   }
   if (h->inject == FF_INJECT_CONFIDENCE_TIMEOUT && !(h->conf_tau_cm > 0.0f)) {
@@ -1549,6 +1551,11 @@ static ff_status frame_finish(ff_handle *h, const FramePlan &plan, MapFrame &mf,
   if (h->leaves_used > h->cfg.leaves_max) h->meshing_ok = false;
   h->queued = nq;
   h->d_queue_last = mf.queue;
+  if (mf.conf) {
+    h->conf_last = mf.conf;
+    h->conf_w = plan.W;
+    h->conf_h = plan.H;
+  }
   h->frames++;
   mesh_note_frame(h->mesh);
   if (queued) *queued = (int32_t)nq;
@@ -1768,11 +1775,8 @@ static ff_status network_buffers(ff_handle *h, int c, int W, int H, MapFrame *mf
   const size_t npx = (size_t)W * H;
   FCK(ensure_network(h, npx * network_images(c, npx), npx));
   for (int k = 0; k < c; k++) {
-    h->d_conf = h->d_ring_conf + (size_t)h->upd_pending * h->ring_pix + npx * k;
-    mf[k].conf = h->h_batch->f[k].conf = h->d_conf;
+    mf[k].conf = h->h_batch->f[k].conf = h->d_ring_conf + (size_t)h->upd_pending * h->ring_pix + npx * k;
   }
-  h->conf_w = W;
-  h->conf_h = H;
   return FF_OK;
 }
 
@@ -2559,13 +2563,13 @@ ff_status ff_set_confidence(ff_handle *h, const float *params, int n_params, flo
 
 ff_status ff_get_confidence_map(ff_handle *h, float *out, int *width, int *height) {
   if (!h) return FF_ERR_BAD_ARG;
-  if (!(h->conf_tau_cm > 0.0f) || !h->d_conf || !h->conf_w)
+  if (!(h->conf_tau_cm > 0.0f) || !h->conf_last)
     return set_err(h, FF_ERR_BAD_ARG, "ff_get_confidence_map: no learned weight or no frame yet");
   if (width) *width = h->conf_w;
   if (height) *height = h->conf_h;
   if (out) {
     CK(cudaSetDevice(h->cfg.device));
-    CK(cudaMemcpyAsync(out, h->d_conf, sizeof(float) * (size_t)h->conf_w * h->conf_h, cudaMemcpyDeviceToHost,
+    CK(cudaMemcpyAsync(out, h->conf_last, sizeof(float) * (size_t)h->conf_w * h->conf_h, cudaMemcpyDeviceToHost,
                        h->stream));
     CK(cudaStreamSynchronize(h->stream));
   }
