@@ -1112,6 +1112,7 @@ struct FramePlan {
   // the counters reach the host before the leaf finalisation: their queued
   // count does not yet hold the frame's new leaves
   bool counters_early = false;
+  bool skip_update = false;  // a sequence's frame behind the one that failed: placed, not updated
 };
 
 
@@ -1260,7 +1261,7 @@ static ff_status frame_prepare(ff_handle *h, const uint16_t *d_depth, const uint
     const int pc = h->prof.begin(ST_CONFIDENCE, cs);
     CK(cnn_features(d_depth, 1, W, H, scaling, kf, h->d_feat, cs));
     CK(cnn_forward(h->d_cnn_params, h->d_feat, 1, W, H, h->d_a1, h->d_a2, h->d_conf, h->conf_tau_cm,
-                   &h->d_cnt->cnn_error, cs));
+                   &h->d_cnt->cnn_error, 0, cs));
     if (h->inject == FF_INJECT_CONFIDENCE_TIMEOUT) {
       // the word the network sets when one of its waits gives up
       CK(cudaMemsetAsync(&h->d_cnt->cnn_error, 0xFF, sizeof(uint32_t), cs));
@@ -1480,7 +1481,7 @@ static ff_status frame_finish(ff_handle *h, const FramePlan &plan, MapFrame &mf,
   // as well); the call then reports FF_ERR_TIMEOUT.
   const bool insert_timeout = (hc.error & ERR_SPIN_TIMEOUT) != 0;
   const bool cnn_failed = hc.cnn_error != 0;
-  const bool skip_update = insert_timeout || cnn_failed;
+  const bool skip_update = insert_timeout || cnn_failed || plan.skip_update;
   const uint32_t leaves_before = plan.leaves_before;
   const int W = plan.W, H = plan.H;
   h->branches_used = std::min(hc.branches_used, h->cfg.branches_max);
@@ -1796,11 +1797,10 @@ static ff_status network_launch(ff_handle *h, int c, int W, int H, const uint16_
     const int pc = h->prof.begin(ST_CONFIDENCE, cs);
     CK(cnn_features_of(images, m, W, H, scaling, h->d_feat, cs));
     CK(cnn_forward(h->d_cnn_params, h->d_feat, m, W, H, h->d_a1, h->d_a2, const_cast<float *>(mf[i].conf),
-                   h->conf_tau_cm, &h->d_seq_cnt[0].cnn_error, cs));
+                   h->conf_tau_cm, &h->d_seq_cnt[i].cnn_error, (int)(sizeof(Counters) / sizeof(uint32_t)), cs));
     // depth -> features -> a1 -> a2 -> confidence, each written once and read once
     h->prof.end(pc, (double)npx * m * ((2 + 16) + (16 + 32) + (32 + 32) + (32 + 4)), cs);
   }
-  CK(cnn_spread_error(h->d_seq_cnt, c, cs));
   if (h->inject == FF_INJECT_CONFIDENCE_TIMEOUT) {
     // the first frame's network reports a wait that gave up
     CK(cudaMemsetAsync(&h->d_seq_cnt[0].cnn_error, 0xFF, sizeof(uint32_t), cs));
@@ -1887,10 +1887,21 @@ static ff_status sequence_chunk(ff_handle *h, bool after_pass, int c, const uint
   }
   CK(cudaMemcpyAsync(h->h_seq_cnt, h->d_seq_cnt, sizeof(Counters) * c, cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
+  // A network's wait that gave up may be known only after frames behind the
+  // failing one were placed and marked (the chain does not wait for the
+  // networks): none of them is updated, so their marks go, before any pass can
+  // run, and the bookkeeping of their bricks is done all the same.
+  int placed = 0, failed = c;
+  for (; placed < c && !(h->h_seq_cnt[placed].error & ERR_SEQ_HALT); placed++)
+    if (h->h_seq_cnt[placed].cnn_error) failed = std::min(failed, placed);
+  if (failed < placed) {
+    launch_unmark(h->d_upd_mask, h->d_upd_list, h->d_upd_count, (1u << (h->upd_pending + failed)) - 1u, s);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(s));
+  }
   h->seq_images = true;
   ff_status st = FF_OK;
-  for (int k = 0; k < c; k++) {
-    if (h->h_seq_cnt[k].error & ERR_SEQ_HALT) break;
+  for (int k = 0; k < placed; k++) {
     h->cur_slot = h->upd_pending;
     h->d_cnt = h->d_seq_cnt + k;
     h->h_cnt = h->h_seq_cnt + k;
@@ -1898,12 +1909,22 @@ static ff_status sequence_chunk(ff_handle *h, bool after_pass, int c, const uint
     plan[k].frame = h->frames + 1;
     plan[k].counters_early = false;  // read after the finalisation: the new leaves are counted
     h->pi_insert = pi_ins[k];        // (its bytes follow from the frame's counters)
-    st = frame_finish(h, plan[k], mf[k], -1, -1, queued ? queued + k : nullptr);
-    if (st != FF_OK) break;
-    done++;
+    plan[k].skip_update = k > failed;
+    const ff_status sk = frame_finish(h, plan[k], mf[k], -1, -1, queued && k <= failed ? queued + k : nullptr);
+    if (sk == FF_OK) {
+      done++;
+      continue;
+    }
+    if (st == FF_OK) st = sk;
+    if (k < failed || !h->h_seq_cnt[k].cnn_error) break;
   }
   h->seq_images = false;
   h->pi_insert = -1;
+  if (failed < placed && !h->upd_pending) {
+    // no pass follows that would empty the list
+    CK(join_fuse(h));
+    CK(cudaMemsetAsync(h->d_upd_count, 0, sizeof(uint32_t), s));
+  }
   // the next chunk's counters start clean of this one's halts
   CK(cudaMemsetAsync(h->d_seq_cnt, 0, sizeof(Counters) * c, s));
   return st;
@@ -2633,7 +2654,7 @@ ff_status ff_cnn_forward(const void *d_params, void *d_packed, const void *d_fea
   if (!d_params || !d_packed || !d_feat || !d_a1 || !d_a2 || !d_out || n <= 0 || width <= 0 || height <= 0)
     return cnn_bad("ff_cnn_forward: bad argument");
   CKN(cnn_forward((const __nv_bfloat16 *)d_params, (const __nv_bfloat16 *)d_feat, n, width, height,
-                  (__nv_bfloat16 *)d_a1, (__nv_bfloat16 *)d_a2, d_out, tau_m > 0.0f ? tau_m * 100.0f : 0.0f, nullptr,
+                  (__nv_bfloat16 *)d_a1, (__nv_bfloat16 *)d_a2, d_out, tau_m > 0.0f ? tau_m * 100.0f : 0.0f, nullptr, 0,
                   (cudaStream_t)stream));
   return FF_OK;
 }

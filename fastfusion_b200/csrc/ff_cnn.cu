@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
                                                              const __nv_bfloat16 *__restrict__ w,
                                                              const __nv_bfloat16 *__restrict__ bias,
                                                              void *__restrict__ out, float inv_tau,
-                                                             uint32_t *__restrict__ err) {
+                                                             uint32_t *__restrict__ err, int err_stride) {
   using I = CqIn<C>;
   using A = CqAcc<C, NB>;
   extern __shared__ __align__(1024) uint8_t rsm[];
@@ -467,7 +467,12 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (*stop && tid == 0 && err) atomicOr(err, ERR_SPIN_TIMEOUT);
+  if (*stop && tid == 0 && err) {
+    // every image the block had a share of
+    const int64_t of_image = (int64_t)strips * quads;
+    for (int64_t i = total * blockIdx.x / gridDim.x / of_image; i * of_image < total * (blockIdx.x + 1) / gridDim.x; i++)
+      atomicOr(err + i * err_stride, ERR_SPIN_TIMEOUT);
+  }
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(A::COLS));
 }
@@ -1500,11 +1505,11 @@ cudaError_t tile_map(CUtensorMap *m, const void *base, int C, int W, int H, int 
 
 template <int C, int NB, int MODE>
 void conv(const __nv_bfloat16 *in, int n, int W, int H, const __nv_bfloat16 *w, const __nv_bfloat16 *b, void *out,
-          float inv_tau, uint32_t *err, cudaStream_t s) {
+          float inv_tau, uint32_t *err, int err_stride, cudaStream_t s) {
   const int64_t quads = (int64_t)((W + CQ_OUT - 1) / CQ_OUT) * n * ((H + 3) / 4);
   note_launch();
   k_conv_quads<C, NB, MODE><<<(int)std::min<int64_t>(148, quads), CQ_THREADS, cq_smem_bytes<C, NB>(), s>>>(
-      in, W, H, n, w, b, out, inv_tau, err);
+      in, W, H, n, w, b, out, inv_tau, err, err_stride);
 }
 
 template <int IN>
@@ -1552,30 +1557,17 @@ cudaError_t cnn_features(const uint16_t *depth, int n, int W, int H, float scali
   return cudaSuccess;
 }
 
-// A batch's error word (the first frame's) in every frame of it: which image's
-// wait gave up is not known.
-__global__ void k_cnn_spread_error(Counters *cnt, int n) {
-  const uint32_t e = cnt[0].cnn_error;
-  if (e && (int)threadIdx.x < n) cnt[threadIdx.x].cnn_error = e;
-}
-
-cudaError_t cnn_spread_error(Counters *cnt, int n, cudaStream_t s) {
-  note_launch();
-  k_cnn_spread_error<<<1, 32, 0, s>>>(cnt, n);
-  return cudaGetLastError();
-}
-
 cudaError_t cnn_forward(const __nv_bfloat16 *params, const __nv_bfloat16 *feat, int n, int W, int H,
-                        __nv_bfloat16 *a1, __nv_bfloat16 *a2, float *out, float tau_cm, uint32_t *err,
+                        __nv_bfloat16 *a1, __nv_bfloat16 *a2, float *out, float tau_cm, uint32_t *err, int err_stride,
                         cudaStream_t s) {
   cudaError_t e = ensure_attrs();
   if (e != cudaSuccess) return e;
-  conv<8, 16, CONV_RELU_BF16>(feat, n, W, H, params + P_W1, params + P_B1, a1, 0.0f, err, s);
-  conv<16, 16, CONV_RELU_BF16>(a1, n, W, H, params + P_W2, params + P_B2, a2, 0.0f, err, s);
+  conv<8, 16, CONV_RELU_BF16>(feat, n, W, H, params + P_W1, params + P_B1, a1, 0.0f, err, err_stride, s);
+  conv<16, 16, CONV_RELU_BF16>(a1, n, W, H, params + P_W2, params + P_B2, a2, 0.0f, err, err_stride, s);
   if (tau_cm > 0.0f)
-    conv<16, 1, CONV_CONF>(a2, n, W, H, params + P_W3, params + P_B3, out, 1.0f / tau_cm, err, s);
+    conv<16, 1, CONV_CONF>(a2, n, W, H, params + P_W3, params + P_B3, out, 1.0f / tau_cm, err, err_stride, s);
   else
-    conv<16, 1, CONV_F32>(a2, n, W, H, params + P_W3, params + P_B3, out, 0.0f, err, s);
+    conv<16, 1, CONV_F32>(a2, n, W, H, params + P_W3, params + P_B3, out, 0.0f, err, err_stride, s);
   return cudaGetLastError();
 }
 

@@ -393,6 +393,19 @@ void launch_fuse_multi(const FuseBatch &fb, int storage, bool rcp_host, int grid
   }
 }
 
+// The marks of frames that will not be updated, taken away from the bricks listed
+// for the next pass (a brick without a mark left stays listed: the pass leaves
+// its voxels as they are).
+__global__ void k_unmark(uint32_t *mask, const uint32_t *list, const uint32_t *count, uint32_t keep) {
+  const uint32_t n = *count;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) mask[list[i]] &= keep;
+}
+
+void launch_unmark(uint32_t *mask, const uint32_t *list, const uint32_t *count, uint32_t keep, cudaStream_t s) {
+  note_launch();
+  k_unmark<<<148, 256, 0, s>>>(mask, list, count, keep);
+}
+
 // ---------------------------------------------------------------------------
 // Halo exchange of a sharded map: the bricks a part owns whose voxels changed
 // since its last export, as records (uint32 leaf index, 12 bytes of padding,

@@ -126,6 +126,8 @@ struct FuseBatch {
 
 // Launch the deferred update pass (grid: blocks of 512 threads).
 void launch_fuse_multi(const FuseBatch &fb, int storage, bool rcp_host, int grid, cudaStream_t s);
+// Deferred update: keep only the marks in `keep` of the listed bricks.
+void launch_unmark(uint32_t *mask, const uint32_t *list, const uint32_t *count, uint32_t keep, cudaStream_t s);
 
 // Loop closure: one fused frame removed into the loop arrays
 // (update8AddLoopSSESingleDeleteloop, loopclosure.cpp:15-228).
@@ -315,15 +317,14 @@ struct FeatureImages {
 };
 cudaError_t cnn_features_of(const FeatureImages &images, int n, int W, int H, float scaling, __nv_bfloat16 *feat,
                             cudaStream_t s);
-// The first frame's network error word copied to the other n - 1 frames' (n <= 32).
-cudaError_t cnn_spread_error(Counters *cnt, int n, cudaStream_t s);
 cudaError_t cnn_features(const uint16_t *depth, int n, int W, int H, float scaling, const float K[4],
                          __nv_bfloat16 *feat, cudaStream_t s);
 // tau_cm > 0: out = the confidence weight; else out = the network's output.
 // err (may be null): ERR_SPIN_TIMEOUT if a tensor-core wait gave up (the
-// layer's output is then NaN, or zero behind a ReLU).
+// layer's output is then NaN, or zero behind a ReLU); image i's word is
+// err[i * err_stride].
 cudaError_t cnn_forward(const __nv_bfloat16 *params, const __nv_bfloat16 *feat, int n, int W, int H,
-                        __nv_bfloat16 *a1, __nv_bfloat16 *a2, float *out, float tau_cm, uint32_t *err,
+                        __nv_bfloat16 *a1, __nv_bfloat16 *a2, float *out, float tau_cm, uint32_t *err, int err_stride,
                         cudaStream_t s);
 cudaError_t cnn_backward(const __nv_bfloat16 *params, const __nv_bfloat16 *feat, const __nv_bfloat16 *a1,
                          const __nv_bfloat16 *a2, const float *dpred, int n, int W, int H, float *g1, float *g2,

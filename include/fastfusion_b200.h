@@ -143,7 +143,10 @@ ff_status ff_add_map_u16_device(ff_handle *h, const uint16_t *d_depth, const uin
  * runs as one deferred pass before the call returns, so the images are free
  * then.  K + 4k, R + 9k, t + 3k: frame k's camera, as in ff_add_map_u16.
  * On an error the frames before the failing one are fused and queued[] of
- * the later ones is left unset.  The reference fuses one frame per call
+ * the later ones is left unset.  When the failing frame's confidence network
+ * gave up (FF_ERR_TIMEOUT), bricks of some frames behind it may be allocated
+ * as well, and those frames count in ff_stats.frames; none of them is updated,
+ * so the failing frame and the later ones can be added again.  The reference fuses one frame per call
  * (geometryfusion_mipmap_cpu.cpp:1603-2034); this is the frame-batched form. */
 ff_status ff_add_map_sequence_u16_device(ff_handle *h, int n, const uint16_t *const *d_depth,
                                          const uint8_t *const *d_bgr, int width, int height, const double *K,
