@@ -460,8 +460,9 @@ static ff_status grow(ff_handle *h, const int *box_min, const int *box_max) {
 // one map after another (a session per recording, say) does not pay the driver's
 // mapping and unmapping each time: creating, growing and destroying a map of
 // 30,000 bricks took 10.5 of a session's 16 ms.  What destroyed maps leave is kept
-// up to MAP_POOL_KEEP; above that it goes back at the next synchronisation, and
-// all of it does when an allocation fails.
+// up to MAP_POOL_KEEP (of a default map, 2 GB, half); above that it goes back as
+// the map is closed, and all of it does when an allocation of the maps or of the
+// mesher fails and with ff_release_memory.
 //
 // The memory can be used on every stream at once, as cudaMalloc's: the pool's
 // stream has waited for the block's last use.
@@ -499,6 +500,13 @@ static cudaError_t map_pool(MapPool &out) {
   return cudaSuccess;
 }
 
+cudaError_t ffb::trim_map_pool() {
+  MapPool P;
+  cudaError_t e = map_pool(P);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(P.stream);
+  return e == cudaSuccess ? cudaMemPoolTrimTo(P.pool, 0) : e;
+}
+
 static cudaError_t dev_malloc(void **p, size_t bytes) {
   *p = nullptr;
   MapPool P;
@@ -506,10 +514,10 @@ static cudaError_t dev_malloc(void **p, size_t bytes) {
   if (e != cudaSuccess) return e;
   e = cudaMallocFromPoolAsync(p, bytes, P.pool, P.stream);
   if (e == cudaErrorMemoryAllocation) {
-    // what the pool keeps may be in other sizes
+    // what the pools keep may be in other sizes
     cudaGetLastError();
-    cudaStreamSynchronize(P.stream);
-    cudaMemPoolTrimTo(P.pool, 0);
+    trim_map_pool();
+    trim_mesh_pool();
     e = cudaMallocFromPoolAsync(p, bytes, P.pool, P.stream);
   }
   if (e != cudaSuccess) {
@@ -858,6 +866,20 @@ ff_status ff_destroy(ff_handle *h) {
   if (h->ev_host_depth) cudaEventDestroy(h->ev_host_depth);
   if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
   delete h;
+  return FF_OK;
+}
+
+ff_status ff_release_memory(int device) {
+  int ndev = 0;
+  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0) {
+    cudaGetLastError();
+    return FF_ERR_NO_DEVICE;
+  }
+  if (device < 0 || device >= ndev) return FF_ERR_BAD_ARG;
+  if (cudaSetDevice(device) != cudaSuccess || trim_map_pool() != cudaSuccess || trim_mesh_pool() != cudaSuccess) {
+    cudaGetLastError();
+    return FF_ERR_CUDA;
+  }
   return FF_OK;
 }
 

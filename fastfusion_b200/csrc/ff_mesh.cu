@@ -2442,7 +2442,21 @@ static cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s) {
   cudaMemPool_t pool;
   cudaError_t e = pool_of_current_device(pool);
   if (e != cudaSuccess) return e;
-  return cudaMallocFromPoolAsync(p, bytes, pool, s);
+  e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  if (e == cudaErrorMemoryAllocation) {
+    // closed maps may have left what is missing
+    cudaGetLastError();
+    trim_map_pool();
+    e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  }
+  return e;
+}
+
+cudaError_t trim_mesh_pool() {
+  cudaMemPool_t pool;
+  cudaError_t e = pool_of_current_device(pool);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);  // (a closed map's buffers were freed on it)
+  return e == cudaSuccess ? cudaMemPoolTrimTo(pool, 0) : e;
 }
 
 template <typename T>

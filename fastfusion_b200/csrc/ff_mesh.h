@@ -72,4 +72,9 @@ void mesh_next_outputs(MeshState &m, const void **xyz, const void **rgb, const v
 void mesh_invalidate(MeshState &m);
 void mesh_note_frame(MeshState &m);
 
+// Give back to the driver what the current device's pools keep of freed
+// memory: the mesher's, and the maps' (ff_capi.cu).
+cudaError_t trim_mesh_pool();
+cudaError_t trim_map_pool();
+
 }  // namespace ffb

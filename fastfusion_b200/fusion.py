@@ -71,6 +71,7 @@ _vp, _i32, _u32, _u64, _f32, _sz = (ctypes.c_void_p, ctypes.c_int, ctypes.c_uint
 SIGNATURES = {
     "ff_create": (_i32, [ctypes.POINTER(ff_config), ctypes.POINTER(_vp)]),
     "ff_destroy": (_i32, [_vp]),
+    "ff_release_memory": (_i32, [_i32]),
     "ff_set_stream": (_i32, [_vp, _vp]),
     "ff_sync": (_i32, [_vp]),
     "ff_set_tuning": (_i32, [_vp, ctypes.POINTER(ff_tuning)]),
@@ -315,6 +316,13 @@ class MeshBuffer:
             self.close()
         except Exception:
             pass
+
+
+def release_memory(device: int = 0):
+    """Give back to the driver the device memory that closed maps left for later ones."""
+    st = load_library().ff_release_memory(device)
+    if st != FF_OK:
+        raise FFError(st, f"ff_release_memory({device}) failed")
 
 
 class FusionMipMapCPU:

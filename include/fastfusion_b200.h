@@ -94,8 +94,15 @@ typedef struct ff_stats {
  * (geometryfusion_mipmap_cpu.cpp:420-640). */
 ff_status ff_create(const ff_config *cfg, ff_handle **out);
 
-/* Destroy a map and free its device memory (~FusionMipMapCPU). */
+/* Destroy a map and free its device memory (~FusionMipMapCPU).  Up to 1 GB per
+ * device of what closed maps held, and what their mesh buffers held, stays with
+ * the process for the next maps; it goes back to the driver when an allocation
+ * of this library finds the device full, and with ff_release_memory. */
 ff_status ff_destroy(ff_handle *h);
+
+/* Give back to the driver the device memory that closed maps left for later
+ * ones (ff_destroy).  Open maps keep theirs.  No counterpart in the reference. */
+ff_status ff_release_memory(int device);
 
 /* Order this map's device work on the given cudaStream_t (NULL = the
  * library's own stream). */

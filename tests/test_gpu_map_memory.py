@@ -99,3 +99,49 @@ def test_image_that_does_not_fit_leaves_the_map_usable(lib_built):
     torch.cuda.empty_cache()
     assert _same(_fuse(other, 8), want)
     other.close()
+
+
+def test_kept_memory_is_given_back(lib_built):
+    """What closed maps leave: at most 1 GB at once (the rest is back when the
+    call returns), all of it with release_memory."""
+    import torch
+    from fastfusion_b200.fusion import release_memory
+    torch.cuda.synchronize()
+    k = _make()
+    _fuse(k)
+    k.updateMeshes()
+    k.close()
+    release_memory()
+    before = torch.cuda.mem_get_info()[0]
+    k = _make(leaves=400000)  # 2.9 GB
+    _fuse(k)
+    k.updateMeshes()
+    k.close()
+    assert before - torch.cuda.mem_get_info()[0] < (1 << 30) + (256 << 20)
+    release_memory()
+    assert before - torch.cuda.mem_get_info()[0] < 64 << 20
+
+
+def test_mesh_gets_what_closed_maps_left(lib_built):
+    """The device is full but for what closed maps left: a mesh update that needs
+    buffers gets them."""
+    import torch
+    from fastfusion_b200.fusion import release_memory
+    a, b = _make(60000), _make(60000)
+    for m in (a, b):
+        _fuse(m, 8, (640, 480))
+    b.updateMeshes()
+    want = b.getMeshInterleavedMarchingCubes()
+    b.close()
+    release_memory()
+    k = _make(120000)  # 0.9 GB
+    k.close()
+    torch.cuda.synchronize()
+    full = torch.empty(torch.cuda.mem_get_info()[0] - (4 << 20), dtype=torch.uint8, device="cuda")
+    a.updateMeshes()
+    del full
+    torch.cuda.empty_cache()
+    got = a.getMeshInterleavedMarchingCubes()
+    assert len(got.faces) > 0
+    assert got.vertices.tobytes() == want.vertices.tobytes() and np.array_equal(got.faces, want.faces)
+    a.close()
