@@ -337,7 +337,8 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
     const uint32_t count = (uint32_t)(seg.end - seg.r + segs);
     uint32_t sl = 0, par = 1;  // ring slot; parity of the wait for it (at once in the first turn)
     for (uint32_t g = 0; g < count; g++) {
-      if (!tc_wait(empty + sl, par, stop)) break;
+      // (the warp stops as one: its lanes meet below)
+      if (!__all_sync(0xffffffffu, tc_wait(empty + sl, par, stop))) break;
       uint8_t *d = ring + sl * I::QUAD;
       cq_store_px<C>(p[0], d + lrow * I::ROW + lpx * 16);
       cq_store_px<C>(p[1], d + (lrow + 1) * I::ROW + lpx * 16);
@@ -716,7 +717,7 @@ __global__ void __launch_bounds__(RC_THREADS, 1) k_grad_rows(const float *__rest
 #pragma unroll
       for (int k = 0; k < RC_AHEAD; k++) {
         if (g0 + (uint32_t)k >= count) break;
-        ok = tc_wait(empty + sl, par, stop);
+        ok = __all_sync(0xffffffffu, tc_wait(empty + sl, par, stop));  // (the warp stops as one: its lanes meet below)
         if (!ok) break;
         rc_store_px<IN>(p[k][0], dst + sl * I::PAIR);
         rc_store_px<IN>(p[k][1], dst + sl * I::PAIR + I::ROW);
