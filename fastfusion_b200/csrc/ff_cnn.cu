@@ -75,7 +75,7 @@ enum ConvMode { CONV_RELU_BF16 = 0, CONV_F32 = 1, CONV_CONF = 2 };
 // (an MMA about 75 cycles); a block per 128 x 8 pixels with one MMA per tap,
 // N = 16, took 34, 50 and 44 us.  On one image 11, 15 and 10 us against 13, 19
 // and 17.
-constexpr int TC_WAIT_LIMIT = 1 << 20;  // polls (a wait of these kernels takes microseconds)
+constexpr int TC_WAIT_LIMIT = 1 << 24;  // polls (a wait takes microseconds: one that gives up means a fault, not a slow device)
 constexpr int CQ_OUT = 128;      // output pixels of a strip
 constexpr int CQ_PX = 136;       // input pixels of a ring row: 128 + 4, whole 128-byte core matrices
 constexpr int CQ_PLANE = CQ_PX * 16;  // bytes of one 8-channel plane of an input row
