@@ -39,22 +39,24 @@ enum ConvMode { CONV_RELU_BF16 = 0, CONV_F32 = 1, CONV_CONF = 2 };
 // ------------------------------------------------ tensor-core convolution
 //
 // The forward layers as streamed implicit GEMMs on the 5th-generation tensor
-// cores.  Output rows come in groups of four
-// ("quads"): for input row t of the eight that a quad reads and for kernel
-// column kx, one tcgen05.mma (M = 128 pixels, K = 16, BF16, FP32 accumulator
-// in tensor memory) adds
-//   D[pixel p][j * NB + co] += sum over ci of x[t][p + kx][ci] * w[co][ci][t - j][kx]
-// for all four output rows j at once (NB = 16 columns a row, or 1 for the
-// one-channel output), zero where t - j is no row of the kernel.  The shift kx
-// is the start address of the A descriptor; the columns of a t are a window
-// into one strip of column blocks per kx (3 zero blocks, the five ky from the
-// last to the first, 3 zero blocks), so they are the start address of B's.
+// cores.  Output rows come in groups of four ("quads"): for input row t of the
+// eight that a quad reads and for kernel column kx, one tcgen05.mma (M = 128
+// pixels, K = 16, BF16, FP32 accumulator in tensor memory) adds
+//   D[pixel p][16 j + co] += sum over ci of x[t][p + kx][ci] * w[co][ci][t - j][kx]
+// for all output rows j at once that have row t in their window (one to four of
+// them: N = 16 to 64; a row's very first product is an MMA of its own, which
+// sets its columns).  The shift kx is the start address of the A descriptor; the
+// rows of a t are a window into one strip of five column blocks per kx, ky from
+// the last to the first, so they are the start address of B's.
 // Why: an M = 128 MMA reads (128 + N) x 32 bytes of operands from shared
 // memory, 128 bytes a cycle.  One MMA per tap with N = 16 takes 25 x 36 = 900
-// cycles a row; a quad takes 8 x 5 MMAs of 48 (N = 64), 480 a row, though 3 of
-// 8 of its columns' products are with zero blocks.  Every output is the sum of
-// its taps in raster order (K = 16 at a time, the zero blocks between them add
-// nothing), the order the activations' BF16 rounding is defined by.
+// cycles a row; a quad takes 43 MMAs of 36 to 48, 450 a row.  Only products of an
+// output's own window enter its sum, so that an infinite activation stays within
+// the outputs that see it (N = 64 throughout, with zero blocks for the rows out of
+// reach, multiplied it by zero elsewhere); and every output is the sum of its
+// taps in raster order (K = 16 at a time), the order the activations' BF16
+// rounding is defined by.  The one-channel layer runs in the same way, with 15 of
+// its 16 columns a row unused.
 //
 // Operands: K-major, unswizzled canonical layout (8 x 16-byte core matrices,
 // pixels 16 bytes apart, 8-pixel groups 128 (SBO), the two 8-channel halves
@@ -71,10 +73,10 @@ enum ConvMode { CONV_RELU_BF16 = 0, CONV_F32 = 1, CONV_CONF = 2 };
 // block's share running over from one strip to the next.  All waits are
 // bounded.
 //
-// Measured on four 640x480 images: layers 1, 2 and 3 take 25, 29 and 22 us
-// (an MMA about 75 cycles); a block per 128 x 8 pixels with one MMA per tap,
-// N = 16, took 34, 50 and 44 us.  On one image 11, 15 and 10 us against 13, 19
-// and 17.
+// Measured on four 640x480 images: layers 1, 2 and 3 take 25, 29 and 25 us; with
+// zero blocks, 40 MMAs of N = 64 a quad (N = 16 for layer 3, four columns used),
+// 26, 29 and 21; a block per 128 x 8 pixels with one MMA per tap, N = 16, 34, 50
+// and 44.  On one image 11, 13 and 13 us against 12, 15 and 10, and 13, 19 and 17.
 constexpr int TC_WAIT_LIMIT = 1 << 24;  // polls (a wait takes microseconds: one that gives up means a fault, not a slow device)
 constexpr int CQ_OUT = 128;      // output pixels of a strip
 constexpr int CQ_PX = 136;       // input pixels of a ring row: 128 + 4, whole 128-byte core matrices
@@ -91,18 +93,16 @@ struct CqIn {
   static constexpr int QUAD = 4 * ROW;
   static constexpr int NKX = C == 8 ? 3 : 5;  // MMAs per t
 };
-// NB: columns of an output row (its channels, 16 or 1)
-template <int C, int NB>
-struct CqAcc {
-  static constexpr int N = NB == 1 ? 16 : 64;  // columns of an MMA and of an accumulator
-  static constexpr int COLS = CQ_MMA_WARPS * N;
-  // columns of a kx's weight strip: 11 blocks (NB = 1: and the rest of the last window)
-  static constexpr int STRIP = NB == 1 ? 24 : 11 * 16;
-  static constexpr int WBYTES = CqIn<C>::NKX * STRIP * 32;
-};
-template <int C, int NB>
+constexpr int CQ_ACC = 4 * 16;     // columns of an accumulator
+constexpr int CQ_COLS = CQ_MMA_WARPS * CQ_ACC;
+constexpr int CQ_STRIP = 5 * 16;   // columns of a kx's weight strip: a block per ky
+template <int C>
+__host__ __device__ constexpr int cq_weight_bytes() {
+  return CqIn<C>::NKX * CQ_STRIP * 32;
+}
+template <int C>
 constexpr size_t cq_smem_bytes() {
-  return (size_t)CQ_SLOTS * CqIn<C>::QUAD + CqAcc<C, NB>::WBYTES + 256;
+  return (size_t)CQ_SLOTS * CqIn<C>::QUAD + cq_weight_bytes<C>() + 256;
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -114,9 +114,8 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t addr, uint32_t lbo, uint32_
 }
 
 // instruction descriptor: D FP32, A and B BF16, both K-major, M = 128
-template <int N>
-__host__ __device__ constexpr uint32_t tc_idesc() {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
+__host__ __device__ constexpr uint32_t tc_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((128u >> 4) << 24);
 }
 
 // TMA tile loads and a bulk copy, completing on an mbarrier (transaction bytes)
@@ -166,6 +165,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t addr, uint32_t (&v)[16]) {
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
         "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
       : "r"(addr));
+}
+__device__ __forceinline__ void tmem_ld1(uint32_t addr, uint32_t &v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(addr));
 }
 __device__ __forceinline__ void tc_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -233,35 +235,36 @@ __device__ __forceinline__ void cq_store_px(const CqPx<C> &p, uint8_t *d) {
   for (int k = 0; k < C / 8; k++) *reinterpret_cast<uint4 *>(d + k * CQ_PLANE) = p.v[k];
 }
 
-// Element (column n, k) of MMA column kxi's weight strip.  Block i of a strip
-// holds ky = 7 - i (zero unless 0 .. 4), its columns the output channels; k is
-// the input channel (8 channels: of pixel kx = 2 kxi, then of kx + 1).
-template <int C, int NB>
+// Element (column n, k) of MMA column kxi's weight strip, for COUT output
+// channels.  Block i of a strip holds ky = 4 - i, its columns the output channels
+// (zero from COUT on); k is the input channel (8 channels: of pixel kx = 2 kxi,
+// then of kx + 1).
+template <int C, int COUT>
 __device__ __forceinline__ __nv_bfloat16 cq_weight(const __nv_bfloat16 *__restrict__ w, int kxi, int n, int k) {
   constexpr int CIN = C == 8 ? CNN_IN : CNN_HID;
-  const int co = n % NB, ky = 7 - n / NB, kx = C == 8 ? 2 * kxi + (k >> 3) : kxi, ci = k % C;
-  if (ky < 0 || ky > 4 || kx > 4 || ci >= CIN) return __float2bfloat16_rn(0.0f);
+  const int co = n & 15, ky = 4 - (n >> 4), kx = C == 8 ? 2 * kxi + (k >> 3) : kxi, ci = k % C;
+  if (co >= COUT || kx > 4 || ci >= CIN) return __float2bfloat16_rn(0.0f);
   return __ldg(w + (co * CIN + ci) * TAPS + ky * 5 + kx);
 }
 
-template <int C, int NB, int MODE>
+template <int C, int COUT, int MODE>
 __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat16 *__restrict__ in, int W, int H, int n_img,
                                                              const __nv_bfloat16 *__restrict__ w,
                                                              const __nv_bfloat16 *__restrict__ bias,
                                                              void *__restrict__ out, float inv_tau,
                                                              uint32_t *__restrict__ err, int err_stride) {
   using I = CqIn<C>;
-  using A = CqAcc<C, NB>;
+  constexpr int WBYTES = cq_weight_bytes<C>();
   extern __shared__ __align__(1024) uint8_t rsm[];
   uint8_t *ring = rsm;
   uint8_t *wsm = rsm + CQ_SLOTS * I::QUAD;  // [kx][k half][strip column][8] bf16
-  uint64_t *full = reinterpret_cast<uint64_t *>(wsm + A::WBYTES);
+  uint64_t *full = reinterpret_cast<uint64_t *>(wsm + WBYTES);
   uint64_t *empty = full + CQ_SLOTS, *dfull = empty + CQ_SLOTS, *dempty = dfull + CQ_MMA_WARPS,
            *drain = dempty + CQ_MMA_WARPS;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
   volatile uint32_t *stop = tmem_slot + 1;
   static_assert((2 * CQ_SLOTS + 2 * CQ_MMA_WARPS + 2) * 8 <= 256, "barrier words");
-  static_assert(I::QUAD % 128 == 0 && A::WBYTES % 16 == 0, "operand alignment");
+  static_assert(I::QUAD % 128 == 0 && WBYTES % 16 == 0, "operand alignment");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool loader = warp >= CQ_EPI_WARPS && warp < CQ_EPI_WARPS + CQ_LOAD_WARPS;
   const int quads = (H + 3) / 4, strips = (W + CQ_OUT - 1) / CQ_OUT;
@@ -295,14 +298,14 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
     fetch();
   } else {
     // (a thread's weights in flight together)
-    constexpr int SETUP = CQ_THREADS - 32 * CQ_LOAD_WARPS, WN = A::WBYTES / 2, PER = (WN + SETUP - 1) / SETUP;
+    constexpr int SETUP = CQ_THREADS - 32 * CQ_LOAD_WARPS, WN = WBYTES / 2, PER = (WN + SETUP - 1) / SETUP;
     const int t = warp < CQ_EPI_WARPS ? tid : tid - 32 * CQ_LOAD_WARPS;
 #pragma unroll 8
     for (int k = 0; k < PER; k++) {
-      const int i = t + k * SETUP, r = (i >> 3) / A::STRIP;
+      const int i = t + k * SETUP, r = (i >> 3) / CQ_STRIP;
       if (i < WN)
         reinterpret_cast<__nv_bfloat16 *>(wsm)[i] =
-            cq_weight<C, NB>(w, r >> 1, (i >> 3) % A::STRIP, (r & 1) * 8 + (i & 7));
+            cq_weight<C, COUT>(w, r >> 1, (i >> 3) % CQ_STRIP, (r & 1) * 8 + (i & 7));
     }
     // (the ring's pixels 132 .. 135 are never written: the 8-channel layer's
     // last tap pair reads pixel 132 against zero weights)
@@ -311,7 +314,7 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
         *reinterpret_cast<uint4 *>(ring + (i >> 2) * I::ROW + (132 + (i & 3)) * 16) = make_uint4(0u, 0u, 0u, 0u);
     if (warp == 0) {
       asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
-                   "r"(A::COLS));
+                   "r"(CQ_COLS));
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 32) {
@@ -357,7 +360,7 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
       // output quad that reads it, or, reading none of it, after it has
       // passed; so no phase of a slot is missed.
       const uint32_t m = (uint32_t)(warp - CQ_EPI_WARPS - CQ_LOAD_WARPS);
-      const uint32_t rbase = smem_addr(ring), wbase = smem_addr(wsm), acc = tmem + m * A::N;
+      const uint32_t rbase = smem_addr(ring), wbase = smem_addr(wsm), acc = tmem + m * CQ_ACC;
       uint32_t g = 0, dpar = 1;  // the segment's first input quad; parity of the wait for the accumulator
       bool ok = true;
       auto wait_full = [&](uint32_t gi) { return tc_wait(full + gi % CQ_SLOTS, (gi / CQ_SLOTS) & 1, stop); };
@@ -382,13 +385,26 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t s0 = rbase + gi % CQ_SLOTS * I::QUAD, s1 = rbase + (gi + 1) % CQ_SLOTS * I::QUAD;
           constexpr int KXS = C == 8 ? 32 : 16, LBO = C == 8 ? 16 : CQ_PLANE;
-          for (int t = 0; t < 8; t++) {
-            const uint32_t rb = (t < 4 ? s0 : s1) + (t & 3) * I::ROW;
-            const uint32_t wb = wbase + (uint32_t)((7 - t) * NB * 16);
 #pragma unroll
-            for (int kx = 0; kx < I::NKX; kx++)
-              tc_mma(acc, tc_desc(rb + kx * KXS, LBO, 128), tc_desc(wb + kx * A::STRIP * 32, A::STRIP * 16, 128),
-                     tc_idesc<A::N>(), (kx || t) ? 1u : 0u);
+          for (int t = 0; t < 8; t++) {
+            // output rows j0 .. j1, from block 4 - t + j0 (ky = t - j0) on
+            const int j0 = max(t - 4, 0), j1 = min(t, 3);
+            const uint32_t rb = (t < 4 ? s0 : s1) + (t & 3) * I::ROW;
+#pragma unroll
+            for (int kx = 0; kx < I::NKX; kx++) {
+              const uint64_t ad = tc_desc(rb + kx * KXS, LBO, 128);
+              const uint32_t wk = wbase + (uint32_t)(kx * CQ_STRIP * 32);
+              auto mma = [&](int j, int rows, uint32_t accumulate) {
+                tc_mma(acc + 16 * j, ad, tc_desc(wk + (uint32_t)((4 - t + j) * 256), CQ_STRIP * 16, 128),
+                       tc_idesc(16 * rows), accumulate);
+              };
+              if (t < 4 && kx == 0) {  // row t's first product
+                if (t) mma(0, t, 1u);
+                mma(t, 1, 0u);
+              } else {
+                mma(j0, j1 - j0 + 1, 1u);
+              }
+            }
           }
           tc_commit(dfull + m);
           // the input quads this issuer's next output quad does not read
@@ -407,9 +423,9 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
     // accumulators in turn, from the first in every segment
     const int quad = warp & 3, row0 = (warp >> 2) * 2;
     const uint32_t trow = tmem + ((uint32_t)(32 * quad) << 16);
-    float b[NB];
+    float b[COUT];
 #pragma unroll
-    for (int k = 0; k < NB; k++) b[k] = __bfloat162float(__ldg(bias + k));
+    for (int k = 0; k < COUT; k++) b[k] = __bfloat162float(__ldg(bias + k));
     uint32_t par = 0;  // bit d: parity of the next wait for accumulator d
     while (seg.r < seg.end) {
       cq_seg(seg, quads, strips);
@@ -422,12 +438,14 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
         const bool ok = tc_wait(dfull + d, (par >> d) & 1, stop);
         __syncwarp();  // (the reads of tensor memory are by whole warps)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        uint32_t v[2][16];
-        if constexpr (NB == 1) {
-          tmem_ld16(trow + d * A::N, v[0]);  // column j: output row j
+        uint32_t v[2][COUT];
+        const uint32_t at = trow + d * CQ_ACC + row0 * 16;
+        if constexpr (COUT == 1) {
+          tmem_ld1(at, v[0][0]);
+          tmem_ld1(at + 16, v[1][0]);
         } else {
-          tmem_ld16(trow + d * A::N + row0 * 16, v[0]);
-          tmem_ld16(trow + d * A::N + row0 * 16 + 16, v[1]);
+          tmem_ld16(at, v[0]);
+          tmem_ld16(at + 16, v[1]);
         }
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -438,8 +456,8 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
         for (int r = 0; r < 2; r++) {
           if (!inside[r]) continue;
           const size_t px = px0 + (size_t)r * W;
-          if constexpr (NB == 1) {
-            float a = __uint_as_float(row0 ? v[0][2 + r] : v[0][r]) + b[0];
+          if constexpr (COUT == 1) {
+            float a = __uint_as_float(v[r][0]) + b[0];
             if (!ok) a = __uint_as_float(0x7FC00000u);  // NaN: the accumulators were not read
             if (MODE == CONV_CONF) {
               // (1 - r/tau)^2 on [0, tau], 0 beyond: weight falls to exactly zero
@@ -475,7 +493,7 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
       atomicOr(err + i * err_stride, ERR_SPIN_TIMEOUT);
   }
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(A::COLS));
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(CQ_COLS));
 }
 
 // ------------------------------------------------ tensor-core input gradients
@@ -772,7 +790,7 @@ __global__ void __launch_bounds__(RC_THREADS, 1) k_grad_rows(const float *__rest
 #pragma unroll
             for (int ky = 0; ky < I::KY; ky++)
               tc_mma(tmem + m * N, tc_desc(rb[ky] + part * 2 * RC_PLANE, RC_PLANE, 128),
-                     tc_desc(wbase + (uint32_t)(ky * 2 * N * 16), N * 16, 128), tc_idesc<N>(),
+                     tc_desc(wbase + (uint32_t)(ky * 2 * N * 16), N * 16, 128), tc_idesc(N),
                      (ky || part < I::PARTS - 1) ? 1u : 0u);
           tc_commit(dfull + m);
           // the input pairs this issuer's next row does not read
@@ -916,7 +934,7 @@ static_assert(wg_smem_bytes<WG_L1>() > 114 * 1024 && wg_smem_bytes<WG_L2>() > 11
 // M = 128, D FP32, A and B BF16, both M/N-major
 template <int N>
 __host__ __device__ constexpr uint32_t wg_idesc() {
-  return tc_idesc<N>() | (1u << 15) | (1u << 16);
+  return tc_idesc(N) | (1u << 15) | (1u << 16);
 }
 
 template <int KIND>
@@ -1417,10 +1435,10 @@ namespace {
 std::mutex g_attr_mu;
 unsigned long long g_attr_done = 0;  // devices whose kernels have their shared-memory limits set
 
-template <int C, int NB, int MODE>
+template <int C, int COUT, int MODE>
 cudaError_t set_conv_attr() {
-  return cudaFuncSetAttribute(k_conv_quads<C, NB, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)cq_smem_bytes<C, NB>());
+  return cudaFuncSetAttribute(k_conv_quads<C, COUT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)cq_smem_bytes<C>());
 }
 template <int IN>
 cudaError_t set_grad_attr() {
@@ -1504,12 +1522,12 @@ cudaError_t tile_map(CUtensorMap *m, const void *base, int C, int W, int H, int 
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-template <int C, int NB, int MODE>
+template <int C, int COUT, int MODE>
 void conv(const __nv_bfloat16 *in, int n, int W, int H, const __nv_bfloat16 *w, const __nv_bfloat16 *b, void *out,
           float inv_tau, uint32_t *err, int err_stride, cudaStream_t s) {
   const int64_t quads = (int64_t)((W + CQ_OUT - 1) / CQ_OUT) * n * ((H + 3) / 4);
   note_launch();
-  k_conv_quads<C, NB, MODE><<<(int)std::min<int64_t>(148, quads), CQ_THREADS, cq_smem_bytes<C, NB>(), s>>>(
+  k_conv_quads<C, COUT, MODE><<<(int)std::min<int64_t>(148, quads), CQ_THREADS, cq_smem_bytes<C>(), s>>>(
       in, W, H, n, w, b, out, inv_tau, err, err_stride);
 }
 
