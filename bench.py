@@ -84,7 +84,7 @@ STAGE_KERNELS = {
     "mesh_cells": "k_keep_cells+k_gen_levels+k_cell_keys+argsort (k_sort_small or k_rs_*)+k_merge_cells/k_gather_cells",
     "mesh_count": "k_mesh_count",
     "mesh_emit": "k_mesh_emit",
-    "confidence": "k_cnn_features+k_conv x3 (learned weight)",
+    "confidence": "k_cnn_features+k_conv_quads x3 (learned weight)",
 }
 
 

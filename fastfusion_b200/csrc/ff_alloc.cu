@@ -128,9 +128,13 @@ __device__ __forceinline__ void grid_barrier(uint32_t *bar, uint32_t nblocks, Co
 }
 
 constexpr int DD_WARPS = 8;  // tiles (warps) per block
-// blocks that share one launch, per SM (the launch bounds below keep them
-// resident): at 64 registers, so that eight maps of mixed sizes (3,750 tiles of 32
-// rows) fit one launch (91 us in two, 74 in one), and three 1280x960 frames
+// Blocks that share one launch, per SM.  A launch's tiles must all be resident, and
+// frames that do not fit one launch pay its rounds of barriers again, so as
+// many blocks as the registers allow without spilling in the rows' loop: 64 a
+// thread, 256 threads, four blocks fill the register file (the launch bounds below
+// keep them resident; their scratch is 147 of the 228 KB).  4,736 tiles a launch:
+// eight maps of mixed sizes (3,750 tiles of 32 rows) take 74 us; at three blocks,
+// in two launches, 91.
 constexpr int DD_BLOCKS_PER_SM = 4;
 // the largest image, in warps per SM
 constexpr int DD_IMAGE_WARPS_PER_SM = 24;

@@ -186,8 +186,8 @@ struct ff_handle {
   bool seq_images = false;             // the frames being finished are a sequence's (caller images)
 
   // a sequence of one map's frames (ff_add_map_sequence_u16_device): per
-  // frame its voxel keys, processed flags, de-duplication boundaries and
-  // counters (device, and a pinned mirror)
+  // frame its list of cells, de-duplication boundaries and counters (device,
+  // and a pinned mirror)
   int seq_frames = 0;
   size_t seq_pix = 0, seq_bnd = 0;
   uint4 *d_seq_cand = nullptr;
@@ -1390,7 +1390,7 @@ static ff_status frame_issue(ff_handle *lead, int n, const LaunchPlan &lp, bool 
     for (size_t g = 0; g < lp.groups.size(); g++)
       CK(launch_dedupe(lead->h_batch, lead->d_batch, (int)lp.groups[g][0], (int)lp.groups[g][1], lp.groups[g][2], lp.rows,
                        lead->d_barrier + 8 * g, lead->cfg.device, s));
-  lead->prof.end(pi, lp.npix * 2, s);  // the depth image read (the keys and flags it writes stay in L2)
+  lead->prof.end(pi, lp.npix * 2, s);  // the depth image read (the list of cells it writes stays in L2)
   if (!insert) {
     CK(cudaGetLastError());
     return FF_OK;

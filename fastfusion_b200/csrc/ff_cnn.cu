@@ -148,7 +148,8 @@ __device__ __forceinline__ uint32_t mbar_wait(uint32_t bar, uint32_t parity) {
 }
 
 // The three BF16 parts of v (bit patterns in the upper halves): v = hi + mid +
-// lo exactly; an infinity or a NaN stays in hi alone.
+// lo, exactly down to 2^-110 (below that the low part leaves BF16's range); an
+// infinity or a NaN stays in hi alone.
 __device__ __forceinline__ void split3_bf16(float v, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
   hi = __float_as_uint(v) & 0xFFFF0000u;
   float r = v - __uint_as_float(hi);
