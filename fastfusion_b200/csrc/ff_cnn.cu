@@ -52,11 +52,14 @@ enum ConvMode { CONV_RELU_BF16 = 0, CONV_F32 = 1, CONV_CONF = 2 };
 // memory, 128 bytes a cycle.  One MMA per tap with N = 16 takes 25 x 36 = 900
 // cycles a row; a quad takes 43 MMAs of 36 to 48, 450 a row.  Only products of an
 // output's own window enter its sum, so that an infinite activation stays within
-// the outputs that see it (N = 64 throughout, with zero blocks for the rows out of
-// reach, multiplied it by zero elsewhere); and every output is the sum of its
-// taps in raster order (K = 16 at a time), the order the activations' BF16
-// rounding is defined by.  The one-channel layer runs in the same way, with 15 of
-// its 16 columns a row unused.
+// the outputs that see it; and every output is the sum of its taps in raster
+// order (K = 16 at a time), the order the activations' BF16 rounding is defined by.
+//
+// The one-channel layer packs the four rows' columns into one N = 16, the smallest:
+// 40 MMAs of 36 a quad, 360 a row, the strips with zeros for the rows that row t
+// is no part of, which add nothing as long as the input is finite.  Loader warps note
+// where it is not, and a quad that reads such values takes its rows one by one
+// (100 MMAs).
 //
 // Operands: K-major, unswizzled canonical layout (8 x 16-byte core matrices,
 // pixels 16 bytes apart, 8-pixel groups 128 (SBO), the two 8-channel halves
@@ -73,10 +76,11 @@ enum ConvMode { CONV_RELU_BF16 = 0, CONV_F32 = 1, CONV_CONF = 2 };
 // block's share running over from one strip to the next.  All waits are
 // bounded.
 //
-// Measured on four 640x480 images: layers 1, 2 and 3 take 25, 29 and 25 us; with
-// zero blocks, 40 MMAs of N = 64 a quad (N = 16 for layer 3, four columns used),
-// 26, 29 and 21; a block per 128 x 8 pixels with one MMA per tap, N = 16, 34, 50
-// and 44.  On one image 11, 13 and 13 us against 12, 15 and 10, and 13, 19 and 17.
+// Measured on four 640x480 images: layers 1, 2 and 3 take 25, 29 and 22 us, on one
+// image 11, 14 and 10; layers 1 and 2 with N = 64 throughout (40 MMAs a quad, zeros
+// for the rows out of reach, by which an infinite activation is multiplied) 26 and
+// 29, and 12 and 15; layer 3 with 16 columns a row (N = 16 to 64) 25 and 13; a block
+// per 128 x 8 pixels with one MMA per tap, N = 16, 34, 50 and 44, and 13, 19 and 17.
 constexpr int TC_WAIT_LIMIT = 1 << 24;  // polls (a wait takes microseconds: one that gives up means a fault, not a slow device)
 constexpr int CQ_OUT = 128;      // output pixels of a strip
 constexpr int CQ_PX = 136;       // input pixels of a ring row: 128 + 4, whole 128-byte core matrices
@@ -95,14 +99,19 @@ struct CqIn {
 };
 constexpr int CQ_ACC = 4 * 16;     // columns of an accumulator
 constexpr int CQ_COLS = CQ_MMA_WARPS * CQ_ACC;
-constexpr int CQ_STRIP = 5 * 16;   // columns of a kx's weight strip: a block per ky
-template <int C>
-__host__ __device__ constexpr int cq_weight_bytes() {
-  return CqIn<C>::NKX * CQ_STRIP * 32;
+// columns of a kx's weight strip: a block of 16 per ky; one output channel: 3 zeros,
+// a column per ky, zeros
+template <int COUT>
+__host__ __device__ constexpr int cq_strip() {
+  return COUT == 1 ? 24 : 5 * 16;
 }
-template <int C>
+template <int C, int COUT>
+__host__ __device__ constexpr int cq_weight_bytes() {
+  return CqIn<C>::NKX * cq_strip<COUT>() * 32;
+}
+template <int C, int COUT>
 constexpr size_t cq_smem_bytes() {
-  return (size_t)CQ_SLOTS * CqIn<C>::QUAD + cq_weight_bytes<C>() + 256;
+  return (size_t)CQ_SLOTS * CqIn<C>::QUAD + cq_weight_bytes<C, COUT>() + 256;
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -236,15 +245,28 @@ __device__ __forceinline__ void cq_store_px(const CqPx<C> &p, uint8_t *d) {
   for (int k = 0; k < C / 8; k++) *reinterpret_cast<uint4 *>(d + k * CQ_PLANE) = p.v[k];
 }
 
-// Element (column n, k) of MMA column kxi's weight strip, for COUT output
-// channels.  Block i of a strip holds ky = 4 - i, its columns the output channels
-// (zero from COUT on); k is the input channel (8 channels: of pixel kx = 2 kxi,
-// then of kx + 1).
+// The largest of m's and a pixel's values as bit patterns (halves): from 0x7F80 on
+// infinite, NaN or, behind a ReLU not met, negative.
+template <int C>
+__device__ __forceinline__ uint32_t cq_largest(const CqPx<C> &p, uint32_t m) {
+#pragma unroll
+  for (int k = 0; k < C / 8; k++) {
+    m = __vimax3_u16x2(m, p.v[k].x, p.v[k].y);
+    m = __vimax3_u16x2(m, p.v[k].z, p.v[k].w);
+  }
+  return m;
+}
+
+// Element (column n, k) of MMA column kxi's weight strip.  16 output channels:
+// block i of a strip holds ky = 4 - i, its columns the output channels; one:
+// column i holds ky = 7 - i (zero unless 0 .. 4).  k is the input channel (8
+// channels: of pixel kx = 2 kxi, then of kx + 1).
 template <int C, int COUT>
 __device__ __forceinline__ __nv_bfloat16 cq_weight(const __nv_bfloat16 *__restrict__ w, int kxi, int n, int k) {
   constexpr int CIN = C == 8 ? CNN_IN : CNN_HID;
-  const int co = n & 15, ky = 4 - (n >> 4), kx = C == 8 ? 2 * kxi + (k >> 3) : kxi, ci = k % C;
-  if (co >= COUT || kx > 4 || ci >= CIN) return __float2bfloat16_rn(0.0f);
+  const int co = COUT == 1 ? 0 : n & 15, ky = COUT == 1 ? 7 - n : 4 - (n >> 4);
+  const int kx = C == 8 ? 2 * kxi + (k >> 3) : kxi, ci = k % C;
+  if (ky < 0 || ky > 4 || kx > 4 || ci >= CIN) return __float2bfloat16_rn(0.0f);
   return __ldg(w + (co * CIN + ci) * TAPS + ky * 5 + kx);
 }
 
@@ -255,7 +277,7 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
                                                              void *__restrict__ out, float inv_tau,
                                                              uint32_t *__restrict__ err, int err_stride) {
   using I = CqIn<C>;
-  constexpr int WBYTES = cq_weight_bytes<C>();
+  constexpr int STRIP = cq_strip<COUT>(), WBYTES = cq_weight_bytes<C, COUT>();
   extern __shared__ __align__(1024) uint8_t rsm[];
   uint8_t *ring = rsm;
   uint8_t *wsm = rsm + CQ_SLOTS * I::QUAD;  // [kx][k half][strip column][8] bf16
@@ -264,7 +286,14 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
            *drain = dempty + CQ_MMA_WARPS;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
   volatile uint32_t *stop = tmem_slot + 1;
-  static_assert((2 * CQ_SLOTS + 2 * CQ_MMA_WARPS + 2) * 8 <= 256, "barrier words");
+  // one output channel: how an accumulator holds its rows (1: a column each, 16:
+  // 16 columns each), and whether a loader warp's share of a slot has values that
+  // are not finite
+  volatile uint32_t *row_cols = tmem_slot + 2;
+  volatile uint8_t *not_finite = reinterpret_cast<volatile uint8_t *>(tmem_slot + 2 + CQ_MMA_WARPS);
+  static_assert((2 * CQ_SLOTS + 2 * CQ_MMA_WARPS + 2) * 8 + 4 * CQ_MMA_WARPS + CQ_SLOTS * CQ_LOAD_WARPS <= 256 &&
+                    CQ_LOAD_WARPS == 8 && CQ_MMA_WARPS % 2 == 0,
+                "barrier words");
   static_assert(I::QUAD % 128 == 0 && WBYTES % 16 == 0, "operand alignment");
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const bool loader = warp >= CQ_EPI_WARPS && warp < CQ_EPI_WARPS + CQ_LOAD_WARPS;
@@ -303,10 +332,10 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
     const int t = warp < CQ_EPI_WARPS ? tid : tid - 32 * CQ_LOAD_WARPS;
 #pragma unroll 8
     for (int k = 0; k < PER; k++) {
-      const int i = t + k * SETUP, r = (i >> 3) / CQ_STRIP;
+      const int i = t + k * SETUP, r = (i >> 3) / STRIP;
       if (i < WN)
         reinterpret_cast<__nv_bfloat16 *>(wsm)[i] =
-            cq_weight<C, COUT>(w, r >> 1, (i >> 3) % CQ_STRIP, (r & 1) * 8 + (i & 7));
+            cq_weight<C, COUT>(w, r >> 1, (i >> 3) % STRIP, (r & 1) * 8 + (i & 7));
     }
     // (the ring's pixels 132 .. 135 are never written: the 8-channel layer's
     // last tap pair reads pixel 132 against zero weights)
@@ -323,7 +352,7 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(b)), "r"(n));
       };
       for (int k = 0; k < CQ_SLOTS; k++) init(full + k, CQ_LOAD_WARPS), init(empty + k, CQ_MMA_WARPS);
-      for (int k = 0; k < CQ_MMA_WARPS; k++) init(dfull + k, 1), init(dempty + k, CQ_EPI_WARPS);
+      for (int k = 0; k < CQ_MMA_WARPS; k++) init(dfull + k, COUT == 1 ? 2 : 1), init(dempty + k, CQ_EPI_WARPS);
       init(drain, CQ_MMA_WARPS);
       *stop = 0u;
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -347,6 +376,12 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
       cq_store_px<C>(p[0], d + lrow * I::ROW + lpx * 16);
       cq_store_px<C>(p[1], d + (lrow + 1) * I::ROW + lpx * 16);
       if (lt < 16) cq_store_px<C>(p[2], d + (lt >> 2) * I::ROW + (128 + (lt & 3)) * 16);
+      if constexpr (COUT == 1) {
+        uint32_t u = cq_largest<C>(p[1], cq_largest<C>(p[0], 0u));
+        if (lt < 16) u = cq_largest<C>(p[2], u);
+        const bool any = __any_sync(0xffffffffu, (u & 0xFFFFu) >= 0x7F80u || u >= 0x7F800000u);
+        if (lane == 0) not_finite[sl * CQ_LOAD_WARPS + warp - CQ_EPI_WARPS] = any ? 1 : 0;
+      }
       __syncwarp();
       if (lane == 0) tc_arrive(full + sl);
       if (++sl == CQ_SLOTS) sl = 0, par ^= 1;
@@ -386,24 +421,55 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t s0 = rbase + gi % CQ_SLOTS * I::QUAD, s1 = rbase + (gi + 1) % CQ_SLOTS * I::QUAD;
           constexpr int KXS = C == 8 ? 32 : 16, LBO = C == 8 ? 16 : CQ_PLANE;
+          if constexpr (COUT == 1) {
+            const volatile uint32_t *f0 =
+                reinterpret_cast<const volatile uint32_t *>(not_finite + gi % CQ_SLOTS * CQ_LOAD_WARPS);
+            const volatile uint32_t *f1 =
+                reinterpret_cast<const volatile uint32_t *>(not_finite + (gi + 1) % CQ_SLOTS * CQ_LOAD_WARPS);
+            const bool finite = !(f0[0] | f0[1] | f1[0] | f1[1]);
+            row_cols[m] = finite ? 1u : 16u;
+            if (finite) {
 #pragma unroll
-          for (int t = 0; t < 8; t++) {
-            // output rows j0 .. j1, from block 4 - t + j0 (ky = t - j0) on
-            const int j0 = max(t - 4, 0), j1 = min(t, 3);
-            const uint32_t rb = (t < 4 ? s0 : s1) + (t & 3) * I::ROW;
+              for (int t = 0; t < 8; t++) {
+                const uint32_t rb = (t < 4 ? s0 : s1) + (t & 3) * I::ROW;
+                const uint32_t wb = wbase + (uint32_t)((7 - t) * 16);
 #pragma unroll
-            for (int kx = 0; kx < I::NKX; kx++) {
-              const uint64_t ad = tc_desc(rb + kx * KXS, LBO, 128);
-              const uint32_t wk = wbase + (uint32_t)(kx * CQ_STRIP * 32);
-              auto mma = [&](int j, int rows, uint32_t accumulate) {
-                tc_mma(acc + 16 * j, ad, tc_desc(wk + (uint32_t)((4 - t + j) * 256), CQ_STRIP * 16, 128),
-                       tc_idesc(16 * rows), accumulate);
-              };
-              if (t < 4 && kx == 0) {  // row t's first product
-                if (t) mma(0, t, 1u);
-                mma(t, 1, 0u);
-              } else {
-                mma(j0, j1 - j0 + 1, 1u);
+                for (int kx = 0; kx < I::NKX; kx++)
+                  tc_mma(acc, tc_desc(rb + kx * KXS, LBO, 128), tc_desc(wb + kx * STRIP * 32, STRIP * 16, 128),
+                         tc_idesc(16), (kx || t) ? 1u : 0u);
+              }
+            } else {
+              for (int i = 0; i < 4 * 5; i++) {
+                const int j = i / 5, ky = i % 5, t = j + ky;
+                const uint32_t rb = (t < 4 ? s0 : s1) + (t & 3) * I::ROW;
+                const uint32_t wb = wbase + (uint32_t)((7 - ky) * 16);
+#pragma unroll
+                for (int kx = 0; kx < I::NKX; kx++)
+                  tc_mma(acc + 16 * j, tc_desc(rb + kx * KXS, LBO, 128),
+                         tc_desc(wb + kx * STRIP * 32, STRIP * 16, 128), tc_idesc(16), (kx || ky) ? 1u : 0u);
+              }
+            }
+            tc_arrive(dfull + m);  // (row_cols, released to the epilogue: the phase takes this and the commit)
+          } else {
+#pragma unroll
+            for (int t = 0; t < 8; t++) {
+              // output rows j0 .. j1, from block 4 - t + j0 (ky = t - j0) on
+              const int j0 = max(t - 4, 0), j1 = min(t, 3);
+              const uint32_t rb = (t < 4 ? s0 : s1) + (t & 3) * I::ROW;
+#pragma unroll
+              for (int kx = 0; kx < I::NKX; kx++) {
+                const uint64_t ad = tc_desc(rb + kx * KXS, LBO, 128);
+                const uint32_t wk = wbase + (uint32_t)(kx * STRIP * 32);
+                auto mma = [&](int j, int rows, uint32_t accumulate) {
+                  tc_mma(acc + 16 * j, ad, tc_desc(wk + (uint32_t)((4 - t + j) * 256), STRIP * 16, 128),
+                         tc_idesc(16 * rows), accumulate);
+                };
+                if (t < 4 && kx == 0) {  // row t's first product
+                  if (t) mma(0, t, 1u);
+                  mma(t, 1, 0u);
+                } else {
+                  mma(j0, j1 - j0 + 1, 1u);
+                }
               }
             }
           }
@@ -440,10 +506,11 @@ __global__ void __launch_bounds__(CQ_THREADS, 1) k_conv_quads(const __nv_bfloat1
         __syncwarp();  // (the reads of tensor memory are by whole warps)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         uint32_t v[2][COUT];
-        const uint32_t at = trow + d * CQ_ACC + row0 * 16;
+        const uint32_t cols = COUT == 1 && row_cols[d] == 1u ? 1u : 16u;
+        const uint32_t at = trow + d * CQ_ACC + row0 * cols;
         if constexpr (COUT == 1) {
           tmem_ld1(at, v[0][0]);
-          tmem_ld1(at + 16, v[1][0]);
+          tmem_ld1(at + cols, v[1][0]);
         } else {
           tmem_ld16(at, v[0]);
           tmem_ld16(at + 16, v[1]);
@@ -1439,7 +1506,7 @@ unsigned long long g_attr_done = 0;  // devices whose kernels have their shared-
 template <int C, int COUT, int MODE>
 cudaError_t set_conv_attr() {
   return cudaFuncSetAttribute(k_conv_quads<C, COUT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)cq_smem_bytes<C>());
+                              (int)cq_smem_bytes<C, COUT>());
 }
 template <int IN>
 cudaError_t set_grad_attr() {
@@ -1528,7 +1595,7 @@ void conv(const __nv_bfloat16 *in, int n, int W, int H, const __nv_bfloat16 *w, 
           float inv_tau, uint32_t *err, int err_stride, cudaStream_t s) {
   const int64_t quads = (int64_t)((W + CQ_OUT - 1) / CQ_OUT) * n * ((H + 3) / 4);
   note_launch();
-  k_conv_quads<C, COUT, MODE><<<(int)std::min<int64_t>(148, quads), CQ_THREADS, cq_smem_bytes<C>(), s>>>(
+  k_conv_quads<C, COUT, MODE><<<(int)std::min<int64_t>(148, quads), CQ_THREADS, cq_smem_bytes<C, COUT>(), s>>>(
       in, W, H, n, w, b, out, inv_tau, err, err_stride);
 }
 
